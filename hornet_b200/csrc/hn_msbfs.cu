@@ -42,9 +42,8 @@ struct MsState {
     long long* qbase[2];
     unsigned* qoff[2];
     int32_t* chunk[2];
-    unsigned long long* seen;
+    ulonglong2* sn;                 // {seen, nxt} of each vertex, one load for both
     unsigned long long* front[2];
-    unsigned long long* nxt;
     int32_t* touched;
     int32_t* dist;                  // nslots x nV, slot-major
     const int32_t* src;
@@ -55,7 +54,7 @@ struct MsState {
     int prev_nq;                    // size of the previous frontier (its fronts are cleared)
     int bottom_up;                  // bottom-up levels allowed
     int alpha, beta;                // direction switch thresholds
-    long long m_total;              // edges of the graph
+    long long open_edges;           // degrees of the vertices that miss a slot
     unsigned long long all_mask;    // slots that hold at least one source
 };
 
@@ -68,7 +67,7 @@ struct MsGraph {
     long long* qbasebuf = nullptr;
     unsigned* qoffbuf = nullptr;
     int32_t* chunkbuf = nullptr;
-    unsigned long long* masks = nullptr;   // seen, front0, front1, nxt
+    unsigned long long* masks = nullptr;   // {seen, nxt} pairs, front0, front1
     int32_t* touched = nullptr;
     unsigned long long* stat = nullptr;
     unsigned long long* h_stat = nullptr;
@@ -128,10 +127,9 @@ __global__ void k_ms_fill(MsState* st) {
          i += (long long)gridDim.x * blockDim.x) {
         st->dist[i] = kInf;
         if (i < n) {
-            st->seen[i] = 0;
+            st->sn[i] = make_ulonglong2(0ull, 0ull);
             st->front[0][i] = 0;
             st->front[1][i] = 0;
-            st->nxt[i] = 0;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x < 3 * kMaxSlots) st->stat[threadIdx.x] = 0;
@@ -166,7 +164,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_ms_seed(MsState* st) {
             unsigned long long bit = 1ull << b;
             atomicOr(&st->all_mask, bit);
             unsigned long long old = atomicOr(st->front[0] + v, bit);
-            unsigned long long olds = atomicOr(st->seen + v, bit);
+            unsigned long long olds = atomicOr(&st->sn[v].x, bit);
             first = old == 0;
             r = st->vtab[v];
             if (!(olds & bit)) {
@@ -228,8 +226,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
     const unsigned* qoff = st->qoff[cur];
     const int32_t* chunk = st->chunk[cur];
     const unsigned long long* front = st->front[cur];
-    const unsigned long long* seen = st->seen;
-    unsigned long long* nxt = st->nxt;
+    ulonglong2* sn = st->sn;
     const int32_t* pool = st->pool;
     const unsigned nchunks = (total + kMsChunk - 1) / kMsChunk;
     for (unsigned c = blockIdx.x; c < nchunks; c += gridDim.x) {
@@ -273,14 +270,22 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
                     fm[k] = s_front[j];
                 }
             }
+            // bits that an earlier edge of this level has already set in nxt
+            // need no atomic (through L2: an L1 copy would miss them)
             unsigned long long sv[IPT];
 #pragma unroll
-            for (int k = 0; k < IPT; k++) sv[k] = w[k] >= 0 ? __ldca(seen + w[k]) : ~0ull;
+            for (int k = 0; k < IPT; k++) {
+                sv[k] = ~0ull;
+                if (w[k] >= 0) {
+                    const ulonglong2 q = __ldcg(sn + w[k]);
+                    sv[k] = q.x | q.y;
+                }
+            }
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
                 unsigned long long m = fm[k] & ~sv[k];
                 if (m) {
-                    unsigned long long old = atomicOr(nxt + w[k], m);
+                    unsigned long long old = atomicOr(&sn[w[k]].y, m);
                     if (old == 0) touched_here[nt++] = w[k];
                 }
             }
@@ -296,15 +301,83 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
     }
 }
 
-// apply: new bits of every touched vertex; next frontier; clear the old one
+// Bottom-up step of one warp: lane's vertex (record r, missing slots `todo`)
+// takes, for every slot it still misses, the frontier mask of a neighbour on
+// that slot's frontier.  The first kMsLane neighbours are read by the lane
+// itself, four at a time (neighbour ids with one 16-byte load, then their
+// masks together); a list that needs more is read by the whole warp, 64
+// neighbours a step, so a hub costs its warp deg / 64 steps instead of deg.
+// Stops at the step after which nothing is missing.  Called by all lanes.
+constexpr int kMsLane = 16;
+constexpr long long kMsScan = 16;
+
+__device__ __forceinline__ unsigned long long ms_pull(const VRec& r, unsigned long long todo,
+                                                      const int32_t* __restrict__ pool,
+                                                      const unsigned long long* __restrict__ front) {
+    const unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    unsigned long long got = 0;
+    const int32_t* nb = pool + r.off;
+    if (todo) {
+        // blocks of capacity >= 4 are 16-byte aligned and whole
+        const int mine = r.deg < kMsLane ? r.deg : kMsLane;
+        for (int e = 0; e < mine; e += 4) {
+            int4 n4;
+            if (r.cap >= 4) n4 = __ldg(reinterpret_cast<const int4*>(nb + e));
+            else n4 = make_int4(__ldg(nb), r.deg > 1 ? __ldg(nb + 1) : 0, 0, 0);   // cap 1 or 2
+            const int left = r.deg - e;
+            const unsigned long long m0 = front[n4.x];
+            const unsigned long long m1 = left > 1 ? front[n4.y] : 0ull;
+            const unsigned long long m2 = left > 2 ? front[n4.z] : 0ull;
+            const unsigned long long m3 = left > 3 ? front[n4.w] : 0ull;
+            got |= m0 | m1 | m2 | m3;
+            if (!(todo & ~got)) break;
+        }
+    }
+    got &= todo;
+    unsigned more = __ballot_sync(kFull, r.deg > kMsLane && (todo & ~got) != 0);
+    while (more) {
+        const int l = __ffs(more) - 1;
+        more &= more - 1;
+        const int32_t* wn = pool + __shfl_sync(kFull, r.off, l);
+        const int wd = __shfl_sync(kFull, r.deg, l);
+        const unsigned long long wt = __shfl_sync(kFull, todo & ~got, l);
+        unsigned long long acc = 0;
+        for (int e = kMsLane; e < wd; e += 64) {
+            const int e0 = e + lane, e1 = e + 32 + lane;
+            const int a = e0 < wd ? __ldg(wn + e0) : -1;
+            const int b = e1 < wd ? __ldg(wn + e1) : -1;
+            const unsigned long long m = (a >= 0 ? front[a] : 0ull) | (b >= 0 ? front[b] : 0ull);
+            const unsigned lo = __reduce_or_sync(kFull, (unsigned)(m & wt));
+            const unsigned hi = __reduce_or_sync(kFull, (unsigned)((m & wt) >> 32));
+            acc |= ((unsigned long long)hi << 32) | lo;
+            if (!(wt & ~acc)) break;
+        }
+        if (lane == l) got |= acc;
+    }
+    return got;
+}
+
+// apply: new bits of every touched vertex (top-down) or of every vertex that
+// misses a slot (bottom-up), their distances, the next frontier.  kMsApply
+// vertices per thread share one CTA-wide reservation.  Per-slot statistics
+// stay in registers (lane b counts slots b and b + 32, by ballot and warp
+// sum): an atomic per (vertex, slot), 64-bit and on few shared words, had
+// taken most of a level.  512 graphs (8.0 M vertices, 148 M edges), 8 slots:
+// 54.8 ms before, 22.3 ms with these two (lists by warps, statistics in
+// registers), 7.1 ms with {seen, nxt} in one load ahead of each atomic and
+// the direction chosen by the edges that either would read.
+constexpr int kMsApply = 4;
+
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_ms_apply(MsState* st, cudaGraphConditionalHandle cond) {
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
+k_ms_apply(MsState* st, cudaGraphConditionalHandle cond) {
+    const unsigned kFull = 0xFFFFFFFFu;
     __shared__ unsigned long long s_wsum[BLOCK / 32];
     __shared__ unsigned long long s_cb;
     __shared__ unsigned long long s_stat[2 * kMaxSlots];
-    __shared__ int s_last[kMaxSlots];   // written only with this level's number
+    const int lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < 2 * kMaxSlots; i += BLOCK) s_stat[i] = 0;
-    for (int i = threadIdx.x; i < kMaxSlots; i += BLOCK) s_last[i] = 0;
     __syncthreads();
     const int level = st->level;
     const int it = level - 1;
@@ -312,78 +385,109 @@ __global__ void __launch_bounds__(BLOCK) k_ms_apply(MsState* st, cudaGraphCondit
     unsigned long long* cout = &st->cnt[(it + 1) % 3];
     const long long nt = (long long)st->tcnt;
     const int nV = st->nV;
-    const VRec* vtab = st->vtab;
-    unsigned long long* seen = st->seen;
-    unsigned long long* nxt = st->nxt;
+    const VRec* __restrict__ vtab = st->vtab;
+    const int32_t* __restrict__ pool = st->pool;
+    ulonglong2* sn = st->sn;
     unsigned long long* nfront = st->front[nx];
-    const long long stride = (long long)gridDim.x * blockDim.x;
     const bool bu = st->mode == 1;
     const unsigned long long* cfront = st->front[nx ^ 1];
     const unsigned long long all = st->all_mask;
     const int nq_in = (int)(st->cnt[it % 3] & 0xFFFFFFFFull);
     const long long n_items = bu ? (long long)nV : nt;
-    for (long long i0 = blockIdx.x * (long long)blockDim.x; i0 < n_items; i0 += stride) {
-        long long i = i0 + threadIdx.x;
-        bool q = false;
-        int v = 0;
-        VRec r;
-        r.deg = 0;
-        r.off = 0;
-        unsigned long long nw = 0;
-        if (bu && i < n_items) {
-            // bottom-up: v takes, for every slot it still misses, the first
-            // neighbour on that slot's frontier; stops once nothing is missing
-            v = (int)i;
-            unsigned long long todo = all & ~seen[v];
-            if (todo) {
-                r = vtab[v];
-                const int32_t* nb = st->pool + r.off;
-                for (int e = 0; e < r.deg && todo; e++) {
-                    const unsigned long long m = cfront[__ldg(nb + e)] & todo;
-                    nw |= m;
-                    todo &= ~m;
+    int32_t* dist = st->dist;
+    unsigned long long vis0 = 0, vis1 = 0, sc0 = 0, sc1 = 0;   // slots lane, lane + 32
+    long long closed = 0;   // degrees of vertices that miss no slot any more
+    constexpr long long PER = (long long)BLOCK * kMsApply;
+    for (long long i0 = blockIdx.x * PER; i0 < n_items; i0 += (long long)gridDim.x * PER) {
+        int vk[kMsApply], dk[kMsApply];
+        long long ok[kMsApply];
+        unsigned long long mine = 0;   // (degree sum << 32) | queued vertices
+#pragma unroll
+        for (int k = 0; k < kMsApply; k++) {
+            const long long i = i0 + k * BLOCK + threadIdx.x;
+            int v = 0;
+            VRec r;
+            r.deg = 0;
+            r.off = 0;
+            r.cap = 0;
+            unsigned long long nw = 0;
+            if (bu) {
+                unsigned long long sv = 0, todo = 0;
+                if (i < n_items) {
+                    v = (int)i;
+                    sv = sn[v].x;
+                    todo = all & ~sv;
+                    if (todo) {
+                        r = vtab[v];
+                        if (r.deg == 0) todo = 0;
+                    }
                 }
+                nw = ms_pull(r, todo, pool, cfront);
                 if (nw) {
-                    seen[v] |= nw;
+                    sn[v].x = sv | nw;
                     nfront[v] = nw;
+                    if (!(all & ~(sv | nw))) closed += r.deg;
+                }
+            } else if (i < nt) {
+                v = st->touched[i];
+                const ulonglong2 q = sn[v];
+                nw = q.y & ~q.x;
+                sn[v] = make_ulonglong2(q.x | nw, 0ull);
+                nfront[v] = nw;
+                r = vtab[v];
+                if (!(all & ~(q.x | nw))) closed += r.deg;
+            }
+            // the slots that reach any of the warp's vertices now
+            unsigned ulo = __reduce_or_sync(kFull, (unsigned)nw);
+            unsigned uhi = __reduce_or_sync(kFull, (unsigned)(nw >> 32));
+            while (ulo | uhi) {
+                const bool low = ulo != 0;
+                const int b5 = __ffs(low ? ulo : uhi) - 1;
+                if (low) ulo &= ulo - 1; else uhi &= uhi - 1;
+                const int bb = low ? b5 : b5 + 32;
+                const bool has = (nw >> bb) & 1ull;
+                if (has) dist[(long long)bb * nV + v] = level;
+                const unsigned c = __popc(__ballot_sync(kFull, has));
+                // distinct vertices: their degrees sum to at most nE < 2^32
+                const unsigned ds = __reduce_add_sync(kFull, has ? (unsigned)r.deg : 0u);
+                if (lane == b5) {
+                    if (low) { vis0 += c; sc0 += ds; }
+                    else { vis1 += c; sc1 += ds; }
                 }
             }
-        } else if (!bu && i < nt) {
-            v = st->touched[i];
-            unsigned long long x = nxt[v];
-            nxt[v] = 0;
-            nw = x & ~seen[v];
-            seen[v] |= nw;
-            nfront[v] = nw;
-            r = vtab[v];
+            const bool q = nw != 0 && r.deg > 0;
+            vk[k] = v;
+            dk[k] = q ? r.deg : 0;
+            ok[k] = r.off;
+            if (q) mine += ((unsigned long long)r.deg << 32) | 1ull;
         }
-        if (nw) {
-            while (nw) {
-                int bb = __ffsll((long long)nw) - 1;
-                nw &= nw - 1;
-                st->dist[(long long)bb * nV + v] = level;
-                atomicAdd(&s_stat[bb], 1ull);
-                atomicAdd(&s_stat[kMaxSlots + bb], (unsigned long long)r.deg);
-                s_last[bb] = level;
-            }
-            q = r.deg > 0;
-        }
-        unsigned long long mine = q ? (((unsigned long long)r.deg << 32) | 1ull) : 0ull;
+        if (!__syncthreads_or(mine != 0)) continue;   // nothing queued by the CTA
         unsigned long long at = ms_cta_reserve<BLOCK>(mine, cout, s_wsum, &s_cb);
-        if (q) {
-            int pos = (int)(at & 0xFFFFFFFFull);
-            unsigned off = (unsigned)(at >> 32);
-            st->q[nx][pos] = v;
-            st->qbase[nx][pos] = r.off;
-            st->qoff[nx][pos] = off;
-            ms_mark_chunks(st->chunk[nx], off, (unsigned)r.deg, pos);
+#pragma unroll
+        for (int k = 0; k < kMsApply; k++) {
+            if (dk[k]) {
+                const int pos = (int)(at & 0xFFFFFFFFull);
+                const unsigned off = (unsigned)(at >> 32);
+                st->q[nx][pos] = vk[k];
+                st->qbase[nx][pos] = ok[k];
+                st->qoff[nx][pos] = off;
+                ms_mark_chunks(st->chunk[nx], off, (unsigned)dk[k], pos);
+                at += ((unsigned long long)dk[k] << 32) | 1ull;
+            }
         }
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) closed += __shfl_xor_sync(kFull, closed, o);
+    if (lane == 0 && closed)
+        atomicAdd((unsigned long long*)&st->open_edges, (unsigned long long)-closed);
+    if (vis0) { atomicAdd(&s_stat[lane], vis0); atomicAdd(&s_stat[kMaxSlots + lane], sc0); }
+    if (vis1) { atomicAdd(&s_stat[lane + 32], vis1); atomicAdd(&s_stat[kMaxSlots + lane + 32], sc1); }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * kMaxSlots; i += BLOCK)
-        if (s_stat[i]) atomicAdd(st->stat + i, s_stat[i]);
-    for (int i = threadIdx.x; i < kMaxSlots; i += BLOCK)
-        if (s_last[i]) st->stat[2 * kMaxSlots + i] = (unsigned long long)level;
+        if (s_stat[i]) {
+            atomicAdd(st->stat + i, s_stat[i]);
+            if (i < kMaxSlots) st->stat[2 * kMaxSlots + i] = (unsigned long long)level;
+        }
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -398,14 +502,13 @@ __global__ void __launch_bounds__(BLOCK) k_ms_apply(MsState* st, cudaGraphCondit
             st->level = level + 1;
             st->prev_nq = nq_in;
             if (st->bottom_up) {
-                // bottom-up while the next frontier's edges exceed m/alpha;
-                // back to top-down once it holds fewer than nV/beta vertices
+                // bottom-up while the next frontier's edges (which a push
+                // reads) exceed those of the vertices that still miss a slot
+                // (which a pull reads at most) -- alpha / kMsScan, about 1 by
+                // default -- and the frontier holds nV/beta vertices or more
                 const long long mf = (long long)(c >> 32);
-                if (st->mode == 0) {
-                    if (mf * st->alpha > st->m_total) st->mode = 1;
-                } else if ((long long)nn * st->beta < nV) {
-                    st->mode = 0;
-                }
+                const long long open = (long long)atomicAdd((unsigned long long*)&st->open_edges, 0ull);
+                st->mode = mf * st->alpha > kMsScan * open && (long long)nn * st->beta >= nV;
             }
             cudaGraphSetConditional(cond, (nn > 0 && level < nV) ? 1u : 0u);
         }
@@ -563,10 +666,9 @@ extern "C" int hn_bfs_batch(hn_graph_t* g, const int32_t* sources, const int32_t
     h.qoff[1] = mg.qoffbuf + nV + 2;
     h.chunk[0] = mg.chunkbuf;
     h.chunk[1] = mg.chunkbuf + mg.nchunk_cap;
-    h.seen = mg.masks;
-    h.front[0] = mg.masks + nV;
-    h.front[1] = mg.masks + 2 * (size_t)nV;
-    h.nxt = mg.masks + 3 * (size_t)nV;
+    h.sn = (ulonglong2*)mg.masks;
+    h.front[0] = mg.masks + 2 * (size_t)nV;
+    h.front[1] = mg.masks + 3 * (size_t)nV;
     h.touched = mg.touched;
     h.dist = out;
     h.src = d_src.get();
@@ -576,7 +678,7 @@ extern "C" int hn_bfs_batch(hn_graph_t* g, const int32_t* sources, const int32_t
     h.bottom_up = (int)knob(kKnobMsBottomUp);
     h.alpha = (int)knob(kKnobBfsDoAlpha);
     h.beta = (int)knob(kKnobBfsDoBeta);
-    h.m_total = g->nE;
+    h.open_edges = g->nE;
     HN_CUDA(cudaMemcpyAsync(mg.state, &h, sizeof(MsState), cudaMemcpyHostToDevice, s));
     cudaEvent_t ev0 = nullptr;
     if (g_profiling) profile_begin(s, &ev0);

@@ -154,3 +154,27 @@ def test_batch_bottom_up_switching(alpha, beta):
         check(out, st, ref, ref_stats)
     finally:
         H.tune_reset()
+
+
+@pytest.mark.parametrize("block", [128, 256, 512])
+def test_batch_bottom_up_long_lists(block):
+    """Bottom-up levels over lists that a lane leaves to its warp (more than
+    16 neighbours, up to a hub of 5,000), lists of capacity 1, 2 and 4, and
+    vertices that some slots never reach."""
+    rng = np.random.default_rng(2)
+    star = O.build_csr_undirected(5001, np.zeros(5000, np.int32), np.arange(1, 5001, dtype=np.int32))
+    path = O.build_csr_undirected(9, np.arange(8, dtype=np.int32), np.arange(1, 9, dtype=np.int32))
+    g, base = T.disjoint_union([star, T.rmat_graph(11, 16, seed=3), path, T.er_graph(500, 60, seed=1)])
+    h = build(g)
+    srcs = np.concatenate([base, rng.integers(0, g.nV, 36), [5000, int(base[2]) + 8]]).astype(np.int32)
+    slots = np.arange(len(srcs)) % 40
+    ref, ref_stats = oracle_slots(g, srcs, slots, 40)
+    try:
+        H.tune_set("msbfs.block", block)
+        for alpha, beta in ((1 << 20, 1), (1 << 20, 1 << 20), (2, 24)):
+            H.tune_set("bfs.do_alpha", alpha)
+            H.tune_set("bfs.do_beta", beta)
+            out, st = H.BfsTopDown(h).run_batch(srcs, slots=slots.astype(np.int32), nslots=40)
+            check(out, st, ref, ref_stats)
+    finally:
+        H.tune_reset()
