@@ -744,7 +744,7 @@ void build_from_csr(hn_graph* g, int32_t nV, int64_t nE, const long long* d_off,
         uint32_t* va = d_w ? w2.get() : nullptr;
         HN_CUDA(cudaMemsetAsync(&g->alloc->error, 0, sizeof(int), s));
         radix_sort_u64(g, kc, ka, vc, va, (long long)nE, 2 * L, &g->alloc->error, s);
-        if (d_w && vc != sorted_w.get()) std::swap(sorted_w.p, w2.p);
+        if (d_w && vc != sorted_w.get()) sorted_w.swap(w2);
         sorted_adj.alloc((size_t)nE, s);
         HN_LAUNCH(k_keys_dst, grid_for(g, nE, 256), 256, 0, s, (const unsigned long long*)kc,
                   (long long)nE, L, sorted_adj.get());

@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include "hn_internal.cuh"
@@ -48,40 +49,74 @@ struct ProfileScope {
         }                                                                    \
     } while (0)
 
+// Room for the temporary buffers of one call, from one stream-ordered
+// allocation: an update takes about 25 buffers, and at two driver calls each
+// they cost more host time than a small batch's kernels.
+struct Arena {
+    char* p = nullptr;
+    size_t cap = 0, used = 0;
+    cudaStream_t s = nullptr;
+    Arena() = default;
+    void open(size_t bytes, cudaStream_t st) {
+        s = st;
+        HN_CUDA(cudaMallocAsync((void**)&p, bytes, st));
+        cap = bytes;
+    }
+    void* take(size_t bytes) {   // null when it does not fit
+        const size_t at = (used + 255) & ~(size_t)255;
+        if (at + bytes > cap) return nullptr;
+        used = at + bytes;
+        return p + at;
+    }
+    ~Arena() {
+        if (p) cudaFreeAsync(p, s);
+    }
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+};
+
 // Stream-ordered temporary device buffer (cudaMallocAsync on the graph's
-// stream; the memory returns to the device pool, not to the driver).
+// stream; the memory returns to the device pool, not to the driver), or a
+// part of an arena when one is given and has room.
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
     cudaStream_t s = nullptr;
+    bool own = true;
     DevBuf() = default;
-    DevBuf(size_t count, cudaStream_t st) { alloc(count, st); }
-    void alloc(size_t count, cudaStream_t st) {
+    DevBuf(size_t count, cudaStream_t st, Arena* arena = nullptr) { alloc(count, st, arena); }
+    void alloc(size_t count, cudaStream_t st, Arena* arena = nullptr) {
         release();
         s = st;
         n = count;
-        if (count) HN_CUDA(cudaMallocAsync((void**)&p, count * sizeof(T), st));
+        if (!count) return;
+        if (arena) p = (T*)arena->take(count * sizeof(T));
+        own = p == nullptr;
+        if (own) HN_CUDA(cudaMallocAsync((void**)&p, count * sizeof(T), st));
     }
     void release() {
-        if (p) cudaFreeAsync(p, s);
+        if (p && own) cudaFreeAsync(p, s);
         p = nullptr;
         n = 0;
+        own = true;
     }
     ~DevBuf() { release(); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), s(o.s) { o.p = nullptr; o.n = 0; }
+    DevBuf(DevBuf&& o) noexcept { swap(o); }
     DevBuf& operator=(DevBuf&& o) noexcept {
         if (this != &o) {
             release();
-            p = o.p;
-            n = o.n;
-            s = o.s;
-            o.p = nullptr;
-            o.n = 0;
+            swap(o);
         }
         return *this;
+    }
+    void swap(DevBuf& o) noexcept {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+        std::swap(s, o.s);
+        std::swap(own, o.own);
     }
     T* get() const { return p; }
 };
@@ -230,13 +265,14 @@ namespace hn {
 // hn_sort.cu.
 void radix_sort_u64(hn_graph* g, unsigned long long*& keys, unsigned long long*& keys_alt,
                     uint32_t*& vals, uint32_t*& vals_alt, long long n, int bits, int* err,
-                    cudaStream_t s);
+                    cudaStream_t s, Arena* arena = nullptr);
 
 // out[i] = in[0] + ... + in[i-1] (out may be in), on stream s, in OutT.
 // Defined in hn_scan.cu for (int, int), (int, long long), (long long,
 // long long) and (unsigned long long, unsigned long long).
 template <typename InT, typename OutT>
-void exclusive_scan(hn_graph* g, const InT* in, OutT* out, long long n, cudaStream_t s);
+void exclusive_scan(hn_graph* g, const InT* in, OutT* out, long long n, cudaStream_t s,
+                    Arena* arena = nullptr);
 
 // Update entry points call this: a query view never changes the graph.
 inline void require_owner(const hn_graph* g) {

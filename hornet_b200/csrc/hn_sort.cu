@@ -39,6 +39,7 @@ constexpr int kBins = 256;
 constexpr int kMaxPasses = 8;
 constexpr long long kWaitLimit = 1 << 22;
 constexpr int kLook = 4;   // statuses a look-back step reads at once
+constexpr long long kStatusBytes = 64 << 20;
 
 constexpr unsigned long long kFlagAgg = 1ull << 62;    // the tile's own counts
 constexpr unsigned long long kFlagIncl = 2ull << 62;   // counts of tiles 0..t
@@ -48,6 +49,7 @@ struct SortState {
     unsigned ghist[kMaxPasses][kBins];   // keys per digit, per pass
     int tile_ctr[kMaxPasses];            // next tile number, per pass
 };
+static_assert(sizeof(SortState) % 8 == 0, "statuses follow it");
 
 __device__ __forceinline__ unsigned digit_of(unsigned long long k, int shift) {
     return (unsigned)(k >> shift) & 0xFFu;
@@ -272,7 +274,7 @@ int sm_count(const hn_graph* g) {
 // keys are then not sorted).  n < 2^32.
 void radix_sort_u64(hn_graph* g, unsigned long long*& keys, unsigned long long*& keys_alt,
                     uint32_t*& vals, uint32_t*& vals_alt, long long n, int bits, int* err,
-                    cudaStream_t s) {
+                    cudaStream_t s, Arena* arena) {
     if (n <= 1 || bits <= 0) return;
     if (n >= (1ll << 32)) throw Error(HN_ERR_CAPACITY, "radix sort of 2^32 keys or more");
     const int passes = (bits + 7) / 8;
@@ -282,23 +284,30 @@ void radix_sort_u64(hn_graph* g, unsigned long long*& keys, unsigned long long*&
     const int nt = vals ? 256 : 512;
     const long long tile = (long long)nt * kOsIpt;
     const long long ntiles = (n + tile - 1) / tile;
-    DevBuf<SortState> ss(1, s);
-    DevBuf<unsigned long long> status((size_t)ntiles * kBins, s);
-    HN_CUDA(cudaMemsetAsync(ss.get(), 0, sizeof(SortState), s));
+    // the state and every pass's statuses are cleared at once; only when the
+    // statuses would take more than kStatusBytes do the passes share one array
+    const long long per_pass = ntiles * kBins;
+    const bool all = per_pass * passes * (long long)sizeof(unsigned long long) <= kStatusBytes;
+    DevBuf<unsigned long long> mem(sizeof(SortState) / 8 + (size_t)per_pass * (all ? passes : 1), s,
+                                   arena);
+    SortState* ss = (SortState*)mem.get();
+    unsigned long long* status0 = mem.get() + sizeof(SortState) / 8;
+    HN_CUDA(cudaMemsetAsync(mem.get(), 0, all ? mem.n * 8 : sizeof(SortState), s));
     const long long grid0 = std::min<long long>((n + kOsThreads - 1) / kOsThreads,
                                                 (long long)sm_count(g) * 8);
-    HN_LAUNCH(k_rs_hist0, grid0, kOsThreads, 0, s, keys, n, ss.get());
+    HN_LAUNCH(k_rs_hist0, grid0, kOsThreads, 0, s, keys, n, ss);
     for (int p = 0; p < passes; p++) {
         const int shift = 8 * p;
         const int next = p + 1 < passes ? shift + 8 : -1;
-        HN_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(unsigned long long) * ntiles * kBins, s));
+        unsigned long long* status = status0 + (all ? p * per_pass : 0);
+        if (!all) HN_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * per_pass, s));
         if (vals)
             HN_LAUNCH((k_rs_pass<true, 256>), ntiles, 256, 0, s, keys, vals, keys_alt, vals_alt,
-                      n, p, shift, next, status.get(), ss.get(), err);
+                      n, p, shift, next, status, ss, err);
         else
             HN_LAUNCH((k_rs_pass<false, 512>), ntiles, 512, 0, s, keys,
                       (const uint32_t*)nullptr, keys_alt, (uint32_t*)nullptr, n, p, shift, next,
-                      status.get(), ss.get(), err);
+                      status, ss, err);
         std::swap(keys, keys_alt);
         if (vals) std::swap(vals, vals_alt);
     }

@@ -496,49 +496,58 @@ k_scatter_old(const long long* __restrict__ prefix, long long nseg,
 }
 
 // Vertices updated in place whose moved entries span two or more scatter
-// tiles: a warp each stages the moved part [base, deg) (at most kInPlaceMax
+// tiles: a CTA each stages the moved part [base, deg) (at most kInPlaceMax
 // entries) in shared memory, then writes every entry to its new slot, so
-// all reads precede all writes.  Same slot rules as k_scatter_old.
-constexpr int kSpanWarps = 4;
+// all reads precede all writes.  Same slot rules as k_scatter_old.  There are
+// few such vertices (one per tile boundary at most), so what counts is the
+// chain of one of them: with a warp each it took 64 dependent rounds.
+constexpr int kSpanThreads = 256;
 
 template <bool INSERT>
-__global__ void __launch_bounds__(kSpanWarps * 32)
+__global__ void __launch_bounds__(kSpanThreads)
 k_inplace_span(const int32_t* __restrict__ span_list, const int* __restrict__ nspan,
                const int32_t* __restrict__ seg_u, const int32_t* __restrict__ seg_kstart,
                const int32_t* __restrict__ seg_base, const long long* __restrict__ seg_old_off,
                const int32_t* __restrict__ cdst, const VRec* __restrict__ vtab,
                int32_t* __restrict__ pool, long long span_cap) {
-    __shared__ int32_t sA[kSpanWarps][kInPlaceMax];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int32_t* A = sA[w];
+    constexpr int IPT = kInPlaceMax / kSpanThreads;
+    __shared__ int32_t A[kInPlaceMax];
     const int count = *nspan < span_cap ? *nspan : (int)span_cap;
-    for (int i = blockIdx.x * kSpanWarps + w; i < count; i += gridDim.x * kSpanWarps) {
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
         const int s = span_list[i];
         const int base = seg_base[s];
         const int n = vtab[seg_u[s]].deg - base;   // the old degree: commit runs later
         const long long off = seg_old_off[s] + base;
-        for (int j = lane; j < n; j += 32) A[j] = pool[off + j];
-        __syncwarp();
         const int k0 = seg_kstart[s], nb = seg_kstart[s + 1] - k0;
         const int32_t* B = cdst + k0;
-        for (int j = lane; j < n; j += 32) {
-            const int32_t x = A[j];
+        int32_t x[IPT];
+#pragma unroll
+        for (int q = 0; q < IPT; q++) {
+            const int j = q * kSpanThreads + threadIdx.x;
+            x[q] = j < n ? pool[off + j] : 0;
+            if (!INSERT && j < n) A[j] = x[q];
+        }
+        __syncthreads();   // every read of the list before any write
+#pragma unroll
+        for (int q = 0; q < IPT; q++) {
+            const int j = q * kSpanThreads + threadIdx.x;
+            if (j >= n) break;
             if (INSERT) {
-                pool[off + j + lower_bound32(B, nb, x)] = x;
+                pool[off + j + lower_bound32(B, nb, x[q])] = x[q];
             } else {
-                const int lbl = lower_bound32(B, nb, x);
+                const int lbl = lower_bound32(B, nb, x[q]);
                 int ubl = lbl;
-                while (ubl < nb && B[ubl] == x) ubl++;
+                while (ubl < nb && B[ubl] == x[q]) ubl++;
                 bool keep = true;
                 if (ubl > lbl) {
                     int first = j;
-                    if (j > 0 && A[j - 1] == x) first = lower_bound32(A, j, x);
+                    if (j > 0 && A[j - 1] == x[q]) first = lower_bound32(A, j, x[q]);
                     keep = (j - first) >= ubl - lbl;
                 }
-                if (keep) pool[off + j - ubl] = x;
+                if (keep) pool[off + j - ubl] = x[q];
             }
         }
-        __syncwarp();   // A is restaged for the next vertex
+        __syncthreads();   // A is restaged for the next vertex
     }
 }
 
@@ -920,8 +929,325 @@ __global__ void __launch_bounds__(kB) k_tc_delta(const VRec* __restrict__ vtab,
     }
 }
 
+// ---------------------------------------------------------------------------
+// Small batches (at most kSmallBatch entries, unweighted graphs): one kernel
+// up to the host's plan and two after it.  The general pipeline takes 24
+// launches, each a few microseconds of launch and latency for a few
+// microseconds of work at most: 1,000 entries inserted and erased took 430 us,
+// and 110 us this way.
+// ---------------------------------------------------------------------------
+constexpr int kSmallBatch = 2048;
+constexpr long long kArenaBatch = 1 << 20;   // batches whose buffers share one allocation
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallIpt = kSmallBatch / kSmallThreads;
+
+// What the host plans from (pinned; the layout of h_scalar and h_alloc).
+struct SmallPlan {
+    long long kept, nseg;
+    unsigned long long nbig, snap_words;
+};
+
+// Pack, sort, mark, compact and plan in one CTA: the same arrays as the
+// general pipeline's k_pack .. k_plan, by the same rules.  The sort is a
+// bitonic network on the packed keys in shared memory (equal keys are
+// interchangeable: there are no values).
+template <bool INSERT>
+__global__ void __launch_bounds__(kSmallThreads)
+k_small_front(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
+              const unsigned long long* __restrict__ sorted, int n, int nV, int L, unsigned flags,
+              const VRec* __restrict__ vtab, const int32_t* __restrict__ pool, bool in_place,
+              int big_min, int32_t* __restrict__ cdst, int32_t* __restrict__ cseg,
+              int32_t* __restrict__ capos, int32_t* __restrict__ seg_u,
+              int32_t* __restrict__ seg_kstart, long long* __restrict__ seg_work,
+              int32_t* __restrict__ seg_ncap, int32_t* __restrict__ seg_base,
+              long long* __restrict__ seg_old_off, int32_t* __restrict__ big_list,
+              AllocState* __restrict__ st, long long* __restrict__ totals,
+              SmallPlan* __restrict__ h_plan, AllocState* __restrict__ h_alloc) {
+    __shared__ unsigned long long key[kSmallBatch];
+    __shared__ int s_kstart[kSmallBatch + 1];
+    __shared__ int s_u[kSmallBatch];
+    __shared__ int s_apos0[kSmallBatch];        // place of each segment's first kept entry
+    __shared__ int s_keep[kSmallThreads / 32 * kSmallIpt], s_head[kSmallThreads / 32 * kSmallIpt];
+    __shared__ int s_need[kNumClasses], s_push[kNumClasses];
+    __shared__ int s_err, s_kept, s_nseg, s_nbig;
+    __shared__ unsigned long long s_snap;
+    const unsigned kFull = 0xFFFFFFFFu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NW = kSmallThreads / 32;
+    int np = 32;   // keys of the network: a power of two
+    while (np < n) np <<= 1;
+    if (tid == 0) {
+        s_err = 0;
+        s_nbig = 0;
+        s_snap = 0;
+    }
+    if (tid < kNumClasses) s_need[tid] = s_push[tid] = 0;
+    for (int i = tid; i < (int)(sizeof(AllocState) / 4); i += kSmallThreads) ((int*)st)[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < np; i += kSmallThreads) {
+        unsigned long long k = ~0ull;
+        if (i < n) {
+            if (sorted) {
+                k = sorted[i];
+            } else {
+                int u = src[i], v = dst[i];
+                if (u < 0 || u >= nV || v < 0 || v >= nV) {
+                    s_err = 1;
+                    u = v = 0;
+                }
+                k = ((unsigned long long)(unsigned)u << L) | (unsigned)v;
+            }
+        }
+        key[i] = k;
+    }
+    __syncthreads();
+    if (s_err) {   // the batch is refused
+        if (tid == 0) h_alloc->error = HN_ERR_INVALID;
+        return;
+    }
+    if (!sorted) {
+        for (int size = 2; size <= np; size <<= 1) {
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int p = tid; p < np / 2; p += kSmallThreads) {
+                    const int i = 2 * p - (p & (stride - 1)), j = i + stride;
+                    const unsigned long long x = key[i], y = key[j];
+                    if ((x > y) == ((i & size) == 0)) {
+                        key[i] = y;
+                        key[j] = x;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+    }
+    // mark: element i = r * kSmallThreads + tid
+    const unsigned long long mask = (1ull << L) - 1;
+    bool keep[kSmallIpt], head[kSmallIpt];
+    int apos[kSmallIpt];
+#pragma unroll
+    for (int r = 0; r < kSmallIpt; r++) {
+        const int i = r * kSmallThreads + tid;
+        keep[r] = head[r] = false;
+        apos[r] = 0;
+        if (i < n) {
+            const unsigned long long k = key[i];
+            const bool first = i == 0 || key[i - 1] != k;
+            head[r] = i == 0 || (key[i - 1] >> L) != (k >> L);
+            if (first || !(flags & HN_DEDUP_BATCH)) {
+                const int u = (int)(k >> L), x = (int)(k & mask);
+                const VRec v = vtab[u];
+                const int32_t* a = pool + v.off;
+                if (INSERT) {
+                    const int ub = upper_bound32(a, v.deg, x);
+                    keep[r] = !(first && (flags & HN_DEDUP_GRAPH) && ub > 0 && a[ub - 1] == x);
+                    apos[r] = ub;
+                } else {
+                    int rank = 0;   // among the batch's copies of (u, x)
+                    if (!first) rank = i - (int)lower_bound_dev((const unsigned long long*)key, (long long)i, k);
+                    const int lo = lower_bound32(a, v.deg, x);
+                    int cg = 0;
+                    if (lo < v.deg && a[lo] == x) cg = upper_bound32(a, v.deg, x) - lo;
+                    keep[r] = rank < cg;
+                    apos[r] = lo;
+                }
+            }
+        }
+        const unsigned bk = __ballot_sync(kFull, keep[r]), bh = __ballot_sync(kFull, head[r]);
+        if (lane == 0) {
+            s_keep[r * NW + warp] = __popc(bk);
+            s_head[r * NW + warp] = __popc(bh);
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {   // exclusive scans of the warps' counts, in element order
+        int ck = 0, ch = 0;
+#pragma unroll
+        for (int r = 0; r < kSmallIpt; r++) {
+            const int vk = s_keep[r * NW + lane], vh = s_head[r * NW + lane];
+            int ik = vk, ih = vh;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int yk = __shfl_up_sync(kFull, ik, o), yh = __shfl_up_sync(kFull, ih, o);
+                if (lane >= o) {
+                    ik += yk;
+                    ih += yh;
+                }
+            }
+            s_keep[r * NW + lane] = ck + ik - vk;
+            s_head[r * NW + lane] = ch + ih - vh;
+            ck += __shfl_sync(kFull, ik, 31);
+            ch += __shfl_sync(kFull, ih, 31);
+        }
+        if (lane == 0) {
+            s_kept = ck;
+            s_nseg = ch;
+            s_kstart[ch] = ck;
+            seg_kstart[ch] = ck;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSmallIpt; r++) {
+        const int i = r * kSmallThreads + tid;
+        const unsigned lt = (1u << lane) - 1u;
+        const unsigned bk = __ballot_sync(kFull, keep[r]), bh = __ballot_sync(kFull, head[r]);
+        const int pos = s_keep[r * NW + warp] + __popc(bk & lt);
+        const int seg = s_head[r * NW + warp] + __popc(bh & lt) + (head[r] ? 1 : 0) - 1;
+        if (head[r]) {
+            s_u[seg] = (int)(key[i] >> L);
+            s_kstart[seg] = pos;
+            seg_u[seg] = s_u[seg];
+            seg_kstart[seg] = pos;
+        }
+        if (keep[r]) {
+            cdst[pos] = (int)(key[i] & mask);
+            cseg[pos] = seg;
+            capos[pos] = apos[r];
+            s_apos0[pos] = apos[r];
+        }
+    }
+    __syncthreads();
+    // plan: the rules of k_plan
+    const int nseg = s_nseg;
+    for (int s0 = 0; s0 < nseg; s0 += kSmallThreads) {
+        const int s = s0 + tid;
+        if (s >= nseg) break;
+        const int k0 = s_kstart[s], k = s_kstart[s + 1] - k0;
+        const VRec r = vtab[s_u[s]];
+        int ncap = -1, base = 0;
+        const bool big = k > 0 && r.deg >= big_min;
+        if (k > 0) {
+            const int nd = INSERT ? r.deg + k : r.deg - k;
+            ncap = pow2_ceil(nd);
+            bool here = in_place && nd > 0 && ncap == r.cap && (!big || k <= kHubSnap);
+            if (here) {
+                base = s_apos0[k0];
+                if (big) {
+                    const int nch = (r.deg - base + kBigChunk - 1) / kBigChunk;
+                    if (nch > 1) atomicAdd(&s_snap, (unsigned long long)(nch - 1) * k);
+                } else {
+                    here = r.deg - base <= kInPlaceMax;
+                }
+            }
+            if (here) {
+                ncap = kInPlace;
+            } else {
+                base = 0;
+                if (ncap > 0) atomicAdd(&s_need[cap_class(ncap)], 1);
+                if (r.cap > 0) atomicAdd(&s_push[cap_class(r.cap)], 1);
+            }
+        }
+        seg_ncap[s] = ncap;
+        seg_base[s] = base;
+        seg_work[s] = k > 0 && !big ? r.deg - base : 0;
+        seg_old_off[s] = r.off;
+        if (big) big_list[atomicAdd(&s_nbig, 1)] = s;
+    }
+    __syncthreads();
+    if (tid < kNumClasses) {
+        h_alloc->need[tid] = s_need[tid];
+        h_alloc->push[tid] = s_push[tid];
+    }
+    if (tid == 0) {
+        seg_work[nseg] = 0;
+        totals[0] = s_kept;
+        totals[1] = nseg;
+        h_alloc->error = 0;
+        h_plan->kept = s_kept;
+        h_plan->nseg = nseg;
+        h_plan->nbig = (unsigned long long)s_nbig;
+        h_plan->snap_words = s_snap;
+    }
+}
+
+// After the host's plan and k_assign, when the batch touches no hub: a CTA
+// per touched vertex moves its old entries, places its batch entries and
+// commits its record (k_scatter_old, k_inplace_span, k_scatter_new and
+// k_commit of the general pipeline).  A list of at most kInPlaceMax
+// moved entries is read into registers before anything is written, which
+// makes the in-place move safe; a longer one (big_min above its default)
+// moves to a new block and is streamed.
+constexpr int kApplyThreads = 128;
+
+template <bool INSERT>
+__global__ void __launch_bounds__(kApplyThreads)
+k_small_apply(const int32_t* __restrict__ seg_u, const int32_t* __restrict__ seg_kstart,
+              const int32_t* __restrict__ seg_ncap, const int32_t* __restrict__ seg_base,
+              const long long* __restrict__ seg_new_off, const int32_t* __restrict__ cdst,
+              const int32_t* __restrict__ capos, Plan plan, long long* const* __restrict__ fl,
+              AllocState* st, int32_t* __restrict__ pool, VRec* __restrict__ vtab) {
+    constexpr int IPT = kInPlaceMax / kApplyThreads;
+    __shared__ int32_t A[INSERT ? 1 : kInPlaceMax];
+    const int s = blockIdx.x;
+    const int ncap = seg_ncap[s];
+    if (ncap == -1) return;   // unchanged
+    const int u = seg_u[s];
+    const VRec r = vtab[u];
+    const int k0 = seg_kstart[s], nb = seg_kstart[s + 1] - k0;
+    const int32_t* B = cdst + k0;
+    const bool here = ncap == kInPlace;
+    const long long new_off = seg_new_off[s];
+    const int base = seg_base[s];
+    const int n = r.deg - base;
+    const long long from = r.off + base;
+    int32_t x[IPT];
+    const bool reg = n <= kInPlaceMax;   // always when in place
+    if (reg) {
+#pragma unroll
+        for (int q = 0; q < IPT; q++) {
+            const int j = q * kApplyThreads + threadIdx.x;
+            if (j < n) {
+                x[q] = pool[from + j];
+                if (!INSERT) A[j] = x[q];
+            }
+        }
+    }
+    __syncthreads();   // every read of the list before any write
+    const long long to = new_off + base;
+    auto place = [&](int j, int32_t v, const int32_t* old) {
+        if (INSERT) {
+            pool[to + j + lower_bound32(B, nb, v)] = v;
+        } else {
+            const int lbl = lower_bound32(B, nb, v);
+            int ubl = lbl;
+            while (ubl < nb && B[ubl] == v) ubl++;
+            bool keep = true;
+            if (ubl > lbl) {
+                int first = j;
+                if (j > 0 && old[j - 1] == v) first = lower_bound32(old, j, v);
+                keep = (j - first) >= ubl - lbl;
+            }
+            if (keep) pool[to + j - ubl] = v;
+        }
+    };
+    if (reg) {
+#pragma unroll
+        for (int q = 0; q < IPT; q++) {
+            const int j = q * kApplyThreads + threadIdx.x;
+            if (j < n) place(j, x[q], A);
+        }
+    } else {
+        for (int j = threadIdx.x; j < n; j += kApplyThreads) place(j, pool[from + j], pool + from);
+    }
+    if (INSERT)
+        for (int p = threadIdx.x; p < nb; p += kApplyThreads)
+            pool[new_off + p + capos[k0 + p]] = B[p];
+    if (threadIdx.x == 0) {
+        VRec nr;
+        nr.deg = INSERT ? r.deg + nb : r.deg - nb;
+        nr.cap = here ? r.cap : ncap;
+        nr.off = here ? r.off : ncap > 0 ? new_off : 0;
+        if (!here && r.cap > 0) {
+            const int c = cap_class(r.cap);
+            fl[c][plan.push_base[c] + atomicAdd(&st->prank[c], 1)] = r.off;
+        }
+        vtab[u] = nr;
+    }
+}
+
 void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* applied,
-                unsigned long long* new_triangles = nullptr) {
+                unsigned long long* new_triangles = nullptr,
+                const unsigned long long* sorted = nullptr) {
     cudaStream_t s = g->stream;
     const long long n = b->n;
     if (applied) *applied = 0;
@@ -929,17 +1255,48 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     const int L = g->key_bits;
     AllocState* st = g->alloc;
 
-    // 1. pack + sort
-    DevBuf<unsigned long long> keys(n, s), keys2(n, s);
-    HN_CUDA(cudaMemsetAsync(st, 0, sizeof(AllocState), s));
-    HN_LAUNCH(k_pack, grid_for(g, n, kB), kB, 0, s, b->src, b->dst, n, g->nV, L, keys.get(), st);
+    // one allocation for the buffers below, for batches whose buffers are small
+    Arena arena;
+    if (n <= kArenaBatch) arena.open((size_t)n * 144 + (1 << 16), s);
+    Arena* ar = arena.cap ? &arena : nullptr;
+    const bool small = n <= kSmallBatch && !g->weighted && !new_triangles;
+    DevBuf<int32_t> cdst(n, s, ar), cseg(n, s, ar), seg_u(n, s, ar), seg_kstart(n + 1, s, ar),
+        seg_ncap(n, s, ar), seg_base(n, s, ar), capos(n, s, ar), big_list(n + 1, s, ar);
+    DevBuf<long long> seg_work(n + 1, s, ar), seg_new_off(n, s, ar), seg_old_off(n, s, ar);
+    DevBuf<uint32_t> cw;
+    long long* totals = g->d_scalar;
+    // weighted graphs keep every list on the tile path, which moves the
+    // weights with their neighbours, and move every touched list
+    const int big_min = g->weighted ? INT_MAX : (int)knob(kKnobUpdateBigMin);
+    const bool in_place = !g->weighted && knob(kKnobUpdateInPlace) != 0;
+    if (small) {
+        SmallPlan* h_plan = (SmallPlan*)g->h_scalar;
+        if (insert)
+            HN_LAUNCH(k_small_front<true>, 1, kSmallThreads, 0, s, b->src, b->dst, sorted, (int)n,
+                      g->nV, L, flags, g->vtab, g->pool, in_place, big_min, cdst.get(), cseg.get(),
+                      capos.get(), seg_u.get(), seg_kstart.get(), seg_work.get(), seg_ncap.get(),
+                      seg_base.get(), seg_old_off.get(), big_list.get(), st, totals, h_plan,
+                      g->h_alloc);
+        else
+            HN_LAUNCH(k_small_front<false>, 1, kSmallThreads, 0, s, b->src, b->dst, sorted, (int)n,
+                      g->nV, L, flags, g->vtab, g->pool, in_place, big_min, cdst.get(), cseg.get(),
+                      capos.get(), seg_u.get(), seg_kstart.get(), seg_work.get(), seg_ncap.get(),
+                      seg_base.get(), seg_old_off.get(), big_list.get(), st, totals, h_plan,
+                      g->h_alloc);
+    } else {
+    // 1. pack + sort (`sorted`: the keys come sorted)
+    DevBuf<unsigned long long> keys, keys2(n, s, ar);
     // weights travel with their keys (a stable sort keeps the batch order
-    // of equal edges)
+    // of equal edges); a sorted run has none
     const bool carry_w = insert && g->weighted && b->has_w;
     DevBuf<uint32_t> wv, wv2;
+    HN_CUDA(cudaMemsetAsync(st, 0, sizeof(AllocState), s));
+    if (!sorted) {
+    keys.alloc(n, s, ar);
+    HN_LAUNCH(k_pack, grid_for(g, n, kB), kB, 0, s, b->src, b->dst, n, g->nV, L, keys.get(), st);
     if (carry_w) {
-        wv.alloc(n, s);
-        wv2.alloc(n, s);
+        wv.alloc(n, s, ar);
+        wv2.alloc(n, s, ar);
         HN_CUDA(cudaMemcpyAsync(wv.get(), b->w, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
     }
     if (knob(kKnobUpdateOwnSort)) {
@@ -947,9 +1304,9 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
         unsigned long long* ka = keys2.get();
         uint32_t* vc = carry_w ? wv.get() : nullptr;
         uint32_t* va = carry_w ? wv2.get() : nullptr;
-        radix_sort_u64(g, kc, ka, vc, va, n, 2 * L, &st->error, s);
-        if (kc != keys.get()) std::swap(keys.p, keys2.p);
-        if (carry_w && vc != wv.get()) std::swap(wv.p, wv2.p);
+        radix_sort_u64(g, kc, ka, vc, va, n, 2 * L, &st->error, s, ar);
+        if (kc != keys.get()) keys.swap(keys2);
+        if (carry_w && vc != wv.get()) wv.swap(wv2);
     } else {
         // the library sort, kept for comparison (update.own_sort 0)
         ProfileScope ps("cub_sort_keys", s);
@@ -960,63 +1317,56 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
             HN_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, db, dw, (int)n, 0, 2 * L, s));
             DevBuf<char> tmp(tb, s);
             HN_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tb, db, dw, (int)n, 0, 2 * L, s));
-            if (dw.Current() != wv.get()) std::swap(wv.p, wv2.p);
+            if (dw.Current() != wv.get()) wv.swap(wv2);
         } else {
             HN_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (int)n, 0, 2 * L, s));
             DevBuf<char> tmp(tb, s);
             HN_CUDA(cub::DeviceRadixSort::SortKeys(tmp.get(), tb, db, (int)n, 0, 2 * L, s));
         }
         count_launch();
-        if (db.Current() != keys.get()) std::swap(keys.p, keys2.p);
+        if (db.Current() != keys.get()) keys.swap(keys2);
     }
     wv2.release();
+    }
+    const unsigned long long* ks = sorted ? sorted : keys.get();
     // 2. mark  (keys2 reused as the counter values)
     unsigned long long* val = keys2.get();
     // each entry's place in its old list (insert: old entries <= it; erase:
     // old entries below it), kept for the compacted entries
-    DevBuf<int32_t> apos(n, s), capos(n, s);
+    DevBuf<int32_t> apos(n, s, ar);
     if (insert)
-        HN_LAUNCH(k_mark_insert, grid_for(g, n, kB), kB, 0, s, keys.get(), n, L, flags, g->vtab,
+        HN_LAUNCH(k_mark_insert, grid_for(g, n, kB), kB, 0, s, ks, n, L, flags, g->vtab,
                   g->pool, val, apos.get(), (const AllocState*)st);
     else
-        HN_LAUNCH(k_mark_erase, grid_for(g, n, kB), kB, 0, s, keys.get(), n, L, flags, g->vtab,
+        HN_LAUNCH(k_mark_erase, grid_for(g, n, kB), kB, 0, s, ks, n, L, flags, g->vtab,
                   g->pool, val, apos.get(), (const AllocState*)st);
     // 3. scan + compact
-    DevBuf<unsigned long long> scan(n, s);
-    exclusive_scan(g, (const unsigned long long*)val, scan.get(), n, s);
-    DevBuf<int32_t> cdst(n, s), cseg(n, s), seg_u(n, s), seg_kstart(n + 1, s), seg_ncap(n, s),
-        seg_base(n, s);
-    DevBuf<long long> seg_work(n + 1, s), seg_new_off(n, s), seg_old_off(n, s);
-    long long* totals = g->d_scalar;
-    DevBuf<uint32_t> cw;
-    if (carry_w) cw.alloc(n, s);
-    HN_LAUNCH(k_compact, grid_for(g, n, kB), kB, 0, s, keys.get(), val, scan.get(), n, L,
+    DevBuf<unsigned long long> scan(n, s, ar);
+    exclusive_scan(g, (const unsigned long long*)val, scan.get(), n, s, ar);
+    if (carry_w) cw.alloc(n, s, ar);
+    HN_LAUNCH(k_compact, grid_for(g, n, kB), kB, 0, s, ks, val, scan.get(), n, L,
               cdst.get(), cseg.get(), seg_u.get(), seg_kstart.get(), totals,
               (const uint32_t*)wv.get(), cw.get(), (const int32_t*)apos.get(), capos.get());
     wv.release();
     apos.release();
     keys2.release();
     scan.release();
-    // 4. plan (weighted graphs keep every list on the tile path, which moves
-    // the weights with their neighbours)
-    const int big_min = g->weighted ? INT_MAX : (int)knob(kKnobUpdateBigMin);
-    DevBuf<int32_t> big_list(n + 1, s);
-    DevBuf<unsigned long long> big_ctr(2, s);   // [0] hubs listed, [1] snapshot slots
+    // 4. plan
+    DevBuf<unsigned long long> big_ctr(2, s, ar);   // [0] hubs listed, [1] snapshot slots
     HN_CUDA(cudaMemsetAsync(big_ctr.get(), 0, 2 * sizeof(unsigned long long), s));
-    // weighted graphs move every touched list (the weights travel with it)
-    const bool in_place = !g->weighted && knob(kKnobUpdateInPlace) != 0;
     HN_LAUNCH(k_plan, grid_for(g, n + 1, kB), kB, 0, s, seg_u.get(), seg_kstart.get(), totals,
               insert, g->vtab, (const int32_t*)capos.get(), in_place,
               seg_work.get(), seg_ncap.get(), seg_base.get(), seg_old_off.get(), st, big_min,
               big_list.get(), (int*)big_ctr.get(), big_ctr.get() + 1);
-    // 5. host plan (the one synchronisation of the batch)
-    cudaEvent_t plan_ev = nullptr;   // profiled: the stream's idle time across the plan
-    if (g_profiling) profile_begin(s, &plan_ev);
     HN_CUDA(cudaMemcpyAsync(g->h_scalar, totals, 2 * sizeof(long long), cudaMemcpyDeviceToHost,
                             s));
     HN_CUDA(cudaMemcpyAsync(g->h_alloc, st, sizeof(AllocState), cudaMemcpyDeviceToHost, s));
     HN_CUDA(cudaMemcpyAsync(g->h_scalar + 2, big_ctr.get(), 2 * sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, s));
+    }
+    // 5. host plan (the one synchronisation of the batch)
+    cudaEvent_t plan_ev = nullptr;   // profiled: the stream's idle time across the plan
+    if (g_profiling) profile_begin(s, &plan_ev);
     HN_CUDA(cudaStreamSynchronize(s));
     const int nbig = *(const int*)(g->h_scalar + 2);
     const long long snap_words = g->h_scalar[3];
@@ -1061,8 +1411,20 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     HN_LAUNCH(k_assign, grid_for(g, nseg, kB), kB, 0, s, seg_ncap.get(), nseg, plan,
               (long long* const*)g->d_fl, st, (const long long*)seg_old_off.get(),
               seg_new_off.get());
+    if (small && nbig == 0) {
+        if (insert)
+            HN_LAUNCH(k_small_apply<true>, nseg, kApplyThreads, 0, s, seg_u.get(),
+                      seg_kstart.get(), seg_ncap.get(), seg_base.get(), seg_new_off.get(),
+                      cdst.get(), capos.get(), plan, (long long* const*)g->d_fl, st, g->pool,
+                      g->vtab);
+        else
+            HN_LAUNCH(k_small_apply<false>, nseg, kApplyThreads, 0, s, seg_u.get(),
+                      seg_kstart.get(), seg_ncap.get(), seg_base.get(), seg_new_off.get(),
+                      cdst.get(), capos.get(), plan, (long long* const*)g->d_fl, st, g->pool,
+                      g->vtab);
+    } else {
     // 7. scatter-merge
-    exclusive_scan(g, (const long long*)seg_work.get(), seg_work.get(), nseg + 1, s);
+    exclusive_scan(g, (const long long*)seg_work.get(), seg_work.get(), nseg + 1, s, ar);
     // tiles are read from the device prefix; the grid is persistent
     // five CTAs per SM (the shared-memory limit of the tile): each tile waits
     // on a short chain of dependent loads, so more resident tiles hide it
@@ -1072,12 +1434,12 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     DevBuf<unsigned long long> chunk_pre;
     DevBuf<int32_t> snap;
     if (nbig > 0) {
-        chunk_pre.alloc((size_t)nbig + 1, s);
+        chunk_pre.alloc((size_t)nbig + 1, s, ar);
         HN_LAUNCH(k_big_chunks, grid_for(g, (long long)nbig + 1, kB), kB, 0, s, big_list.get(),
                   nbig, seg_u.get(), seg_kstart.get(), seg_ncap.get(), seg_base.get(),
                   seg_old_off.get(), seg_new_off.get(), g->vtab, chunk_pre.get());
         exclusive_scan(g, (const unsigned long long*)chunk_pre.get(), chunk_pre.get(),
-                       (long long)nbig + 1, s);
+                       (long long)nbig + 1, s, ar);
         const long long grid_big = (long long)g->info.sms * 8;
         if (snap_words > 0) {
             snap.alloc((size_t)snap_words, s);
@@ -1111,7 +1473,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     // tile boundary, and the work is at most nE entries
     const long long span_cap = (g->nE + nseg) / Tile::TILE + 2;
     DevBuf<int32_t> span_list(span_cap, s);
-    DevBuf<int> nspan(1, s);
+    DevBuf<int> nspan(1, s, ar);
     HN_CUDA(cudaMemsetAsync(nspan.get(), 0, sizeof(int), s));
     const long long grid_span = (long long)g->info.sms * 8;
     if (insert) {
@@ -1119,7 +1481,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
                   seg_u.get(), seg_kstart.get(), seg_new_off.get(), cdst.get(),
                   seg_old_off.get(), seg_ncap.get(), seg_base.get(), g->pool, splits.get(),
                   (long long)splits.n - 1, g->wpool, span_list.get(), nspan.get(), span_cap);
-        HN_LAUNCH(k_inplace_span<true>, grid_span, kSpanWarps * 32, 0, s, span_list.get(),
+        HN_LAUNCH(k_inplace_span<true>, grid_span, kSpanThreads, 0, s, span_list.get(),
                   nspan.get(), seg_u.get(), seg_kstart.get(), seg_base.get(), seg_old_off.get(),
                   cdst.get(), g->vtab, g->pool, span_cap);
         HN_LAUNCH(k_scatter_new, grid_for(g, kept, kB), kB, 0, s, cdst.get(), cseg.get(),
@@ -1130,7 +1492,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
                   nseg, seg_u.get(), seg_kstart.get(), seg_new_off.get(), cdst.get(),
                   seg_old_off.get(), seg_ncap.get(), seg_base.get(), g->pool, splits.get(),
                   (long long)splits.n - 1, g->wpool, span_list.get(), nspan.get(), span_cap);
-        HN_LAUNCH(k_inplace_span<false>, grid_span, kSpanWarps * 32, 0, s, span_list.get(),
+        HN_LAUNCH(k_inplace_span<false>, grid_span, kSpanThreads, 0, s, span_list.get(),
                   nspan.get(), seg_u.get(), seg_kstart.get(), seg_base.get(), seg_old_off.get(),
                   cdst.get(), g->vtab, g->pool, span_cap);
     }
@@ -1138,6 +1500,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     HN_LAUNCH(k_commit, grid_for(g, nseg, kB), kB, 0, s, seg_u.get(), seg_kstart.get(),
               seg_ncap.get(), seg_new_off.get(), nseg, insert, plan, (long long* const*)g->d_fl,
               st, g->vtab);
+    }
     for (int c = 0; c < kNumClasses; c++)
         g->fl_count[c] = plan.push_base[c] + g->h_alloc->push[c];
     g->bump_host = bump;
@@ -1185,23 +1548,17 @@ __global__ void k_net_mark(const unsigned long long* __restrict__ keys,
     }
 }
 
+// The net insert and erase sets, as sorted keys.
 __global__ void k_net_split(const unsigned long long* __restrict__ keys,
                             const unsigned long long* __restrict__ val,
-                            const unsigned long long* __restrict__ scan, long long n, int L,
-                            int32_t* ins_src, int32_t* ins_dst, int32_t* del_src,
-                            int32_t* del_dst, long long* totals) {
-    const unsigned long long mask = (1ull << L) - 1;
+                            const unsigned long long* __restrict__ scan, long long n,
+                            unsigned long long* __restrict__ ins,
+                            unsigned long long* __restrict__ del, long long* totals) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long v = val[i], at = scan[i];
-        const int32_t u = (int32_t)(keys[i] >> L), w = (int32_t)(keys[i] & mask);
-        if (v & 0xFFFFFFFFull) {
-            ins_src[at & 0xFFFFFFFFull] = u;
-            ins_dst[at & 0xFFFFFFFFull] = w;
-        } else if (v >> 32) {
-            del_src[at >> 32] = u;
-            del_dst[at >> 32] = w;
-        }
+        if (v & 0xFFFFFFFFull) ins[at & 0xFFFFFFFFull] = keys[i];
+        else if (v >> 32) del[at >> 32] = keys[i];
         if (i == n - 1) {
             totals[0] = (long long)((at + v) & 0xFFFFFFFFull);
             totals[1] = (long long)((at + v) >> 32);
@@ -1358,15 +1715,18 @@ int hn_update_coalesced(hn_graph_t* g, int64_t n, const int32_t* src, const int3
     HN_CUDA(cudaSetDevice(g->device));
     cudaStream_t s = g->stream;
     const int L = g->key_bits;
+    Arena arena;
+    if (n <= kArenaBatch) arena.open((size_t)n * 80 + (1 << 16), s);
+    Arena* ar = arena.cap ? &arena : nullptr;
     DevBuf<int32_t> hs, hd;
     DevBuf<unsigned char> hops;
     const int32_t* d_src = src;
     const int32_t* d_dst = dst;
     const unsigned char* d_ops = ops;
     if (mem == HN_MEM_HOST) {
-        hs.alloc((size_t)n, s);
-        hd.alloc((size_t)n, s);
-        hops.alloc((size_t)n, s);
+        hs.alloc((size_t)n, s, ar);
+        hd.alloc((size_t)n, s, ar);
+        hops.alloc((size_t)n, s, ar);
         HN_CUDA(cudaMemcpyAsync(hs.get(), src, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
         HN_CUDA(cudaMemcpyAsync(hd.get(), dst, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
         HN_CUDA(cudaMemcpyAsync(hops.get(), ops, (size_t)n, cudaMemcpyHostToDevice, s));
@@ -1375,8 +1735,8 @@ int hn_update_coalesced(hn_graph_t* g, int64_t n, const int32_t* src, const int3
         d_ops = hops.get();
     }
     AllocState* st = g->alloc;
-    DevBuf<unsigned long long> keys((size_t)n, s), keys2((size_t)n, s);
-    DevBuf<uint32_t> ops2((size_t)n, s), ops1((size_t)n, s);
+    DevBuf<unsigned long long> keys((size_t)n, s, ar), keys2((size_t)n, s, ar);
+    DevBuf<uint32_t> ops2((size_t)n, s, ar), ops1((size_t)n, s, ar);
     HN_CUDA(cudaMemsetAsync(st, 0, sizeof(AllocState), s));
     HN_LAUNCH(k_pack, grid_for(g, n, kB), kB, 0, s, d_src, d_dst, n, g->nV, L, keys.get(), st);
     HN_LAUNCH(k_widen_ops, grid_for(g, n, kB), kB, 0, s, d_ops, n, ops1.get());
@@ -1386,21 +1746,21 @@ int hn_update_coalesced(hn_graph_t* g, int64_t n, const int32_t* src, const int3
         unsigned long long* ka = keys2.get();
         uint32_t* vc = ops1.get();
         uint32_t* va = ops2.get();
-        radix_sort_u64(g, kc, ka, vc, va, n, 2 * L, &st->error, s);
-        if (kc != keys.get()) std::swap(keys.p, keys2.p);
-        if (vc != ops1.get()) std::swap(ops1.p, ops2.p);
+        radix_sort_u64(g, kc, ka, vc, va, n, 2 * L, &st->error, s, ar);
+        if (kc != keys.get()) keys.swap(keys2);
+        if (vc != ops1.get()) ops1.swap(ops2);
     }
     unsigned long long* val = keys2.get();
     HN_LAUNCH(k_net_mark, grid_for(g, n, kB), kB, 0, s, keys.get(), ops1.get(), n, val,
               (const AllocState*)st);
-    DevBuf<unsigned long long> scan((size_t)n, s);
-    exclusive_scan(g, (const unsigned long long*)val, scan.get(), n, s);
+    DevBuf<unsigned long long> scan((size_t)n, s, ar);
+    exclusive_scan(g, (const unsigned long long*)val, scan.get(), n, s, ar);
     hn_batch bi, bd;
     bi.g = bd.g = g;
     bi.device = bd.device = g->device;
-    DevBuf<int32_t> is((size_t)n, s), id((size_t)n, s), ds((size_t)n, s), dd((size_t)n, s);
-    HN_LAUNCH(k_net_split, grid_for(g, n, kB), kB, 0, s, keys.get(), val, scan.get(), n, L,
-              is.get(), id.get(), ds.get(), dd.get(), g->d_scalar);
+    DevBuf<unsigned long long> ins((size_t)n, s, ar), del((size_t)n, s, ar);
+    HN_LAUNCH(k_net_split, grid_for(g, n, kB), kB, 0, s, keys.get(), val, scan.get(), n, ins.get(),
+              del.get(), g->d_scalar);
     HN_CUDA(cudaMemcpyAsync(g->h_scalar, g->d_scalar, 2 * sizeof(long long),
                             cudaMemcpyDeviceToHost, s));
     HN_CUDA(cudaMemcpyAsync(g->h_alloc, st, sizeof(AllocState), cudaMemcpyDeviceToHost, s));
@@ -1415,13 +1775,10 @@ int hn_update_coalesced(hn_graph_t* g, int64_t n, const int32_t* src, const int3
     keys.release();
     keys2.release();
     scan.release();
-    bd.src = ds.get();
-    bd.dst = dd.get();
-    bi.src = is.get();
-    bi.dst = id.get();
-    // the two sets are disjoint, so their order does not matter
-    run_update(g, &bd, HN_DEDUP_BATCH, false, erased);
-    run_update(g, &bi, HN_DEDUP_BATCH | HN_DEDUP_GRAPH, true, inserted);
+    // the two sets are disjoint, so their order does not matter; both come
+    // out of the split sorted
+    run_update(g, &bd, HN_DEDUP_BATCH, false, erased, nullptr, del.get());
+    run_update(g, &bi, HN_DEDUP_BATCH | HN_DEDUP_GRAPH, true, inserted, nullptr, ins.get());
     HN_API_END
 }
 
