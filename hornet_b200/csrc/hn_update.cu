@@ -32,6 +32,7 @@
 #include <climits>
 
 #include "hn_graph.cuh"
+#include "hn_window.cuh"
 
 namespace hn {
 namespace {
@@ -195,7 +196,7 @@ __global__ void k_compact(const unsigned long long* __restrict__ keys,
 // is rewritten (insert: base = the old entries <= the smallest batch entry;
 // erase: base = the old entries below the smallest deleted one); a list
 // moved by the tiles only when that part has at most kInPlaceMax entries,
-// so that one warp can stage it, a hub only when it has at most kHubSnap
+// so that one warp moves it, a hub only when it has at most kHubSnap
 // batch entries (the slots snapshotted per chunk boundary).  Other vertices move to a new block (seg_ncap = new capacity, 0 for
 // an emptied list, -1 for a vertex without batch entries) and their whole
 // list is the work.  seg_work[s] = entries the scatter moves (0 for hubs,
@@ -313,13 +314,8 @@ k_assign(const int32_t* __restrict__ seg_ncap, long long nseg, Plan plan,
     }
 }
 
-// Scatter tiles: 256 threads x 4 items, five CTAs per SM (the shared-memory
-// limit of a tile).  128 x 8, 128 x 4 (ten per SM) and 256 x 2 (eight per
-// SM) measured 13-52 % slower on the 10M-edge batch.
 constexpr int kSB = 256;
-constexpr int kScatterCtas = 5;
-using Tile = LbTile<kSB, 4>;
-constexpr int kStage = 512;    // batch entries of a tile staged in shared memory
+constexpr int kScatterTile = 1024;   // elements of a warp's scatter tile
 
 __device__ __forceinline__ int lower_bound32(const int32_t* a, int n, int32_t x) {
     int lo = 0, hi = n;
@@ -341,213 +337,117 @@ __device__ __forceinline__ int upper_bound32(const int32_t* a, int n, int32_t x)
 
 // Old adjacency of every changed vertex -> its place in the new block, or
 // in its own block for a vertex updated in place (only its entries from
-// seg_base on are work items).  The batch entries the tile's segments search
-// are one contiguous run of cdst (the segments are consecutive sources and
-// cdst is sorted by source): when the run has at most kStage entries it is
-// staged in shared memory, so the per-item searches do not wait on global
-// loads.
+// seg_base on are work items).  A warp per merge-path tile, in windows of 32
+// touched vertices; an item's batch entries (few: 1.7 a vertex on a uniform
+// 10M batch) are searched where they are.
 //
-// In place, an entry's new slot may be another entry's old slot, so every
-// item's value and destination are read and computed before the barrier
-// and stored after it.  That orders the reads before the writes within the
-// CTA; a vertex updated in place whose items span two tiles (two CTAs)
-// would not be ordered, so the tiles leave it alone and the tile holding
-// its first item lists it for k_inplace_span, which moves it whole.
+// In place, an entry's new slot may be another entry's old slot.  An insert
+// moves entries right, so the rows of a window go from last to first, an
+// erase moves them left, from first to last; a row group's loads all precede
+// its stores.  A vertex updated in place must be moved by one warp for that:
+// the one whose tile holds its first item moves all of it (at most
+// kInPlaceMax entries), past the tile's end if need be, and the next tile
+// skips it.
 template <bool INSERT>
-__global__ void __launch_bounds__(kSB, kScatterCtas)
+__global__ void __launch_bounds__(kSB)
 k_scatter_old(const long long* __restrict__ prefix, long long nseg,
-              const int32_t* __restrict__ seg_u, const int32_t* __restrict__ seg_kstart,
-              const long long* __restrict__ seg_new_off, const int32_t* __restrict__ cdst,
+              const int32_t* __restrict__ seg_kstart, const long long* __restrict__ seg_new_off,
+              const int32_t* __restrict__ cdst, const int32_t* __restrict__ capos,
               const long long* __restrict__ seg_old_off, const int32_t* __restrict__ seg_ncap,
-              const int32_t* __restrict__ seg_base, int32_t* __restrict__ pool,
-              const long long* __restrict__ splits, long long split_tiles,
-              uint32_t* __restrict__ wpool, int32_t* __restrict__ span_list,
-              int* __restrict__ nspan, long long span_cap) {
-    __shared__ Tile t;
-    __shared__ long long s_old[Tile::TILE + 1];   // old slot of item e: s_old[b] + e
-    __shared__ long long s_new[Tile::TILE + 1];   // slot before the batch shift: s_new[b] + e
-    __shared__ int s_k0[Tile::TILE + 1];   // the batch list of segment b, narrowed to
-    __shared__ int s_k1[Tile::TILE + 1];   // the old values this tile holds: [k0, k1)
-    __shared__ int s_kb[Tile::TILE + 1];   // batch entries of the segment before k0
-    __shared__ int32_t s_cd[kStage];       // cdst[K0, K1) of this tile
-    __shared__ int s_K0, s_K1;
+              const int32_t* __restrict__ seg_base, int32_t* pool,
+              const long long* __restrict__ splits, uint32_t* wpool) {
+    constexpr int ROWS = 4;
+    const unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
     const long long total = prefix[nseg];
-    long long ntiles = (total + nseg + Tile::TILE - 1) / Tile::TILE;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        if (threadIdx.x == 0) {   // the previous tile ended with a barrier
-            s_K0 = INT_MAX;
-            s_K1 = INT_MIN;
+    const long long ntiles = (total + nseg + kScatterTile - 1) / kScatterTile;
+    const long long nwarps = (long long)gridDim.x * (kSB / 32);
+    for (long long tile = blockIdx.x * (long long)(kSB / 32) + (threadIdx.x >> 5); tile < ntiles;
+         tile += nwarps) {
+        WarpTile wt = warp_tile(splits, tile, kScatterTile, total, nseg);
+        if (wt.nitems == 0) continue;
+        const long long tend = wt.item0 + wt.nitems;
+        // the tile's last vertex in place: to its end (uniform)
+        if (seg_ncap[wt.seg1] == kInPlace) {
+            const long long f = prefix[wt.seg1], en = prefix[wt.seg1 + 1];
+            if (f >= wt.item0 && f < tend && en > tend) wt.nitems = (int)(en - wt.item0);
         }
-        int n = lb_tile_load(t, prefix, nseg, total, tile, splits, split_tiles);
-        for (int b = threadIdx.x; b <= t.nends; b += kSB) {
-            long long s = t.seg0 + b;
-            s_k0[b] = 0;
-            s_k1[b] = -1;   // marks a segment this tile does not move
-            if (s < nseg) {
-                const long long st0 = t.seg_start(b);
-                const long long en = t.ends[b], tend = t.item0 + n;
-                if (seg_ncap[s] == kInPlace && (st0 < t.item0 || en > tend)) {
-                    // in place and spanning tiles: listed once, by the tile
-                    // holding its first item
-                    if (st0 >= t.item0 && st0 < tend) {
-                        // one vertex per tile boundary at most, so the
-                        // list (one entry per tile) never fills
-                        const int at = atomicAdd(nspan, 1);
-                        if (at < span_cap) span_list[at] = (int)s;
+        for (long long s0 = wt.seg0; s0 <= wt.seg1; s0 += 32) {
+            const long long s = s0 + lane < nseg ? s0 + lane : nseg;
+            const long long first = prefix[s];
+            const long long next = s0 + 32 <= nseg ? prefix[s0 + 32] : total;
+            const WarpWindow w = warp_window(wt, s0, first, next);
+            if (w.n == 0) continue;
+            // the lane's segment (its record before the window's compaction)
+            long long so = 0, sn = 0;   // slot of item e: so + e, before the shift sn + e
+            int k0 = 0, nb = -1, rb = 0;   // batch list; index of item e in the list: rb + e
+            if (s <= wt.seg1 && s < nseg) {
+                const long long en = prefix[s + 1];
+                if (first < en && first < tend && en > wt.item0) {
+                    const int base = seg_base[s];
+                    // (in place from an earlier tile: moved there)
+                    if (seg_ncap[s] != kInPlace || first >= wt.item0) {
+                        k0 = seg_kstart[s];
+                        nb = seg_kstart[s + 1] - k0;
+                        so = seg_old_off[s] + base - first + wt.item0;
+                        sn = seg_new_off[s] + base - first + wt.item0;
+                        rb = base + (int)(wt.item0 - first);
                     }
-                    continue;
-                }
-                const int base = seg_base[s];
-                const long long old_off = seg_old_off[s] + base;
-                s_old[b] = old_off - st0;
-                s_new[b] = seg_new_off[s] + base - st0;
-                const int k0 = seg_kstart[s], k1 = seg_kstart[s + 1];
-                // a segment with a long batch list (a hub hit by many
-                // updates) searches only the batch entries that can fall
-                // between this tile's first and last old value; short lists
-                // are searched whole
-                const long long lo_e = st0 > t.item0 ? st0 : t.item0;
-                const long long hi_e = en < tend ? en : tend;
-                int blo = 0, bhi = k1 - k0;
-                if (lo_e < hi_e && k1 - k0 > 8) {   // short batch lists: searched whole
-                    const int32_t a_lo = pool[old_off + (lo_e - st0)];
-                    const int32_t a_hi = pool[old_off + (hi_e - 1 - st0)];
-                    blo = (int)lower_bound_dev(cdst + k0, (long long)(k1 - k0), a_lo);
-                    bhi = (int)upper_bound_dev(cdst + k0, (long long)(k1 - k0), a_hi);
-                }
-                s_k0[b] = k0 + blo;
-                s_k1[b] = k0 + bhi;
-                s_kb[b] = blo;
-                if (bhi > blo) {
-                    atomicMin(&s_K0, k0 + blo);
-                    atomicMax(&s_K1, k0 + bhi);
                 }
             }
-        }
-        __syncthreads();
-        // all of this thread's old-list loads first (the pool is both read
-        // and written here, so a plain loop would wait for each store)
-        constexpr int IPT = Tile::TILE / kSB;
-        int xs[IPT], bs[IPT];
-        uint32_t ws[IPT];
+            so = __shfl_sync(kFull, so, w.lane_of);
+            sn = __shfl_sync(kFull, sn, w.lane_of);
+            k0 = __shfl_sync(kFull, k0, w.lane_of);
+            nb = __shfl_sync(kFull, nb, w.lane_of);
+            rb = __shfl_sync(kFull, rb, w.lane_of);
+            const int row0 = w.begin & ~31;
+            const int groups = (w.end - row0 + 32 * ROWS - 1) / (32 * ROWS);
+            for (int q = 0; q < groups; q++) {
+                const int r = row0 + 32 * ROWS * (INSERT ? groups - 1 - q : q);
+                int32_t x[ROWS];
+                uint32_t y[ROWS];
+                long long to[ROWS];   // -1: no item, deleted, or another tile's
+                int bk[ROWS], bn[ROWS], br[ROWS];
 #pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            const int i = threadIdx.x + k * kSB;
-            bs[k] = -1;
-            ws[k] = 0;
-            if (i < n) {
-                const int b = t.seg[i];
-                if (s_k1[b] >= s_k0[b]) {
-                    bs[k] = b;
-                    xs[k] = pool[s_old[b] + t.item0 + i];
-                    if (wpool) ws[k] = wpool[s_old[b] + t.item0 + i];
+                for (int k = 0; k < ROWS; k++) {
+                    const int row = r + 32 * k, e = row + lane;
+                    to[k] = -1;
+                    x[k] = 0;
+                    if (row >= w.end) continue;   // uniform
+                    const int j = warp_owner(w, row) & 31;
+                    const long long a = __shfl_sync(kFull, so, j), b = __shfl_sync(kFull, sn, j);
+                    bk[k] = __shfl_sync(kFull, k0, j);
+                    bn[k] = __shfl_sync(kFull, nb, j);
+                    br[k] = INSERT ? 0 : __shfl_sync(kFull, rb, j);
+                    if (e >= w.begin && e < w.end && bn[k] >= 0) {
+                        x[k] = pool[a + e];
+                        if (wpool) y[k] = wpool[a + e];
+                        to[k] = b + e;
+                    }
                 }
+                __syncwarp();   // every read of the group before any write
+#pragma unroll
+                for (int k = 0; k < ROWS; k++) {
+                    if (to[k] < 0) continue;
+                    const int32_t* B = cdst + bk[k];
+                    const int lb = lower_bound32(B, bn[k], x[k]);
+                    if (INSERT) {
+                        to[k] += lb;
+                    } else {
+                        int ub = lb;
+                        while (ub < bn[k] && B[ub] == x[k]) ub++;
+                        // the first (ub - lb) copies of x go: ranks count from
+                        // the first copy's slot, recorded at marking
+                        const int rank = br[k] + r + 32 * k + lane - (ub > lb ? capos[bk[k] + lb] : 0);
+                        if (ub > lb && rank < ub - lb) continue;
+                        to[k] -= ub;
+                    }
+                    pool[to[k]] = x[k];
+                    if (wpool) wpool[to[k]] = y[k];
+                }
+                __syncwarp();
             }
         }
-        // stage the tile's batch run while those loads are in flight
-        const int K0 = s_K0, K1 = s_K1;
-        const bool staged = K1 > K0 && K1 - K0 <= kStage;   // uniform in the CTA
-        if (staged) {
-            for (int i = threadIdx.x; i < K1 - K0; i += kSB) s_cd[i] = cdst[K0 + i];
-            __syncthreads();
-        }
-        long long to[IPT];   // destination slot, -1 = the entry is deleted
-#pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            to[k] = -1;
-            if (bs[k] < 0) continue;
-            const int b = bs[k];
-            const int x = xs[k];
-            const long long e = t.item0 + threadIdx.x + k * kSB;   // global item
-            const int nb = s_k1[b] - s_k0[b];
-            // read only when nb > 0, and then [s_k0[b], s_k1[b]) lies in [K0, K1)
-            const int32_t* B = staged ? s_cd + (s_k0[b] - K0) : cdst + s_k0[b];
-            if (INSERT) {
-                to[k] = s_new[b] + e + s_kb[b] + lower_bound32(B, nb, x);
-            } else {
-                // every batch copy of x lies inside the narrowed range
-                // batch entries below x, then its copies (few): one search
-                const long long lbl = lower_bound32(B, nb, x);
-                long long ubl = lbl;
-                while (ubl < nb && B[ubl] == x) ubl++;
-                long long cnt = ubl - lbl;  // copies of x to delete
-                bool keep = true;
-                if (cnt > 0) {
-                    // rank of this copy among equal values of the old list
-                    // (the entries before seg_base are all below x)
-                    long long r = e - t.seg_start(b);
-                    const int32_t* A = pool + s_old[b] + t.seg_start(b);
-                    long long first = r;
-                    if (r > 0 && A[r - 1] == x) first = lower_bound_dev(A, r, x);
-                    keep = (r - first) >= cnt;
-                }
-                if (keep) to[k] = s_new[b] + e - (s_kb[b] + ubl);
-            }
-        }
-        __syncthreads();   // every read of this tile's lists before any write
-#pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            if (to[k] < 0) continue;
-            pool[to[k]] = xs[k];
-            if (wpool) wpool[to[k]] = ws[k];
-        }
-        __syncthreads();
-    }
-}
-
-// Vertices updated in place whose moved entries span two or more scatter
-// tiles: a CTA each stages the moved part [base, deg) (at most kInPlaceMax
-// entries) in shared memory, then writes every entry to its new slot, so
-// all reads precede all writes.  Same slot rules as k_scatter_old.  There are
-// few such vertices (one per tile boundary at most), so what counts is the
-// chain of one of them: with a warp each it took 64 dependent rounds.
-constexpr int kSpanThreads = 256;
-
-template <bool INSERT>
-__global__ void __launch_bounds__(kSpanThreads)
-k_inplace_span(const int32_t* __restrict__ span_list, const int* __restrict__ nspan,
-               const int32_t* __restrict__ seg_u, const int32_t* __restrict__ seg_kstart,
-               const int32_t* __restrict__ seg_base, const long long* __restrict__ seg_old_off,
-               const int32_t* __restrict__ cdst, const VRec* __restrict__ vtab,
-               int32_t* __restrict__ pool, long long span_cap) {
-    constexpr int IPT = kInPlaceMax / kSpanThreads;
-    __shared__ int32_t A[kInPlaceMax];
-    const int count = *nspan < span_cap ? *nspan : (int)span_cap;
-    for (int i = blockIdx.x; i < count; i += gridDim.x) {
-        const int s = span_list[i];
-        const int base = seg_base[s];
-        const int n = vtab[seg_u[s]].deg - base;   // the old degree: commit runs later
-        const long long off = seg_old_off[s] + base;
-        const int k0 = seg_kstart[s], nb = seg_kstart[s + 1] - k0;
-        const int32_t* B = cdst + k0;
-        int32_t x[IPT];
-#pragma unroll
-        for (int q = 0; q < IPT; q++) {
-            const int j = q * kSpanThreads + threadIdx.x;
-            x[q] = j < n ? pool[off + j] : 0;
-            if (!INSERT && j < n) A[j] = x[q];
-        }
-        __syncthreads();   // every read of the list before any write
-#pragma unroll
-        for (int q = 0; q < IPT; q++) {
-            const int j = q * kSpanThreads + threadIdx.x;
-            if (j >= n) break;
-            if (INSERT) {
-                pool[off + j + lower_bound32(B, nb, x[q])] = x[q];
-            } else {
-                const int lbl = lower_bound32(B, nb, x[q]);
-                int ubl = lbl;
-                while (ubl < nb && B[ubl] == x[q]) ubl++;
-                bool keep = true;
-                if (ubl > lbl) {
-                    int first = j;
-                    if (j > 0 && A[j - 1] == x[q]) first = lower_bound32(A, j, x[q]);
-                    keep = (j - first) >= ubl - lbl;
-                }
-                if (keep) pool[off + j - ubl] = x[q];
-            }
-        }
-        __syncthreads();   // A is restaged for the next vertex
     }
 }
 
@@ -641,9 +541,12 @@ __global__ void k_big_snap(const int32_t* __restrict__ big_list, int nbig,
                            const long long* __restrict__ seg_new_off,
                            const VRec* __restrict__ vtab, const unsigned long long* __restrict__ pre,
                            const int32_t* __restrict__ pool, int32_t* __restrict__ snap) {
-    // a thread per chunk: a boundary keeps only k (<= kHubSnap) slots
+    // a warp per chunk (its k <= kHubSnap slots side by side: a thread per
+    // chunk copied them one after the other, 30 us for a 300K-entry batch)
     const int total = (int)(pre[nbig] >> 32);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    for (int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < total; q += nwarps) {
         const int i = big_hub_of(pre, nbig, q);
         const int c = q - (int)(pre[i] >> 32);
         const BigHub h = big_hub(big_list[i], seg_u, seg_kstart, seg_ncap, seg_base, seg_old_off,
@@ -651,7 +554,7 @@ __global__ void k_big_snap(const int32_t* __restrict__ big_list, int nbig,
         if (!h.in_place || c + 1 >= h.nch) continue;   // no boundary after this chunk
         const long long r1 = (long long)h.base + (long long)(c + 1) * kBigChunk;
         int32_t* out = snap + (pre[i] & 0xFFFFFFFFull) + (long long)c * h.nb;
-        for (int t = 0; t < h.nb; t++) {
+        for (int t = lane; t < h.nb; t += 32) {
             const long long r = INSERT ? r1 + t : r1 - h.nb + t;
             if (r < h.deg) out[t] = pool[h.old_off + r];
         }
@@ -1162,8 +1065,8 @@ k_small_front(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
 
 // After the host's plan and k_assign, when the batch touches no hub: a CTA
 // per touched vertex moves its old entries, places its batch entries and
-// commits its record (k_scatter_old, k_inplace_span, k_scatter_new and
-// k_commit of the general pipeline).  A list of at most kInPlaceMax
+// commits its record (k_scatter_old, k_scatter_new and k_commit of the
+// general pipeline).  A list of at most kInPlaceMax
 // moved entries is read into registers before anything is written, which
 // makes the in-place move safe; a longer one (big_min above its default)
 // moves to a new block and is streamed.
@@ -1425,12 +1328,10 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     } else {
     // 7. scatter-merge
     exclusive_scan(g, (const long long*)seg_work.get(), seg_work.get(), nseg + 1, s, ar);
-    // tiles are read from the device prefix; the grid is persistent
-    // five CTAs per SM (the shared-memory limit of the tile): each tile waits
-    // on a short chain of dependent loads, so more resident tiles hide it
-    const long long grid_sc = (long long)g->info.sms * kScatterCtas;
+    // the work is known on the device only: a persistent grid
+    const long long grid_sc = (long long)g->info.sms * 8;
     DevBuf<long long> splits;
-    lb_splits(g, seg_work.get(), nseg, g->nE, Tile::TILE, splits);
+    lb_splits(g, seg_work.get(), nseg, g->nE, kScatterTile, splits);
     DevBuf<unsigned long long> chunk_pre;
     DevBuf<int32_t> snap;
     if (nbig > 0) {
@@ -1443,7 +1344,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
         const long long grid_big = (long long)g->info.sms * 8;
         if (snap_words > 0) {
             snap.alloc((size_t)snap_words, s);
-            const long long grid_snap = grid_for(g, nbig * 8ll, kB);   // ~8 chunks a hub
+            const long long grid_snap = grid_for(g, nbig * 8ll, kB / 32);   // ~8 chunks a hub
             if (insert)
                 HN_LAUNCH(k_big_snap<true>, grid_snap, kB, 0, s, big_list.get(), nbig, seg_u.get(),
                           seg_kstart.get(), seg_ncap.get(), seg_base.get(), seg_old_off.get(),
@@ -1469,32 +1370,19 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
                       (const int32_t*)capos.get(), g->vtab, g->pool,
                       (const unsigned long long*)chunk_pre.get(), (const int32_t*)snap.get());
     }
-    // in-place vertices whose moved entries span tiles: at most one per
-    // tile boundary, and the work is at most nE entries
-    const long long span_cap = (g->nE + nseg) / Tile::TILE + 2;
-    DevBuf<int32_t> span_list(span_cap, s);
-    DevBuf<int> nspan(1, s, ar);
-    HN_CUDA(cudaMemsetAsync(nspan.get(), 0, sizeof(int), s));
-    const long long grid_span = (long long)g->info.sms * 8;
     if (insert) {
-        HN_LAUNCH(k_scatter_old<true>, grid_sc, kSB, 0, s, seg_work.get(), nseg,
-                  seg_u.get(), seg_kstart.get(), seg_new_off.get(), cdst.get(),
-                  seg_old_off.get(), seg_ncap.get(), seg_base.get(), g->pool, splits.get(),
-                  (long long)splits.n - 1, g->wpool, span_list.get(), nspan.get(), span_cap);
-        HN_LAUNCH(k_inplace_span<true>, grid_span, kSpanThreads, 0, s, span_list.get(),
-                  nspan.get(), seg_u.get(), seg_kstart.get(), seg_base.get(), seg_old_off.get(),
-                  cdst.get(), g->vtab, g->pool, span_cap);
+        HN_LAUNCH(k_scatter_old<true>, grid_sc, kSB, 0, s, (const long long*)seg_work.get(), nseg,
+                  seg_kstart.get(), seg_new_off.get(), cdst.get(), (const int32_t*)capos.get(),
+                  seg_old_off.get(), seg_ncap.get(), seg_base.get(), g->pool,
+                  (const long long*)splits.get(), g->wpool);
         HN_LAUNCH(k_scatter_new, grid_for(g, kept, kB), kB, 0, s, cdst.get(), cseg.get(),
                   (const int32_t*)capos.get(), totals, seg_kstart.get(), seg_new_off.get(),
                   g->pool, (const uint32_t*)cw.get(), g->wpool);
     } else {
-        HN_LAUNCH(k_scatter_old<false>, grid_sc, kSB, 0, s, seg_work.get(),
-                  nseg, seg_u.get(), seg_kstart.get(), seg_new_off.get(), cdst.get(),
-                  seg_old_off.get(), seg_ncap.get(), seg_base.get(), g->pool, splits.get(),
-                  (long long)splits.n - 1, g->wpool, span_list.get(), nspan.get(), span_cap);
-        HN_LAUNCH(k_inplace_span<false>, grid_span, kSpanThreads, 0, s, span_list.get(),
-                  nspan.get(), seg_u.get(), seg_kstart.get(), seg_base.get(), seg_old_off.get(),
-                  cdst.get(), g->vtab, g->pool, span_cap);
+        HN_LAUNCH(k_scatter_old<false>, grid_sc, kSB, 0, s, (const long long*)seg_work.get(), nseg,
+                  seg_kstart.get(), seg_new_off.get(), cdst.get(), (const int32_t*)capos.get(),
+                  seg_old_off.get(), seg_ncap.get(), seg_base.get(), g->pool,
+                  (const long long*)splits.get(), g->wpool);
     }
     // 8. commit
     HN_LAUNCH(k_commit, grid_for(g, nseg, kB), kB, 0, s, seg_u.get(), seg_kstart.get(),
