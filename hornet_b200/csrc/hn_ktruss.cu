@@ -24,8 +24,11 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstddef>
+#include <cstring>
 
 #include "hn_graph.cuh"
+#include "hn_gridsync.cuh"
 #include "hn_tc.cuh"
 
 namespace hn {
@@ -33,11 +36,8 @@ namespace {
 
 constexpr int kB = 256;
 
-// Device state of the peel rounds.  Every kernel of a round reads its
-// arrays and counts from here, so one instantiated CUDA graph (a WHILE node
-// around the round's kernels) serves every round of every K: the frontier
-// buffers swap, the lists shrink and K advances on the device or between
-// graph launches, never as baked-in kernel arguments.
+// Device state of the host-driven peel rounds (ktruss.device_rounds = 0):
+// every kernel of a round reads its arrays and counts from here.
 struct KtPeel {
     const long long* off;     // current adjacency lists (rebuilt as edges die)
     const int32_t* adj;
@@ -95,12 +95,13 @@ __global__ void k_kt_init(const int32_t* __restrict__ adj, const int32_t* __rest
 }
 
 // Positions of the current lists whose (canonical) edge is still alive.
+// (alive as bytes, or state: alive iff INT_MAX)
 __global__ void k_kt_live_pos(const int32_t* __restrict__ canon, long long n,
                               const unsigned char* __restrict__ alive,
-                              int32_t* __restrict__ flag) {
+                              const int32_t* __restrict__ state, int32_t* __restrict__ flag) {
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n;
          p += (long long)gridDim.x * blockDim.x)
-        flag[p] = alive[canon[p]] ? 1 : 0;
+        flag[p] = state ? state[canon[p]] == INT_MAX : alive[canon[p]] != 0;
 }
 
 // List shrinking: a vertex's new offset is the new slot of its first old
@@ -293,10 +294,9 @@ __global__ void k_kt_mark(const KtPeel* st, unsigned char* __restrict__ inF) {
         inF[NF[i]] = 1;
 }
 
-// End of a round (one thread): the peeled edges leave the alive count, the
-// next frontier becomes the current one, and the WHILE loop continues while
-// it is non-empty.
-__global__ void k_kt_advance(KtPeel* st, cudaGraphConditionalHandle cond, int in_graph) {
+// End of a round (one thread): the peeled edges leave the alive count and the
+// next frontier becomes the current one.
+__global__ void k_kt_advance(KtPeel* st) {
     st->remaining -= st->nf;
     st->rounds++;
     int32_t* t = st->F;
@@ -305,7 +305,6 @@ __global__ void k_kt_advance(KtPeel* st, cudaGraphConditionalHandle cond, int in
     st->nf = st->nNF;
     st->nNF = 0;
     st->nheavy = 0;
-    if (in_graph) cudaGraphSetConditional(cond, st->nf > 0 ? 1u : 0u);
 }
 
 // Start of a K (one thread): its value, empty frontier counters.
@@ -314,6 +313,321 @@ __global__ void k_kt_begin(KtPeel* st, int K) {
     st->nf = 0;
     st->nNF = 0;
     st->nheavy = 0;
+}
+
+// ---------------------------------------------------------------------------
+// k_kt_run: the peel rounds of K after K in one cooperative launch
+// (ktruss.device_rounds = 1).  A K ends with the compaction of the alive
+// list, which also gives the next K that peels anything.  The kernel returns
+// when no edge is left or when at most half of the entries of the adjacency
+// lists are alive (the host then rebuilds the lists).
+//
+// Most rounds are small (a hundred thousand vertices: 62 values of K, several
+// hundred rounds of a few edges), so what counts is the length of a round's
+// chain of dependent steps:
+//   * one grid barrier a round.  There is no retire or mark pass: state[e] is
+//     kAlive or the round in which e is (or was) on the frontier, so in round
+//     r an edge is on the frontier iff state = r, dead iff state < r, and an
+//     edge that drops below K - 2 now gets state r + 1 and its truss number
+//     when it is appended;
+//   * a frontier of at most kKtFew edges is staged by every CTA for itself
+//     (endpoints and list bounds, with the prefix of their 32-entry chunks),
+//     and the chunks go round-robin to all warps, one binary search a lane;
+//   * a larger one is taken 32 edges a warp: lanes finish those with at most
+//     kKtTiny entries alone, the warp the others, except that lists above
+//     kKtHeavy are left to a CTA each after another barrier.
+// ---------------------------------------------------------------------------
+constexpr int kKtThreads = 512;
+constexpr int kKtFew = 512;      // edges staged per CTA (one per thread)
+constexpr int kKtTiny = 4;
+constexpr int kKtHeavy = 256;
+constexpr int kAlive = INT_MAX;
+
+struct KtCtl {
+    GridBar bar;
+    const long long* off;     // adjacency lists (dead entries stay until rebuilt)
+    const int32_t* adj;
+    const int32_t* canon;
+    int32_t* F;               // frontier of this round (canonical edge ids)
+    int32_t* NF;              // ... and of the next
+    int32_t* L;               // alive edges at the start of this K
+    int32_t* L2;
+    long long lm;             // entries of adj
+    // copied to the host after the launch
+    int K, nL, minsup, error;
+    long long remaining;
+    int round;                // number of the current round, from 1
+    int nf, nNF, nheavy, nL2, stop, swapped, pad;
+};
+
+struct KtArgs {
+    KtCtl* ctl;
+    const int32_t* src;       // endpoints of each edge id
+    const int32_t* eadj;
+    int32_t* state;
+    int32_t* sup;
+    int32_t* truss;
+    int32_t* heavy;
+};
+
+// x loses a triangle; the thread that takes it below K - 2 puts it on the
+// next frontier.
+__device__ __forceinline__ void kt_drop(const KtArgs& a, int x, int K, int round, int32_t* NF) {
+    if (atomicSub(a.sup + x, 1) == K - 2) {
+        a.state[x] = round + 1;
+        a.truss[x] = K - 1;
+        NF[atomicAdd(&a.ctl->nNF, 1)] = x;
+    }
+}
+
+// kt_triangle for the states above (read through L2: they change during the
+// launch).
+__device__ __forceinline__ void kt_common(const KtArgs& a, int e, int e1, int e2, int K, int round,
+                                          int32_t* NF) {
+    const int s1 = __ldcg(a.state + e1), s2 = __ldcg(a.state + e2);
+    if (s1 < round || s2 < round) return;   // the triangle is already gone
+    const bool f1 = s1 == round, f2 = s2 == round;
+    if (!f1 && !f2) {
+        kt_drop(a, e1, K, round, NF);
+        kt_drop(a, e2, K, round, NF);
+    } else if (f1 && !f2) {
+        if (e < e1) kt_drop(a, e2, K, round, NF);
+    } else if (!f1 && f2) {
+        if (e < e2) kt_drop(a, e1, K, round, NF);
+    }
+}
+
+__device__ __forceinline__ int kt_lower(const int32_t* __restrict__ a, int n, int x) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(a + mid) < x) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+struct KtEdge {   // a frontier edge: the shorter list [pa, pa + na), the longer one
+    int e, pa, pb, na, nb;
+};
+
+__device__ __forceinline__ KtEdge kt_edge(const KtArgs& a, const long long* __restrict__ off, int e) {
+    KtEdge k;
+    const int u = __ldg(a.src + e), v = __ldg(a.eadj + e);
+    const int au = (int)__ldg(off + u), la = (int)__ldg(off + u + 1) - au;
+    const int bv = (int)__ldg(off + v), lb = (int)__ldg(off + v + 1) - bv;
+    const bool sw = la > lb;
+    k.e = e;
+    k.pa = sw ? bv : au;
+    k.pb = sw ? au : bv;
+    k.na = sw ? lb : la;
+    k.nb = sw ? la : lb;
+    return k;
+}
+
+__global__ void __launch_bounds__(kKtThreads, 2) k_kt_run(const __grid_constant__ KtArgs a) {
+    __shared__ struct {
+        const long long* off;
+        const int32_t* adj;
+        const int32_t* canon;
+        int32_t *F, *NF, *L, *L2;
+        int K, nL, nf, nheavy, round, stop, error;
+        unsigned gen;
+    } s;
+    __shared__ int s_e[kKtFew], s_pa[kKtFew], s_pb[kKtFew], s_na[kKtFew], s_nb[kKtFew];
+    __shared__ int s_pre[kKtFew + 1], s_ws[kKtThreads / 32];
+    const unsigned kFull = 0xFFFFFFFFu;
+    KtCtl* ctl = a.ctl;
+    volatile KtCtl* vc = a.ctl;   // read and written by the CTA that seals a phase
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int gw = blockIdx.x * (kKtThreads / 32) + warp;
+    const int nwarps = gridDim.x * (kKtThreads / 32);
+    const long long gt = blockIdx.x * (long long)kKtThreads + threadIdx.x;
+    const long long nt = (long long)gridDim.x * kKtThreads;
+    auto load = [&] {
+        s.off = vc->off;
+        s.adj = vc->adj;
+        s.canon = vc->canon;
+        s.F = vc->F;
+        s.NF = vc->NF;
+        s.L = vc->L;
+        s.L2 = vc->L2;
+        s.K = vc->K;
+        s.nL = vc->nL;
+        s.nf = vc->nf;
+        s.nheavy = vc->nheavy;
+        s.round = vc->round;
+        s.stop = vc->stop;
+    };
+    auto sync = [&](auto seal) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (!grid_barrier(&ctl->bar, s.gen, seal)) {
+                *(volatile int*)&ctl->error = HN_ERR_TIMEOUT;
+                s.error = 1;
+            }
+            load();
+        }
+        __syncthreads();
+        return s.error == 0;
+    };
+    auto nothing = [] {};
+    // the round is over: the next frontier becomes the current one
+    auto end_round = [&] {
+        vc->remaining = vc->remaining - vc->nf;
+        vc->round = vc->round + 1;
+        int32_t* t = vc->F;
+        vc->F = vc->NF;
+        vc->NF = t;
+        vc->nf = vc->nNF;
+        vc->nNF = 0;
+        vc->nheavy = 0;
+    };
+    if (threadIdx.x == 0) {
+        s.error = 0;
+        s.gen = *(volatile unsigned*)&ctl->bar.gen;   // it moves only after this CTA arrives
+        load();
+    }
+    __syncthreads();
+    while (true) {
+        // the frontier of K: alive edges with support < K - 2
+        {
+            const int nL = s.nL, K = s.K, round = s.round;
+            for (long long i0 = gt - lane; i0 < nL; i0 += nt) {
+                const long long i = i0 + lane;
+                const int e = i < nL ? __ldcg(s.L + i) : 0;
+                const bool take = i < nL && __ldcg(a.sup + e) < K - 2;
+                const int p = warp_append(&ctl->nf, take);
+                if (take) {
+                    s.F[p] = e;
+                    a.state[e] = round;
+                    a.truss[e] = K - 1;
+                }
+            }
+            if (!sync(nothing)) return;
+        }
+        while (s.nf > 0) {
+            const int nf = s.nf, K = s.K, round = s.round;
+            int32_t* const NF = s.NF;
+            const int32_t* __restrict__ adj = s.adj;
+            const int32_t* __restrict__ canon = s.canon;
+            auto probe = [&](int e, int pa, int pb, int nb, int i) {
+                const int w = __ldg(adj + pa + i);
+                const int p = kt_lower(adj + pb, nb, w);
+                if (p < nb && __ldg(adj + pb + p) == w)
+                    kt_common(a, e, __ldg(canon + pa + i), __ldg(canon + pb + p), K, round, NF);
+            };
+            if (nf <= kKtFew) {
+                int chunks = 0;
+                if ((int)threadIdx.x < nf) {
+                    const KtEdge k = kt_edge(a, s.off, __ldcg(s.F + threadIdx.x));
+                    s_e[threadIdx.x] = k.e;
+                    s_pa[threadIdx.x] = k.pa;
+                    s_pb[threadIdx.x] = k.pb;
+                    s_na[threadIdx.x] = k.na;
+                    s_nb[threadIdx.x] = k.nb;
+                    chunks = (k.na + 31) >> 5;
+                }
+                int incl = chunks;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                if (lane == 31) s_ws[warp] = incl;
+                __syncthreads();
+                int before = 0;
+                for (int q = 0; q < warp; q++) before += s_ws[q];
+                s_pre[threadIdx.x] = before + incl - chunks;
+                if (threadIdx.x == kKtThreads - 1) s_pre[kKtThreads] = before + incl;
+                __syncthreads();
+                const int total = s_pre[nf < kKtThreads ? nf : kKtThreads];
+                for (int c = gw; c < total; c += nwarps) {
+                    int lo = 0, hi = nf;   // last edge with s_pre <= c
+                    while (hi - lo > 1) {
+                        const int mid = (lo + hi) >> 1;
+                        if (s_pre[mid] <= c) lo = mid; else hi = mid;
+                    }
+                    const int i = (c - s_pre[lo]) * 32 + lane;
+                    if (i < s_na[lo]) probe(s_e[lo], s_pa[lo], s_pb[lo], s_nb[lo], i);
+                }
+                if (!sync(end_round)) return;
+                continue;
+            }
+            const int want = (nf + nwarps - 1) / nwarps;
+            const int per = want < 32 ? want : 32;
+            for (long long f0 = (long long)gw * per; f0 < nf; f0 += (long long)nwarps * per) {
+                KtEdge k{0, 0, 0, 0, 0};
+                if (lane < per && f0 + lane < nf) k = kt_edge(a, s.off, __ldcg(s.F + f0 + lane));
+                const bool big = k.na > kKtHeavy;
+                const int slot = warp_append(&ctl->nheavy, big);
+                if (big) a.heavy[slot] = k.e;
+                const bool tiny = per > 1 && k.na <= kKtTiny;
+                if (tiny)
+                    for (int i = 0; i < k.na; i++) probe(k.e, k.pa, k.pb, k.nb, i);
+                __syncwarp();
+                unsigned coop = __ballot_sync(kFull, !big && !tiny && k.na > 0);
+                while (coop) {
+                    const int l = __ffs(coop) - 1;
+                    coop &= coop - 1;
+                    const int we = __shfl_sync(kFull, k.e, l);
+                    const int wpa = __shfl_sync(kFull, k.pa, l), wpb = __shfl_sync(kFull, k.pb, l);
+                    const int wna = __shfl_sync(kFull, k.na, l), wnb = __shfl_sync(kFull, k.nb, l);
+                    for (int i = lane; i < wna; i += 32) probe(we, wpa, wpb, wnb, i);
+                    __syncwarp();
+                }
+            }
+            if (!sync(nothing)) return;
+            if (s.nheavy > 0) {
+                const int nh = s.nheavy;
+                for (int h = blockIdx.x; h < nh; h += gridDim.x) {
+                    const KtEdge k = kt_edge(a, s.off, __ldcg(a.heavy + h));
+                    for (int i = threadIdx.x; i < k.na; i += kKtThreads)
+                        probe(k.e, k.pa, k.pb, k.nb, i);
+                }
+            }
+            if (!sync(end_round)) return;
+        }
+        // the edges left, and the smallest support among them
+        {
+            const int nL = s.nL;
+            int mn = 0x7FFFFFFF;
+            for (long long i0 = gt - lane; i0 < nL; i0 += nt) {
+                const long long i = i0 + lane;
+                const int e = i < nL ? __ldcg(s.L + i) : 0;
+                const bool take = i < nL && __ldcg(a.state + e) == kAlive;
+                const int p = warp_append(&ctl->nL2, take);
+                if (take) {
+                    s.L2[p] = e;
+                    mn = min(mn, __ldcg(a.sup + e));
+                }
+            }
+            mn = __reduce_min_sync(kFull, mn);
+            if (lane == 0 && mn != 0x7FFFFFFF) atomicMin(&ctl->minsup, mn);
+            if (!sync([&] {
+                    const int left = vc->nL2;
+                    int32_t* t = vc->L;
+                    vc->L = vc->L2;
+                    vc->L2 = t;
+                    vc->swapped = vc->swapped ^ 1;
+                    vc->nL = left;
+                    vc->nL2 = 0;
+                    const int next = vc->minsup + 3, k1 = vc->K + 1;
+                    vc->minsup = 0x7FFFFFFF;
+                    vc->stop = left == 0 || 4LL * left <= vc->lm;
+                    if (left > 0) vc->K = next > k1 ? next : k1;
+                    vc->nf = 0;
+                }))
+                return;
+            if (s.stop) return;
+        }
+    }
+}
+
+__global__ void k_kt_state(const unsigned char* __restrict__ alive, long long m,
+                           int32_t* __restrict__ state) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m;
+         e += (long long)gridDim.x * blockDim.x)
+        state[e] = alive[e] ? kAlive : 0;
 }
 
 __global__ void k_kt_out(const int32_t* __restrict__ canon, const int32_t* __restrict__ truss,
@@ -396,7 +710,7 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
         HN_CUDA(cudaMemcpyAsync(minsup, &big, sizeof(int), cudaMemcpyHostToDevice, s));
         HN_LAUNCH(k_kt_compact, grid_for(g, n, kB), kB, 0, s, in, n, alive.get(), sup.get(),
                   L2.get(), nL, minsup);
-        std::swap(L.p, L2.p);
+        L.swap(L2);
         HN_CUDA(cudaMemcpyAsync(g->h_scalar, cnt, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
         HN_CUDA(cudaStreamSynchronize(s));
         return ((int*)g->h_scalar)[4];
@@ -410,14 +724,14 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
     int32_t* lcanon = canon.get();
     long long lm = m;
     DevBuf<long long> coff;
-    DevBuf<int32_t> cadj, ccanon, cflag;
+    DevBuf<int32_t> cadj, ccanon, cflag, state;
     auto shrink_lists = [&]() {
         const long long keep = 2LL * n_alive;
         if (keep * 2 > lm) return;
         cflag.alloc((size_t)lm + 1, s);
         HN_CUDA(cudaMemsetAsync(cflag.get() + lm, 0, sizeof(int32_t), s));
         HN_LAUNCH(k_kt_live_pos, grid_for(g, lm, kB), kB, 0, s, (const int32_t*)lcanon, lm,
-                  alive.get(), cflag.get());
+                  alive.get(), (const int32_t*)state.get(), cflag.get());
         // new slot of every live entry: an exclusive scan of the live flags;
         // a vertex's new offset is the new slot of its first old entry
         DevBuf<long long> pos((size_t)lm + 1, s), noff((size_t)nV + 1, s);
@@ -437,123 +751,98 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
         lm = keep;
         cflag.release();
     };
-    // the peel rounds of one K: a CUDA graph whose WHILE node repeats
-    // peel -> heavy peel -> retire -> mark -> advance until a round finds no
-    // new frontier, with no host round trip between rounds
-    DevBuf<KtPeel> st(1, s);
-    KtPeel* h_st = nullptr;
-    HN_CUDA(cudaMallocHost((void**)&h_st, sizeof(KtPeel)));
-    struct HostFree {
-        KtPeel* p;
-        ~HostFree() { cudaFreeHost(p); }
-    } h_st_free{h_st};
-    *h_st = KtPeel{loff, ladj, lcanon, F.get(), NF.get(), 0, 0, 0, K, remaining, 0};
-    HN_CUDA(cudaMemcpyAsync(st.get(), h_st, sizeof(KtPeel), cudaMemcpyHostToDevice, s));
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    struct GraphFree {
-        cudaGraph_t* g;
-        cudaGraphExec_t* e;
-        ~GraphFree() {
-            if (*e) cudaGraphExecDestroy(*e);
-            if (*g) cudaGraphDestroy(*g);
-        }
-    } graph_free{&graph, &exec};
     const bool device_rounds = knob(kKnobKtDeviceRounds) != 0;
     if (device_rounds) {
-        HN_CUDA(cudaGraphCreate(&graph, 0));
-        cudaGraphConditionalHandle cond;
-        HN_CUDA(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = cond;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cnode;
-        HN_CUDA(cudaGraphAddNode(&cnode, graph, nullptr, 0, &cp));
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        KtPeel* a_st = st.get();
-        const int32_t* a_src = src.get();
-        const int32_t* a_eadj = adj.get();
-        const unsigned char* a_alive_c = alive.get();
-        unsigned char* a_alive = alive.get();
-        const unsigned char* a_inF_c = inF.get();
-        unsigned char* a_inF = inF.get();
-        int32_t* a_sup = sup.get();
-        int32_t* a_heavy = H.get();
-        const int32_t* a_heavy_c = H.get();
-        int32_t* a_truss = truss.get();
-        const unsigned sms = (unsigned)g->info.sms;
-        void* peel_args[] = {&a_st, &a_src, &a_eadj, &a_alive_c, &a_inF_c, &a_sup, &a_heavy};
-        void* heavy_args[] = {&a_st, &a_src, &a_eadj, &a_heavy_c, &a_alive_c, &a_inF_c, &a_sup};
-        void* retire_args[] = {&a_st, &a_alive, &a_inF, &a_truss};
-        void* mark_args[] = {&a_st, &a_inF};
-        int one = 1;
-        void* adv_args[] = {&a_st, &cond, &one};
-        struct N {
-            void* f;
-            unsigned grid, block;
-            void** args;
-        } nodes[] = {{(void*)k_kt_peel, sms * 16, 128, peel_args},
-                     {(void*)k_kt_peel_heavy, sms * 8, 256, heavy_args},
-                     {(void*)k_kt_retire, sms * 8, kB, retire_args},
-                     {(void*)k_kt_mark, sms * 8, kB, mark_args},
-                     {(void*)k_kt_advance, 1, 1, adv_args}};
-        cudaGraphNode_t prev = nullptr;
-        for (const N& n : nodes) {
-            cudaKernelNodeParams p = {};
-            p.func = n.f;
-            p.gridDim = dim3(n.grid);
-            p.blockDim = dim3(n.block);
-            p.kernelParams = n.args;
-            cudaGraphNode_t node;
-            HN_CUDA(cudaGraphAddKernelNode(&node, body, prev ? &prev : nullptr, prev ? 1 : 0, &p));
-            prev = node;
+        // all K in cooperative launches, one between two list rebuilds
+        DevBuf<KtCtl> ctl(1, s);
+        state.alloc((size_t)m, s);
+        HN_LAUNCH(k_kt_state, grid_for(g, m, kB), kB, 0, s, (const unsigned char*)alive.get(), m,
+                  state.get());
+        int round = 1;
+        const int ms = ((int*)g->h_scalar)[5];
+        if (ms + 3 > K) K = ms + 3;
+        KtArgs a{ctl.get(), src.get(), adj.get(), state.get(), sup.get(), truss.get(), H.get()};
+        while (remaining > 0) {
+            KtCtl h{};
+            h.off = loff;
+            h.adj = ladj;
+            h.canon = lcanon;
+            h.F = F.get();
+            h.NF = NF.get();
+            h.L = L.get();
+            h.L2 = L2.get();
+            h.lm = lm;
+            h.K = K;
+            h.nL = n_alive;
+            h.minsup = INT_MAX;
+            h.remaining = remaining;
+            h.round = round;
+            HN_CUDA(cudaMemcpyAsync(ctl.get(), &h, sizeof(KtCtl), cudaMemcpyHostToDevice, s));
+            void* args[] = {&a};
+            cudaEvent_t ev = nullptr;
+            if (g_profiling) profile_begin(s, &ev);
+            HN_CUDA(cudaLaunchCooperativeKernel((void*)k_kt_run, dim3(2u * g->info.sms),
+                                                dim3(kKtThreads), args, 0, s));
+            if (ev) profile_end("k_kt_run", s, ev);
+            count_launch();
+            // the part of the state that the host reads
+            constexpr size_t from = offsetof(KtCtl, K);
+            static_assert(sizeof(KtCtl) - from <= 16 * sizeof(long long), "pinned scalars");
+            HN_CUDA(cudaMemcpyAsync(g->h_scalar, (const char*)ctl.get() + from,
+                                    sizeof(KtCtl) - from, cudaMemcpyDeviceToHost, s));
+            HN_CUDA(cudaStreamSynchronize(s));
+            std::memcpy((char*)&h + from, g->h_scalar, sizeof(KtCtl) - from);
+            if (h.error) throw Error(h.error, "k-truss: a bounded wait gave up");
+            if (h.swapped) L.swap(L2);
+            remaining = h.remaining;
+            n_alive = h.nL;
+            K = h.K;
+            round = h.round;
+            if (remaining <= 0) break;
+            shrink_lists();
         }
-        HN_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+        K--;   // no edge is left at K (K = 3 on a graph without edges)
     }
-    while (true) {
+    // host-driven rounds (ktruss.device_rounds = 0): launches sized to each
+    // frontier, one read-back of the next frontier's size per round
+    DevBuf<KtPeel> st(1, s);
+    KtPeel h_peel{loff, ladj, lcanon, F.get(), NF.get(), 0, 0, 0, K, remaining, 0};
+    KtPeel* h_st = &h_peel;
+    if (!device_rounds)
+        HN_CUDA(cudaMemcpyAsync(st.get(), h_st, sizeof(KtPeel), cudaMemcpyHostToDevice, s));
+    while (!device_rounds) {
         if (remaining <= 0) { K--; break; }
         const int ms = ((int*)g->h_scalar)[5];
         if (ms + 3 > K) K = ms + 3;
         HN_LAUNCH(k_kt_begin, 1, 1, 0, s, st.get(), K);
         HN_LAUNCH(k_kt_frontier, grid_for(g, n_alive, kB), kB, 0, s, L.get(), n_alive,
                   sup.get(), alive.get(), inF.get(), st.get());
-        const long long rounds_before = h_st->rounds;
-        if (device_rounds) {
-            HN_CUDA(cudaGraphLaunch(exec, s));
-        } else {
-            // host-driven rounds: launches sized to each frontier, one
-            // read-back of the next frontier's size per round
-            HN_CUDA(cudaMemcpyAsync(&h_st->nf, &st.get()->nf, sizeof(int), cudaMemcpyDeviceToHost,
-                                    s));
+        HN_CUDA(cudaMemcpyAsync(&h_st->nf, &st.get()->nf, sizeof(int), cudaMemcpyDeviceToHost,
+                                s));
+        HN_CUDA(cudaStreamSynchronize(s));
+        int nf = h_st->nf;
+        while (nf > 0) {
+            HN_LAUNCH(k_kt_peel, grid_for(g, nf, 128), 128, 0, s, st.get(), src.get(),
+                      (const int32_t*)adj.get(), (const unsigned char*)alive.get(),
+                      (const unsigned char*)inF.get(), sup.get(), H.get());
+            HN_LAUNCH(k_kt_peel_heavy, std::min<long long>(nf, (long long)g->info.sms * 8),
+                      256, 0, s, st.get(), src.get(), (const int32_t*)adj.get(),
+                      (const int32_t*)H.get(), (const unsigned char*)alive.get(),
+                      (const unsigned char*)inF.get(), sup.get());
+            HN_LAUNCH(k_kt_retire, grid_for(g, nf, kB), kB, 0, s, (const KtPeel*)st.get(),
+                      alive.get(), inF.get(), truss.get());
+            HN_LAUNCH(k_kt_mark, grid_for(g, nf, kB), kB, 0, s, (const KtPeel*)st.get(),
+                      inF.get());
+            HN_LAUNCH(k_kt_advance, 1, 1, 0, s, st.get());
+            HN_CUDA(cudaMemcpyAsync(&h_st->nf, &st.get()->nf, sizeof(int),
+                                    cudaMemcpyDeviceToHost, s));
             HN_CUDA(cudaStreamSynchronize(s));
-            int nf = h_st->nf;
-            while (nf > 0) {
-                HN_LAUNCH(k_kt_peel, grid_for(g, nf, 128), 128, 0, s, st.get(), src.get(),
-                          (const int32_t*)adj.get(), (const unsigned char*)alive.get(),
-                          (const unsigned char*)inF.get(), sup.get(), H.get());
-                HN_LAUNCH(k_kt_peel_heavy, std::min<long long>(nf, (long long)g->info.sms * 8),
-                          256, 0, s, st.get(), src.get(), (const int32_t*)adj.get(),
-                          (const int32_t*)H.get(), (const unsigned char*)alive.get(),
-                          (const unsigned char*)inF.get(), sup.get());
-                HN_LAUNCH(k_kt_retire, grid_for(g, nf, kB), kB, 0, s, (const KtPeel*)st.get(),
-                          alive.get(), inF.get(), truss.get());
-                HN_LAUNCH(k_kt_mark, grid_for(g, nf, kB), kB, 0, s, (const KtPeel*)st.get(),
-                          inF.get());
-                HN_LAUNCH(k_kt_advance, 1, 1, 0, s, st.get(), (cudaGraphConditionalHandle)0, 0);
-                HN_CUDA(cudaMemcpyAsync(&h_st->nf, &st.get()->nf, sizeof(int),
-                                        cudaMemcpyDeviceToHost, s));
-                HN_CUDA(cudaStreamSynchronize(s));
-                nf = h_st->nf;
-            }
+            nf = h_st->nf;
         }
         // the state comes back with the alive-list compaction's read-back
         HN_CUDA(cudaMemcpyAsync(h_st, st.get(), sizeof(KtPeel), cudaMemcpyDeviceToHost, s));
         n_alive = compact(L.get(), n_alive);
         remaining = h_st->remaining;
-        if (device_rounds)
-            count_launch((int)(5 * (h_st->rounds - rounds_before)));   // kernels the WHILE node ran
         if (remaining <= 0) { K--; break; }
         const long long* old_off = loff;
         shrink_lists();
