@@ -11,13 +11,15 @@
 // atomicCAS, finds use intermediate pointer jumping — driven by the
 // neighbour-sampling schedule of Afforest (Sutton, Ben-Nun & Barak,
 // IPDPS 2018):
-//   1. every vertex links with its first kSample neighbours;
-//   2. compress; the most frequent root among 256 evenly spaced vertices
-//      is taken as the giant component G;
-//   3. only vertices outside G (with more than kSample neighbours) link
-//      with the rest of their neighbours — an edge from G to a vertex
-//      outside G is seen from the outside end, edges inside G are already
-//      implied — so on power-law graphs most edges are never read;
+//   1. every vertex starts under its first neighbour when that is smaller
+//      (lists are sorted, so the first is the smallest: a link without an
+//      atomic), then links with its second one;
+//   2. the most frequent root of 256 evenly spaced vertices is taken as the
+//      giant component G; compress;
+//   3. only vertices outside G link with the rest of their neighbours — an
+//      edge from G to a vertex outside G is seen from the outside end, edges
+//      inside G are already implied — so on power-law graphs most edges are
+//      never read;
 //   4. compress and count roots.
 // Parents only ever point to smaller ids, so each root is the minimum id of
 // its component: the labels come out canonical with no relabelling, and no
@@ -44,14 +46,6 @@ __device__ __forceinline__ int find_root(int* __restrict__ parent, int v) {
     return cur;
 }
 
-__global__ void k_cc_init(int* __restrict__ parent, int nV) {
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nV;
-         v += (long long)gridDim.x * blockDim.x)
-        parent[v] = (int)v;
-}
-
-constexpr int kSample = 2;
-
 __device__ __forceinline__ void cc_link(int* __restrict__ parent, int u, int v) {
     int ru = find_root(parent, u);
     int rv = find_root(parent, v);
@@ -64,54 +58,99 @@ __device__ __forceinline__ void cc_link(int* __restrict__ parent, int u, int v) 
     }
 }
 
-// 1. link every vertex with its first kSample neighbours.  Each thread
-// takes kVerts vertices per round and issues all their record and
-// neighbour loads before the first link (each link is a chain of dependent
-// parent reads, so the loads of one vertex alone leave the SM waiting).
+// 1a. parent[v] = v's first neighbour when smaller, else v; second[v] = its
+// second neighbour, kNone when it has none, kBoth for a vertex smaller than
+// all its neighbours (1b links it with its first two).  This is the only
+// pass over all records and lists (a 16-byte record and a sector of the list
+// per vertex, from HBM); the passes below read parent and second.  Each
+// thread issues the loads of kVerts vertices before it stores.
 constexpr int kVerts = 4;
-__global__ void k_cc_sample(const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
-                            int nV, int* __restrict__ parent) {
+constexpr int kNone = -1, kBoth = -2;
+__global__ void __launch_bounds__(kB)
+k_cc_init(const VRec* __restrict__ vtab, const int32_t* __restrict__ pool, int nV,
+          int* __restrict__ parent, int* __restrict__ second) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long v0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; v0 < nV;
          v0 += kVerts * stride) {
-        int deg[kVerts];
-        long long off[kVerts];
+        VRec r[kVerts];
 #pragma unroll
         for (int j = 0; j < kVerts; j++) {
             const long long v = v0 + j * stride;
-            deg[j] = 0;
-            off[j] = 0;
-            if (v < nV) {
-                const VRec r = vtab[v];
-                deg[j] = r.deg < kSample ? r.deg : kSample;
-                off[j] = r.off;
+            r[j].deg = 0;
+            if (v < nV) r[j] = vtab[v];
+        }
+        int a[kVerts], b[kVerts];
+#pragma unroll
+        for (int j = 0; j < kVerts; j++) {
+            a[j] = b[j] = -1;
+            if (r[j].deg > 1) {   // blocks of two slots or more start on 8 bytes
+                const int2 q = __ldg(reinterpret_cast<const int2*>(pool + r[j].off));
+                a[j] = q.x;
+                b[j] = q.y;
+            } else if (r[j].deg == 1) {
+                a[j] = __ldg(pool + r[j].off);
             }
         }
-        int nb[kVerts][kSample];
 #pragma unroll
-        for (int j = 0; j < kVerts; j++)
-#pragma unroll
-            for (int i = 0; i < kSample; i++) nb[j][i] = i < deg[j] ? __ldg(pool + off[j] + i) : -1;
-#pragma unroll
-        for (int j = 0; j < kVerts; j++)
-#pragma unroll
-            for (int i = 0; i < kSample; i++)
-                if (nb[j][i] >= 0) cc_link(parent, (int)(v0 + j * stride), nb[j][i]);
+        for (int j = 0; j < kVerts; j++) {
+            const long long v = v0 + j * stride;
+            if (v >= nV) break;
+            const bool up = a[j] >= 0 && a[j] < v;
+            parent[v] = up ? a[j] : (int)v;
+            second[v] = up ? b[j] : a[j] >= 0 ? kBoth : kNone;
+        }
     }
 }
 
-__global__ void k_cc_compress(int* __restrict__ parent, int nV) {
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nV;
-         v += (long long)gridDim.x * blockDim.x)
-        parent[v] = find_root(parent, (int)v);
+// 1b. the second links.  Most find both ends under one parent or grandparent
+// already (hubs have small ids), which four vertices' loads together decide
+// before any walk to the roots; skipping such a link changes no component.
+__global__ void k_cc_sample(const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
+                            const int* __restrict__ second, int nV, int* __restrict__ parent) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long v0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; v0 < nV;
+         v0 += kVerts * stride) {
+        int w[kVerts];
+#pragma unroll
+        for (int j = 0; j < kVerts; j++)
+            w[j] = v0 + j * stride < nV ? second[v0 + j * stride] : kNone;
+        int a[kVerts], b[kVerts];
+#pragma unroll
+        for (int j = 0; j < kVerts; j++) {
+            a[j] = b[j] = 0;
+            if (w[j] >= 0) {
+                a[j] = parent[v0 + j * stride];
+                b[j] = parent[w[j]];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kVerts; j++) {
+            if (w[j] >= 0 && a[j] != b[j]) {
+                a[j] = parent[a[j]];
+                b[j] = parent[b[j]];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kVerts; j++) {
+            if (w[j] == kNone || (w[j] >= 0 && a[j] == b[j])) continue;
+            const int v = (int)(v0 + j * stride);
+            if (w[j] >= 0) {
+                cc_link(parent, v, w[j]);
+            } else {
+                const VRec r = vtab[v];
+                cc_link(parent, v, pool[r.off]);
+                if (r.deg > 1) cc_link(parent, v, pool[r.off + 1]);
+            }
+        }
+    }
 }
 
 // 2. most frequent root among 256 evenly spaced vertices (one CTA of 256)
-__global__ void k_cc_giant(const int* __restrict__ parent, int nV, int* __restrict__ giant) {
+__global__ void k_cc_giant(int* __restrict__ parent, int nV, int* __restrict__ giant) {
     __shared__ int s_r[256];
     int t = threadIdx.x;
     long long v = (long long)t * nV / 256;
-    s_r[t] = parent[v < nV ? v : nV - 1];
+    s_r[t] = find_root(parent, (int)(v < nV ? v : nV - 1));
     __syncthreads();
     int mine = s_r[t], c = 0;
     for (int i = 0; i < 256; i++) c += (s_r[i] == mine);
@@ -125,21 +164,27 @@ __global__ void k_cc_giant(const int* __restrict__ parent, int nV, int* __restri
     if (t == 0) *giant = 0x7FFFFFFF - (int)(s_key & 0xFFFFFFFFull);
 }
 
-// 3a. vertices outside the giant component with unread neighbours
-__global__ void k_cc_worklist(const VRec* __restrict__ vtab, const int* __restrict__ parent,
-                              int nV, const int* __restrict__ giant, int* __restrict__ list,
+// 2b, 3a. compress; list the vertices outside the giant component that may
+// have unread neighbours
+__global__ void k_cc_worklist(const int* __restrict__ second, int* __restrict__ parent, int nV,
+                              const int* __restrict__ giant, int* __restrict__ list,
                               int* __restrict__ nlist) {
     const int gr = *giant;
     for (long long v0 = blockIdx.x * (long long)blockDim.x; v0 < nV;
          v0 += (long long)gridDim.x * blockDim.x) {
         long long v = v0 + threadIdx.x;
-        bool take = v < nV && vtab[v].deg > kSample && parent[v] != gr;
+        bool take = false;
+        if (v < nV) {
+            const int r = find_root(parent, (int)v);
+            parent[v] = r;
+            take = r != gr && second[v] != kNone;
+        }
         int p = warp_append(nlist, take);
         if (take) list[p] = (int)v;
     }
 }
 
-// 3b. one warp per listed vertex: link with neighbours kSample..deg-1
+// 3b. one warp per listed vertex: link with the neighbours after the first
 __global__ void k_cc_rest(const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
                           const int* __restrict__ list, const int* __restrict__ nlist,
                           int* __restrict__ parent) {
@@ -150,7 +195,7 @@ __global__ void k_cc_rest(const VRec* __restrict__ vtab, const int32_t* __restri
     for (long long i = wid; i < n; i += nw) {
         int v = list[i];
         VRec r = vtab[v];
-        for (int k = kSample + lane; k < r.deg; k += 32) cc_link(parent, v, pool[r.off + k]);
+        for (int k = 1 + lane; k < r.deg; k += 32) cc_link(parent, v, pool[r.off + k]);
     }
 }
 
@@ -220,35 +265,38 @@ extern "C" int hn_cc(hn_graph_t* g, int mode, int32_t* labels, int mem, int32_t*
         if (n_components) *n_components = 0;
         return HN_OK;
     }
-    DevBuf<int> parent((size_t)nV, s), list((size_t)nV, s);
+    // minimum-id labels for a device array are computed in place
+    const bool direct = mem == HN_MEM_DEVICE && mode == HN_CC_MIN_ID;
+    DevBuf<int> buf, second((size_t)nV, s), list((size_t)nV, s);
+    if (!direct) buf.alloc((size_t)nV, s);
+    int* parent = direct ? (int*)labels : buf.get();
     int* cnt = (int*)(g->d_scalar + 2);  // [0] giant root, [1] worklist size
     HN_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(int), s));
-    HN_LAUNCH(k_cc_init, grid_for(g, nV, kB), kB, 0, s, parent.get(), nV);
-    HN_LAUNCH(k_cc_sample, grid_for(g, nV, kB), kB, 0, s, g->vtab, g->pool, nV, parent.get());
-    HN_LAUNCH(k_cc_compress, grid_for(g, nV, kB), kB, 0, s, parent.get(), nV);
-    HN_LAUNCH(k_cc_giant, 1, 256, 0, s, parent.get(), nV, cnt);
-    HN_LAUNCH(k_cc_worklist, grid_for(g, nV, kB), kB, 0, s, g->vtab, parent.get(), nV, cnt,
-              list.get(), cnt + 1);
+    HN_LAUNCH(k_cc_init, grid_for(g, nV, kB), kB, 0, s, g->vtab, g->pool, nV, parent,
+              second.get());
+    HN_LAUNCH(k_cc_sample, grid_for(g, nV, kB), kB, 0, s, g->vtab, g->pool,
+              (const int*)second.get(), nV, parent);
+    HN_LAUNCH(k_cc_giant, 1, 256, 0, s, parent, nV, cnt);
+    HN_LAUNCH(k_cc_worklist, grid_for(g, nV, kB), kB, 0, s, (const int*)second.get(), parent, nV,
+              cnt, list.get(), cnt + 1);
     HN_LAUNCH(k_cc_rest, (long long)g->info.sms * 8, kB, 0, s, g->vtab, g->pool, list.get(),
-              cnt + 1, parent.get());
+              cnt + 1, parent);
     HN_CUDA(cudaMemsetAsync(g->d_scalar, 0, 2 * sizeof(long long), s));
-    HN_LAUNCH(k_cc_finish, grid_for(g, nV, kB), kB, 0, s, parent.get(), nV, (int*)g->d_scalar);
-    int32_t* out = mem == HN_MEM_DEVICE ? labels : nullptr;
+    HN_LAUNCH(k_cc_finish, grid_for(g, nV, kB), kB, 0, s, parent, nV, (int*)g->d_scalar);
+    int32_t* out = parent;
     DevBuf<int32_t> tmp;
-    if (!out) {
-        tmp.alloc((size_t)nV, s);
-        out = tmp.get();
-    }
-    if (mode == HN_CC_MIN_ID) {
-        HN_CUDA(cudaMemcpyAsync(out, parent.get(), sizeof(int32_t) * nV, cudaMemcpyDeviceToDevice,
-                                s));
-    } else {
+    if (mode == HN_CC_REFERENCE) {
+        out = labels;
+        if (mem == HN_MEM_HOST) {
+            tmp.alloc((size_t)nV, s);
+            out = tmp.get();
+        }
         DevBuf<int> mx((size_t)nV, s);
         HN_CUDA(cudaMemsetAsync(mx.get(), 0xFF, sizeof(int) * nV, s));
-        HN_LAUNCH(k_cc_maxid, grid_for(g, nV, kB), kB, 0, s, parent.get(), nV, mx.get());
+        HN_LAUNCH(k_cc_maxid, grid_for(g, nV, kB), kB, 0, s, parent, nV, mx.get());
         unsigned long long* key = (unsigned long long*)(g->d_scalar + 1);
         HN_LAUNCH(k_max_degree_key, grid_for(g, nV, kB), kB, 0, s, g->vtab, nV, key);
-        HN_LAUNCH(k_cc_refcolor, grid_for(g, nV, kB), kB, 0, s, parent.get(), mx.get(), nV, key,
+        HN_LAUNCH(k_cc_refcolor, grid_for(g, nV, kB), kB, 0, s, parent, mx.get(), nV, key,
                   out);
     }
     if (mem == HN_MEM_HOST)
