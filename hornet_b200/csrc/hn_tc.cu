@@ -15,12 +15,21 @@
 //   pass 2  compact the kept neighbours (lists stay sorted).
 // The intersection is vertex-centric with N+(u) in a shared-memory hash
 // table (see the comment above k_tc_warp).
+//
+// Counts of graphs whose edges are not local in vertex id (build_by_rank) use
+// another orientation: vertices are renumbered by rank in the (degree, id)
+// order, so that the ends of most probes are among the kWin highest numbers,
+// where membership in N+(u) is one bit of an 8 KB shared bitmap instead of a
+// hash lookup.
 #include <cub/cub.cuh>
 
+#include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "hn_graph.cuh"
 #include "hn_tc.cuh"
+#include "hn_window.cuh"
 
 namespace hn {
 
@@ -125,6 +134,177 @@ k_orient_fill(const long long* __restrict__ prefix, int nV, const VRec* __restri
         offp[u] = pos[prefix[u]];
 }
 
+// ---------------------------------------------------------------------------
+// Orientation by rank.  rank = position in the (degree, id) order; vertex u's
+// oriented list is stored under rank[u] and holds ranks, so u -> v iff
+// rank[u] < rank[v].  One random 4-byte read per edge decides the direction
+// (a vertex record is 16 bytes) and the decision is kept as one bit per edge,
+// so the fill reads ranks of kept edges only.  Lists are not sorted.
+// ---------------------------------------------------------------------------
+constexpr int kWinBits = 16;
+constexpr int kWin = 1 << kWinBits;          // ranks of the shared bitmap
+constexpr int kRankTile = 1024;
+
+__global__ void k_rank_keys(const VRec* __restrict__ vtab, int nV,
+                            unsigned long long* __restrict__ keys) {
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nV;
+         v += (long long)gridDim.x * blockDim.x)
+        keys[v] = ((unsigned long long)v << 32) | (unsigned)vtab[v].deg;
+}
+
+__global__ void k_rank_of(const unsigned long long* __restrict__ keys, int nV,
+                          int32_t* __restrict__ rank, int32_t* __restrict__ inv) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nV;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int v = (int)(keys[i] >> 32);
+        rank[v] = (int)i;
+        inv[i] = v;
+    }
+}
+
+// Of evenly spaced edges, those whose ends are less than kWin ids apart.
+__global__ void k_local_sample(const long long* __restrict__ prefix, int nV, long long m,
+                               const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
+                               int samples, int* __restrict__ local) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool near = false;
+    if (i < samples) {
+        const long long e = (long long)((double)i / samples * m);
+        const long long u = upper_bound_dev(prefix, (long long)nV + 1, e) - 1;
+        const int v = pool[vtab[u].off + (e - prefix[u])];
+        near = u - v < kWin && v - u < kWin;
+    }
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, near);
+    if ((threadIdx.x & 31) == 0 && b) atomicAdd(local, __popc(b));
+}
+
+// Pass 1 (FILL = false): the direction of every edge, one bit each in
+// `kept`, and the kept edges of each vertex in cnt[rank].  Pass 2: every
+// window reserves its segments' kept edges (cnt is the cursor) and writes
+// their ranks.  A warp per merge-path tile, windows of 32 vertices; a row of
+// 32 edges is one word of `kept` (shared by two windows at their seam).
+template <bool FILL>
+__global__ void __launch_bounds__(kB)
+k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
+              const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
+              const int32_t* __restrict__ rank, unsigned* __restrict__ kept,
+              int* __restrict__ cnt, const long long* __restrict__ offp,
+              int32_t* __restrict__ fwd, const long long* __restrict__ splits,
+              long long ntiles) {
+    constexpr int ROWS = 4;
+    const unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const long long tile = blockIdx.x * (long long)(kB / 32) + (threadIdx.x >> 5);
+    if (tile >= ntiles) return;
+    const WarpTile wt = warp_tile(splits, tile, kRankTile, nE, nV);
+    if (wt.nitems == 0) return;
+    for (long long v0 = wt.seg0; v0 <= wt.seg1; v0 += 32) {
+        const long long v = v0 + lane < nV ? v0 + lane : nV;
+        const long long first = prefix[v];
+        const long long next = v0 + 32 <= nV ? prefix[v0 + 32] : nE;
+        const long long off = v < nV ? vtab[v].off : 0;
+        const int rv = v < nV ? rank[v] : 0;
+        const WarpWindow w = warp_window(wt, v0, first, next);
+        if (w.n == 0) continue;
+        const long long base = __shfl_sync(kFull, off - first, w.lane_of) + wt.item0;
+        const int ru = __shfl_sync(kFull, rv, w.lane_of);   // rank of the lane's segment
+        // the lane's own segment [w.start, send)
+        int send = __shfl_down_sync(kFull, w.start, 1);
+        if (lane >= w.n - 1) send = w.end;
+        const int row0 = w.begin - (int)((wt.item0 + w.begin) & 31);
+        // bits of the row that belong to the lane's segment
+        auto own = [&](int row) {
+            const int lo = w.start > row ? w.start - row : 0;
+            const int hi = send - row < 32 ? send - row : 32;
+            if (lane >= w.n || lo >= hi || hi <= 0 || lo > 31) return 0u;
+            return (hi == 32 ? kFull : (1u << hi) - 1u) & ~((1u << lo) - 1u);
+        };
+        if (!FILL) {
+            int mine = 0;
+            for (int r = row0; r < w.end; r += 32 * ROWS) {
+                int x[ROWS], u[ROWS];
+#pragma unroll
+                for (int k = 0; k < ROWS; k++) {
+                    const int row = r + 32 * k, e = row + lane;
+                    x[k] = -1;
+                    u[k] = 0;
+                    if (row < w.end) {   // uniform
+                        const int j = warp_owner(w, row) & 31;
+                        const long long b = __shfl_sync(kFull, base, j);
+                        u[k] = __shfl_sync(kFull, ru, j);
+                        if (e >= w.begin && e < w.end) x[k] = __ldcs(pool + b + e);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < ROWS; k++) {
+                    const int row = r + 32 * k;
+                    if (row >= w.end) break;   // uniform
+                    const bool keep = x[k] >= 0 && rank[x[k]] > u[k];
+                    const unsigned b = __ballot_sync(kFull, keep);
+                    mine += __popc(b & own(row));
+                    if (lane == 0 && b) {
+                        unsigned* word = kept + ((wt.item0 + row) >> 5);
+                        if (row >= w.begin && row + 32 <= w.end) *word = b;
+                        else atomicOr(word, b);
+                    }
+                }
+            }
+            if (lane < w.n && mine) atomicAdd(cnt + ru, mine);
+        } else {
+            int mine = 0;
+            for (int row = row0; row < w.end; row += 32) {
+                const unsigned b = kept[(wt.item0 + row) >> 5];
+                mine += __popc(b & own(row));
+            }
+            // the next slot of the lane's segment
+            long long at = lane < w.n && mine ? offp[ru] + atomicAdd(cnt + ru, mine) : 0;
+            for (int r = row0; r < w.end; r += 32 * ROWS) {
+                int x[ROWS];
+                long long to[ROWS];
+#pragma unroll
+                for (int k = 0; k < ROWS; k++) {
+                    const int row = r + 32 * k, e = row + lane;
+                    x[k] = -1;
+                    to[k] = 0;
+                    if (row >= w.end) continue;   // uniform
+                    const int j = warp_owner(w, row) & 31;
+                    const unsigned b = kept[(wt.item0 + row) >> 5];
+                    const unsigned seg = own(row);
+                    const unsigned sj = __shfl_sync(kFull, seg, j);
+                    const long long t0 = __shfl_sync(kFull, at, j);
+                    const long long pb = __shfl_sync(kFull, base, j);
+                    if (e >= w.begin && e < w.end && (b >> lane & 1u)) {
+                        to[k] = t0 + __popc(b & sj & ((1u << lane) - 1u));
+                        x[k] = __ldcs(pool + pb + e);
+                    }
+                    at += __popc(b & seg);
+                }
+#pragma unroll
+                for (int k = 0; k < ROWS; k++)
+                    if (x[k] >= 0) fwd[to[k]] = rank[x[k]];
+            }
+        }
+    }
+}
+
+__global__ void k_max_int(const int* __restrict__ a, int n, int* __restrict__ out) {
+    int mx = 0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x)
+        mx = max(mx, a[i]);
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    if ((threadIdx.x & 31) == 0 && mx) atomicMax(out, mx);
+}
+
+// counts under ranks -> counts under vertex ids
+__global__ void k_unrank(const unsigned long long* __restrict__ in,
+                         const int32_t* __restrict__ inv, int nV,
+                         unsigned long long* __restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nV;
+         i += (long long)gridDim.x * blockDim.x)
+        out[inv[i]] = in[i];
+}
+
 // Candidate lists.  The oriented edge x -> y contributes |N+(x) ∩ N+(y)|
 // triangles whichever endpoint counts it, so it is counted by the endpoint
 // whose out-list is the longer: that list is the hash table, the shorter
@@ -133,9 +313,18 @@ k_orient_fill(const long long* __restrict__ prefix, int nV, const VRec* __restri
 // x -> z (owner counts credit the tail x).  Order inside C(z) is immaterial.
 __device__ __forceinline__ bool cand_flip(long long dx, long long dy) { return dy > dx; }
 
+// d+ of every vertex as one int: the candidate passes read it at random, once
+// per oriented edge.
+__global__ void k_dplus(const long long* __restrict__ offp, int nV, int* __restrict__ dplus) {
+    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < nV;
+         u += (long long)gridDim.x * blockDim.x)
+        dplus[u] = (int)(offp[u + 1] - offp[u]);
+}
+
 template <bool FILL>
 __global__ void __launch_bounds__(kB)
-k_cand(const long long* __restrict__ offp, int nV, const int32_t* __restrict__ fwd,
+k_cand(const long long* __restrict__ offp, const int* __restrict__ dplus, int nV,
+       const int32_t* __restrict__ fwd,
        int* __restrict__ cnt /*count pass: sizes; fill pass: cursors*/,
        const long long* __restrict__ coff, int32_t* __restrict__ cand,
        const long long* __restrict__ splits, long long split_tiles,
@@ -160,7 +349,7 @@ k_cand(const long long* __restrict__ offp, int nV, const int32_t* __restrict__ f
                 const int b = t.seg[i];
                 const long long dx = t.ends[b] - t.seg_start(b);
                 const int y = fwd[t.item0 + i];
-                const long long dy = offp[y + 1] - offp[y];
+                const long long dy = dplus[y];
                 ys[k] = y;
                 keep[k] = cand_flip(dx, dy) ? 0 : 1;
             }
@@ -228,6 +417,8 @@ k_cand(const long long* __restrict__ offp, int nV, const int32_t* __restrict__ f
 constexpr int kTcWarps = 8;
 constexpr int kWarpCap = 512;
 constexpr int kWarpTab = 2 * kWarpCap;
+constexpr int kWarpWin = kWarpTab * 32;   // numbers of a warp's bitmap (in its table's place)
+constexpr long long kWinWork = 8192;
 constexpr int kCtaCap = 16384;   // largest tc.cta_table_cap: 160 KB tables
 #ifndef HN_TC_PAIR_ILP
 #define HN_TC_PAIR_ILP 8
@@ -335,6 +526,7 @@ struct TcView {
     const int32_t* feid;     // edge id of each fwd entry
     const int32_t* ceid;     // edge id of each candidate entry
     int* esup;               // per-edge triangle counts
+    int wb = INT_MAX;        // by rank: first rank of the bitmap window; by id: INT_MAX
 };
 
 // One triangle {u, v, w} found from u: credit its three edges (MODE 3).
@@ -352,12 +544,22 @@ __device__ __forceinline__ void tc_credit_edges(int* esup, int e_uv, int e_vw, i
 // [min N+(u), max N+(u)] by two binary searches, then the group's pairs are
 // dealt round-robin to the lanes (one search over the 33-entry prefix per
 // lane per group).
-template <int MODE, bool TAB>
+//
+// KIND: how membership in N+(u) is decided.  kSearch: binary search of the
+// sorted list; kHash: the hash table; kBits: one bit of the bitmap `win` of
+// the numbers [wb, wb + wn), which hold all of N+(u); kBitsHash: the bitmap
+// for w >= wb (wb + wn is past the last number), the table below it.
+enum { kSearch, kHash, kBits, kBitsHash };
+constexpr int kTcLong = 64;   // kBits: lists taken by the whole warp from this length on
+
+template <int MODE, int KIND>
 __device__ __forceinline__ unsigned long long tc_vertex_warp(
     int u, const int32_t* __restrict__ L, int du, const int32_t* __restrict__ C, int dc,
     const int* tab, const unsigned* filt, const int* teid, int bits,
     int narrow_min, int* s_next, const TcView& g, int* s_pref /*33*/, long long* s_vb /*32*/,
-    int* s_v /*32*/, unsigned* s_fc /*32*/, unsigned long long* __restrict__ per_vertex) {
+    int* s_v /*32*/, unsigned* s_fc /*32*/, unsigned long long* __restrict__ per_vertex,
+    const unsigned* win = nullptr, int wb = 0, unsigned wn = 0) {
+    constexpr bool TAB = KIND == kHash || KIND == kBitsHash;
     const int lane = threadIdx.x & 31;
     const int lo_w = L[0], hi_w = L[du - 1];
     unsigned long long cnt = 0, cnt_u = 0;   // all hits; MODE 2: hits owned by u
@@ -384,7 +586,7 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
             // cost more than the few extra filter probes)
             int lo = 0, hi = n;
             int s0 = 0;
-            if (n > narrow_min) {
+            if (KIND != kBits && n > narrow_min) {
                 while (lo < hi) { int m = (lo + hi) >> 1; if (lst[m] < lo_w) lo = m + 1; else hi = m; }
                 s0 = lo;
                 hi = n;
@@ -394,6 +596,49 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
             }
             xb = b0 + s0;
             dx = lo - s0;
+        }
+        if (KIND == kBits) {
+            // long lists (most of a hub's): the whole warp on one list, four
+            // rows in flight.  An entry then costs its load and one bit of
+            // shared memory; the dealt pairs below also find their candidate.
+            unsigned longs = __ballot_sync(0xFFFFFFFFu, dx >= kTcLong);
+            while (longs) {
+                const int l = __ffs(longs) - 1;
+                longs &= longs - 1;
+                const int32_t* q = g.fwd + __shfl_sync(0xFFFFFFFFu, xb, l);
+                const int n = __shfl_sync(0xFFFFFFFFu, dx, l);
+                const int vl = __shfl_sync(0xFFFFFFFFu, v, l);
+                const bool fl = __shfl_sync(0xFFFFFFFFu, (int)flp, l) != 0;
+                unsigned h = 0;
+                for (int i = lane; i < n; i += 128) {
+                    unsigned wi[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)   // past the end: outside the window
+                        wi[j] = i + 32 * j < n ? (unsigned)(q[i + 32 * j] - wb) : 0xFFFFFFFFu;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        if (wi[j] >= wn) continue;
+                        const unsigned hit = (win[wi[j] >> 5] >> (wi[j] & 31)) & 1u;
+                        h += hit;
+                        if (MODE == 1 && hit) atomicAdd(per_vertex + (int)wi[j] + wb, 1ull);
+                    }
+                }
+                cnt += h;
+                if (MODE == 1 || MODE == 2) {
+                    const unsigned all = __reduce_add_sync(0xFFFFFFFFu, h);
+                    if (lane == 0 && all) {
+                        if (MODE == 1) {
+                            atomicAdd(per_vertex + u, (unsigned long long)all);
+                            atomicAdd(per_vertex + vl, (unsigned long long)all);
+                        } else if (fl) {
+                            atomicAdd(per_vertex + vl, (unsigned long long)all);
+                        } else {
+                            cnt_u += all;
+                        }
+                    }
+                }
+            }
+            if (dx >= kTcLong) dx = 0;
         }
         int incl = dx;
         for (int o = 1; o < 32; o <<= 1) {
@@ -464,7 +709,14 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
                     if (!FULL && w < 0) continue;
                     bool hit;
                     int e_uw = 0;   // MODE 3: edge (u, w)
-                    if (TAB) {
+                    if (KIND == kBits) {
+                        // (a candidate's list may leave the window)
+                        const unsigned i = (unsigned)(w - wb);
+                        hit = i < wn && ((win[i >> 5] >> (i & 31)) & 1u);
+                    } else if (KIND == kBitsHash && w >= wb) {
+                        const unsigned i = (unsigned)(w - wb);
+                        hit = (win[i >> 5] >> (i & 31)) & 1u;
+                    } else if (TAB) {
                         const unsigned f = tc_fbit(w, bits);
                         bool more;
                         unsigned slot;
@@ -639,8 +891,33 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
             const int dc = (int)(g.coff[u + 1] - cb);
             if (du == 0 || dc == 0) continue;
             if (du <= small_du && dc <= small_dc) continue;   // k_tc_thread's
+            // ids of N+(u) close enough for a bitmap in place of the table (in
+            // id order its ends are the list's; by rank, the last numbers)
+            int wb = INT_MAX;
+            unsigned wn = 0;
+            bool to_cta = false;
+            if (MODE != 3) {
+                if (g.wb != INT_MAX) {
+                    const int b = nV - kWarpWin;
+                    if (u >= b) {
+                        wb = b;
+                        wn = kWarpWin;
+                    }
+                } else {
+                    const int first = g.fwd[ub];
+                    const unsigned span = (unsigned)(g.fwd[ub + du - 1] - first) + 1;
+                    if (span <= (unsigned)kWarpWin) {
+                        wb = first;
+                        wn = span;
+                    } else {
+                        // a CTA has room for twice the bits, and is worth its
+                        // set-up from a few thousand pairs on
+                        to_cta = span <= (unsigned)kWin && (long long)dc * du > kWinWork;
+                    }
+                }
+            }
             // every probed list of u is at most du long: dc * du bounds u's pairs
-            if (du > warp_cap || (long long)dc * du > warp_work) {
+            if (du > warp_cap || (long long)dc * du > warp_work || to_cta) {
                 // listed: one work item (u, chunk) per item_cands candidates;
                 // mid items from the front of `big`, huge items from the back
                 if (lane == 0) {
@@ -657,6 +934,23 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
                 }
                 continue;
             }
+            if (MODE != 3 && wn) {
+                unsigned* win = (unsigned*)tab;
+                for (unsigned i = lane; i < (wn + 127) / 128; i += 32)
+                    reinterpret_cast<uint4*>(win)[i] = make_uint4(0u, 0u, 0u, 0u);
+                __syncwarp();
+                for (int i = lane; i < du; i += 32) {
+                    const unsigned x = (unsigned)(g.fwd[ub + i] - wb);
+                    atomicOr(win + (x >> 5), 1u << (x & 31));
+                }
+                __syncwarp();
+                mine += tc_vertex_warp<MODE, kBits>(
+                    u, g.fwd + ub, du, g.cand + cb, dc, nullptr, nullptr, nullptr, 0, narrow_min,
+                    nullptr, g, s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, wb,
+                    wn);
+                __syncwarp();
+                continue;
+            }
             int bits = 32 - __clz(2 * du - 1);   // table of 2^bits >= 2*du slots
             if (bits < 5) bits = 5;
             unsigned* filt = s_filt[warp];
@@ -669,7 +963,7 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
                 if (MODE == 3) teid[h] = g.feid[ub + i];
             }
             __syncwarp();
-            const unsigned long long cu = tc_vertex_warp<MODE, true>(
+            const unsigned long long cu = tc_vertex_warp<MODE, kHash>(
                 u, g.fwd + ub, du, g.cand + cb, dc, tab, filt, teid, bits, narrow_min, nullptr, g,
                 s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex);
             mine += cu;
@@ -695,7 +989,11 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
 // lists share `big` (items (u << 32) | chunk, each item_cands(d+(u))
 // candidates of u): mid from the front (counters[1] entries), huge from the
 // back (counters[2] entries).
-template <int MODE>
+// WIN: an 8 KB bitmap in front of the table.  By rank it holds the members
+// among the last kWin ranks and the table those below (none for u among them;
+// no list exceeds `cap`, checked by the host); by id, all members when they
+// are less than kWin ids apart.
+template <int MODE, bool WIN>
 __global__ void __launch_bounds__(kTcWarps * 32, 4)
 k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
          unsigned long long* __restrict__ total_out, const int* __restrict__ counters,
@@ -721,31 +1019,63 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         const long long cb = g.coff[u] + (long long)ch * ipc;
         const int rest = (int)(g.coff[u + 1] - cb);
         const int dc = rest < ipc ? rest : ipc;
-        const int* tab = nullptr;
-        unsigned* filt = (unsigned*)(s_dyn + tc_table_slots(cap));
+        unsigned* win = (unsigned*)s_dyn;                  // WIN: kWin bits
+        int* slots = s_dyn + (WIN ? kWin / 32 : 0);
+        unsigned* filt = (unsigned*)(slots + tc_table_slots(cap));
         int* teid = MODE == 3 ? (int*)(filt + tc_table_slots(cap) / 4) : nullptr;
+        int wb = INT_MAX;
+        unsigned wn = kWin;
+        bool hash = du <= cap;
+        if (WIN) {
+            if (g.wb != INT_MAX) {
+                wb = g.wb;
+                hash = u < wb;
+            } else {
+                const int first = g.fwd[ub];
+                const unsigned span = (unsigned)(g.fwd[ub + du - 1] - first) + 1;
+                if (span <= (unsigned)kWin) {
+                    wb = first;
+                    wn = span;
+                    hash = false;
+                }
+            }
+        }
+        const bool bm = wb != INT_MAX;   // uniform in the CTA
         int bits = 0;
         if (threadIdx.x == 0) s_next = 0;
-        if (du <= cap) {
+        if (WIN && bm)
+            for (int j = threadIdx.x; j < (int)((wn + 127) / 128); j += blockDim.x)
+                reinterpret_cast<uint4*>(win)[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (hash) {
             bits = 32 - __clz(2 * du - 1);
             if (bits < 5) bits = 5;
-            for (int j = threadIdx.x; j < (1 << bits); j += blockDim.x) s_dyn[j] = -1;
+            for (int j = threadIdx.x; j < (1 << bits); j += blockDim.x) slots[j] = -1;
             for (int j = threadIdx.x; j < (1 << (bits - 2)); j += blockDim.x) filt[j] = 0u;
+        }
+        if ((WIN && bm) || hash) {
             __syncthreads();
             for (int j = threadIdx.x; j < du; j += blockDim.x) {
-                const unsigned h = tab_insert_f(s_dyn, filt, bits, g.fwd[ub + j]);
-                if (MODE == 3) teid[h] = g.feid[ub + j];
+                const int w = g.fwd[ub + j];
+                if (WIN && w >= wb) {
+                    const unsigned i = (unsigned)(w - wb);
+                    atomicOr(win + (i >> 5), 1u << (i & 31));
+                } else {
+                    const unsigned h = tab_insert_f(slots, filt, bits, w);
+                    if (MODE == 3) teid[h] = g.feid[ub + j];
+                }
             }
-            tab = s_dyn;
         }
         __syncthreads();
-        const unsigned long long cu =
-            tab ? tc_vertex_warp<MODE, true>(u, g.fwd + ub, du, g.cand + cb, dc, tab, filt, teid,
-                                             bits, narrow_min, &s_next, g, s_pref[warp],
-                                             s_vb[warp], s_v[warp], s_fc[warp], per_vertex)
-                : tc_vertex_warp<MODE, false>(u, g.fwd + ub, du, g.cand + cb, dc, tab, filt, teid,
-                                              bits, narrow_min, &s_next, g, s_pref[warp],
-                                              s_vb[warp], s_v[warp], s_fc[warp], per_vertex);
+        auto run = [&](auto kind) {
+            return tc_vertex_warp<MODE, decltype(kind)::value>(
+                u, g.fwd + ub, du, g.cand + cb, dc, slots, filt, teid, bits, narrow_min, &s_next, g,
+                s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, wb, wn);
+        };
+        unsigned long long cu;
+        if (WIN && bm) cu = hash ? run(std::integral_constant<int, kBitsHash>())
+                                 : run(std::integral_constant<int, kBits>());
+        else cu = hash ? run(std::integral_constant<int, kHash>())
+                       : run(std::integral_constant<int, kSearch>());
         mine += cu;
         __syncthreads();
     }
@@ -782,6 +1112,70 @@ void build_oriented(hn_graph* g, Oriented& o, const int32_t* canon) {
               canon ? o.feid.get() : (int32_t*)nullptr);
 }
 
+// The orientation by rank, when it pays: true and o filled.  It does when
+// most edges join vertices of more than kWin apart in id (otherwise, as in a
+// union of small graphs, id order keeps the lists of neighbours close in
+// memory, which ranks would scatter) and every oriented list fits the CTA
+// kernel's table (unsorted lists cannot be searched).
+static bool build_by_rank(hn_graph* g, Oriented& o) {
+    cudaStream_t s = g->stream;
+    const int nV = g->nV;
+    const long long m = g->nE;
+    if (m == 0 || m > 0x7FFFFFFFll || nV <= kWin || !knob(kKnobTcFlip)) return false;
+    o.prefix.alloc((size_t)nV + 1, s);
+    degree_prefix(g, nullptr, nV, o.prefix.get());
+    constexpr int kSamples = 16384;
+    int* local = (int*)(g->d_scalar + 4);   // [0] local samples, [1] longest oriented list
+    HN_CUDA(cudaMemsetAsync(local, 0, 2 * sizeof(int), s));
+    HN_LAUNCH(k_local_sample, kSamples / 256, 256, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
+              kSamples, local);
+    HN_CUDA(cudaMemcpyAsync(g->h_scalar + 4, local, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    HN_CUDA(cudaStreamSynchronize(s));
+    if (2 * *(const int*)(g->h_scalar + 4) > kSamples) return false;
+    // ranks: vertices sorted by degree, stably (so by id among equals)
+    DevBuf<int32_t> rank((size_t)nV, s);
+    o.inv.alloc((size_t)nV, s);
+    {
+        DevBuf<unsigned long long> k1((size_t)nV, s), k2((size_t)nV, s);
+        HN_LAUNCH(k_rank_keys, grid_for(g, nV, kB), kB, 0, s, g->vtab, nV, k1.get());
+        unsigned long long *kc = k1.get(), *ka = k2.get();
+        uint32_t *v1 = nullptr, *v2 = nullptr;
+        HN_CUDA(cudaMemsetAsync(&g->alloc->error, 0, sizeof(int), s));
+        radix_sort_u64(g, kc, ka, v1, v2, nV, 32, &g->alloc->error, s);
+        check_device_error(g);   // unsorted keys are no permutation
+        HN_LAUNCH(k_rank_of, grid_for(g, nV, kB), kB, 0, s, (const unsigned long long*)kc, nV,
+                  rank.get(), o.inv.get());
+    }
+    const long long ntiles = (m + nV + kRankTile - 1) / kRankTile;
+    const long long grid = (ntiles + kB / 32 - 1) / (kB / 32);
+    DevBuf<long long> splits;
+    lb_splits(g, o.prefix.get(), nV, m, kRankTile, splits);
+    DevBuf<unsigned> kept((size_t)m / 32 + 2, s);
+    DevBuf<int> cnt((size_t)nV + 1, s);
+    HN_CUDA(cudaMemsetAsync(kept.get(), 0, sizeof(unsigned) * kept.n, s));
+    HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * cnt.n, s));
+    HN_LAUNCH(k_rank_orient<false>, grid, kB, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
+              (const int32_t*)rank.get(), kept.get(), cnt.get(), (const long long*)nullptr,
+              (int32_t*)nullptr, (const long long*)splits.get(), ntiles);
+    HN_LAUNCH(k_max_int, grid_for(g, nV, kB), kB, 0, s, (const int*)cnt.get(), nV, local + 1);
+    HN_CUDA(cudaMemcpyAsync(g->h_scalar + 4, local, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    o.offp.alloc((size_t)nV + 1, s);
+    exclusive_scan(g, (const int*)cnt.get(), o.offp.get(), (long long)nV + 1, s);
+    HN_CUDA(cudaStreamSynchronize(s));
+    if (((const int*)(g->h_scalar + 4))[1] > knob(kKnobTcCtaTableCap)) return false;
+    HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * cnt.n, s));
+    o.fwd.alloc((size_t)(m + 4), s);
+    HN_LAUNCH(k_rank_orient<true>, grid, kB, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
+              (const int32_t*)rank.get(), kept.get(), cnt.get(), (const long long*)o.offp.get(),
+              o.fwd.get(), (const long long*)splits.get(), ntiles);
+    o.wb = nV - kWin;
+    return true;
+}
+
+void build_for_counting(hn_graph* g, Oriented& o) {
+    if (!build_by_rank(g, o)) build_oriented(g, o);
+}
+
 // C(z) for every vertex z: offsets coff (nV+1) and lists cand.
 void build_candidates(hn_graph* g, const Oriented& o, DevBuf<long long>& coff,
                       DevBuf<int32_t>& cand, DevBuf<int32_t>* ceid) {
@@ -795,13 +1189,17 @@ void build_candidates(hn_graph* g, const Oriented& o, DevBuf<long long>& coff,
     const long long grid = (long long)g->info.sms * 8;
     coff.alloc((size_t)nV + 1, s);
     cand.alloc((size_t)m + 4, s);
-    HN_LAUNCH(k_cand<false>, grid, kB, 0, s, o.offp.get(), nV, o.fwd.get(), cnt.get(),
+    DevBuf<int> dplus((size_t)nV, s);
+    HN_LAUNCH(k_dplus, grid_for(g, nV, kB), kB, 0, s, (const long long*)o.offp.get(), nV, dplus.get());
+    HN_LAUNCH(k_cand<false>, grid, kB, 0, s, o.offp.get(), (const int*)dplus.get(), nV,
+              o.fwd.get(), cnt.get(),
               (const long long*)nullptr, (int32_t*)nullptr, splits.get(), (long long)splits.n - 1,
               (const int32_t*)nullptr, (int32_t*)nullptr);
     exclusive_scan(g, (const int*)cnt.get(), coff.get(), (long long)nV + 1, s);
     HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * ((size_t)nV + 1), s));
     if (ceid) ceid->alloc((size_t)m + 4, s);
-    HN_LAUNCH(k_cand<true>, grid, kB, 0, s, o.offp.get(), nV, o.fwd.get(), cnt.get(),
+    HN_LAUNCH(k_cand<true>, grid, kB, 0, s, o.offp.get(), (const int*)dplus.get(), nV,
+              o.fwd.get(), cnt.get(),
               (const long long*)coff.get(), cand.get(), splits.get(), (long long)splits.n - 1,
               ceid ? (const int32_t*)o.feid.get() : (const int32_t*)nullptr,
               ceid ? ceid->get() : (int32_t*)nullptr);
@@ -818,7 +1216,7 @@ constexpr size_t tc_table_bytes(int cap, bool eid = false) {
 }
 constexpr int kCtaCapEid = 8192;   // largest table with edge ids (147 KB)
 
-template <int MODE>
+template <int MODE, bool WIN>
 void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_counts,
                      unsigned long long* d_total, int* counters, long long* big,
                      long long big_cap, bool flipped) {
@@ -826,29 +1224,35 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     const long long gw = (long long)g->info.sms * knob(kKnobTcWarpCtasPerSm);
     const int warp_cap = (int)knob(kKnobTcWarpCap);
     const int chunk = (int)knob(kKnobTcChunk);
-    const int narrow_min = (int)knob(kKnobTcNarrowMin);
-    const long long warp_work = knob(kKnobTcWarpWork), item_work = knob(kKnobTcItemWork);
+    const bool by_rank = view.wb != INT_MAX;
+    // lists by rank are not sorted: nothing to narrow
+    const int narrow_min = by_rank ? INT_MAX : (int)knob(kKnobTcNarrowMin);
+    // by rank, with a bitmap to set up per item and cheaper pairs: items four
+    // times as long on graphs with enough of them (rmat scale 22, 46,000 items:
+    // 30.6 -> 27.3 ms)
+    const long long warp_work = knob(kKnobTcWarpWork);
+    const long long item_work = knob(kKnobTcItemWork) * (by_rank && g->nE >= (1ll << 26) ? 4 : 1);
     constexpr bool eid = MODE == 3;
     const int cap_max = eid ? kCtaCapEid : kCtaCap;
     const int mid_cap = (int)knob(kKnobTcMidCap);
     const int cta_cap = (int)std::min<long long>(knob(kKnobTcCtaTableCap), cap_max);
-    const size_t dyn_mid = tc_table_bytes(mid_cap, eid), dyn_huge = tc_table_bytes(cta_cap, eid);
+    constexpr size_t win = WIN ? kWin / 8 : 0;
+    const size_t dyn_mid = win + tc_table_bytes(mid_cap, eid);
+    const size_t dyn_huge = win + tc_table_bytes(cta_cap, eid);
     const size_t dyn_warp = eid ? (size_t)kTcWarps * kWarpTab * sizeof(int) : 0;
-    static bool attr_set = false;   // one attribute per instantiation
-    if (!attr_set) {
-        HN_CUDA(cudaFuncSetAttribute(k_tc_cta<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)tc_table_bytes(cap_max, eid)));
-        HN_CUDA(cudaFuncSetAttribute(k_tc_warp<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)dyn_warp));
-        attr_set = true;
-    }
+    // (set per call: the attributes belong to the device in use)
+    HN_CUDA(cudaFuncSetAttribute(k_tc_cta<MODE, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(win + tc_table_bytes(cap_max, eid))));
+    HN_CUDA(cudaFuncSetAttribute(k_tc_warp<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)dyn_warp));
     int mid_per_sm = 0;
-    HN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mid_per_sm, k_tc_cta<MODE>,
+    HN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mid_per_sm, k_tc_cta<MODE, WIN>,
                                                           kTcWarps * 32, dyn_mid));
     if (mid_per_sm < 1) mid_per_sm = 1;
     // small vertices by thread (only with the smaller-side assignment, which
-    // bounds every probed list by d+(u))
-    const int small_du = flipped ? (int)knob(kKnobTcThreadDu) : 0;
+    // bounds every probed list by d+(u),
+    // and sorted lists, which it merges)
+    const int small_du = flipped && !by_rank ? (int)knob(kKnobTcThreadDu) : 0;
     const int small_dc = (int)knob(kKnobTcThreadDc);
     if (small_du > 0)
         HN_LAUNCH(k_tc_thread<MODE>, (long long)g->info.sms * 8, 256, 0, s, view, g->nV, small_du,
@@ -856,9 +1260,9 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     HN_LAUNCH(k_tc_warp<MODE>, gw, kTcWarps * 32, dyn_warp, s, view, g->nV, d_counts, d_total,
               counters, big, big_cap, warp_cap, mid_cap, warp_work, item_work, chunk, narrow_min,
               small_du, small_dc);
-    HN_LAUNCH(k_tc_cta<MODE>, (long long)g->info.sms * mid_per_sm, kTcWarps * 32, dyn_mid, s, view,
+    HN_LAUNCH((k_tc_cta<MODE, WIN>), (long long)g->info.sms * mid_per_sm, kTcWarps * 32, dyn_mid, s, view,
               g->nV, d_counts, d_total, counters, big, big_cap, item_work, narrow_min, 0, mid_cap);
-    HN_LAUNCH(k_tc_cta<MODE>, (long long)g->info.sms, kTcWarps * 32, dyn_huge, s, view, g->nV,
+    HN_LAUNCH((k_tc_cta<MODE, WIN>), (long long)g->info.sms, kTcWarps * 32, dyn_huge, s, view, g->nV,
               d_counts, d_total, counters, big, big_cap, item_work, narrow_min, 1, cta_cap);
 }
 
@@ -896,11 +1300,16 @@ unsigned long long run_counting(hn_graph* g, const Oriented& o, int mode,
     }
     if (d_counts) HN_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * g->nV, s));
     long long* bp = big.get();
+    view.wb = o.wb;
+    auto count = [&](auto m) {   // (edge supports need the table's slots)
+        constexpr int M = decltype(m)::value;
+        launch_counting<M, M != 3>(g, view, d_counts, d_total, counters, bp, big_cap, flipped);
+    };
     switch (mode) {
-        case 0: launch_counting<0>(g, view, nullptr, d_total, counters, bp, big_cap, flipped); break;
-        case 1: launch_counting<1>(g, view, d_counts, d_total, counters, bp, big_cap, flipped); break;
-        case 2: launch_counting<2>(g, view, d_counts, d_total, counters, bp, big_cap, flipped); break;
-        default: launch_counting<3>(g, view, nullptr, d_total, counters, bp, big_cap, flipped);
+        case 0: count(std::integral_constant<int, 0>()); break;
+        case 1: count(std::integral_constant<int, 1>()); break;
+        case 2: count(std::integral_constant<int, 2>()); break;
+        default: count(std::integral_constant<int, 3>());
     }
     read_scalars(g, 1);
     return (unsigned long long)g->h_scalar[0];
@@ -910,7 +1319,15 @@ unsigned long long run_counting(hn_graph* g, const Oriented& o, int mode,
 
 unsigned long long count_triangles(hn_graph* g, const Oriented& o, unsigned long long* d_counts,
                                    int mode) {
-    return run_counting(g, o, d_counts ? mode : 0, d_counts, nullptr);
+    if (!d_counts || o.wb == INT_MAX)
+        return run_counting(g, o, d_counts ? mode : 0, d_counts, nullptr);
+    // counted under ranks, then handed out under vertex ids
+    DevBuf<unsigned long long> by_rank((size_t)g->nV, g->stream);
+    const unsigned long long t = run_counting(g, o, mode, by_rank.get(), nullptr);
+    HN_LAUNCH(k_unrank, grid_for(g, g->nV, kB), kB, 0, g->stream,
+              (const unsigned long long*)by_rank.get(), (const int32_t*)o.inv.get(), g->nV, d_counts);
+    HN_CUDA(cudaStreamSynchronize(g->stream));
+    return t;
 }
 
 unsigned long long edge_support(hn_graph* g, const Oriented& o, int32_t* sup) {
@@ -934,7 +1351,7 @@ extern "C" int hn_tc(hn_graph_t* g, uint64_t* per_vertex, int mem, uint64_t* tot
         return HN_OK;
     }
     Oriented o;
-    build_oriented(g, o);
+    build_for_counting(g, o);
     DevBuf<unsigned long long> pv;
     unsigned long long* d_pv = nullptr;
     if (per_vertex) {
@@ -965,7 +1382,7 @@ extern "C" int hn_tc_owner(hn_graph_t* g, uint64_t* counts, int mem, uint64_t* t
         return HN_OK;
     }
     Oriented o;
-    build_oriented(g, o);
+    build_for_counting(g, o);
     DevBuf<unsigned long long> buf;
     unsigned long long* d_c = (unsigned long long*)counts;
     if (mem == HN_MEM_HOST) {

@@ -1,6 +1,8 @@
 // Degree-oriented graph used by triangle counting.
 #pragma once
 
+#include <climits>
+
 #include "hn_graph.cuh"
 
 namespace hn {
@@ -10,12 +12,20 @@ struct Oriented {
     DevBuf<long long> offp;    // oriented offsets (nV+1)
     DevBuf<int32_t> fwd;       // oriented, sorted neighbour lists
     DevBuf<int32_t> feid;      // edge id of each fwd entry (when built with canon)
+    // orientation by rank (build_for_counting): offp is indexed by rank and
+    // fwd holds ranks, unsorted
+    DevBuf<int32_t> inv;       // vertex of each rank
+    int wb = INT_MAX;          // first rank of the bitmap window; INT_MAX: by id
 };
 
 // Build N+(u) = {v in N(u) : (deg u, u) < (deg v, v)} for every vertex.
 // With canon (an id per CSR position, nE entries), feid[p] = canon of the
 // CSR position the oriented entry p came from.
 void build_oriented(hn_graph* g, Oriented& o, const int32_t* canon = nullptr);
+
+// The same orientation for the counts only, under vertex ids or under ranks
+// in the (degree, id) order, whichever the graph's edges favour.
+void build_for_counting(hn_graph* g, Oriented& o);
 
 // Triangles of the oriented graph.  With d_counts (device array of nV
 // entries): mode 1 = per-vertex counts (each triangle credited to its three

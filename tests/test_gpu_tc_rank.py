@@ -1,0 +1,78 @@
+"""Triangle counts by the rank orientation (graphs of more than 65,536
+vertices whose edges are not local in id): totals, per-vertex and owner
+counts equal the id orientation's (tc.flip = 0 never ranks) and the oracle's,
+with lists below, across and inside the bitmap window."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import hornet_b200 as H
+from oracle import oracle as O
+from tests import helpers as T
+
+pytestmark = pytest.mark.gpu
+
+
+def build(g):
+    return H.Hornet(H.HornetInit(g.nV, g.nE, g.off32(), g.adj, sorted_adjacency=True))
+
+
+def owner(h):
+    out = np.zeros(h.nV(), np.uint64)
+    total = ctypes.c_uint64()
+    H._check(H.lib().hn_tc_owner(h.handle, out.ctypes.data_as(ctypes.c_void_p), H.HN_MEM_HOST,
+                                 ctypes.byref(total)))
+    return out, total.value
+
+
+def graph(kind):
+    rng = np.random.default_rng(3)
+    if kind == "rmat":
+        return T.rmat_graph(18, 8, seed=2)
+    if kind == "uniform":       # every list mostly below the window
+        return T.er_graph(200_001, 24, seed=4)
+    if kind == "sparse_core":   # a dense core of scattered ids, lists across the window's edge
+        n = 70_000
+        core = rng.permutation(n)[:600].astype(np.int32)
+        s = [core[rng.integers(0, 600, 120_000)], rng.integers(0, n, 150_000).astype(np.int32)]
+        d = [core[rng.integers(0, 600, 120_000)], core[rng.integers(0, 600, 150_000)]]
+        return O.build_csr_undirected(n, np.concatenate(s), np.concatenate(d))
+    return O.build_csr_undirected(65_537, rng.integers(0, 65_537, 400_000).astype(np.int32),
+                                  rng.integers(0, 65_537, 400_000).astype(np.int32))
+
+
+@pytest.mark.parametrize("kind", ["rmat", "uniform", "sparse_core", "just_over"])
+def test_rank_orientation(kind):
+    g = graph(kind)
+    h = build(g)
+    ref = O.tc(g)
+    tc = H.TriangleCounting2(h)
+    for knobs in ({}, {"tc.warp_cap": 32, "tc.warp_work": 1024, "tc.mid_cap": 32,
+                       "tc.item_work": 1024}):
+        try:
+            for k, v in knobs.items():
+                H.tune_set(k, v)
+            assert tc.run() == ref
+            assert tc.run(per_vertex=True) == ref
+            pv = tc.copyTCToHost().copy()
+            ow, total = owner(h)
+            H.tune_set("tc.flip", 0)
+            assert total == ref == int(ow.sum())
+            assert tc.run(per_vertex=True) == ref
+            np.testing.assert_array_equal(pv, tc.copyTCToHost())
+            ow0, _ = owner(h)
+            np.testing.assert_array_equal(ow, ow0)
+        finally:
+            H.tune_reset()
+
+
+def test_lists_too_long_for_the_table_go_by_id():
+    """tc.cta_table_cap below the longest oriented list: no ranking."""
+    g = T.rmat_graph(17, 16, seed=6, n_vertices=100_003)
+    h = build(g)
+    try:
+        H.tune_set("tc.cta_table_cap", 64)
+        assert H.TriangleCounting2(h).run() == O.tc(g)
+    finally:
+        H.tune_reset()
