@@ -12,7 +12,9 @@
 // list has at most kLaneMax entries (probing each entry of the shorter list
 // in the longer one by a binary search narrowed from the previous hit);
 // longer pairs are appended to a list that a second kernel spreads over the
-// whole grid, one warp per pair, lanes striding the shorter list.  (The
+// whole grid, one warp per pair, lanes striding the shorter list, and a CTA
+// per pair whose shorter list exceeds kWarpMax entries (a hub seed's pair
+// with another hub: a warp of its own took as long as all the rest).  (The
 // heavy pairs of one seed sit side by side in the pair order, so leaving
 // them to the warp that met them would serialise them.)  Per-seed sums are
 // warp-aggregated before one atomic.
@@ -23,6 +25,7 @@ namespace {
 
 constexpr int kTclBlock = 256;
 constexpr int kLaneMax = 8;
+constexpr int kWarpMax = 128;
 
 // entries of a[0..na) that occur in b[0..nb) (both sorted, no duplicates)
 __device__ __forceinline__ unsigned common_seq(const int32_t* __restrict__ a, int na,
@@ -58,7 +61,7 @@ __global__ void __launch_bounds__(kTclBlock) k_tcl_pairs(const VRec* __restrict_
                                                          const int32_t* __restrict__ seeds,
                                                          const long long* __restrict__ prefix,
                                                          int n, unsigned long long* counts,
-                                                         long long* heavy_list,
+                                                         long long* heavy_list, long long cap,
                                                          unsigned long long* heavy_n) {
     const int lane = threadIdx.x & 31;
     const long long total = prefix[n];
@@ -93,12 +96,17 @@ __global__ void __launch_bounds__(kTclBlock) k_tcl_pairs(const VRec* __restrict_
             if (na <= kLaneMax) c = common_seq(a, na, b, nb);
             else heavy = true;
         }
-        const unsigned hm = __ballot_sync(0xFFFFFFFFu, heavy);
-        if (hm) {
-            unsigned long long at = 0;
-            if (lane == 0) at = atomicAdd(heavy_n, (unsigned long long)__popc(hm));
-            at = __shfl_sync(0xFFFFFFFFu, at, 0);
-            if (heavy) heavy_list[at + __popc(hm & ((1u << lane) - 1u))] = p;
+        // the warps' pairs from the front of the list, the CTAs' from its end
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const bool mine = heavy && (na > kWarpMax) == (q == 1);
+            const unsigned hm = __ballot_sync(0xFFFFFFFFu, mine);
+            if (hm) {
+                unsigned long long at = 0;
+                if (lane == 0) at = atomicAdd(heavy_n + q, (unsigned long long)__popc(hm));
+                at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(hm & ((1u << lane) - 1u));
+                if (mine) heavy_list[q ? cap - 1 - (long long)at : (long long)at] = p;
+            }
         }
         // lanes of one seed are contiguous: one atomic per run of equal i,
         // issued by the run's last lane with the run's sum
@@ -120,42 +128,63 @@ __global__ void __launch_bounds__(kTclBlock) k_tcl_pairs(const VRec* __restrict_
     }
 }
 
-// One warp per listed heavy pair: lanes stride the shorter list and probe
-// the longer one.
+// A pair (v, u) of the list: its seed, its shorter and its longer list.
+struct TclPair {
+    const int32_t *a, *b;
+    int i, na, nb;
+};
+
+__device__ __forceinline__ TclPair tcl_pair(const VRec* __restrict__ vtab,
+                                            const int32_t* __restrict__ pool,
+                                            const int32_t* __restrict__ seeds,
+                                            const long long* __restrict__ prefix, int n,
+                                            long long p) {
+    int lo = 0, hi = n;   // last i with prefix[i] <= p
+    while (hi - lo > 1) {
+        int mid = (lo + hi) >> 1;
+        if (__ldg(prefix + mid) <= p) lo = mid; else hi = mid;
+    }
+    const VRec rv = vtab[seeds[lo]];
+    const VRec ru = vtab[__ldg(pool + rv.off + (p - __ldg(prefix + lo)))];
+    const bool sw = rv.deg > ru.deg;
+    TclPair r;
+    r.i = lo;
+    r.a = pool + (sw ? ru.off : rv.off);
+    r.b = pool + (sw ? rv.off : ru.off);
+    r.na = sw ? ru.deg : rv.deg;
+    r.nb = sw ? rv.deg : ru.deg;
+    return r;
+}
+
+// The listed pairs: a warp, or a CTA, strides the shorter list and probes the
+// longer one.
 __global__ void __launch_bounds__(kTclBlock) k_tcl_heavy(const VRec* __restrict__ vtab,
                                                          const int32_t* __restrict__ pool,
                                                          const int32_t* __restrict__ seeds,
                                                          const long long* __restrict__ prefix,
                                                          int n, unsigned long long* counts,
                                                          const long long* __restrict__ heavy_list,
+                                                         long long cap,
                                                          const unsigned long long* heavy_n) {
     const int lane = threadIdx.x & 31;
-    const long long nh = (long long)*heavy_n;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long h = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); h < nh;
-         h += warps) {
-        const long long p = heavy_list[h];
-        int lo = 0, hi = n;   // last i with prefix[i] <= p
-        while (hi - lo > 1) {
-            int mid = (lo + hi) >> 1;
-            if (__ldg(prefix + mid) <= p) lo = mid; else hi = mid;
-        }
-        const int i = lo;
-        const VRec rv = vtab[seeds[i]];
-        const int32_t u = __ldg(pool + rv.off + (p - __ldg(prefix + i)));
-        const VRec ru = vtab[u];
-        const int32_t* a = pool + rv.off;
-        const int32_t* b = pool + ru.off;
-        int na = rv.deg, nb = ru.deg;
-        if (na > nb) {
-            const int32_t* t = a; a = b; b = t;
-            int tn = na; na = nb; nb = tn;
-        }
+    const long long nw = (long long)heavy_n[0], nc = (long long)heavy_n[1];
+    for (long long h = blockIdx.x; h < nc; h += gridDim.x) {
+        const TclPair q = tcl_pair(vtab, pool, seeds, prefix, n, heavy_list[cap - 1 - h]);
         unsigned c = 0;
-        for (int j = lane; j < na; j += 32) c += find_sorted(b, nb, __ldg(a + j)) ? 1u : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-        if (lane == 0 && c) atomicAdd(counts + i, (unsigned long long)c);
+        for (int j = threadIdx.x; j < q.na; j += kTclBlock)
+            c += find_sorted(q.b, q.nb, __ldg(q.a + j)) ? 1u : 0u;
+        c = __reduce_add_sync(0xFFFFFFFFu, c);
+        if (lane == 0 && c) atomicAdd(counts + q.i, (unsigned long long)c);
+    }
+    const long long warps = (long long)gridDim.x * (kTclBlock >> 5);
+    for (long long h = (long long)blockIdx.x * (kTclBlock >> 5) + (threadIdx.x >> 5); h < nw;
+         h += warps) {
+        const TclPair q = tcl_pair(vtab, pool, seeds, prefix, n, heavy_list[h]);
+        unsigned c = 0;
+        for (int j = lane; j < q.na; j += 32)
+            c += find_sorted(q.b, q.nb, __ldg(q.a + j)) ? 1u : 0u;
+        c = __reduce_add_sync(0xFFFFFFFFu, c);
+        if (lane == 0 && c) atomicAdd(counts + q.i, (unsigned long long)c);
     }
 }
 
@@ -217,11 +246,11 @@ extern "C" int hn_tc_local(hn_graph_t* g, const int32_t* seeds, int32_t k, uint6
     const long long pairs = g->h_scalar[4];
     DevBuf<long long> heavy((size_t)pairs + 1, s);
     unsigned long long* heavy_n = (unsigned long long*)(g->d_scalar + 5);
-    HN_CUDA(cudaMemsetAsync(heavy_n, 0, sizeof(unsigned long long), s));
+    HN_CUDA(cudaMemsetAsync(heavy_n, 0, 2 * sizeof(unsigned long long), s));
     HN_LAUNCH(k_tcl_pairs, (long long)g->info.sms * 8, kTclBlock, 0, s, g->vtab, g->pool, d_seeds,
-              prefix.get(), k, d_counts, heavy.get(), heavy_n);
+              prefix.get(), k, d_counts, heavy.get(), pairs + 1, heavy_n);
     HN_LAUNCH(k_tcl_heavy, (long long)g->info.sms * 8, kTclBlock, 0, s, g->vtab, g->pool,
-              d_seeds, prefix.get(), k, d_counts, (const long long*)heavy.get(),
+              d_seeds, prefix.get(), k, d_counts, (const long long*)heavy.get(), pairs + 1,
               (const unsigned long long*)heavy_n);
     HN_LAUNCH(k_tcl_half, grid_for(g, k, 256), 256, 0, s, d_counts, k);
     if (mem == HN_MEM_HOST)
