@@ -628,6 +628,10 @@ void ensure_free_list(hn_graph* g, int c, long long count) {
 }
 
 void degree_prefix(hn_graph* g, const int32_t* verts, int32_t n, long long* prefix) {
+    if (!verts) {
+        degree_scan(g->vtab, n, prefix, g->stream);
+        return;
+    }
     HN_LAUNCH(k_degrees, grid_for(g, (long long)n + 1, 256), 256, 0, g->stream, g->vtab, verts,
               n, prefix);
     exclusive_scan(g, (const long long*)prefix, prefix, (long long)n + 1, g->stream);

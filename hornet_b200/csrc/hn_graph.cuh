@@ -274,6 +274,9 @@ template <typename InT, typename OutT>
 void exclusive_scan(hn_graph* g, const InT* in, OutT* out, long long n, cudaStream_t s,
                     Arena* arena = nullptr);
 
+// prefix[v] = degrees of the vertices before v, v = 0..nV (hn_scan.cu).
+void degree_scan(const VRec* vtab, int nV, long long* prefix, cudaStream_t s);
+
 // Update entry points call this: a query view never changes the graph.
 inline void require_owner(const hn_graph* g) {
     if (g->parent) throw Error(HN_ERR_STATE, "a query view cannot update the graph");

@@ -36,6 +36,18 @@ __device__ __forceinline__ T warp_incl_t(T x, int lane) {
     return x;
 }
 
+// An input as a number; a vertex record counts as its degree, so that degree
+// prefixes need no pass of their own over the records.
+template <typename OutT, typename InT>
+__device__ __forceinline__ OutT scan_in(const InT* in, long long i) {
+    return (OutT)in[i];
+}
+template <typename OutT>
+__device__ __forceinline__ OutT scan_in(const VRec* in, long long i) {
+    return (OutT)in[i].deg;
+}
+
+// (n inputs; outputs past them, if any, take the total)
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_reduce(const InT* __restrict__ in, long long n, OutT* __restrict__ sums) {
@@ -45,7 +57,7 @@ k_scan_reduce(const InT* __restrict__ in, long long n, OutT* __restrict__ sums) 
     OutT acc = 0;
 #pragma unroll
     for (int j = 0; j < kScanIpt; j++)
-        if (base + j * kScanThreads < n) acc += (OutT)in[base + j * kScanThreads];
+        if (base + j * kScanThreads < n) acc += scan_in<OutT>(in, base + j * kScanThreads);
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
     if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = acc;
@@ -99,7 +111,8 @@ __device__ __forceinline__ int scan_slot(int i) { return i + (i >> 5); }
 
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_down(const InT* in, OutT* out, long long n, const OutT* __restrict__ prefix) {
+k_scan_down(const InT* in, long long n_in, OutT* out, long long n,
+            const OutT* __restrict__ prefix) {
     __shared__ OutT s_buf[kScanTile + kScanTile / 32];
     __shared__ OutT s_w[kScanThreads / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -109,7 +122,7 @@ k_scan_down(const InT* in, OutT* out, long long n, const OutT* __restrict__ pref
 #pragma unroll
     for (int j = 0; j < kScanIpt; j++) {
         const int i = j * kScanThreads + threadIdx.x;
-        s_buf[scan_slot(i)] = t0 + i < n ? (OutT)in[t0 + i] : (OutT)0;
+        s_buf[scan_slot(i)] = t0 + i < n_in ? scan_in<OutT>(in, t0 + i) : (OutT)0;
     }
     __syncthreads();
     OutT v[kScanIpt];
@@ -142,13 +155,13 @@ k_scan_down(const InT* in, OutT* out, long long n, const OutT* __restrict__ pref
 constexpr long long kScanOne = 16384;
 
 template <typename InT, typename OutT>
-__global__ void __launch_bounds__(kTopThreads) k_scan_one(const InT* in, OutT* out, int n) {
+__global__ void __launch_bounds__(kTopThreads) k_scan_one(const InT* in, int n_in, OutT* out, int n) {
     __shared__ OutT s_w[2][kTopThreads / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     OutT v[kScanIpt], nv[kScanIpt];
     const int b0 = threadIdx.x * kScanIpt;
 #pragma unroll
-    for (int j = 0; j < kScanIpt; j++) nv[j] = b0 + j < n ? (OutT)in[b0 + j] : (OutT)0;
+    for (int j = 0; j < kScanIpt; j++) nv[j] = b0 + j < n_in ? scan_in<OutT>(in, b0 + j) : (OutT)0;
     OutT carry = 0;
     for (int c0 = 0, buf = 0; c0 < n; c0 += kTopThreads * kScanIpt, buf ^= 1) {
         const int b = c0 + b0, bn = b + kTopThreads * kScanIpt;
@@ -157,7 +170,7 @@ __global__ void __launch_bounds__(kTopThreads) k_scan_one(const InT* in, OutT* o
         for (int j = 0; j < kScanIpt; j++) {
             v[j] = nv[j];
             mine += v[j];
-            nv[j] = bn + j < n ? (OutT)in[bn + j] : (OutT)0;
+            nv[j] = bn + j < n_in ? scan_in<OutT>(in, bn + j) : (OutT)0;
         }
         const OutT incl = warp_incl_t(mine, lane);
         if (lane == 31) s_w[buf][w] = incl;
@@ -174,24 +187,34 @@ __global__ void __launch_bounds__(kTopThreads) k_scan_one(const InT* in, OutT* o
     }
 }
 
+// n outputs from n_in <= n inputs
+template <typename InT, typename OutT>
+void scan(const InT* in, long long n_in, OutT* out, long long n, cudaStream_t s, Arena* arena) {
+    if (n <= 0) return;
+    if (n <= kScanOne) {
+        HN_LAUNCH((k_scan_one<InT, OutT>), 1, kTopThreads, 0, s, in, (int)n_in, out, (int)n);
+        return;
+    }
+    const long long nt = (n + kScanTile - 1) / kScanTile;
+    if (nt > 0x7FFFFFFFll) throw Error(HN_ERR_CAPACITY, "prefix sum over too many elements");
+    DevBuf<OutT> sums((size_t)nt, s, arena);
+    HN_LAUNCH((k_scan_reduce<InT, OutT>), nt, kScanThreads, 0, s, in, n_in, sums.get());
+    HN_LAUNCH(k_scan_tiles<OutT>, 1, kTopThreads, 0, s, sums.get(), nt);
+    HN_LAUNCH((k_scan_down<InT, OutT>), nt, kScanThreads, 0, s, in, n_in, out, n,
+              (const OutT*)sums.get());
+}
+
 }  // namespace
 
 template <typename InT, typename OutT>
 void exclusive_scan(hn_graph* g, const InT* in, OutT* out, long long n, cudaStream_t s,
                     Arena* arena) {
-    if (n <= 0) return;
-    if (n <= kScanOne) {
-        HN_LAUNCH((k_scan_one<InT, OutT>), 1, kTopThreads, 0, s, in, out, (int)n);
-        return;
-    }
-    const long long nt = (n + kScanTile - 1) / kScanTile;
-    if (nt > 0x7FFFFFFFll) throw Error(HN_ERR_CAPACITY, "prefix sum over too many elements");
     (void)g;
-    DevBuf<OutT> sums((size_t)nt, s, arena);
-    HN_LAUNCH((k_scan_reduce<InT, OutT>), nt, kScanThreads, 0, s, in, n, sums.get());
-    HN_LAUNCH(k_scan_tiles<OutT>, 1, kTopThreads, 0, s, sums.get(), nt);
-    HN_LAUNCH((k_scan_down<InT, OutT>), nt, kScanThreads, 0, s, in, out, n,
-              (const OutT*)sums.get());
+    scan(in, n, out, n, s, arena);
+}
+
+void degree_scan(const VRec* vtab, int nV, long long* prefix, cudaStream_t s) {
+    scan(vtab, (long long)nV, prefix, (long long)nV + 1, s, nullptr);
 }
 
 template void exclusive_scan<int, int>(hn_graph*, const int*, int*, long long, cudaStream_t, Arena*);

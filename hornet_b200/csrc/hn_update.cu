@@ -315,7 +315,9 @@ k_assign(const int32_t* __restrict__ seg_ncap, long long nseg, Plan plan,
 }
 
 constexpr int kSB = 256;
-constexpr int kScatterTile = 1024;   // elements of a warp's scatter tile
+// Elements of a warp's scatter tile (256 measured 30 % slower on a 300K-entry
+// batch: a tile's first loads are a chain of their own).
+constexpr int kScatterTile = 1024;
 
 __device__ __forceinline__ int lower_bound32(const int32_t* a, int n, int32_t x) {
     int lo = 0, hi = n;
@@ -834,10 +836,9 @@ __global__ void __launch_bounds__(kB) k_tc_delta(const VRec* __restrict__ vtab,
 
 // ---------------------------------------------------------------------------
 // Small batches (at most kSmallBatch entries, unweighted graphs): one kernel
-// up to the host's plan and two after it.  The general pipeline takes 24
+// up to the host's plan and one after it.  The general pipeline takes 24
 // launches, each a few microseconds of launch and latency for a few
-// microseconds of work at most: 1,000 entries inserted and erased took 430 us,
-// and 110 us this way.
+// microseconds of work at most.
 // ---------------------------------------------------------------------------
 constexpr int kSmallBatch = 2048;
 constexpr long long kArenaBatch = 1 << 20;   // batches whose buffers share one allocation
@@ -909,8 +910,11 @@ k_small_front(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
         return;
     }
     if (!sorted) {
+        // thread t keeps keys t and t + kSmallThreads in registers across the
+        // strides below 32, which are exchanges within a warp
         for (int size = 2; size <= np; size <<= 1) {
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            int stride = size >> 1;
+            for (; stride >= 32; stride >>= 1) {
                 for (int p = tid; p < np / 2; p += kSmallThreads) {
                     const int i = 2 * p - (p & (stride - 1)), j = i + stride;
                     const unsigned long long x = key[i], y = key[j];
@@ -921,6 +925,20 @@ k_small_front(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
                 }
                 __syncthreads();
             }
+#pragma unroll
+            for (int r = 0; r < kSmallIpt; r++) {
+                const int i = r * kSmallThreads + tid;
+                if (r * kSmallThreads + (tid & ~31) < np) {   // whole warps
+                    unsigned long long x = key[i];
+                    for (int o = stride; o > 0; o >>= 1) {
+                        const unsigned long long y = __shfl_xor_sync(kFull, x, o);
+                        const bool low = (i & o) == 0, up = (i & size) == 0;
+                        x = (low == up) == (x > y) ? y : x;
+                    }
+                    key[i] = x;
+                }
+            }
+            __syncthreads();
         }
     }
     // mark: element i = r * kSmallThreads + tid
