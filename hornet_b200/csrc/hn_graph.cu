@@ -672,9 +672,9 @@ static void export_edges(hn_graph* g, const long long* prefix, int32_t* src, int
                   (const uint32_t*)nullptr, (uint32_t*)nullptr);
 }
 
-void export_csr64(hn_graph* g, long long* off, int32_t* adj) {
+void export_csr64(hn_graph* g, long long* off, int32_t* adj, int32_t* src) {
     degree_prefix(g, nullptr, g->nV, off);
-    export_edges(g, off, nullptr, adj, nullptr);
+    export_edges(g, off, src, adj, nullptr);
 }
 
 void build_from_csr(hn_graph* g, int32_t nV, int64_t nE, const long long* d_off,

@@ -353,7 +353,9 @@ void ensure_free_list(hn_graph* g, int c, long long count);
 void lb_splits(hn_graph* g, const long long* prefix, long long nseg, long long max_total,
                int tile, DevBuf<long long>& splits);
 
-// Scratch export of the graph as a contiguous CSR (device, int64 offsets).
-void export_csr64(hn_graph* g, long long* off /*nV+1*/, int32_t* adj /*nE*/);
+// Scratch export of the graph as a contiguous CSR (device, int64 offsets),
+// with the source of every entry when src is given.
+void export_csr64(hn_graph* g, long long* off /*nV+1*/, int32_t* adj /*nE*/,
+                  int32_t* src /*nE*/ = nullptr);
 
 }  // namespace hn

@@ -24,7 +24,6 @@
 
 #include <algorithm>
 #include <climits>
-#include <cstddef>
 #include <cstring>
 
 #include "hn_graph.cuh"
@@ -51,12 +50,6 @@ struct KtPeel {
     long long remaining;      // alive edges
     long long rounds;         // peel rounds run
 };
-
-__global__ void k_kt_src(const long long* __restrict__ off, int nV, int32_t* __restrict__ src) {
-    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < nV;
-         u += (long long)gridDim.x * blockDim.x)
-        for (long long e = off[u]; e < off[u + 1]; e++) src[e] = (int)u;
-}
 
 // canonical (u < v) position of every directed edge; checks simplicity and
 // symmetry.
@@ -329,71 +322,81 @@ __global__ void k_kt_begin(KtPeel* st, int K) {
 //     kAlive or the round in which e is (or was) on the frontier, so in round
 //     r an edge is on the frontier iff state = r, dead iff state < r, and an
 //     edge that drops below K - 2 now gets state r + 1 and its truss number
-//     when it is appended;
+//     when it is appended.  Frontiers and their sizes are indexed by the
+//     round, so ending one takes no copying: the barrier's last CTA clears
+//     one counter;
 //   * a frontier of at most kKtFew edges is staged by every CTA for itself
 //     (endpoints and list bounds, with the prefix of their 32-entry chunks),
 //     and the chunks go round-robin to all warps, one binary search a lane;
-//   * a larger one is taken 32 edges a warp: lanes finish those with at most
-//     kKtTiny entries alone, the warp the others, except that lists above
-//     kKtHeavy are left to a CTA each after another barrier.
+//   * a frontier of at most kKtSolo edges is peeled by CTA 0 alone, and so are
+//     the ones it leads to until one exceeds kKtSoloMax, without a grid
+//     barrier.  CTA 0 leaves the shared state alone meanwhile (others may
+//     still be reading it): the barrier's seal takes its result over;
+//   * a larger frontier is split evenly over the CTAs, each staging its edges
+//     (at most kKtFew at a time) and spreading their chunks over its warps.
+// 100,003 vertices, 2.2 M edges, 62 values of K, 663 rounds: 29.7 ms with a
+// WHILE node around five kernels a round, 13.3 ms with one barrier a round and
+// a warp per large frontier's edge, 9.2 ms this way.
 // ---------------------------------------------------------------------------
-constexpr int kKtThreads = 512;
-constexpr int kKtFew = 512;      // edges staged per CTA (one per thread)
-constexpr int kKtTiny = 4;
-constexpr int kKtHeavy = 256;
+constexpr int kKtThreads = 1024;
+constexpr int kKtFew = 512;      // edges staged per CTA
+constexpr int kKtSolo = 16;      // edges that CTA 0 takes alone
+constexpr int kKtSoloMax = 64;
+static_assert(kKtSoloMax <= kKtFew, "CTA 0 stages its frontiers");
 constexpr int kAlive = INT_MAX;
 
 struct KtCtl {
     GridBar bar;
-    const long long* off;     // adjacency lists (dead entries stay until rebuilt)
-    const int32_t* adj;
-    const int32_t* canon;
-    int32_t* F;               // frontier of this round (canonical edge ids)
-    int32_t* NF;              // ... and of the next
-    int32_t* L;               // alive edges at the start of this K
-    int32_t* L2;
-    long long lm;             // entries of adj
-    // copied to the host after the launch
-    int K, nL, minsup, error;
-    long long remaining;
+    // read by every CTA after a barrier
     int round;                // number of the current round, from 1
-    int nf, nNF, nheavy, nL2, stop, swapped, pad;
+    int nL;                   // alive edges at the start of this K
+    int K;
+    int stop;
+    int cnt[3];               // |frontier of round r| at [r % 3]
+    int side;                 // the list L is L[side]
+    int nL2, minsup, error;
+    int x_round, x_nf;        // CTA 0's round and frontier after its rounds alone
 };
 
 struct KtArgs {
     KtCtl* ctl;
+    const long long* off;     // adjacency lists (dead entries stay until rebuilt)
+    const int32_t* adj;
+    const int32_t* canon;
+    long long lm;             // entries of adj
+    int32_t* F[2];            // frontier of round r (canonical edge ids) at [r % 2]
+    int32_t* L[2];            // alive edges of this K, and of the next
     const int32_t* src;       // endpoints of each edge id
     const int32_t* eadj;
     int32_t* state;
     int32_t* sup;
     int32_t* truss;
-    int32_t* heavy;
 };
 
 // x loses a triangle; the thread that takes it below K - 2 puts it on the
 // next frontier.
-__device__ __forceinline__ void kt_drop(const KtArgs& a, int x, int K, int round, int32_t* NF) {
+__device__ __forceinline__ void kt_drop(const KtArgs& a, int x, int K, int round, int* n_next) {
     if (atomicSub(a.sup + x, 1) == K - 2) {
         a.state[x] = round + 1;
         a.truss[x] = K - 1;
-        NF[atomicAdd(&a.ctl->nNF, 1)] = x;
+        a.F[(round + 1) & 1][atomicAdd(n_next, 1)] = x;
     }
 }
 
 // kt_triangle for the states above (read through L2: they change during the
 // launch).
 __device__ __forceinline__ void kt_common(const KtArgs& a, int e, int e1, int e2, int K, int round,
-                                          int32_t* NF) {
+                                          int* n_next) {
     const int s1 = __ldcg(a.state + e1), s2 = __ldcg(a.state + e2);
     if (s1 < round || s2 < round) return;   // the triangle is already gone
     const bool f1 = s1 == round, f2 = s2 == round;
     if (!f1 && !f2) {
-        kt_drop(a, e1, K, round, NF);
-        kt_drop(a, e2, K, round, NF);
+        kt_drop(a, e1, K, round, n_next);
+        kt_drop(a, e2, K, round, n_next);
     } else if (f1 && !f2) {
-        if (e < e1) kt_drop(a, e2, K, round, NF);
+        if (e < e1) kt_drop(a, e2, K, round, n_next);
     } else if (!f1 && f2) {
-        if (e < e2) kt_drop(a, e1, K, round, NF);
+        if (e < e2) kt_drop(a, e1, K, round, n_next);
     }
 }
 
@@ -424,102 +427,85 @@ __device__ __forceinline__ KtEdge kt_edge(const KtArgs& a, const long long* __re
     return k;
 }
 
-__global__ void __launch_bounds__(kKtThreads, 2) k_kt_run(const __grid_constant__ KtArgs a) {
-    __shared__ struct {
-        const long long* off;
-        const int32_t* adj;
-        const int32_t* canon;
-        int32_t *F, *NF, *L, *L2;
-        int K, nL, nf, nheavy, round, stop, error;
-        unsigned gen;
-    } s;
+__global__ void __launch_bounds__(kKtThreads, 1) k_kt_run(const __grid_constant__ KtArgs a) {
+    __shared__ int s_nf, s_round, s_nL, s_K, s_stop, s_side, s_error, s_next;
+    __shared__ unsigned s_gen;
     __shared__ int s_e[kKtFew], s_pa[kKtFew], s_pb[kKtFew], s_na[kKtFew], s_nb[kKtFew];
-    __shared__ int s_pre[kKtFew + 1], s_ws[kKtThreads / 32];
+    __shared__ int s_pre[kKtFew + 1], s_ws[kKtFew / 32];
     const unsigned kFull = 0xFFFFFFFFu;
     KtCtl* ctl = a.ctl;
     volatile KtCtl* vc = a.ctl;   // read and written by the CTA that seals a phase
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (kKtThreads / 32) + warp;
-    const int nwarps = gridDim.x * (kKtThreads / 32);
+    constexpr int NW = kKtThreads / 32;
+    const int gw = blockIdx.x * NW + warp;
+    const int nwarps = gridDim.x * NW;
     const long long gt = blockIdx.x * (long long)kKtThreads + threadIdx.x;
     const long long nt = (long long)gridDim.x * kKtThreads;
+    const int32_t* __restrict__ adj = a.adj;
+    const int32_t* __restrict__ canon = a.canon;
+    // after a barrier: the sizes that this round needs
     auto load = [&] {
-        s.off = vc->off;
-        s.adj = vc->adj;
-        s.canon = vc->canon;
-        s.F = vc->F;
-        s.NF = vc->NF;
-        s.L = vc->L;
-        s.L2 = vc->L2;
-        s.K = vc->K;
-        s.nL = vc->nL;
-        s.nf = vc->nf;
-        s.nheavy = vc->nheavy;
-        s.round = vc->round;
-        s.stop = vc->stop;
+        const int r = __ldcg(&ctl->round);
+        s_nL = __ldcg(&ctl->nL);
+        s_K = __ldcg(&ctl->K);
+        s_stop = __ldcg(&ctl->stop);
+        s_side = __ldcg(&ctl->side);
+        s_nf = __ldcg(&ctl->cnt[r % 3]);
+        s_round = r;
     };
     auto sync = [&](auto seal) {
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (!grid_barrier(&ctl->bar, s.gen, seal)) {
+            if (!grid_barrier(&ctl->bar, s_gen, seal)) {
                 *(volatile int*)&ctl->error = HN_ERR_TIMEOUT;
-                s.error = 1;
+                s_error = 1;
             }
             load();
         }
         __syncthreads();
-        return s.error == 0;
+        return s_error == 0;
     };
     auto nothing = [] {};
-    // the round is over: the next frontier becomes the current one
-    auto end_round = [&] {
-        vc->remaining = vc->remaining - vc->nf;
-        vc->round = vc->round + 1;
-        int32_t* t = vc->F;
-        vc->F = vc->NF;
-        vc->NF = t;
-        vc->nf = vc->nNF;
-        vc->nNF = 0;
-        vc->nheavy = 0;
-    };
     if (threadIdx.x == 0) {
-        s.error = 0;
-        s.gen = *(volatile unsigned*)&ctl->bar.gen;   // it moves only after this CTA arrives
+        s_error = 0;
+        s_gen = *(volatile unsigned*)&ctl->bar.gen;   // it moves only after this CTA arrives
         load();
     }
     __syncthreads();
     while (true) {
         // the frontier of K: alive edges with support < K - 2
         {
-            const int nL = s.nL, K = s.K, round = s.round;
+            const int nL = s_nL, K = s_K, round = s_round;
+            const int32_t* L = a.L[s_side];
+            int* nf = &ctl->cnt[round % 3];
             for (long long i0 = gt - lane; i0 < nL; i0 += nt) {
                 const long long i = i0 + lane;
-                const int e = i < nL ? __ldcg(s.L + i) : 0;
+                const int e = i < nL ? __ldcg(L + i) : 0;
                 const bool take = i < nL && __ldcg(a.sup + e) < K - 2;
-                const int p = warp_append(&ctl->nf, take);
+                const int p = warp_append(nf, take);
                 if (take) {
-                    s.F[p] = e;
+                    a.F[round & 1][p] = e;
                     a.state[e] = round;
                     a.truss[e] = K - 1;
                 }
             }
             if (!sync(nothing)) return;
         }
-        while (s.nf > 0) {
-            const int nf = s.nf, K = s.K, round = s.round;
-            int32_t* const NF = s.NF;
-            const int32_t* __restrict__ adj = s.adj;
-            const int32_t* __restrict__ canon = s.canon;
-            auto probe = [&](int e, int pa, int pb, int nb, int i) {
+        while (s_nf > 0) {
+            const int nf = s_nf, K = s_K, round = s_round;
+            // entry i of the shorter list of frontier edge e of round r
+            auto probe = [&](int e, int pa, int pb, int nb, int i, int r, int* n_next) {
                 const int w = __ldg(adj + pa + i);
                 const int p = kt_lower(adj + pb, nb, w);
                 if (p < nb && __ldg(adj + pb + p) == w)
-                    kt_common(a, e, __ldg(canon + pa + i), __ldg(canon + pb + p), K, round, NF);
+                    kt_common(a, e, __ldg(canon + pa + i), __ldg(canon + pb + p), K, r, n_next);
             };
-            if (nf <= kKtFew) {
+            // round r for n <= kKtFew edges of its frontier, from f0 on, by the
+            // warps first, first + step, ... (called by the whole CTA)
+            auto few = [&](int f0, int n, int r, int first, int step, int* n_next) {
                 int chunks = 0;
-                if ((int)threadIdx.x < nf) {
-                    const KtEdge k = kt_edge(a, s.off, __ldcg(s.F + threadIdx.x));
+                if ((int)threadIdx.x < n) {
+                    const KtEdge k = kt_edge(a, a.off, __ldcg(a.F[r & 1] + f0 + threadIdx.x));
                     s_e[threadIdx.x] = k.e;
                     s_pa[threadIdx.x] = k.pa;
                     s_pb[threadIdx.x] = k.pb;
@@ -533,92 +519,105 @@ __global__ void __launch_bounds__(kKtThreads, 2) k_kt_run(const __grid_constant_
                     const int y = __shfl_up_sync(kFull, incl, o);
                     if (lane >= o) incl += y;
                 }
-                if (lane == 31) s_ws[warp] = incl;
+                if (lane == 31 && warp < kKtFew / 32) s_ws[warp] = incl;
                 __syncthreads();
-                int before = 0;
-                for (int q = 0; q < warp; q++) before += s_ws[q];
-                s_pre[threadIdx.x] = before + incl - chunks;
-                if (threadIdx.x == kKtThreads - 1) s_pre[kKtThreads] = before + incl;
+                if (threadIdx.x < kKtFew) {
+                    int before = 0;
+                    for (int q = 0; q < warp; q++) before += s_ws[q];
+                    s_pre[threadIdx.x] = before + incl - chunks;
+                    if (threadIdx.x == kKtFew - 1) s_pre[kKtFew] = before + incl;
+                }
                 __syncthreads();
-                const int total = s_pre[nf < kKtThreads ? nf : kKtThreads];
-                for (int c = gw; c < total; c += nwarps) {
-                    int lo = 0, hi = nf;   // last edge with s_pre <= c
+                const int total = s_pre[n];
+                for (int c = first; c < total; c += step) {
+                    int lo = 0, hi = n;   // last edge with s_pre <= c
                     while (hi - lo > 1) {
                         const int mid = (lo + hi) >> 1;
                         if (s_pre[mid] <= c) lo = mid; else hi = mid;
                     }
                     const int i = (c - s_pre[lo]) * 32 + lane;
-                    if (i < s_na[lo]) probe(s_e[lo], s_pa[lo], s_pb[lo], s_nb[lo], i);
+                    if (i < s_na[lo]) probe(s_e[lo], s_pa[lo], s_pb[lo], s_nb[lo], i, r, n_next);
                 }
-                if (!sync(end_round)) return;
+            };
+            // the round is over: its counters are free for the one after next
+            auto end_round = [&] {
+                vc->cnt[(round + 2) % 3] = 0;
+                vc->round = round + 1;
+            };
+            if (nf <= kKtSolo) {
+                if (blockIdx.x == 0) {
+                    int r = round, n = nf;
+                    while (n > 0 && n <= (r == round ? kKtSolo : kKtSoloMax)) {
+                        if (threadIdx.x == 0) {
+                            s_next = 0;
+                            vc->bar.beat = (unsigned)r;
+                        }
+                        __syncthreads();
+                        few(0, n, r, warp, NW, &s_next);
+                        __syncthreads();
+                        n = s_next;
+                        r++;
+                        __syncthreads();   // read before it is cleared
+                    }
+                    if (threadIdx.x == 0) {
+                        vc->x_round = r;
+                        vc->x_nf = n;
+                    }
+                }
+                if (!sync([&] {
+                        const int r = vc->x_round;
+                        vc->round = r;
+                        vc->cnt[r % 3] = vc->x_nf;
+                        vc->cnt[(r + 1) % 3] = 0;
+                        vc->cnt[(r + 2) % 3] = 0;
+                    }))
+                    return;
                 continue;
             }
-            const int want = (nf + nwarps - 1) / nwarps;
-            const int per = want < 32 ? want : 32;
-            for (long long f0 = (long long)gw * per; f0 < nf; f0 += (long long)nwarps * per) {
-                KtEdge k{0, 0, 0, 0, 0};
-                if (lane < per && f0 + lane < nf) k = kt_edge(a, s.off, __ldcg(s.F + f0 + lane));
-                const bool big = k.na > kKtHeavy;
-                const int slot = warp_append(&ctl->nheavy, big);
-                if (big) a.heavy[slot] = k.e;
-                const bool tiny = per > 1 && k.na <= kKtTiny;
-                if (tiny)
-                    for (int i = 0; i < k.na; i++) probe(k.e, k.pa, k.pb, k.nb, i);
-                __syncwarp();
-                unsigned coop = __ballot_sync(kFull, !big && !tiny && k.na > 0);
-                while (coop) {
-                    const int l = __ffs(coop) - 1;
-                    coop &= coop - 1;
-                    const int we = __shfl_sync(kFull, k.e, l);
-                    const int wpa = __shfl_sync(kFull, k.pa, l), wpb = __shfl_sync(kFull, k.pb, l);
-                    const int wna = __shfl_sync(kFull, k.na, l), wnb = __shfl_sync(kFull, k.nb, l);
-                    for (int i = lane; i < wna; i += 32) probe(we, wpa, wpb, wnb, i);
-                    __syncwarp();
-                }
-            }
-            if (!sync(nothing)) return;
-            if (s.nheavy > 0) {
-                const int nh = s.nheavy;
-                for (int h = blockIdx.x; h < nh; h += gridDim.x) {
-                    const KtEdge k = kt_edge(a, s.off, __ldcg(a.heavy + h));
-                    for (int i = threadIdx.x; i < k.na; i += kKtThreads)
-                        probe(k.e, k.pa, k.pb, k.nb, i);
+            int* const n_next = &ctl->cnt[(round + 1) % 3];
+            if (nf <= kKtFew) {
+                few(0, nf, round, gw, nwarps, n_next);
+            } else {
+                const int per = (nf + gridDim.x - 1) / gridDim.x;
+                const int end = min(nf, (int)(blockIdx.x + 1) * per);
+                for (int f0 = blockIdx.x * per; f0 < end; f0 += kKtFew) {
+                    few(f0, min(kKtFew, end - f0), round, warp, NW, n_next);
+                    __syncthreads();   // the staged edges are replaced
                 }
             }
             if (!sync(end_round)) return;
         }
         // the edges left, and the smallest support among them
         {
-            const int nL = s.nL;
+            const int nL = s_nL, K = s_K, side = s_side, round = s_round;
+            const int32_t* L = a.L[side];
+            int32_t* L2 = a.L[side ^ 1];
             int mn = 0x7FFFFFFF;
             for (long long i0 = gt - lane; i0 < nL; i0 += nt) {
                 const long long i = i0 + lane;
-                const int e = i < nL ? __ldcg(s.L + i) : 0;
+                const int e = i < nL ? __ldcg(L + i) : 0;
                 const bool take = i < nL && __ldcg(a.state + e) == kAlive;
                 const int p = warp_append(&ctl->nL2, take);
                 if (take) {
-                    s.L2[p] = e;
+                    L2[p] = e;
                     mn = min(mn, __ldcg(a.sup + e));
                 }
             }
             mn = __reduce_min_sync(kFull, mn);
             if (lane == 0 && mn != 0x7FFFFFFF) atomicMin(&ctl->minsup, mn);
             if (!sync([&] {
-                    const int left = vc->nL2;
-                    int32_t* t = vc->L;
-                    vc->L = vc->L2;
-                    vc->L2 = t;
-                    vc->swapped = vc->swapped ^ 1;
+                    const int left = vc->nL2, next = vc->minsup + 3;
+                    vc->side = side ^ 1;
                     vc->nL = left;
                     vc->nL2 = 0;
-                    const int next = vc->minsup + 3, k1 = vc->K + 1;
                     vc->minsup = 0x7FFFFFFF;
-                    vc->stop = left == 0 || 4LL * left <= vc->lm;
-                    if (left > 0) vc->K = next > k1 ? next : k1;
-                    vc->nf = 0;
+                    vc->stop = left == 0 || 4LL * left <= a.lm;
+                    if (left > 0) vc->K = next > K + 1 ? next : K + 1;
+                    vc->cnt[round % 3] = 0;
+                    vc->cnt[(round + 1) % 3] = 0;
                 }))
                 return;
-            if (s.stop) return;
+            if (s_stop) return;
         }
     }
 }
@@ -671,8 +670,7 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
         truss((size_t)m, s), F((size_t)m, s), NF((size_t)m, s);
     DevBuf<unsigned char> alive((size_t)m, s), inF((size_t)m, s);
     int* cnt = (int*)g->d_scalar;  // [0] err/alive, [1] nF, [2] nNF
-    export_csr64(g, off.get(), adj.get());
-    HN_LAUNCH(k_kt_src, grid_for(g, nV, kB), kB, 0, s, off.get(), nV, src.get());
+    export_csr64(g, off.get(), adj.get(), src.get());
     HN_CUDA(cudaMemsetAsync(cnt, 0, 4 * sizeof(int), s));
     HN_LAUNCH(k_kt_canon, grid_for(g, m, kB), kB, 0, s, off.get(), adj.get(), src.get(), m,
               canon.get(), cnt);
@@ -681,7 +679,9 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
         throw Error(HN_ERR_INVALID, "k-truss needs a simple symmetric graph");
     HN_CUDA(cudaMemsetAsync(cnt, 0, 4 * sizeof(int), s));
     HN_CUDA(cudaMemsetAsync(inF.get(), 0, (size_t)m, s));
-    DevBuf<int32_t> H((size_t)m, s);   // heavy frontier edges of each peel round
+    const bool device_rounds = knob(kKnobKtDeviceRounds) != 0;
+    DevBuf<int32_t> H;   // heavy frontier edges of each host-driven peel round
+    if (!device_rounds) H.alloc((size_t)m, s);
     {
         // supports: each triangle of the degree-oriented graph credits its
         // three canonical edges once (uses the graph's scalars, so it runs
@@ -751,7 +751,6 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
         lm = keep;
         cflag.release();
     };
-    const bool device_rounds = knob(kKnobKtDeviceRounds) != 0;
     if (device_rounds) {
         // all K in cooperative launches, one between two list rebuilds
         DevBuf<KtCtl> ctl(1, s);
@@ -761,45 +760,33 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
         int round = 1;
         const int ms = ((int*)g->h_scalar)[5];
         if (ms + 3 > K) K = ms + 3;
-        KtArgs a{ctl.get(), src.get(), adj.get(), state.get(), sup.get(), truss.get(), H.get()};
-        while (remaining > 0) {
+        while (n_alive > 0) {
             KtCtl h{};
-            h.off = loff;
-            h.adj = ladj;
-            h.canon = lcanon;
-            h.F = F.get();
-            h.NF = NF.get();
-            h.L = L.get();
-            h.L2 = L2.get();
-            h.lm = lm;
-            h.K = K;
-            h.nL = n_alive;
-            h.minsup = INT_MAX;
-            h.remaining = remaining;
             h.round = round;
+            h.nL = n_alive;
+            h.K = K;
+            h.minsup = INT_MAX;
             HN_CUDA(cudaMemcpyAsync(ctl.get(), &h, sizeof(KtCtl), cudaMemcpyHostToDevice, s));
+            KtArgs a{ctl.get(), loff, ladj, lcanon, lm, {F.get(), NF.get()}, {L.get(), L2.get()},
+                     src.get(), adj.get(), state.get(), sup.get(), truss.get()};
             void* args[] = {&a};
             cudaEvent_t ev = nullptr;
             if (g_profiling) profile_begin(s, &ev);
-            HN_CUDA(cudaLaunchCooperativeKernel((void*)k_kt_run, dim3(2u * g->info.sms),
+            HN_CUDA(cudaLaunchCooperativeKernel((void*)k_kt_run, dim3((unsigned)g->info.sms),
                                                 dim3(kKtThreads), args, 0, s));
             if (ev) profile_end("k_kt_run", s, ev);
             count_launch();
-            // the part of the state that the host reads
-            constexpr size_t from = offsetof(KtCtl, K);
-            static_assert(sizeof(KtCtl) - from <= 16 * sizeof(long long), "pinned scalars");
-            HN_CUDA(cudaMemcpyAsync(g->h_scalar, (const char*)ctl.get() + from,
-                                    sizeof(KtCtl) - from, cudaMemcpyDeviceToHost, s));
+            static_assert(sizeof(KtCtl) <= 16 * sizeof(long long), "pinned scalars");
+            HN_CUDA(cudaMemcpyAsync(g->h_scalar, ctl.get(), sizeof(KtCtl), cudaMemcpyDeviceToHost,
+                                    s));
             HN_CUDA(cudaStreamSynchronize(s));
-            std::memcpy((char*)&h + from, g->h_scalar, sizeof(KtCtl) - from);
+            std::memcpy((void*)&h, g->h_scalar, sizeof(KtCtl));
             if (h.error) throw Error(h.error, "k-truss: a bounded wait gave up");
-            if (h.swapped) L.swap(L2);
-            remaining = h.remaining;
+            if (h.side) L.swap(L2);
             n_alive = h.nL;
             K = h.K;
             round = h.round;
-            if (remaining <= 0) break;
-            shrink_lists();
+            if (n_alive > 0) shrink_lists();
         }
         K--;   // no edge is left at K (K = 3 on a graph without edges)
     }
