@@ -42,7 +42,7 @@ struct KnobDef {
 };
 const KnobDef kKnobs[kNumKnobs] = {
     {"bfs.ctas_per_sm", 9, 1, 16, false},
-    {"bfs.do_alpha", 14, 1, 1 << 20, false},
+    {"bfs.do_alpha", 4, 1, 1 << 20, false},
     {"bfs.do_beta", 24, 1, 1 << 20, false},
     {"msbfs.block", 256, 128, 512, true},
     {"msbfs.ctas_per_sm", 4, 1, 8, false},

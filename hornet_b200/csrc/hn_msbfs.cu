@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
 // neighbours a step, so a hub costs its warp deg / 64 steps instead of deg.
 // Stops at the step after which nothing is missing.  Called by all lanes.
 constexpr int kMsLane = 16;
-constexpr long long kMsScan = 16;
+constexpr long long kMsScan = 4;
 
 __device__ __forceinline__ unsigned long long ms_pull(const VRec& r, unsigned long long todo,
                                                       const int32_t* __restrict__ pool,

@@ -94,7 +94,7 @@ int hn_profile_report(char* buf, int64_t len);
  *   bfs.ctas_per_sm     CTAs per SM of the BFS level kernel, 128 threads
  *                       each (1..16, 9)
  *   bfs.do_alpha        direction-optimising switch to bottom-up when the
- *                       frontier's edges exceed unexplored edges / alpha (14)
+ *                       frontier's edges exceed unexplored edges / alpha (4)
  *   bfs.do_beta         back to top-down below nV / beta frontier vertices (24)
  *   msbfs.block         batched-BFS block size: 128, 256 or 512 (256)
  *   msbfs.ctas_per_sm   batched-BFS CTAs per SM (1..8, 4)
@@ -132,14 +132,15 @@ int hn_profile_report(char* buf, int64_t len);
  *   bfs.host_levels     1: launch the BFS levels one by one from the host
  *                       (for per-level profiling) instead of the CUDA
  *                       graph's device-side loop (0..1, 0)
- *   bfs.kernel          BFS level kernel: 1 = independent warps on 256-edge
- *                       chunks, 0 = 128-thread CTAs on 1024-edge chunks
+ *   bfs.kernel          1 = a BFS in one cooperative launch (independent warps
+ *                       on 256-edge chunks), 0 = a kernel per level in a CUDA
+ *                       graph, 128-thread CTAs on 1024-edge chunks
  *                       (bfs.ctas_per_sm, bfs.dynamic_chunks and
  *                       bfs.warp_strided apply to it) (0..1, 1)
- *   bfs.warp_ctas_per_sm  CTAs per SM of the warp-chunk level kernel, 256
- *                       threads each (1..8, 4)
- *   ktruss.device_rounds  1: the peel rounds of each K run in a CUDA graph
- *                       (WHILE node, no host round trip per round); 0: one
+ *   bfs.warp_ctas_per_sm  256s of threads per SM of the one-launch BFS, of
+ *                       which three fill an SM's registers (1..8, 4)
+ *   ktruss.device_rounds  1: the peel rounds of all K run in cooperative
+ *                       launches (no host round trip per round or K); 0: one
  *                       host round trip per round, launches sized to the
  *                       frontier (0..1, 1)
  *   update.big_min      old lists of at least this many entries (hubs) are
@@ -339,7 +340,7 @@ int hn_bfs_do(hn_graph_t* g, const int32_t* sources, int32_t k, int32_t* dist,
               int mem, hn_bfs_stats_t* stats);
 
 /* Instrumentation: per-level device time (microseconds, from the GPU's
- * global timer at each level's end inside the BFS CUDA graph) and frontier
+ * global timer at each level's end) and frontier
  * edges of the latest hn_bfs / hn_bfs_multi / hn_bfs_do source on this
  * graph, for its first min(levels, max_levels, 32) levels.  us and edges
  * may be NULL.  No reference counterpart (the reference times whole runs
