@@ -29,6 +29,11 @@ constexpr int kSeedBlock = 256;       // the single seeding CTA
 constexpr int kMsChunk = 2048;        // edges per chunk (block x items per thread)
 constexpr int kMaxSlots = 64;
 
+// A level pushes and applies the touched vertices it listed, pulls (apply
+// does the work), or pushes without a list and applies in a pass over all
+// vertices.
+enum { kMsPush, kMsPull, kMsPushAll };
+
 struct MsState {
     unsigned long long cnt[3];      // frontier counters: (edge total << 32) | size
     unsigned long long tcnt;        // touched vertices this level
@@ -49,7 +54,7 @@ struct MsState {
     const int32_t* src;
     const int32_t* slot;
     int nsrc;
-    int mode;                       // 0 top-down (push + apply), 1 bottom-up (apply scans)
+    int mode;                       // kMsPush, kMsPull or kMsPushAll
     unsigned long long* stat;       // [3*kMaxSlots]: visited, scanned, last level per slot
     int prev_nq;                    // size of the previous frontier (its fronts are cleared)
     int bottom_up;                  // bottom-up levels allowed
@@ -220,7 +225,8 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
              i += (long long)gridDim.x * BLOCK)
             pf[pq[i]] = 0ull;
     }
-    if (st->mode == 1) return;   // bottom-up level: apply does the work
+    if (st->mode == kMsPull) return;   // apply does the work
+    const bool listed = st->mode == kMsPush;
     const int32_t* q = st->q[cur];
     const long long* qbase = st->qbase[cur];
     const unsigned* qoff = st->qoff[cur];
@@ -285,8 +291,12 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
             for (int k = 0; k < IPT; k++) {
                 unsigned long long m = fm[k] & ~sv[k];
                 if (m) {
-                    unsigned long long old = atomicOr(&sn[w[k]].y, m);
-                    if (old == 0) touched_here[nt++] = w[k];
+                    if (listed) {
+                        unsigned long long old = atomicOr(&sn[w[k]].y, m);
+                        if (old == 0) touched_here[nt++] = w[k];
+                    } else {
+                        atomicOr(&sn[w[k]].y, m);
+                    }
                 }
             }
         }
@@ -310,6 +320,11 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_ms_push(MsState* st) {
 // Stops at the step after which nothing is missing.  Called by all lanes.
 constexpr int kMsLane = 16;
 constexpr long long kMsScan = 4;
+// Edges of a frontier that may touch more than one in kMsAll vertices are
+// pushed without a list of the touched: a pass over all vertices reads their
+// masks in order, writes distances to neighbouring words and queues the next
+// frontier in vertex order, where the list's order is that of the edges.
+constexpr long long kMsAll = 4;
 
 __device__ __forceinline__ unsigned long long ms_pull(const VRec& r, unsigned long long todo,
                                                       const int32_t* __restrict__ pool,
@@ -358,8 +373,9 @@ __device__ __forceinline__ unsigned long long ms_pull(const VRec& r, unsigned lo
     return got;
 }
 
-// apply: new bits of every touched vertex (top-down) or of every vertex that
-// misses a slot (bottom-up), their distances, the next frontier.  kMsApply
+// apply: new bits of every touched vertex (listed, or all vertices with bits
+// in nxt) or of every vertex that misses a slot (pull), their distances, the
+// next frontier.  kMsApply
 // vertices per thread share one CTA-wide reservation.  Per-slot statistics
 // stay in registers (lane b counts slots b and b + 32, by ballot and warp
 // sum): an atomic per (vertex, slot), 64-bit and on few shared words, had
@@ -389,11 +405,12 @@ k_ms_apply(MsState* st, cudaGraphConditionalHandle cond) {
     const int32_t* __restrict__ pool = st->pool;
     ulonglong2* sn = st->sn;
     unsigned long long* nfront = st->front[nx];
-    const bool bu = st->mode == 1;
+    const int mode = st->mode;
+    const bool bu = mode == kMsPull;
     const unsigned long long* cfront = st->front[nx ^ 1];
     const unsigned long long all = st->all_mask;
     const int nq_in = (int)(st->cnt[it % 3] & 0xFFFFFFFFull);
-    const long long n_items = bu ? (long long)nV : nt;
+    const long long n_items = mode == kMsPush ? nt : (long long)nV;
     int32_t* dist = st->dist;
     unsigned long long vis0 = 0, vis1 = 0, sc0 = 0, sc1 = 0;   // slots lane, lane + 32
     long long closed = 0;   // degrees of vertices that miss no slot any more
@@ -428,14 +445,16 @@ k_ms_apply(MsState* st, cudaGraphConditionalHandle cond) {
                     nfront[v] = nw;
                     if (!(all & ~(sv | nw))) closed += r.deg;
                 }
-            } else if (i < nt) {
-                v = st->touched[i];
+            } else if (i < n_items) {
+                v = mode == kMsPush ? st->touched[i] : (int)i;
                 const ulonglong2 q = sn[v];
-                nw = q.y & ~q.x;
-                sn[v] = make_ulonglong2(q.x | nw, 0ull);
-                nfront[v] = nw;
-                r = vtab[v];
-                if (!(all & ~(q.x | nw))) closed += r.deg;
+                if (q.y) {   // (always, of a touched vertex)
+                    nw = q.y & ~q.x;
+                    sn[v] = make_ulonglong2(q.x | nw, 0ull);
+                    nfront[v] = nw;
+                    r = vtab[v];
+                    if (!(all & ~(q.x | nw))) closed += r.deg;
+                }
             }
             // the slots that reach any of the warp's vertices now
             unsigned ulo = __reduce_or_sync(kFull, (unsigned)nw);
@@ -501,15 +520,17 @@ k_ms_apply(MsState* st, cudaGraphConditionalHandle cond) {
             st->tcnt = 0;
             st->level = level + 1;
             st->prev_nq = nq_in;
+            // pull while the next frontier's edges (which a push reads) exceed
+            // those of the vertices that still miss a slot (which a pull reads
+            // at most) -- alpha / kMsScan, about 1 by default -- and the
+            // frontier holds nV/beta vertices or more
+            const long long mf = (long long)(c >> 32);
+            int next = mf * kMsAll > nV ? kMsPushAll : kMsPush;
             if (st->bottom_up) {
-                // bottom-up while the next frontier's edges (which a push
-                // reads) exceed those of the vertices that still miss a slot
-                // (which a pull reads at most) -- alpha / kMsScan, about 1 by
-                // default -- and the frontier holds nV/beta vertices or more
-                const long long mf = (long long)(c >> 32);
                 const long long open = (long long)atomicAdd((unsigned long long*)&st->open_edges, 0ull);
-                st->mode = mf * st->alpha > kMsScan * open && (long long)nn * st->beta >= nV;
+                if (mf * st->alpha > kMsScan * open && (long long)nn * st->beta >= nV) next = kMsPull;
             }
+            st->mode = next;
             cudaGraphSetConditional(cond, (nn > 0 && level < nV) ? 1u : 0u);
         }
     }

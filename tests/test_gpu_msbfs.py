@@ -178,3 +178,27 @@ def test_batch_bottom_up_long_lists(block):
             check(out, st, ref, ref_stats)
     finally:
         H.tune_reset()
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1, 700])
+@pytest.mark.parametrize("slots", [1, 9])
+def test_batch_levels_without_a_touched_list(extra, slots):
+    """Frontiers of about nV / 4 edges: one more and the level records no
+    list of touched vertices.  Two hubs share leaves, which lead on to more
+    vertices; some slots start at a leaf or an isolated vertex."""
+    n = 4000
+    d = n // 4 + extra - 1
+    leaves = np.arange(2, 2 + d)
+    s = np.concatenate([np.zeros(d), [0], np.ones(d // 2), leaves[: d // 3]]).astype(np.int32)
+    t = np.concatenate([leaves, [1], leaves[: d // 2], leaves[: d // 3] + d]).astype(np.int32)
+    g = O.build_csr_undirected(n, s, t)
+    h = build(g)
+    srcs = np.array([0, 2, n - 1, 1, d, 2 + d, 0, 5, 9][:slots], np.int32)
+    ref, ref_stats = oracle_slots(g, srcs, range(slots), slots)
+    try:
+        for bu in (0, 1):
+            H.tune_set("msbfs.bottom_up", bu)
+            out, st = H.BfsTopDown(h).run_batch(srcs)
+            check(out, st, ref, ref_stats)
+    finally:
+        H.tune_reset()
