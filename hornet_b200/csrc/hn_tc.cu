@@ -17,10 +17,10 @@
 // table (see the comment above k_tc_warp).
 //
 // Counts of graphs whose edges are not local in vertex id (build_by_rank) use
-// another orientation: vertices are renumbered by rank in the (degree, id)
-// order, so that the ends of most probes are among the kWin highest numbers,
-// where membership in N+(u) is one bit of an 8 KB shared bitmap instead of a
-// hash lookup.
+// another orientation: vertices are renumbered by descending rank in the
+// (degree, id) order, so that nearly all probes are among the first kWin
+// numbers, where membership in N+(u) is one bit of a 16 KB shared bitmap
+// instead of a hash lookup.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -135,14 +135,17 @@ k_orient_fill(const long long* __restrict__ prefix, int nV, const VRec* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Orientation by rank.  rank = position in the (degree, id) order; vertex u's
-// oriented list is stored under rank[u] and holds ranks, so u -> v iff
-// rank[u] < rank[v].  One random 4-byte read per edge decides the direction
-// (a vertex record is 16 bytes) and the decision is kept as one bit per edge,
-// so the fill reads ranks of kept edges only.  Lists are not sorted.
+// Orientation by rank.  number = position in the descending (degree, id)
+// order; vertex u's oriented list is stored under number[u] and holds
+// numbers, so u -> v iff number[v] < number[u].  One random 4-byte read per
+// edge decides the direction (a vertex record is 16 bytes) and the decision
+// is kept as one bit per edge, so the fill reads numbers of kept edges only.
+// Lists are not sorted; each starts on 16 bytes and is padded to a multiple
+// of four entries with kPad.
 // ---------------------------------------------------------------------------
-constexpr int kWinBits = 16;
-constexpr int kWin = 1 << kWinBits;          // ranks of the shared bitmap
+constexpr int kPad = INT_MAX;
+constexpr int kWin = 1 << 17;   // numbers of the CTA kernel's bitmap (16 KB)
+constexpr int kLocal = 1 << 17;  // ids closer than this are local
 constexpr int kRankTile = 1024;
 
 __global__ void k_rank_keys(const VRec* __restrict__ vtab, int nV,
@@ -157,12 +160,12 @@ __global__ void k_rank_of(const unsigned long long* __restrict__ keys, int nV,
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nV;
          i += (long long)gridDim.x * blockDim.x) {
         const int v = (int)(keys[i] >> 32);
-        rank[v] = (int)i;
-        inv[i] = v;
+        rank[v] = nV - 1 - (int)i;
+        inv[nV - 1 - i] = v;
     }
 }
 
-// Of evenly spaced edges, those whose ends are less than kWin ids apart.
+// Of evenly spaced edges, those whose ends are less than kLocal ids apart.
 __global__ void k_local_sample(const long long* __restrict__ prefix, int nV, long long m,
                                const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
                                int samples, int* __restrict__ local) {
@@ -172,16 +175,16 @@ __global__ void k_local_sample(const long long* __restrict__ prefix, int nV, lon
         const long long e = (long long)((double)i / samples * m);
         const long long u = upper_bound_dev(prefix, (long long)nV + 1, e) - 1;
         const int v = pool[vtab[u].off + (e - prefix[u])];
-        near = u - v < kWin && v - u < kWin;
+        near = u - v < kLocal && v - u < kLocal;
     }
     const unsigned b = __ballot_sync(0xFFFFFFFFu, near);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(local, __popc(b));
 }
 
 // Pass 1 (FILL = false): the direction of every edge, one bit each in
-// `kept`, and the kept edges of each vertex in cnt[rank].  Pass 2: every
+// `kept`, and the kept edges of each vertex in cnt[number].  Pass 2: every
 // window reserves its segments' kept edges (cnt is the cursor) and writes
-// their ranks.  A warp per merge-path tile, windows of 32 vertices; a row of
+// their numbers.  A warp per merge-path tile, windows of 32 vertices; a row of
 // 32 edges is one word of `kept` (shared by two windows at their seam).
 template <bool FILL>
 __global__ void __launch_bounds__(kB)
@@ -207,7 +210,7 @@ k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
         const WarpWindow w = warp_window(wt, v0, first, next);
         if (w.n == 0) continue;
         const long long base = __shfl_sync(kFull, off - first, w.lane_of) + wt.item0;
-        const int ru = __shfl_sync(kFull, rv, w.lane_of);   // rank of the lane's segment
+        const int ru = __shfl_sync(kFull, rv, w.lane_of);   // number of the lane's segment
         // the lane's own segment [w.start, send)
         int send = __shfl_down_sync(kFull, w.start, 1);
         if (lane >= w.n - 1) send = w.end;
@@ -239,7 +242,7 @@ k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
                 for (int k = 0; k < ROWS; k++) {
                     const int row = r + 32 * k;
                     if (row >= w.end) break;   // uniform
-                    const bool keep = x[k] >= 0 && rank[x[k]] > u[k];
+                    const bool keep = x[k] >= 0 && rank[x[k]] < u[k];
                     const unsigned b = __ballot_sync(kFull, keep);
                     mine += __popc(b & own(row));
                     if (lane == 0 && b) {
@@ -296,7 +299,20 @@ __global__ void k_max_int(const int* __restrict__ a, int n, int* __restrict__ ou
     if ((threadIdx.x & 31) == 0 && mx) atomicMax(out, mx);
 }
 
-// counts under ranks -> counts under vertex ids
+__global__ void k_padded(const int* __restrict__ cnt, int nV, int* __restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i <= nV;
+         i += (long long)gridDim.x * blockDim.x)
+        out[i] = i < nV ? (cnt[i] + 3) & ~3 : 0;
+}
+
+__global__ void k_pad_lists(const long long* __restrict__ offp, const int* __restrict__ cnt,
+                            int nV, int32_t* __restrict__ fwd) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nV;
+         i += (long long)gridDim.x * blockDim.x)
+        for (long long e = offp[i] + cnt[i]; e < offp[i + 1]; e++) fwd[e] = kPad;
+}
+
+// counts under numbers -> counts under vertex ids
 __global__ void k_unrank(const unsigned long long* __restrict__ in,
                          const int32_t* __restrict__ inv, int nV,
                          unsigned long long* __restrict__ out) {
@@ -347,11 +363,11 @@ k_cand(const long long* __restrict__ offp, const int* __restrict__ dplus, int nV
             ys[k] = -1;
             if (i < n) {
                 const int b = t.seg[i];
-                const long long dx = t.ends[b] - t.seg_start(b);
                 const int y = fwd[t.item0 + i];
-                const long long dy = dplus[y];
-                ys[k] = y;
-                keep[k] = cand_flip(dx, dy) ? 0 : 1;
+                if (y != kPad) {
+                    ys[k] = y;
+                    keep[k] = cand_flip(dplus[t.seg0 + b], dplus[y]) ? 0 : 1;
+                }
             }
         }
         int kept_total;
@@ -417,8 +433,8 @@ k_cand(const long long* __restrict__ offp, const int* __restrict__ dplus, int nV
 constexpr int kTcWarps = 8;
 constexpr int kWarpCap = 512;
 constexpr int kWarpTab = 2 * kWarpCap;
-constexpr int kWarpWin = kWarpTab * 32;   // numbers of a warp's bitmap (in its table's place)
-constexpr long long kWinWork = 8192;
+constexpr int kWarpWin = (kWarpTab - 1) * 32;   // numbers of a warp's bitmap: its table's place,
+                                                // the last word zero
 constexpr int kCtaCap = 16384;   // largest tc.cta_table_cap: 160 KB tables
 #ifndef HN_TC_PAIR_ILP
 #define HN_TC_PAIR_ILP 8
@@ -519,6 +535,7 @@ __device__ __forceinline__ void tc_credit_owner(unsigned long long* counts, int 
 
 struct TcView {
     const long long* offp;   // oriented offsets
+    const int* dplus;        // oriented degrees (by rank the lists are padded)
     const int32_t* fwd;      // oriented lists
     const long long* coff;   // candidate-list offsets
     const int32_t* cand;     // candidate lists C(z)
@@ -526,7 +543,7 @@ struct TcView {
     const int32_t* feid;     // edge id of each fwd entry
     const int32_t* ceid;     // edge id of each candidate entry
     int* esup;               // per-edge triangle counts
-    int wb = INT_MAX;        // by rank: first rank of the bitmap window; by id: INT_MAX
+    bool ranked = false;     // by rank
 };
 
 // One triangle {u, v, w} found from u: credit its three edges (MODE 3).
@@ -546,11 +563,12 @@ __device__ __forceinline__ void tc_credit_edges(int* esup, int e_uv, int e_vw, i
 // lane per group).
 //
 // KIND: how membership in N+(u) is decided.  kSearch: binary search of the
-// sorted list; kHash: the hash table; kBits: one bit of the bitmap `win` of
-// the numbers [wb, wb + wn), which hold all of N+(u); kBitsHash: the bitmap
-// for w >= wb (wb + wn is past the last number), the table below it.
+// sorted list; kHash: the hash table; by rank kBits: one bit of the bitmap
+// `win` of the numbers below wn, which hold all of N+(u), with a zero word
+// behind them; kBitsHash: the bitmap below wn, the table from there on.
 enum { kSearch, kHash, kBits, kBitsHash };
-constexpr int kTcLong = 64;   // kBits: lists taken by the whole warp from this length on
+constexpr int kTcLong = 48;   // kBits: lists taken by the whole warp from this length on
+constexpr int kWinWords = kWin / 32 + 4;   // a zero word behind the bits, 16-byte multiples
 
 template <int MODE, int KIND>
 __device__ __forceinline__ unsigned long long tc_vertex_warp(
@@ -558,7 +576,7 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
     const int* tab, const unsigned* filt, const int* teid, int bits,
     int narrow_min, int* s_next, const TcView& g, int* s_pref /*33*/, long long* s_vb /*32*/,
     int* s_v /*32*/, unsigned* s_fc /*32*/, unsigned long long* __restrict__ per_vertex,
-    const unsigned* win = nullptr, int wb = 0, unsigned wn = 0) {
+    const unsigned* win = nullptr, unsigned wn = 0) {
     constexpr bool TAB = KIND == kHash || KIND == kBitsHash;
     const int lane = threadIdx.x & 31;
     const int lo_w = L[0], hi_w = L[du - 1];
@@ -578,9 +596,9 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
             v = C[idx];
             flp = v < 0;
             if (flp) v = ~v;
-            long long b0 = g.offp[v], b1 = g.offp[v + 1];
+            const long long b0 = g.offp[v];
             const int32_t* lst = g.fwd + b0;
-            int n = (int)(b1 - b0);
+            const int n = g.dplus[v];
             // [first element >= lo_w, first element > hi_w); lists of at most
             // narrow_min entries are probed whole (two dependent searches
             // cost more than the few extra filter probes)
@@ -598,34 +616,42 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
             dx = lo - s0;
         }
         if (KIND == kBits) {
-            // long lists (most of a hub's): the whole warp on one list, four
-            // rows in flight.  An entry then costs its load and one bit of
-            // shared memory; the dealt pairs below also find their candidate.
+            // long lists (nearly all entries): the whole warp on one list,
+            // four entries a lane with one 16-byte load, 256 entries a step.
+            // An entry takes about seven instructions (clamp to the zero word
+            // behind the window, word, bit, add); dealt to lanes one by one,
+            // with their candidate to be found, it took 40.
             unsigned longs = __ballot_sync(0xFFFFFFFFu, dx >= kTcLong);
             while (longs) {
                 const int l = __ffs(longs) - 1;
                 longs &= longs - 1;
-                const int32_t* q = g.fwd + __shfl_sync(0xFFFFFFFFu, xb, l);
-                const int n = __shfl_sync(0xFFFFFFFFu, dx, l);
-                const int vl = __shfl_sync(0xFFFFFFFFu, v, l);
-                const bool fl = __shfl_sync(0xFFFFFFFFu, (int)flp, l) != 0;
+                const int4* q = reinterpret_cast<const int4*>(g.fwd + __shfl_sync(0xFFFFFFFFu, xb, l));
+                const int n4 = (__shfl_sync(0xFFFFFFFFu, dx, l) + 3) >> 2;
                 unsigned h = 0;
-                for (int i = lane; i < n; i += 128) {
-                    unsigned wi[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++)   // past the end: outside the window
-                        wi[j] = i + 32 * j < n ? (unsigned)(q[i + 32 * j] - wb) : 0xFFFFFFFFu;
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if (wi[j] >= wn) continue;
-                        const unsigned hit = (win[wi[j] >> 5] >> (wi[j] & 31)) & 1u;
-                        h += hit;
-                        if (MODE == 1 && hit) atomicAdd(per_vertex + (int)wi[j] + wb, 1ull);
-                    }
+                auto test = [&](int w) {
+                    const unsigned x = min((unsigned)w, wn);
+                    const unsigned hit = __funnelshift_r(win[x >> 5], 0u, x) & 1u;
+                    h += hit;
+                    if (MODE == 1 && hit) atomicAdd(per_vertex + w, 1ull);
+                };
+                for (int i = lane; i < n4; i += 64) {
+                    const int4 a = q[i];
+                    int4 b = make_int4(kPad, kPad, kPad, kPad);
+                    if (i + 32 < n4) b = q[i + 32];
+                    test(a.x);
+                    test(a.y);
+                    test(a.z);
+                    test(a.w);
+                    test(b.x);
+                    test(b.y);
+                    test(b.z);
+                    test(b.w);
                 }
                 cnt += h;
                 if (MODE == 1 || MODE == 2) {
                     const unsigned all = __reduce_add_sync(0xFFFFFFFFu, h);
+                    const int vl = __shfl_sync(0xFFFFFFFFu, v, l);
+                    const bool fl = __shfl_sync(0xFFFFFFFFu, (int)flp, l) != 0;
                     if (lane == 0 && all) {
                         if (MODE == 1) {
                             atomicAdd(per_vertex + u, (unsigned long long)all);
@@ -709,12 +735,8 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
                     if (!FULL && w < 0) continue;
                     bool hit;
                     int e_uw = 0;   // MODE 3: edge (u, w)
-                    if (KIND == kBits) {
-                        // (a candidate's list may leave the window)
-                        const unsigned i = (unsigned)(w - wb);
-                        hit = i < wn && ((win[i >> 5] >> (i & 31)) & 1u);
-                    } else if (KIND == kBitsHash && w >= wb) {
-                        const unsigned i = (unsigned)(w - wb);
+                    if (KIND == kBits || (KIND == kBitsHash && (unsigned)w < wn)) {
+                        const unsigned i = min((unsigned)w, wn);
                         hit = (win[i >> 5] >> (i & 31)) & 1u;
                     } else if (TAB) {
                         const unsigned f = tc_fbit(w, bits);
@@ -805,7 +827,7 @@ k_tc_thread(TcView g, int nV, int small_du, int small_dc,
          x += (long long)gridDim.x * blockDim.x) {
         const int u = (int)x;
         const long long ub = g.offp[u];
-        const int du = (int)(g.offp[u + 1] - ub);
+        const int du = g.dplus[u];
         const long long cb = g.coff[u];
         const int dc = (int)(g.coff[u + 1] - cb);
         if (du == 0 || dc == 0 || du > small_du || dc > small_dc) continue;
@@ -816,7 +838,7 @@ k_tc_thread(TcView g, int nV, int small_du, int small_dc,
             const bool flp = v < 0;
             if (flp) v = ~v;
             const long long vb = g.offp[v];
-            const int dv = (int)(g.offp[v + 1] - vb);
+            const int dv = g.dplus[v];
             const int32_t* Bv = g.fwd + vb;
             unsigned hits = 0;
             for (int i = 0, j = 0; i < du && j < dv;) {
@@ -885,39 +907,14 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         if (u0 >= nV) break;
         int u1 = u0 + chunk < nV ? u0 + chunk : nV;
         for (int u = u0; u < u1; u++) {
-            long long ub = g.offp[u];
-            int du = (int)(g.offp[u + 1] - ub);
+            const long long ub = g.offp[u];
+            const int du = g.dplus[u];
             const long long cb = g.coff[u];
             const int dc = (int)(g.coff[u + 1] - cb);
             if (du == 0 || dc == 0) continue;
             if (du <= small_du && dc <= small_dc) continue;   // k_tc_thread's
-            // ids of N+(u) close enough for a bitmap in place of the table (in
-            // id order its ends are the list's; by rank, the last numbers)
-            int wb = INT_MAX;
-            unsigned wn = 0;
-            bool to_cta = false;
-            if (MODE != 3) {
-                if (g.wb != INT_MAX) {
-                    const int b = nV - kWarpWin;
-                    if (u >= b) {
-                        wb = b;
-                        wn = kWarpWin;
-                    }
-                } else {
-                    const int first = g.fwd[ub];
-                    const unsigned span = (unsigned)(g.fwd[ub + du - 1] - first) + 1;
-                    if (span <= (unsigned)kWarpWin) {
-                        wb = first;
-                        wn = span;
-                    } else {
-                        // a CTA has room for twice the bits, and is worth its
-                        // set-up from a few thousand pairs on
-                        to_cta = span <= (unsigned)kWin && (long long)dc * du > kWinWork;
-                    }
-                }
-            }
             // every probed list of u is at most du long: dc * du bounds u's pairs
-            if (du > warp_cap || (long long)dc * du > warp_work || to_cta) {
+            if (du > warp_cap || (long long)dc * du > warp_work) {
                 // listed: one work item (u, chunk) per item_cands candidates;
                 // mid items from the front of `big`, huge items from the back
                 if (lane == 0) {
@@ -934,20 +931,21 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
                 }
                 continue;
             }
-            if (MODE != 3 && wn) {
+            if (MODE != 3 && g.ranked && u < kWarpWin) {
+                // by rank, among the first numbers: a bitmap in the table's place
                 unsigned* win = (unsigned*)tab;
-                for (unsigned i = lane; i < (wn + 127) / 128; i += 32)
+                for (int i = lane; i < kWarpTab / 4; i += 32)
                     reinterpret_cast<uint4*>(win)[i] = make_uint4(0u, 0u, 0u, 0u);
                 __syncwarp();
                 for (int i = lane; i < du; i += 32) {
-                    const unsigned x = (unsigned)(g.fwd[ub + i] - wb);
+                    const int x = g.fwd[ub + i];
                     atomicOr(win + (x >> 5), 1u << (x & 31));
                 }
                 __syncwarp();
                 mine += tc_vertex_warp<MODE, kBits>(
                     u, g.fwd + ub, du, g.cand + cb, dc, nullptr, nullptr, nullptr, 0, narrow_min,
-                    nullptr, g, s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, wb,
-                    wn);
+                    nullptr, g, s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win,
+                    kWarpWin);
                 __syncwarp();
                 continue;
             }
@@ -989,10 +987,9 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
 // lists share `big` (items (u << 32) | chunk, each item_cands(d+(u))
 // candidates of u): mid from the front (counters[1] entries), huge from the
 // back (counters[2] entries).
-// WIN: an 8 KB bitmap in front of the table.  By rank it holds the members
-// among the last kWin ranks and the table those below (none for u among them;
-// no list exceeds `cap`, checked by the host); by id, all members when they
-// are less than kWin ids apart.
+// WIN (by rank): a 16 KB bitmap in front of the table holds the members among
+// the first kWin numbers, the table the others (none for u in the window; no
+// list exceeds `cap`, checked by the host).
 template <int MODE, bool WIN>
 __global__ void __launch_bounds__(kTcWarps * 32, 4)
 k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
@@ -1013,38 +1010,21 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         const long long item = huge ? big[big_cap - 1 - i] : big[i];
         const int u = (int)(item >> 32);
         const int ch = (int)(item & 0xFFFFFFFF);
-        long long ub = g.offp[u];
-        int du = (int)(g.offp[u + 1] - ub);
+        const long long ub = g.offp[u];
+        const int du = g.dplus[u];
         const int ipc = item_cands(du, item_work);
         const long long cb = g.coff[u] + (long long)ch * ipc;
         const int rest = (int)(g.coff[u + 1] - cb);
         const int dc = rest < ipc ? rest : ipc;
         unsigned* win = (unsigned*)s_dyn;                  // WIN: kWin bits
-        int* slots = s_dyn + (WIN ? kWin / 32 : 0);
+        int* slots = s_dyn + (WIN ? kWinWords : 0);
         unsigned* filt = (unsigned*)(slots + tc_table_slots(cap));
         int* teid = MODE == 3 ? (int*)(filt + tc_table_slots(cap) / 4) : nullptr;
-        int wb = INT_MAX;
-        unsigned wn = kWin;
-        bool hash = du <= cap;
-        if (WIN) {
-            if (g.wb != INT_MAX) {
-                wb = g.wb;
-                hash = u < wb;
-            } else {
-                const int first = g.fwd[ub];
-                const unsigned span = (unsigned)(g.fwd[ub + du - 1] - first) + 1;
-                if (span <= (unsigned)kWin) {
-                    wb = first;
-                    wn = span;
-                    hash = false;
-                }
-            }
-        }
-        const bool bm = wb != INT_MAX;   // uniform in the CTA
+        const bool hash = WIN ? u >= kWin : du <= cap;
         int bits = 0;
         if (threadIdx.x == 0) s_next = 0;
-        if (WIN && bm)
-            for (int j = threadIdx.x; j < (int)((wn + 127) / 128); j += blockDim.x)
+        if (WIN)
+            for (int j = threadIdx.x; j < kWinWords / 4; j += blockDim.x)
                 reinterpret_cast<uint4*>(win)[j] = make_uint4(0u, 0u, 0u, 0u);
         if (hash) {
             bits = 32 - __clz(2 * du - 1);
@@ -1052,13 +1032,12 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
             for (int j = threadIdx.x; j < (1 << bits); j += blockDim.x) slots[j] = -1;
             for (int j = threadIdx.x; j < (1 << (bits - 2)); j += blockDim.x) filt[j] = 0u;
         }
-        if ((WIN && bm) || hash) {
+        if (WIN || hash) {
             __syncthreads();
             for (int j = threadIdx.x; j < du; j += blockDim.x) {
                 const int w = g.fwd[ub + j];
-                if (WIN && w >= wb) {
-                    const unsigned i = (unsigned)(w - wb);
-                    atomicOr(win + (i >> 5), 1u << (i & 31));
+                if (WIN && w < kWin) {
+                    atomicOr(win + (w >> 5), 1u << (w & 31));
                 } else {
                     const unsigned h = tab_insert_f(slots, filt, bits, w);
                     if (MODE == 3) teid[h] = g.feid[ub + j];
@@ -1069,11 +1048,11 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         auto run = [&](auto kind) {
             return tc_vertex_warp<MODE, decltype(kind)::value>(
                 u, g.fwd + ub, du, g.cand + cb, dc, slots, filt, teid, bits, narrow_min, &s_next, g,
-                s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, wb, wn);
+                s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, kWin);
         };
         unsigned long long cu;
-        if (WIN && bm) cu = hash ? run(std::integral_constant<int, kBitsHash>())
-                                 : run(std::integral_constant<int, kBits>());
+        if (WIN) cu = hash ? run(std::integral_constant<int, kBitsHash>())
+                           : run(std::integral_constant<int, kBits>());
         else cu = hash ? run(std::integral_constant<int, kHash>())
                        : run(std::integral_constant<int, kSearch>());
         mine += cu;
@@ -1110,10 +1089,13 @@ void build_oriented(hn_graph* g, Oriented& o, const int32_t* canon) {
     HN_LAUNCH(k_orient_fill, grid, kB, 0, s, o.prefix.get(), nV, g->vtab, g->pool, pos.get(),
               o.fwd.get(), o.offp.get(), splits.get(), (long long)splits.n - 1, canon,
               canon ? o.feid.get() : (int32_t*)nullptr);
+    o.dplus.alloc((size_t)nV, s);
+    HN_LAUNCH(k_dplus, grid_for(g, nV, kB), kB, 0, s, (const long long*)o.offp.get(), nV,
+              o.dplus.get());
 }
 
 // The orientation by rank, when it pays: true and o filled.  It does when
-// most edges join vertices of more than kWin apart in id (otherwise, as in a
+// most edges join vertices of more than kLocal apart in id (otherwise, as in a
 // union of small graphs, id order keeps the lists of neighbours close in
 // memory, which ranks would scatter) and every oriented list fits the CTA
 // kernel's table (unsorted lists cannot be searched).
@@ -1151,24 +1133,29 @@ static bool build_by_rank(hn_graph* g, Oriented& o) {
     DevBuf<long long> splits;
     lb_splits(g, o.prefix.get(), nV, m, kRankTile, splits);
     DevBuf<unsigned> kept((size_t)m / 32 + 2, s);
+    o.dplus.alloc((size_t)nV, s);
     DevBuf<int> cnt((size_t)nV + 1, s);
     HN_CUDA(cudaMemsetAsync(kept.get(), 0, sizeof(unsigned) * kept.n, s));
-    HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * cnt.n, s));
+    HN_CUDA(cudaMemsetAsync(o.dplus.get(), 0, sizeof(int) * (size_t)nV, s));
     HN_LAUNCH(k_rank_orient<false>, grid, kB, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
-              (const int32_t*)rank.get(), kept.get(), cnt.get(), (const long long*)nullptr,
+              (const int32_t*)rank.get(), kept.get(), o.dplus.get(), (const long long*)nullptr,
               (int32_t*)nullptr, (const long long*)splits.get(), ntiles);
-    HN_LAUNCH(k_max_int, grid_for(g, nV, kB), kB, 0, s, (const int*)cnt.get(), nV, local + 1);
+    HN_LAUNCH(k_max_int, grid_for(g, nV, kB), kB, 0, s, (const int*)o.dplus.get(), nV, local + 1);
     HN_CUDA(cudaMemcpyAsync(g->h_scalar + 4, local, sizeof(long long), cudaMemcpyDeviceToHost, s));
     o.offp.alloc((size_t)nV + 1, s);
+    HN_LAUNCH(k_padded, grid_for(g, (long long)nV + 1, kB), kB, 0, s, (const int*)o.dplus.get(),
+              nV, cnt.get());
     exclusive_scan(g, (const int*)cnt.get(), o.offp.get(), (long long)nV + 1, s);
     HN_CUDA(cudaStreamSynchronize(s));
     if (((const int*)(g->h_scalar + 4))[1] > knob(kKnobTcCtaTableCap)) return false;
     HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * cnt.n, s));
-    o.fwd.alloc((size_t)(m + 4), s);
+    o.fwd.alloc((size_t)(m + 3ll * nV + 4), s);
     HN_LAUNCH(k_rank_orient<true>, grid, kB, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
               (const int32_t*)rank.get(), kept.get(), cnt.get(), (const long long*)o.offp.get(),
               o.fwd.get(), (const long long*)splits.get(), ntiles);
-    o.wb = nV - kWin;
+    HN_LAUNCH(k_pad_lists, grid_for(g, nV, kB), kB, 0, s, (const long long*)o.offp.get(),
+              (const int*)o.dplus.get(), nV, o.fwd.get());
+    o.ranked = true;
     return true;
 }
 
@@ -1181,7 +1168,8 @@ void build_candidates(hn_graph* g, const Oriented& o, DevBuf<long long>& coff,
                       DevBuf<int32_t>& cand, DevBuf<int32_t>* ceid) {
     cudaStream_t s = g->stream;
     const int nV = g->nV;
-    const long long m = g->nE;   // bound on the oriented edge count (read on the device)
+    // bound on the oriented entries, pads included (their number is read on the device)
+    const long long m = g->nE + (o.ranked ? 3ll * nV : 0);
     DevBuf<int> cnt((size_t)nV + 1, s);
     HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * ((size_t)nV + 1), s));
     DevBuf<long long> splits;
@@ -1189,16 +1177,14 @@ void build_candidates(hn_graph* g, const Oriented& o, DevBuf<long long>& coff,
     const long long grid = (long long)g->info.sms * 8;
     coff.alloc((size_t)nV + 1, s);
     cand.alloc((size_t)m + 4, s);
-    DevBuf<int> dplus((size_t)nV, s);
-    HN_LAUNCH(k_dplus, grid_for(g, nV, kB), kB, 0, s, (const long long*)o.offp.get(), nV, dplus.get());
-    HN_LAUNCH(k_cand<false>, grid, kB, 0, s, o.offp.get(), (const int*)dplus.get(), nV,
+    HN_LAUNCH(k_cand<false>, grid, kB, 0, s, o.offp.get(), (const int*)o.dplus.get(), nV,
               o.fwd.get(), cnt.get(),
               (const long long*)nullptr, (int32_t*)nullptr, splits.get(), (long long)splits.n - 1,
               (const int32_t*)nullptr, (int32_t*)nullptr);
     exclusive_scan(g, (const int*)cnt.get(), coff.get(), (long long)nV + 1, s);
     HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * ((size_t)nV + 1), s));
     if (ceid) ceid->alloc((size_t)m + 4, s);
-    HN_LAUNCH(k_cand<true>, grid, kB, 0, s, o.offp.get(), (const int*)dplus.get(), nV,
+    HN_LAUNCH(k_cand<true>, grid, kB, 0, s, o.offp.get(), (const int*)o.dplus.get(), nV,
               o.fwd.get(), cnt.get(),
               (const long long*)coff.get(), cand.get(), splits.get(), (long long)splits.n - 1,
               ceid ? (const int32_t*)o.feid.get() : (const int32_t*)nullptr,
@@ -1224,7 +1210,7 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     const long long gw = (long long)g->info.sms * knob(kKnobTcWarpCtasPerSm);
     const int warp_cap = (int)knob(kKnobTcWarpCap);
     const int chunk = (int)knob(kKnobTcChunk);
-    const bool by_rank = view.wb != INT_MAX;
+    constexpr bool by_rank = WIN;
     // lists by rank are not sorted: nothing to narrow
     const int narrow_min = by_rank ? INT_MAX : (int)knob(kKnobTcNarrowMin);
     // by rank, with a bitmap to set up per item and cheaper pairs: items four
@@ -1234,9 +1220,12 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     const long long item_work = knob(kKnobTcItemWork) * (by_rank && g->nE >= (1ll << 26) ? 4 : 1);
     constexpr bool eid = MODE == 3;
     const int cap_max = eid ? kCtaCapEid : kCtaCap;
-    const int mid_cap = (int)knob(kKnobTcMidCap);
+    // (by rank the bitmap holds most members: a smaller table leaves room for
+    // four CTAs an SM)
+    const int mid_cap = by_rank ? (int)std::min<long long>(knob(kKnobTcMidCap), 2048)
+                                : (int)knob(kKnobTcMidCap);
     const int cta_cap = (int)std::min<long long>(knob(kKnobTcCtaTableCap), cap_max);
-    constexpr size_t win = WIN ? kWin / 8 : 0;
+    constexpr size_t win = WIN ? kWinWords * sizeof(int) : 0;
     const size_t dyn_mid = win + tc_table_bytes(mid_cap, eid);
     const size_t dyn_huge = win + tc_table_bytes(cta_cap, eid);
     const size_t dyn_warp = eid ? (size_t)kTcWarps * kWarpTab * sizeof(int) : 0;
@@ -1286,7 +1275,8 @@ unsigned long long run_counting(hn_graph* g, const Oriented& o, int mode,
     // supports always use the lists)
     DevBuf<long long> coff;
     DevBuf<int32_t> cand, ceid;
-    TcView view{o.offp.get(), o.fwd.get(), o.offp.get(), o.fwd.get(), nullptr, nullptr, nullptr};
+    TcView view{o.offp.get(), o.dplus.get(), o.fwd.get(), o.offp.get(), o.fwd.get(), nullptr,
+                nullptr, nullptr};
     const bool flipped = mode == 3 || knob(kKnobTcFlip);
     if (flipped) {
         build_candidates(g, o, coff, cand, mode == 3 ? &ceid : nullptr);
@@ -1300,10 +1290,13 @@ unsigned long long run_counting(hn_graph* g, const Oriented& o, int mode,
     }
     if (d_counts) HN_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * g->nV, s));
     long long* bp = big.get();
-    view.wb = o.wb;
-    auto count = [&](auto m) {   // (edge supports need the table's slots)
+    view.ranked = o.ranked;
+    auto count = [&](auto m) {   // (edge supports are counted under ids)
         constexpr int M = decltype(m)::value;
-        launch_counting<M, M != 3>(g, view, d_counts, d_total, counters, bp, big_cap, flipped);
+        if (M != 3 && o.ranked)
+            launch_counting<M, M != 3>(g, view, d_counts, d_total, counters, bp, big_cap, flipped);
+        else
+            launch_counting<M, false>(g, view, d_counts, d_total, counters, bp, big_cap, flipped);
     };
     switch (mode) {
         case 0: count(std::integral_constant<int, 0>()); break;
@@ -1319,9 +1312,9 @@ unsigned long long run_counting(hn_graph* g, const Oriented& o, int mode,
 
 unsigned long long count_triangles(hn_graph* g, const Oriented& o, unsigned long long* d_counts,
                                    int mode) {
-    if (!d_counts || o.wb == INT_MAX)
+    if (!d_counts || !o.ranked)
         return run_counting(g, o, d_counts ? mode : 0, d_counts, nullptr);
-    // counted under ranks, then handed out under vertex ids
+    // counted under numbers, then handed out under vertex ids
     DevBuf<unsigned long long> by_rank((size_t)g->nV, g->stream);
     const unsigned long long t = run_counting(g, o, mode, by_rank.get(), nullptr);
     HN_LAUNCH(k_unrank, grid_for(g, g->nV, kB), kB, 0, g->stream,

@@ -1,8 +1,6 @@
 // Degree-oriented graph used by triangle counting.
 #pragma once
 
-#include <climits>
-
 #include "hn_graph.cuh"
 
 namespace hn {
@@ -12,10 +10,12 @@ struct Oriented {
     DevBuf<long long> offp;    // oriented offsets (nV+1)
     DevBuf<int32_t> fwd;       // oriented, sorted neighbour lists
     DevBuf<int32_t> feid;      // edge id of each fwd entry (when built with canon)
-    // orientation by rank (build_for_counting): offp is indexed by rank and
-    // fwd holds ranks, unsorted
-    DevBuf<int32_t> inv;       // vertex of each rank
-    int wb = INT_MAX;          // first rank of the bitmap window; INT_MAX: by id
+    DevBuf<int> dplus;         // oriented degrees (nV)
+    // orientation by rank (build_for_counting): offp and dplus are indexed by
+    // number (0 = highest rank) and fwd holds numbers, unsorted, each list on
+    // 16 bytes and padded to four entries
+    DevBuf<int32_t> inv;       // vertex of each number
+    bool ranked = false;
 };
 
 // Build N+(u) = {v in N(u) : (deg u, u) < (deg v, v)} for every vertex.

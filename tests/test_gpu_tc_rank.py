@@ -1,7 +1,8 @@
-"""Triangle counts by the rank orientation (graphs of more than 65,536
+"""Triangle counts by the rank orientation (graphs of more than 131,072
 vertices whose edges are not local in id): totals, per-vertex and owner
 counts equal the id orientation's (tc.flip = 0 never ranks) and the oracle's,
-with lists below, across and inside the bitmap window."""
+with lists inside, across and beyond the bitmap windows (32,736 numbers for a
+warp, 131,072 for a CTA)."""
 import ctypes
 
 import numpy as np
@@ -30,16 +31,16 @@ def graph(kind):
     rng = np.random.default_rng(3)
     if kind == "rmat":
         return T.rmat_graph(18, 8, seed=2)
-    if kind == "uniform":       # every list mostly below the window
+    if kind == "uniform":       # lists mostly beyond the windows
         return T.er_graph(200_001, 24, seed=4)
     if kind == "sparse_core":   # a dense core of scattered ids, lists across the window's edge
-        n = 70_000
+        n = 140_000
         core = rng.permutation(n)[:600].astype(np.int32)
-        s = [core[rng.integers(0, 600, 120_000)], rng.integers(0, n, 150_000).astype(np.int32)]
-        d = [core[rng.integers(0, 600, 120_000)], core[rng.integers(0, 600, 150_000)]]
+        s = [core[rng.integers(0, 600, 240_000)], rng.integers(0, n, 300_000).astype(np.int32)]
+        d = [core[rng.integers(0, 600, 240_000)], core[rng.integers(0, 600, 300_000)]]
         return O.build_csr_undirected(n, np.concatenate(s), np.concatenate(d))
-    return O.build_csr_undirected(65_537, rng.integers(0, 65_537, 400_000).astype(np.int32),
-                                  rng.integers(0, 65_537, 400_000).astype(np.int32))
+    return O.build_csr_undirected(131_073, rng.integers(0, 131_073, 900_000).astype(np.int32),
+                                  rng.integers(0, 131_073, 900_000).astype(np.int32))
 
 
 @pytest.mark.parametrize("kind", ["rmat", "uniform", "sparse_core", "just_over"])
@@ -69,7 +70,7 @@ def test_rank_orientation(kind):
 
 def test_lists_too_long_for_the_table_go_by_id():
     """tc.cta_table_cap below the longest oriented list: no ranking."""
-    g = T.rmat_graph(17, 16, seed=6, n_vertices=100_003)
+    g = T.rmat_graph(18, 8, seed=6, n_vertices=140_003)
     h = build(g)
     try:
         H.tune_set("tc.cta_table_cap", 64)
