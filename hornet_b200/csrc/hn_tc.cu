@@ -8,19 +8,15 @@
 // directed edges by log-degree pair with 64-bit global atomics (two passes)
 // and runs ~37 intersection launches.
 //
-// Here the orientation is built on the device from the (always sorted)
-// undirected adjacency in two merge-path balanced passes around one scan:
-//   pass 1  keep flag of every edge (needs deg(v): one 16-byte record read),
-//   scan    flag positions = the oriented CSR,
-//   pass 2  compact the kept neighbours (lists stay sorted).
-// The intersection is vertex-centric with N+(u) in a shared-memory hash
-// table (see the comment above k_tc_warp).
+// Here the orientation is built on the device in two passes over the (always
+// sorted) undirected adjacency: one decides every edge's direction and counts,
+// one writes the kept neighbours (k_orient).  The intersection is
+// vertex-centric (see the comment above k_tc_warp): N+(u) is a bitmap in shared
+// memory, or a hash table where it spans too many numbers.
 //
-// Counts of graphs whose edges are not local in vertex id (build_by_rank) use
-// another orientation: vertices are renumbered by descending rank in the
-// (degree, id) order, so that nearly all probes are among the first kWin
-// numbers, where membership in N+(u) is one bit of a 16 KB shared bitmap
-// instead of a hash lookup.
+// Counts of graphs whose edges are not local in vertex id use numbers by
+// descending rank in the (degree, id) order in place of ids, so that nearly
+// all probes are among the first kWin numbers, a 16 KB bitmap.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -135,18 +131,18 @@ k_orient_fill(const long long* __restrict__ prefix, int nV, const VRec* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Orientation by rank.  number = position in the descending (degree, id)
-// order; vertex u's oriented list is stored under number[u] and holds
-// numbers, so u -> v iff number[v] < number[u].  One random 4-byte read per
-// edge decides the direction (a vertex record is 16 bytes) and the decision
-// is kept as one bit per edge, so the fill reads numbers of kept edges only.
-// Lists are not sorted; each starts on 16 bytes and is padded to a multiple
-// of four entries with kPad.
+// Orientation for counts.  A vertex's number is its id, or (ranked) its
+// position in the descending (degree, id) order; its oriented list is stored
+// under its number and holds numbers.  One 4-byte read per edge (the other
+// end's degree or number; a vertex record is 16 bytes) decides the direction,
+// kept as one bit per edge.  Lists are in the order of ids (not sorted by
+// rank); each starts on 16 bytes and is padded to a multiple of four entries
+// with kPad.
 // ---------------------------------------------------------------------------
 constexpr int kPad = INT_MAX;
 constexpr int kWin = 1 << 17;   // numbers of the CTA kernel's bitmap (16 KB)
 constexpr int kLocal = 1 << 17;  // ids closer than this are local
-constexpr int kRankTile = 1024;
+constexpr int kOrientTile = 1024;
 
 __global__ void k_rank_keys(const VRec* __restrict__ vtab, int nV,
                             unsigned long long* __restrict__ keys) {
@@ -181,36 +177,56 @@ __global__ void k_local_sample(const long long* __restrict__ prefix, int nV, lon
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(local, __popc(b));
 }
 
+__global__ void k_degree_of(const VRec* __restrict__ vtab, int nV, int32_t* __restrict__ deg) {
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nV;
+         v += (long long)gridDim.x * blockDim.x)
+        deg[v] = vtab[v].deg;
+}
+
 // Pass 1 (FILL = false): the direction of every edge, one bit each in
-// `kept`, and the kept edges of each vertex in cnt[number].  Pass 2: every
-// window reserves its segments' kept edges (cnt is the cursor) and writes
-// their numbers.  A warp per merge-path tile, windows of 32 vertices; a row of
-// 32 edges is one word of `kept` (shared by two windows at their seam).
-template <bool FILL>
+// `kept`, the kept edges of each vertex in cnt[number], and those of each
+// tile's last vertex in that tile in last[tile].  Pass 2 writes the numbers of
+// the kept edges; a vertex that began in earlier tiles has their `last` edges
+// before it.  key: numbers (RANKED) or degrees.  A warp per merge-path tile,
+// windows of 32 vertices; a row of 32 edges is one word of `kept` (shared by
+// two windows at their seam).
+// R-MAT scale 22 (128 M edges): 1.26 ms both passes; the flags, scan and fill
+// of build_oriented 3.4 ms (148 M edges in 512 graphs: 2.9 ms).
+template <bool FILL, bool RANKED>
 __global__ void __launch_bounds__(kB)
-k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
-              const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
-              const int32_t* __restrict__ rank, unsigned* __restrict__ kept,
-              int* __restrict__ cnt, const long long* __restrict__ offp,
-              int32_t* __restrict__ fwd, const long long* __restrict__ splits,
-              long long ntiles) {
+k_orient(const long long* __restrict__ prefix, int nV, long long nE,
+         const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
+         const int32_t* __restrict__ key, unsigned* __restrict__ kept,
+         int* __restrict__ cnt, int* __restrict__ last, const long long* __restrict__ offp,
+         int32_t* __restrict__ fwd, const long long* __restrict__ splits, long long ntiles) {
     constexpr int ROWS = 4;
     const unsigned kFull = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     const long long tile = blockIdx.x * (long long)(kB / 32) + (threadIdx.x >> 5);
     if (tile >= ntiles) return;
-    const WarpTile wt = warp_tile(splits, tile, kRankTile, nE, nV);
+    const WarpTile wt = warp_tile(splits, tile, kOrientTile, nE, nV);
     if (wt.nitems == 0) return;
+    int before = 0;   // kept edges of the tile's first vertex in earlier tiles
+    if (FILL) {
+        const long long p0 = prefix[wt.seg0];
+        if (p0 < wt.item0) {
+            for (long long j = (p0 + wt.seg0) / kOrientTile + lane; j < tile; j += 32)
+                before += last[j];
+            before = __reduce_add_sync(kFull, before);
+        }
+    }
     for (long long v0 = wt.seg0; v0 <= wt.seg1; v0 += 32) {
         const long long v = v0 + lane < nV ? v0 + lane : nV;
         const long long first = prefix[v];
         const long long next = v0 + 32 <= nV ? prefix[v0 + 32] : nE;
         const long long off = v < nV ? vtab[v].off : 0;
-        const int rv = v < nV ? rank[v] : 0;
+        const int kv = v < nV && (RANKED || !FILL) ? key[v] : 0;
         const WarpWindow w = warp_window(wt, v0, first, next);
         if (w.n == 0) continue;
         const long long base = __shfl_sync(kFull, off - first, w.lane_of) + wt.item0;
-        const int ru = __shfl_sync(kFull, rv, w.lane_of);   // number of the lane's segment
+        const int ku = __shfl_sync(kFull, kv, w.lane_of);   // of the lane's segment
+        const int id = (int)(v0 + w.lane_of);
+        const int number = RANKED ? ku : id;
         // the lane's own segment [w.start, send)
         int send = __shfl_down_sync(kFull, w.start, 1);
         if (lane >= w.n - 1) send = w.end;
@@ -225,16 +241,17 @@ k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
         if (!FILL) {
             int mine = 0;
             for (int r = row0; r < w.end; r += 32 * ROWS) {
-                int x[ROWS], u[ROWS];
+                int x[ROWS], u[ROWS], du[ROWS];
 #pragma unroll
                 for (int k = 0; k < ROWS; k++) {
                     const int row = r + 32 * k, e = row + lane;
                     x[k] = -1;
-                    u[k] = 0;
+                    u[k] = du[k] = 0;
                     if (row < w.end) {   // uniform
                         const int j = warp_owner(w, row) & 31;
                         const long long b = __shfl_sync(kFull, base, j);
-                        u[k] = __shfl_sync(kFull, ru, j);
+                        du[k] = __shfl_sync(kFull, ku, j);
+                        if (!RANKED) u[k] = __shfl_sync(kFull, id, j);
                         if (e >= w.begin && e < w.end) x[k] = __ldcs(pool + b + e);
                     }
                 }
@@ -242,7 +259,11 @@ k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
                 for (int k = 0; k < ROWS; k++) {
                     const int row = r + 32 * k;
                     if (row >= w.end) break;   // uniform
-                    const bool keep = x[k] >= 0 && rank[x[k]] < u[k];
+                    bool keep = false;
+                    if (x[k] >= 0) {
+                        const int kx = key[x[k]];
+                        keep = RANKED ? kx < du[k] : oriented_before(du[k], u[k], kx, x[k]);
+                    }
                     const unsigned b = __ballot_sync(kFull, keep);
                     mine += __popc(b & own(row));
                     if (lane == 0 && b) {
@@ -252,15 +273,12 @@ k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
                     }
                 }
             }
-            if (lane < w.n && mine) atomicAdd(cnt + ru, mine);
+            if (lane < w.n && mine) atomicAdd(cnt + number, mine);
+            if (lane < w.n && id == wt.seg1) last[tile] = mine;
         } else {
-            int mine = 0;
-            for (int row = row0; row < w.end; row += 32) {
-                const unsigned b = kept[(wt.item0 + row) >> 5];
-                mine += __popc(b & own(row));
-            }
             // the next slot of the lane's segment
-            long long at = lane < w.n && mine ? offp[ru] + atomicAdd(cnt + ru, mine) : 0;
+            long long at = 0;
+            if (lane < w.n) at = offp[number] + (id == wt.seg0 ? before : 0);
             for (int r = row0; r < w.end; r += 32 * ROWS) {
                 int x[ROWS];
                 long long to[ROWS];
@@ -284,7 +302,7 @@ k_rank_orient(const long long* __restrict__ prefix, int nV, long long nE,
                 }
 #pragma unroll
                 for (int k = 0; k < ROWS; k++)
-                    if (x[k] >= 0) fwd[to[k]] = rank[x[k]];
+                    if (x[k] >= 0) fwd[to[k]] = RANKED ? key[x[k]] : x[k];
             }
         }
     }
@@ -413,16 +431,25 @@ k_cand(const long long* __restrict__ offp, const int* __restrict__ dplus, int nV
 }
 
 // ---------------------------------------------------------------------------
-// Vertex-centric counting.  For each vertex u, N+(u) goes into an
-// open-addressing hash table in shared memory (multiplicative hash, linear
-// probing, load factor <= 1/2, so every probe sequence ends at an empty
-// slot).  Every oriented edge (u,v) is counted by its tail u: the elements
-// of N+(v) are probed against table(u), after N+(v) is narrowed to
-// [min N+(u), max N+(u)] by two binary searches.  The (v, w) pairs of 32
-// candidates v at a time are dealt to the lanes round-robin (lane l takes
-// pairs l, l+32, ...), so a warp's loads of w read consecutive words of the
-// same list; each lane advances its candidate monotonically (no per-pair
-// search).
+// Vertex-centric counting.  Every edge (u, v) of u's candidate list asks which
+// w of N+(v) are in N+(u), held in shared memory in one of two forms:
+//   a bitmap over the numbers that N+(u) spans (from wb on, wn bits and a zero
+//   bit behind them, to which every other number is clamped): lists N+(v) of
+//   kTcLong entries or more are read by the whole warp, four entries a lane
+//   with one 16-byte load; the 16-byte quads of the shorter lists of 32
+//   candidates are dealt to the lanes round-robin.  An entry takes about seven
+//   instructions, and a quad of a short list ten more;
+//   an open-addressing hash table (multiplicative hash, linear probing, load
+//   factor <= 1/2, so every probe sequence ends at an empty slot) where the
+//   span is too wide, or for edge supports: N+(v) is narrowed to
+//   [min N+(u), max N+(u)] by two binary searches (lists sorted by number),
+//   and the (v, w) pairs of 32 candidates at a time are dealt to the lanes,
+//   about 40 instructions each.
+// R-MAT scale 22, 11.8 G pairs, both kernels: 36.5 ms by tables alone, 24.0
+// with a bitmap and pairs dealt to the lanes, 14.5 this way.  512 graphs (74 M
+// oriented edges), owner counts: 13.4 ms by tables, 6.6 this way.  What bounds
+// it: the shared-memory reads of the bits (random words: about 3.5 wavefronts a
+// warp) beside 47 GB of list reads, mostly from L2.
 //   k_tc_warp: one warp per vertex with d+(u) <= warp_cap (the tc.warp_cap
 //              knob, at most kWarpCap, the table's capacity); vertices handed
 //              out in chunks by an atomic counter; larger ones are listed;
@@ -433,8 +460,17 @@ k_cand(const long long* __restrict__ offp, const int* __restrict__ dplus, int nV
 constexpr int kTcWarps = 8;
 constexpr int kWarpCap = 512;
 constexpr int kWarpTab = 2 * kWarpCap;
-constexpr int kWarpWin = (kWarpTab - 1) * 32;   // numbers of a warp's bitmap: its table's place,
-                                                // the last word zero
+// Bits of a warp's bitmap, the zero one included: 8 KB a warp, three CTAs an
+// SM.  512 graphs of up to 65,536 vertices: k_tc_warp 9.4 ms with 32,768 bits
+// and four CTAs (half of the lists span more ids and are probed by table), 5.1
+// ms this way; R-MAT scale 22: 4.7 and 4.6 ms.
+constexpr unsigned kWarpBits = 65536;
+// Words of shared memory per warp: the table and its filter, in whose place
+// the bitmap goes, and for edge supports the edge id (u, w) of each slot.
+constexpr int tc_warp_words(bool win, bool eid) {
+    const int tab = kWarpTab + kWarpTab / 4 + (eid ? kWarpTab : 0);
+    return win && (int)(kWarpBits / 32) > tab ? (int)(kWarpBits / 32) : tab;
+}
 constexpr int kCtaCap = 16384;   // largest tc.cta_table_cap: 160 KB tables
 #ifndef HN_TC_PAIR_ILP
 #define HN_TC_PAIR_ILP 8
@@ -543,7 +579,6 @@ struct TcView {
     const int32_t* feid;     // edge id of each fwd entry
     const int32_t* ceid;     // edge id of each candidate entry
     int* esup;               // per-edge triangle counts
-    bool ranked = false;     // by rank
 };
 
 // One triangle {u, v, w} found from u: credit its three edges (MODE 3).
@@ -563,12 +598,24 @@ __device__ __forceinline__ void tc_credit_edges(int* esup, int e_uv, int e_vw, i
 // lane per group).
 //
 // KIND: how membership in N+(u) is decided.  kSearch: binary search of the
-// sorted list; kHash: the hash table; by rank kBits: one bit of the bitmap
-// `win` of the numbers below wn, which hold all of N+(u), with a zero word
-// behind them; kBitsHash: the bitmap below wn, the table from there on.
+// sorted list; kHash: the hash table; kBits: one bit of the bitmap `win` of
+// the wn numbers from wb on, which hold all of N+(u), with a zero bit behind
+// them; kBitsHash: the bitmap for those numbers, the table for the others.
 enum { kSearch, kHash, kBits, kBitsHash };
-constexpr int kTcLong = 48;   // kBits: lists taken by the whole warp from this length on
+constexpr int kTcLong = 128;
+constexpr int kQuads = 4;   // kBits: lists read by the whole warp from this length on
 constexpr int kWinWords = kWin / 32 + 4;   // a zero word behind the bits, 16-byte multiples
+
+// Clears the words of a bitmap of wn bits and the zero bit behind them.
+__device__ __forceinline__ void clear_bits(unsigned* win, unsigned wn, int first, int step) {
+    const int quads = (int)(wn >> 7) + 1;
+    for (int j = first; j < quads; j += step)
+        reinterpret_cast<uint4*>(win)[j] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Kernels' WIN: no bitmaps (lists neither aligned nor padded); bitmaps of the
+// first numbers, ranked; bitmaps of the ids that N+(u) spans.
+enum { kNoWin, kRankWin, kIdWin };
 
 template <int MODE, int KIND>
 __device__ __forceinline__ unsigned long long tc_vertex_warp(
@@ -576,10 +623,10 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
     const int* tab, const unsigned* filt, const int* teid, int bits,
     int narrow_min, int* s_next, const TcView& g, int* s_pref /*33*/, long long* s_vb /*32*/,
     int* s_v /*32*/, unsigned* s_fc /*32*/, unsigned long long* __restrict__ per_vertex,
-    const unsigned* win = nullptr, unsigned wn = 0) {
+    const unsigned* win = nullptr, int wb = 0, unsigned wn = 0) {
     constexpr bool TAB = KIND == kHash || KIND == kBitsHash;
     const int lane = threadIdx.x & 31;
-    const int lo_w = L[0], hi_w = L[du - 1];
+    const int lo_w = KIND == kBits ? 0 : L[0], hi_w = KIND == kBits ? 0 : L[du - 1];
     unsigned long long cnt = 0, cnt_u = 0;   // all hits; MODE 2: hits owned by u
     auto claim = [&](int c) {
         if (!s_next) return c + 32;
@@ -616,36 +663,39 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
             dx = lo - s0;
         }
         if (KIND == kBits) {
-            // long lists (nearly all entries): the whole warp on one list,
-            // four entries a lane with one 16-byte load, 256 entries a step.
-            // An entry takes about seven instructions (clamp to the zero word
-            // behind the window, word, bit, add); dealt to lanes one by one,
-            // with their candidate to be found, it took 40.
+            unsigned h = 0;
+            auto test1 = [&](int w) {
+                const unsigned x = min((unsigned)(w - wb), wn);
+                const unsigned hit = __funnelshift_r(win[x >> 5], 0u, x) & 1u;
+                h += hit;
+                if (MODE == 1 && hit) atomicAdd(per_vertex + w, 1ull);
+            };
+            auto test = [&](const int4& q) {
+                test1(q.x);
+                test1(q.y);
+                test1(q.z);
+                test1(q.w);
+            };
+            const int4 none = make_int4(kPad, kPad, kPad, kPad);
+            const int n4 = (dx + 3) >> 2;
+            // long lists: the whole warp on one, two loads in flight
             unsigned longs = __ballot_sync(0xFFFFFFFFu, dx >= kTcLong);
             while (longs) {
                 const int l = __ffs(longs) - 1;
                 longs &= longs - 1;
                 const int4* q = reinterpret_cast<const int4*>(g.fwd + __shfl_sync(0xFFFFFFFFu, xb, l));
-                const int n4 = (__shfl_sync(0xFFFFFFFFu, dx, l) + 3) >> 2;
-                unsigned h = 0;
-                auto test = [&](int w) {
-                    const unsigned x = min((unsigned)w, wn);
-                    const unsigned hit = __funnelshift_r(win[x >> 5], 0u, x) & 1u;
-                    h += hit;
-                    if (MODE == 1 && hit) atomicAdd(per_vertex + w, 1ull);
-                };
-                for (int i = lane; i < n4; i += 64) {
-                    const int4 a = q[i];
-                    int4 b = make_int4(kPad, kPad, kPad, kPad);
-                    if (i + 32 < n4) b = q[i + 32];
-                    test(a.x);
-                    test(a.y);
-                    test(a.z);
-                    test(a.w);
-                    test(b.x);
-                    test(b.y);
-                    test(b.z);
-                    test(b.w);
+                const int n = __shfl_sync(0xFFFFFFFFu, n4, l);
+                h = 0;
+                for (int i0 = 0; i0 < n; i0 += 64) {
+                    const int i = i0 + lane;
+                    const int4 a = i < n ? q[i] : none;
+                    if (i0 + 32 < n) {
+                        const int4 b = i + 32 < n ? q[i + 32] : none;
+                        test(a);
+                        test(b);
+                    } else {
+                        test(a);
+                    }
                 }
                 cnt += h;
                 if (MODE == 1 || MODE == 2) {
@@ -664,7 +714,81 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
                     }
                 }
             }
-            if (dx >= kTcLong) dx = 0;
+            // the others: their 16-byte quads dealt to the lanes round-robin,
+            // kQuads in flight a lane
+            const int m4 = dx >= kTcLong ? 0 : n4;
+            int incl = m4;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            s_pref[lane + 1] = incl;
+            if (lane == 0) s_pref[0] = 0;
+            s_vb[lane] = xb;
+            if (MODE == 1) s_v[lane] = v;
+            if (MODE == 2) {   // the owner of v's triangles: v (flipped), or u
+                s_v[lane] = idx < dc && flp ? v : -1;
+                s_fc[lane] = 0;
+            }
+            __syncwarp();
+            const int T = s_pref[32];
+            if (lane < T) {
+                int a = 0, b = 32;   // candidate slot of quad `lane`
+                while (b - a > 1) {
+                    const int mid = (a + b) >> 1;
+                    if (s_pref[mid] <= lane) a = mid; else b = mid;
+                }
+                int end = s_pref[a + 1];
+                // quad k of the group: base[k]
+                const int4* base = reinterpret_cast<const int4*>(g.fwd + s_vb[a]) - s_pref[a];
+                for (int k0 = lane; k0 < T; k0 += 32 * kQuads) {
+                    int4 q[kQuads];
+                    int va[kQuads];
+#pragma unroll
+                    for (int j = 0; j < kQuads; j++) {
+                        const int k = k0 + 32 * j;
+                        q[j] = none;
+                        va[j] = a;
+                        if (k < T) {
+                            if (k >= end) {   // the candidate holding quad k
+                                a++;
+                                if (s_pref[a + 1] <= k) {
+                                    int hi = 32;
+                                    while (hi - a > 1) {
+                                        const int mid = (a + hi) >> 1;
+                                        if (s_pref[mid] <= k) a = mid; else hi = mid;
+                                    }
+                                }
+                                end = s_pref[a + 1];
+                                base = reinterpret_cast<const int4*>(g.fwd + s_vb[a]) - s_pref[a];
+                            }
+                            q[j] = base[k];
+                            va[j] = a;
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kQuads; j++) {
+                        h = 0;
+                        test(q[j]);
+                        cnt += h;
+                        if (MODE == 1 && h) {
+                            atomicAdd(per_vertex + u, (unsigned long long)h);
+                            atomicAdd(per_vertex + s_v[va[j]], (unsigned long long)h);
+                        }
+                        if (MODE == 2 && h) {
+                            if (s_v[va[j]] >= 0) atomicAdd(s_fc + va[j], h);
+                            else cnt_u += h;
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            if (MODE == 2) {   // flipped candidates own their triangles
+                if (s_v[lane] >= 0 && s_fc[lane])
+                    atomicAdd(per_vertex + s_v[lane], (unsigned long long)s_fc[lane]);
+                __syncwarp();
+            }
+            continue;
         }
         int incl = dx;
         for (int o = 1; o < 32; o <<= 1) {
@@ -735,8 +859,8 @@ __device__ __forceinline__ unsigned long long tc_vertex_warp(
                     if (!FULL && w < 0) continue;
                     bool hit;
                     int e_uw = 0;   // MODE 3: edge (u, w)
-                    if (KIND == kBits || (KIND == kBitsHash && (unsigned)w < wn)) {
-                        const unsigned i = min((unsigned)w, wn);
+                    if (KIND == kBitsHash && (unsigned)(w - wb) < wn) {
+                        const unsigned i = (unsigned)(w - wb);
                         hit = (win[i >> 5] >> (i & 31)) & 1u;
                     } else if (TAB) {
                         const unsigned f = tc_fbit(w, bits);
@@ -880,25 +1004,22 @@ k_tc_thread(TcView g, int nV, int small_du, int small_dc,
 
 // Five CTAs per SM for the plain count (48 registers, no spills); the
 // modes that credit vertices or edges carry more state and get 64.
-template <int MODE>
-__global__ void __launch_bounds__(kTcWarps * 32, MODE == 0 ? 5 : 4)
+template <int MODE, int WIN>
+__global__ void __launch_bounds__(kTcWarps * 32, WIN != kNoWin ? 3 : MODE == 0 ? 5 : 4)
 k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
           unsigned long long* __restrict__ total_out,
           int* __restrict__ counters /*[0] next vertex, [1] mid, [2] huge list size*/,
           long long* __restrict__ big, long long big_cap, int warp_cap, int mid_cap,
           long long warp_work, long long item_work, int chunk, int narrow_min, int small_du,
           int small_dc) {
-    __shared__ __align__(16) int s_tab[kTcWarps][kWarpTab];
-    __shared__ unsigned s_filt[kTcWarps][kWarpTab / 4];
-    // MODE 3: edge id (u, w) of each table slot, kWarpTab per warp (dynamic)
-    extern __shared__ int s_teid[];
+    extern __shared__ __align__(16) int s_dyn[];   // tc_warp_words per warp
     __shared__ int s_pref[kTcWarps][33];
     __shared__ long long s_vb[kTcWarps][32];
     __shared__ int s_v[kTcWarps][32];
     __shared__ unsigned s_fc[kTcWarps][32];   // MODE 2: hits owned by each candidate
     __shared__ unsigned long long s_sum[kTcWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int* tab = s_tab[warp];
+    int* tab = s_dyn + warp * tc_warp_words(WIN != kNoWin, MODE == 3);
     unsigned long long mine = 0;
     while (true) {
         int u0 = 0;
@@ -931,31 +1052,38 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
                 }
                 continue;
             }
-            if (MODE != 3 && g.ranked && u < kWarpWin) {
-                // by rank, among the first numbers: a bitmap in the table's place
+            // the numbers that a bitmap in the table's place would hold
+            int wb = 0;
+            unsigned wn = 0;
+            if (WIN == kRankWin) {
+                wn = (unsigned)u;
+            } else if (WIN == kIdWin) {
+                wb = g.fwd[ub];
+                wn = (unsigned)(g.fwd[ub + du - 1] - wb) + 1u;
+            }
+            if (WIN != kNoWin && wn < kWarpBits) {
                 unsigned* win = (unsigned*)tab;
-                for (int i = lane; i < kWarpTab / 4; i += 32)
-                    reinterpret_cast<uint4*>(win)[i] = make_uint4(0u, 0u, 0u, 0u);
+                clear_bits(win, wn, lane, 32);
                 __syncwarp();
                 for (int i = lane; i < du; i += 32) {
-                    const int x = g.fwd[ub + i];
+                    const int x = g.fwd[ub + i] - wb;
                     atomicOr(win + (x >> 5), 1u << (x & 31));
                 }
                 __syncwarp();
                 mine += tc_vertex_warp<MODE, kBits>(
                     u, g.fwd + ub, du, g.cand + cb, dc, nullptr, nullptr, nullptr, 0, narrow_min,
                     nullptr, g, s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win,
-                    kWarpWin);
+                    wb, wn);
                 __syncwarp();
                 continue;
             }
             int bits = 32 - __clz(2 * du - 1);   // table of 2^bits >= 2*du slots
             if (bits < 5) bits = 5;
-            unsigned* filt = s_filt[warp];
+            unsigned* filt = (unsigned*)(tab + kWarpTab);
             for (int i = lane; i < (1 << bits); i += 32) tab[i] = -1;
             for (int i = lane; i < (1 << (bits - 2)); i += 32) filt[i] = 0u;
             __syncwarp();
-            int* teid = MODE == 3 ? s_teid + warp * kWarpTab : nullptr;
+            int* teid = MODE == 3 ? tab + kWarpTab + kWarpTab / 4 : nullptr;
             for (int i = lane; i < du; i += 32) {
                 const unsigned h = tab_insert_f(tab, filt, bits, g.fwd[ub + i]);
                 if (MODE == 3) teid[h] = g.feid[ub + i];
@@ -987,10 +1115,11 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
 // lists share `big` (items (u << 32) | chunk, each item_cands(d+(u))
 // candidates of u): mid from the front (counters[1] entries), huge from the
 // back (counters[2] entries).
-// WIN (by rank): a 16 KB bitmap in front of the table holds the members among
-// the first kWin numbers, the table the others (none for u in the window; no
-// list exceeds `cap`, checked by the host).
-template <int MODE, bool WIN>
+// WIN: a 16 KB bitmap in front of the table.  Ranked it holds the members among
+// the first kWin numbers, the table the others (none for u <= kWin); under ids
+// all of an N+(u) that spans at most kWin, else the table does.  No list
+// exceeds `cap` (checked by the host).
+template <int MODE, int WIN>
 __global__ void __launch_bounds__(kTcWarps * 32, 4)
 k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
          unsigned long long* __restrict__ total_out, const int* __restrict__ counters,
@@ -1017,27 +1146,36 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         const int rest = (int)(g.coff[u + 1] - cb);
         const int dc = rest < ipc ? rest : ipc;
         unsigned* win = (unsigned*)s_dyn;                  // WIN: kWin bits
-        int* slots = s_dyn + (WIN ? kWinWords : 0);
+        int* slots = s_dyn + (WIN != kNoWin ? kWinWords : 0);
         unsigned* filt = (unsigned*)(slots + tc_table_slots(cap));
         int* teid = MODE == 3 ? (int*)(filt + tc_table_slots(cap) / 4) : nullptr;
-        const bool hash = WIN ? u >= kWin : du <= cap;
+        int wb = 0;
+        unsigned wn = 0;
+        bool hash = du <= cap;
+        if (WIN == kRankWin) {
+            wn = (unsigned)min(u, kWin);
+            hash = u > kWin;
+        } else if (WIN == kIdWin) {
+            wb = g.fwd[ub];
+            wn = (unsigned)(g.fwd[ub + du - 1] - wb) + 1u;
+            hash = wn > kWin;
+        }
         int bits = 0;
         if (threadIdx.x == 0) s_next = 0;
-        if (WIN)
-            for (int j = threadIdx.x; j < kWinWords / 4; j += blockDim.x)
-                reinterpret_cast<uint4*>(win)[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (WIN == kRankWin || (WIN == kIdWin && !hash)) clear_bits(win, wn, threadIdx.x, blockDim.x);
         if (hash) {
             bits = 32 - __clz(2 * du - 1);
             if (bits < 5) bits = 5;
             for (int j = threadIdx.x; j < (1 << bits); j += blockDim.x) slots[j] = -1;
             for (int j = threadIdx.x; j < (1 << (bits - 2)); j += blockDim.x) filt[j] = 0u;
         }
-        if (WIN || hash) {
+        if (WIN != kNoWin || hash) {
             __syncthreads();
             for (int j = threadIdx.x; j < du; j += blockDim.x) {
                 const int w = g.fwd[ub + j];
-                if (WIN && w < kWin) {
-                    atomicOr(win + (w >> 5), 1u << (w & 31));
+                if (WIN == kRankWin ? w < kWin : WIN == kIdWin && !hash) {
+                    const int x = w - wb;
+                    atomicOr(win + (x >> 5), 1u << (x & 31));
                 } else {
                     const unsigned h = tab_insert_f(slots, filt, bits, w);
                     if (MODE == 3) teid[h] = g.feid[ub + j];
@@ -1048,13 +1186,18 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         auto run = [&](auto kind) {
             return tc_vertex_warp<MODE, decltype(kind)::value>(
                 u, g.fwd + ub, du, g.cand + cb, dc, slots, filt, teid, bits, narrow_min, &s_next, g,
-                s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, kWin);
+                s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, wb, wn);
         };
         unsigned long long cu;
-        if (WIN) cu = hash ? run(std::integral_constant<int, kBitsHash>())
-                           : run(std::integral_constant<int, kBits>());
-        else cu = hash ? run(std::integral_constant<int, kHash>())
-                       : run(std::integral_constant<int, kSearch>());
+        if (WIN == kRankWin)
+            cu = hash ? run(std::integral_constant<int, kBitsHash>())
+                      : run(std::integral_constant<int, kBits>());
+        else if (WIN == kIdWin)
+            cu = hash ? run(std::integral_constant<int, kHash>())
+                      : run(std::integral_constant<int, kBits>());
+        else
+            cu = hash ? run(std::integral_constant<int, kHash>())
+                      : run(std::integral_constant<int, kSearch>());
         mine += cu;
         __syncthreads();
     }
@@ -1094,30 +1237,33 @@ void build_oriented(hn_graph* g, Oriented& o, const int32_t* canon) {
               o.dplus.get());
 }
 
-// The orientation by rank, when it pays: true and o filled.  It does when
-// most edges join vertices of more than kLocal apart in id (otherwise, as in a
-// union of small graphs, id order keeps the lists of neighbours close in
-// memory, which ranks would scatter) and every oriented list fits the CTA
-// kernel's table (unsorted lists cannot be searched).
-static bool build_by_rank(hn_graph* g, Oriented& o) {
+// The orientation for bitmaps: true and o filled, or false where build_oriented
+// has to do: tc.flip = 0, numbers too close to kPad, a list too long for the
+// CTA kernel's table (by rank it could not be searched).  Ranked when most
+// edges join vertices of more than kLocal apart in id; otherwise, as in a
+// union of small graphs, ids keep the lists of neighbours close in memory,
+// which ranks would scatter, and lists span few of them.
+static bool build_padded(hn_graph* g, Oriented& o) {
     cudaStream_t s = g->stream;
     const int nV = g->nV;
     const long long m = g->nE;
-    if (m == 0 || m > 0x7FFFFFFFll || nV <= kWin || !knob(kKnobTcFlip)) return false;
+    if (m == 0 || m > 0x7FFFFFFFll || nV > kPad - 2 * kWin || !knob(kKnobTcFlip)) return false;
     o.prefix.alloc((size_t)nV + 1, s);
     degree_prefix(g, nullptr, nV, o.prefix.get());
-    constexpr int kSamples = 16384;
     int* local = (int*)(g->d_scalar + 4);   // [0] local samples, [1] longest oriented list
     HN_CUDA(cudaMemsetAsync(local, 0, 2 * sizeof(int), s));
-    HN_LAUNCH(k_local_sample, kSamples / 256, 256, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
-              kSamples, local);
-    HN_CUDA(cudaMemcpyAsync(g->h_scalar + 4, local, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    HN_CUDA(cudaStreamSynchronize(s));
-    if (2 * *(const int*)(g->h_scalar + 4) > kSamples) return false;
-    // ranks: vertices sorted by degree, stably (so by id among equals)
-    DevBuf<int32_t> rank((size_t)nV, s);
-    o.inv.alloc((size_t)nV, s);
-    {
+    bool ranked = false;
+    if (nV > kLocal) {
+        constexpr int kSamples = 16384;
+        HN_LAUNCH(k_local_sample, kSamples / 256, 256, 0, s, o.prefix.get(), nV, m, g->vtab,
+                  g->pool, kSamples, local);
+        HN_CUDA(cudaMemcpyAsync(g->h_scalar + 4, local, sizeof(long long), cudaMemcpyDeviceToHost, s));
+        HN_CUDA(cudaStreamSynchronize(s));
+        ranked = 2 * *(const int*)(g->h_scalar + 4) <= kSamples;
+    }
+    DevBuf<int32_t> key((size_t)nV, s);   // numbers, or degrees
+    if (ranked) {   // vertices sorted by degree, stably (so by id among equals)
+        o.inv.alloc((size_t)nV, s);
         DevBuf<unsigned long long> k1((size_t)nV, s), k2((size_t)nV, s);
         HN_LAUNCH(k_rank_keys, grid_for(g, nV, kB), kB, 0, s, g->vtab, nV, k1.get());
         unsigned long long *kc = k1.get(), *ka = k2.get();
@@ -1126,20 +1272,33 @@ static bool build_by_rank(hn_graph* g, Oriented& o) {
         radix_sort_u64(g, kc, ka, v1, v2, nV, 32, &g->alloc->error, s);
         check_device_error(g);   // unsorted keys are no permutation
         HN_LAUNCH(k_rank_of, grid_for(g, nV, kB), kB, 0, s, (const unsigned long long*)kc, nV,
-                  rank.get(), o.inv.get());
+                  key.get(), o.inv.get());
+    } else {
+        HN_LAUNCH(k_degree_of, grid_for(g, nV, kB), kB, 0, s, g->vtab, nV, key.get());
     }
-    const long long ntiles = (m + nV + kRankTile - 1) / kRankTile;
+    const long long ntiles = (m + nV + kOrientTile - 1) / kOrientTile;
     const long long grid = (ntiles + kB / 32 - 1) / (kB / 32);
     DevBuf<long long> splits;
-    lb_splits(g, o.prefix.get(), nV, m, kRankTile, splits);
+    lb_splits(g, o.prefix.get(), nV, m, kOrientTile, splits);
     DevBuf<unsigned> kept((size_t)m / 32 + 2, s);
+    DevBuf<int> last((size_t)ntiles, s);
     o.dplus.alloc((size_t)nV, s);
     DevBuf<int> cnt((size_t)nV + 1, s);
     HN_CUDA(cudaMemsetAsync(kept.get(), 0, sizeof(unsigned) * kept.n, s));
+    HN_CUDA(cudaMemsetAsync(last.get(), 0, sizeof(int) * last.n, s));
     HN_CUDA(cudaMemsetAsync(o.dplus.get(), 0, sizeof(int) * (size_t)nV, s));
-    HN_LAUNCH(k_rank_orient<false>, grid, kB, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
-              (const int32_t*)rank.get(), kept.get(), o.dplus.get(), (const long long*)nullptr,
-              (int32_t*)nullptr, (const long long*)splits.get(), ntiles);
+    auto orient = [&](auto fill) {
+        auto launch = [&](auto by_rank) {
+            constexpr bool FILL = decltype(fill)::value, RANKED = decltype(by_rank)::value;
+            HN_LAUNCH((k_orient<FILL, RANKED>), grid, kB, 0, s, (const long long*)o.prefix.get(), nV,
+                      m, (const VRec*)g->vtab, (const int32_t*)g->pool, (const int32_t*)key.get(),
+                      kept.get(), o.dplus.get(), last.get(), (const long long*)o.offp.get(),
+                      o.fwd.get(), (const long long*)splits.get(), ntiles);
+        };
+        if (ranked) launch(std::true_type());
+        else launch(std::false_type());
+    };
+    orient(std::false_type());
     HN_LAUNCH(k_max_int, grid_for(g, nV, kB), kB, 0, s, (const int*)o.dplus.get(), nV, local + 1);
     HN_CUDA(cudaMemcpyAsync(g->h_scalar + 4, local, sizeof(long long), cudaMemcpyDeviceToHost, s));
     o.offp.alloc((size_t)nV + 1, s);
@@ -1148,19 +1307,17 @@ static bool build_by_rank(hn_graph* g, Oriented& o) {
     exclusive_scan(g, (const int*)cnt.get(), o.offp.get(), (long long)nV + 1, s);
     HN_CUDA(cudaStreamSynchronize(s));
     if (((const int*)(g->h_scalar + 4))[1] > knob(kKnobTcCtaTableCap)) return false;
-    HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * cnt.n, s));
     o.fwd.alloc((size_t)(m + 3ll * nV + 4), s);
-    HN_LAUNCH(k_rank_orient<true>, grid, kB, 0, s, o.prefix.get(), nV, m, g->vtab, g->pool,
-              (const int32_t*)rank.get(), kept.get(), cnt.get(), (const long long*)o.offp.get(),
-              o.fwd.get(), (const long long*)splits.get(), ntiles);
+    orient(std::true_type());
     HN_LAUNCH(k_pad_lists, grid_for(g, nV, kB), kB, 0, s, (const long long*)o.offp.get(),
               (const int*)o.dplus.get(), nV, o.fwd.get());
-    o.ranked = true;
+    o.padded = true;
+    o.ranked = ranked;
     return true;
 }
 
 void build_for_counting(hn_graph* g, Oriented& o) {
-    if (!build_by_rank(g, o)) build_oriented(g, o);
+    if (!build_padded(g, o)) build_oriented(g, o);
 }
 
 // C(z) for every vertex z: offsets coff (nV+1) and lists cand.
@@ -1169,7 +1326,7 @@ void build_candidates(hn_graph* g, const Oriented& o, DevBuf<long long>& coff,
     cudaStream_t s = g->stream;
     const int nV = g->nV;
     // bound on the oriented entries, pads included (their number is read on the device)
-    const long long m = g->nE + (o.ranked ? 3ll * nV : 0);
+    const long long m = g->nE + (o.padded ? 3ll * nV : 0);
     DevBuf<int> cnt((size_t)nV + 1, s);
     HN_CUDA(cudaMemsetAsync(cnt.get(), 0, sizeof(int) * ((size_t)nV + 1), s));
     DevBuf<long long> splits;
@@ -1202,7 +1359,7 @@ constexpr size_t tc_table_bytes(int cap, bool eid = false) {
 }
 constexpr int kCtaCapEid = 8192;   // largest table with edge ids (147 KB)
 
-template <int MODE, bool WIN>
+template <int MODE, int WIN>
 void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_counts,
                      unsigned long long* d_total, int* counters, long long* big,
                      long long big_cap, bool flipped) {
@@ -1210,7 +1367,7 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     const long long gw = (long long)g->info.sms * knob(kKnobTcWarpCtasPerSm);
     const int warp_cap = (int)knob(kKnobTcWarpCap);
     const int chunk = (int)knob(kKnobTcChunk);
-    constexpr bool by_rank = WIN;
+    constexpr bool by_rank = WIN == kRankWin;
     // lists by rank are not sorted: nothing to narrow
     const int narrow_min = by_rank ? INT_MAX : (int)knob(kKnobTcNarrowMin);
     // by rank, with a bitmap to set up per item and cheaper pairs: items four
@@ -1220,19 +1377,19 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     const long long item_work = knob(kKnobTcItemWork) * (by_rank && g->nE >= (1ll << 26) ? 4 : 1);
     constexpr bool eid = MODE == 3;
     const int cap_max = eid ? kCtaCapEid : kCtaCap;
-    // (by rank the bitmap holds most members: a smaller table leaves room for
-    // four CTAs an SM)
-    const int mid_cap = by_rank ? (int)std::min<long long>(knob(kKnobTcMidCap), 2048)
+    // (the bitmap holds most members: a smaller table leaves room for four CTAs
+    // an SM)
+    const int mid_cap = WIN != kNoWin ? (int)std::min<long long>(knob(kKnobTcMidCap), 2048)
                                 : (int)knob(kKnobTcMidCap);
     const int cta_cap = (int)std::min<long long>(knob(kKnobTcCtaTableCap), cap_max);
-    constexpr size_t win = WIN ? kWinWords * sizeof(int) : 0;
+    constexpr size_t win = WIN != kNoWin ? kWinWords * sizeof(int) : 0;
     const size_t dyn_mid = win + tc_table_bytes(mid_cap, eid);
     const size_t dyn_huge = win + tc_table_bytes(cta_cap, eid);
-    const size_t dyn_warp = eid ? (size_t)kTcWarps * kWarpTab * sizeof(int) : 0;
+    constexpr size_t dyn_warp = sizeof(int) * kTcWarps * tc_warp_words(WIN != kNoWin, eid);
     // (set per call: the attributes belong to the device in use)
     HN_CUDA(cudaFuncSetAttribute(k_tc_cta<MODE, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(win + tc_table_bytes(cap_max, eid))));
-    HN_CUDA(cudaFuncSetAttribute(k_tc_warp<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HN_CUDA(cudaFuncSetAttribute((k_tc_warp<MODE, WIN>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dyn_warp));
     int mid_per_sm = 0;
     HN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mid_per_sm, k_tc_cta<MODE, WIN>,
@@ -1246,7 +1403,7 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     if (small_du > 0)
         HN_LAUNCH(k_tc_thread<MODE>, (long long)g->info.sms * 8, 256, 0, s, view, g->nV, small_du,
                   small_dc, d_counts, d_total);
-    HN_LAUNCH(k_tc_warp<MODE>, gw, kTcWarps * 32, dyn_warp, s, view, g->nV, d_counts, d_total,
+    HN_LAUNCH((k_tc_warp<MODE, WIN>), gw, kTcWarps * 32, dyn_warp, s, view, g->nV, d_counts, d_total,
               counters, big, big_cap, warp_cap, mid_cap, warp_work, item_work, chunk, narrow_min,
               small_du, small_dc);
     HN_LAUNCH((k_tc_cta<MODE, WIN>), (long long)g->info.sms * mid_per_sm, kTcWarps * 32, dyn_mid, s, view,
@@ -1290,13 +1447,17 @@ unsigned long long run_counting(hn_graph* g, const Oriented& o, int mode,
     }
     if (d_counts) HN_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * g->nV, s));
     long long* bp = big.get();
-    view.ranked = o.ranked;
-    auto count = [&](auto m) {   // (edge supports are counted under ids)
+    auto count = [&](auto m) {   // (edge supports are counted with tables)
         constexpr int M = decltype(m)::value;
-        if (M != 3 && o.ranked)
-            launch_counting<M, M != 3>(g, view, d_counts, d_total, counters, bp, big_cap, flipped);
-        else
-            launch_counting<M, false>(g, view, d_counts, d_total, counters, bp, big_cap, flipped);
+        auto launch = [&](auto win) {
+            launch_counting<M, decltype(win)::value>(g, view, d_counts, d_total, counters, bp,
+                                                     big_cap, flipped);
+        };
+        if constexpr (M != 3) {
+            if (o.ranked) return launch(std::integral_constant<int, kRankWin>());
+            if (o.padded) return launch(std::integral_constant<int, kIdWin>());
+        }
+        launch(std::integral_constant<int, kNoWin>());
     };
     switch (mode) {
         case 0: count(std::integral_constant<int, 0>()); break;

@@ -11,11 +11,11 @@ struct Oriented {
     DevBuf<int32_t> fwd;       // oriented, sorted neighbour lists
     DevBuf<int32_t> feid;      // edge id of each fwd entry (when built with canon)
     DevBuf<int> dplus;         // oriented degrees (nV)
-    // orientation by rank (build_for_counting): offp and dplus are indexed by
-    // number (0 = highest rank) and fwd holds numbers, unsorted, each list on
-    // 16 bytes and padded to four entries
-    DevBuf<int32_t> inv;       // vertex of each number
-    bool ranked = false;
+    // build_for_counting: offp and dplus are indexed by number (the id, or
+    // ranked 0 = highest rank) and fwd holds numbers, in the order of ids;
+    // padded: each list starts on 16 bytes and is padded to four entries
+    DevBuf<int32_t> inv;       // ranked: vertex of each number
+    bool padded = false, ranked = false;
 };
 
 // Build N+(u) = {v in N(u) : (deg u, u) < (deg v, v)} for every vertex.

@@ -1,7 +1,7 @@
-"""Triangle counts by the rank orientation (graphs of more than 131,072
+"""Triangle counts by bitmaps: the rank orientation (graphs of more than 131,072
 vertices whose edges are not local in id): totals, per-vertex and owner
 counts equal the id orientation's (tc.flip = 0 never ranks) and the oracle's,
-with lists inside, across and beyond the bitmap windows (32,736 numbers for a
+with lists inside, across and beyond the bitmaps (65,535 numbers for a
 warp, 131,072 for a CTA)."""
 import ctypes
 
@@ -77,3 +77,47 @@ def test_lists_too_long_for_the_table_go_by_id():
         assert H.TriangleCounting2(h).run() == O.tc(g)
     finally:
         H.tune_reset()
+
+
+@pytest.mark.parametrize("case", ["union", "small", "one_tile", "hub"])
+def test_close_ids_use_bitmaps_of_ids(case):
+    """Lists under ids that span less than a warp's bitmap (65,536 ids), than
+    a CTA's (131,072), and more; one vertex's list across many tiles."""
+    rng = np.random.default_rng(8)
+    if case == "union":
+        parts = [T.rmat_graph(13, 16, seed=1), T.er_graph(90_000, 40, seed=2),
+                 T.rmat_graph(17, 8, seed=3, n_vertices=70_001), T.er_graph(300, 150, seed=4),
+                 T.er_graph(140_000, 12, seed=9)]
+        g, _ = T.disjoint_union(parts)
+    elif case == "small":
+        g = T.rmat_graph(10, 40, seed=5)
+    elif case == "one_tile":
+        g = T.er_graph(40, 9, seed=6)
+    else:
+        n = 40_000       # two vertices joined to nearly all, which form short lists
+        a = rng.permutation(n)[:39_000].astype(np.int32)
+        s = [np.full(39_000, 7, np.int32), np.full(39_000, 39_991, np.int32), a[:-1]]
+        d = [a, a[::-1].copy(), a[1:]]
+        s, d = np.concatenate(s), np.concatenate(d)
+        keep = s != d
+        g = O.build_csr_undirected(n, s[keep], d[keep])
+    h = build(g)
+    ref = O.tc(g)
+    tc = H.TriangleCounting2(h)
+    for knobs in ({}, {"tc.warp_cap": 32, "tc.warp_work": 1024, "tc.mid_cap": 32,
+                       "tc.item_work": 1024}, {"tc.thread_du": 0}):
+        try:
+            for k, v in knobs.items():
+                H.tune_set(k, v)
+            assert tc.run() == ref
+            assert tc.run(per_vertex=True) == ref
+            pv = tc.copyTCToHost().copy()
+            ow, total = owner(h)
+            assert total == ref == int(ow.sum())
+            H.tune_set("tc.flip", 0)
+            assert tc.run(per_vertex=True) == ref
+            np.testing.assert_array_equal(pv, tc.copyTCToHost())
+            ow0, _ = owner(h)
+            np.testing.assert_array_equal(ow, ow0)
+        finally:
+            H.tune_reset()
