@@ -655,6 +655,11 @@ __device__ __forceinline__ void tc_credit_edges(int* esup, int e_uv, int e_vw, i
 enum { kSearch, kHash, kBits, kBitsHash };
 constexpr int kTcLong = 128;
 constexpr int kQuads = 4;   // kBits: lists read by the whole warp from this length on
+// CTAs an SM of the bitmap-only kernel: it waits on list loads, so occupancy
+// pays.  Totals (32 registers), R-MAT scale 22: 9.7 ms at 4, 9.1 at 5, 8.8 at 8;
+// owner counts, which spill below 48 registers, 512 graphs: 1.43 ms at 4, 1.38 at
+// 5, 1.59 at 8.  Tables in the same kernel (62 registers): 10.0 and 1.46 ms.
+__host__ __device__ constexpr int bits_ctas(int mode) { return mode == 0 ? 8 : 5; }
 constexpr int kWinWords = kWin / 32 + 4;   // a zero word behind the bits, 16-byte multiples
 
 // Clears the words of a bitmap of wn bits and the zero bit behind them.
@@ -1166,12 +1171,13 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
 // lists share `big` (items (u << 32) | chunk, each item_cands(d+(u))
 // candidates of u): mid from the front (counters[1] entries), huge from the
 // back (counters[2] entries).
-// WIN: a 16 KB bitmap in front of the table.  Ranked it holds the members among
-// the first kWin numbers, the table the others (none for u <= kWin); under ids
-// all of an N+(u) that spans at most kWin, else the table does.  No list
-// exceeds `cap` (checked by the host).
-template <int MODE, int WIN>
-__global__ void __launch_bounds__(kTcWarps * 32, 4)
+// WIN: the vertices whose N+(u) fits a 16 KB bitmap (ranked, the first kWin + 1
+// numbers; under ids, spans of at most kWin) are a launch of their own over both
+// lists (BITS), which needs no table and fewer registers (bits_ctas an SM).  The
+// others have the table, ranked with the bitmap of the members among the first
+// kWin numbers in front of it.  No list exceeds `cap` (checked by the host).
+template <int MODE, int WIN, bool BITS>
+__global__ void __launch_bounds__(kTcWarps * 32, BITS ? bits_ctas(MODE) : 4)
 k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
          unsigned long long* __restrict__ total_out, const int* __restrict__ counters,
          const long long* __restrict__ big, long long big_cap, long long item_work, int narrow_min,
@@ -1184,10 +1190,10 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
     __shared__ unsigned long long s_sum[kTcWarps];
     __shared__ int s_next;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nbig = counters[huge ? 2 : 1];
+    const int nhuge = BITS || huge ? counters[2] : 0, nmid = BITS || !huge ? counters[1] : 0;
     unsigned long long mine = 0;
-    for (int i = blockIdx.x; i < nbig; i += gridDim.x) {
-        const long long item = huge ? big[big_cap - 1 - i] : big[i];
+    for (int i = blockIdx.x; i < nhuge + nmid; i += gridDim.x) {
+        const long long item = i < nhuge ? big[big_cap - 1 - i] : big[i - nhuge];
         const int u = (int)(item >> 32);
         const int ch = (int)(item & 0xFFFFFFFF);
         const long long ub = g.offp[u];
@@ -1196,10 +1202,6 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
         const long long cb = g.coff[u] + (long long)ch * ipc;
         const int rest = (int)(g.coff[u + 1] - cb);
         const int dc = rest < ipc ? rest : ipc;
-        unsigned* win = (unsigned*)s_dyn;                  // WIN: kWin bits
-        int* slots = s_dyn + (WIN != kNoWin ? kWinWords : 0);
-        unsigned* filt = (unsigned*)(slots + tc_table_slots(cap));
-        int* teid = MODE == 3 ? (int*)(filt + tc_table_slots(cap) / 4) : nullptr;
         int wb = 0;
         unsigned wn = 0;
         bool hash = du <= cap;
@@ -1211,20 +1213,25 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
             wn = (unsigned)(g.fwd[ub + du - 1] - wb) + 1u;
             hash = wn > kWin;
         }
+        if (WIN != kNoWin && hash == BITS) continue;   // the other launch's
+        unsigned* win = (unsigned*)s_dyn;                  // BITS or ranked: kWin bits
+        int* slots = s_dyn + (WIN == kRankWin ? kWinWords : 0);
+        unsigned* filt = (unsigned*)(slots + tc_table_slots(cap));
+        int* teid = MODE == 3 ? (int*)(filt + tc_table_slots(cap) / 4) : nullptr;
         int bits = 0;
         if (threadIdx.x == 0) s_next = 0;
-        if (WIN == kRankWin || (WIN == kIdWin && !hash)) clear_bits(win, wn, threadIdx.x, blockDim.x);
-        if (hash) {
+        if (BITS || WIN == kRankWin) clear_bits(win, wn, threadIdx.x, blockDim.x);
+        if (!BITS && hash) {
             bits = 32 - __clz(2 * du - 1);
             if (bits < 5) bits = 5;
             for (int j = threadIdx.x; j < (1 << bits); j += blockDim.x) slots[j] = -1;
             for (int j = threadIdx.x; j < (1 << (bits - 2)); j += blockDim.x) filt[j] = 0u;
         }
-        if (WIN != kNoWin || hash) {
+        if (BITS || hash) {
             __syncthreads();
             for (int j = threadIdx.x; j < du; j += blockDim.x) {
                 const int w = g.fwd[ub + j];
-                if (WIN == kRankWin ? w < kWin : WIN == kIdWin && !hash) {
+                if (BITS || (WIN == kRankWin && w < kWin)) {
                     const int x = w - wb;
                     atomicOr(win + (x >> 5), 1u << (x & 31));
                 } else {
@@ -1240,15 +1247,10 @@ k_tc_cta(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
                 s_pref[warp], s_vb[warp], s_v[warp], s_fc[warp], per_vertex, win, wb, wn);
         };
         unsigned long long cu;
-        if (WIN == kRankWin)
-            cu = hash ? run(std::integral_constant<int, kBitsHash>())
-                      : run(std::integral_constant<int, kBits>());
-        else if (WIN == kIdWin)
-            cu = hash ? run(std::integral_constant<int, kHash>())
-                      : run(std::integral_constant<int, kBits>());
-        else
-            cu = hash ? run(std::integral_constant<int, kHash>())
-                      : run(std::integral_constant<int, kSearch>());
+        if (BITS) cu = run(std::integral_constant<int, kBits>());
+        else if (WIN == kRankWin) cu = run(std::integral_constant<int, kBitsHash>());
+        else if (WIN == kIdWin || hash) cu = run(std::integral_constant<int, kHash>());
+        else cu = run(std::integral_constant<int, kSearch>());
         mine += cu;
         __syncthreads();
     }
@@ -1427,7 +1429,12 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     cudaStream_t s = g->stream;
     const long long gw = (long long)g->info.sms * knob(kKnobTcWarpCtasPerSm);
     const int warp_cap = (int)knob(kKnobTcWarpCap);
-    const int chunk = (int)knob(kKnobTcChunk);
+    // vertices that a warp takes at a time: fewer on small graphs, where 16
+    // heavy ones in a row kept one warp busy after the others had finished
+    // (100,003 vertices, 2.2 M edges: 3.0 ms at 16, 0.8 at 1; 4.2 M vertices:
+    // 6.6 ms at 1, 4.6 at 8 and 16)
+    const int chunk = (int)std::max(1ll, std::min<long long>(knob(kKnobTcChunk),
+                                                             g->nV / (g->info.sms * 512ll)));
     constexpr bool by_rank = WIN == kRankWin;
     // lists by rank are not sorted: nothing to narrow
     const int narrow_min = by_rank ? INT_MAX : (int)knob(kKnobTcNarrowMin);
@@ -1443,17 +1450,19 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     const int mid_cap = WIN != kNoWin ? (int)std::min<long long>(knob(kKnobTcMidCap), 2048)
                                 : (int)knob(kKnobTcMidCap);
     const int cta_cap = (int)std::min<long long>(knob(kKnobTcCtaTableCap), cap_max);
-    constexpr size_t win = WIN != kNoWin ? kWinWords * sizeof(int) : 0;
+    constexpr size_t bits = kWinWords * sizeof(int);
+    constexpr size_t win = WIN == kRankWin ? bits : 0;   // in front of the tables
     const size_t dyn_mid = win + tc_table_bytes(mid_cap, eid);
     const size_t dyn_huge = win + tc_table_bytes(cta_cap, eid);
     constexpr size_t dyn_warp = sizeof(int) * kTcWarps * tc_warp_words(WIN != kNoWin, eid);
     // (set per call: the attributes belong to the device in use)
-    HN_CUDA(cudaFuncSetAttribute(k_tc_cta<MODE, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HN_CUDA(cudaFuncSetAttribute((k_tc_cta<MODE, WIN, false>),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(win + tc_table_bytes(cap_max, eid))));
     HN_CUDA(cudaFuncSetAttribute((k_tc_warp<MODE, WIN>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dyn_warp));
     int mid_per_sm = 0;
-    HN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mid_per_sm, k_tc_cta<MODE, WIN>,
+    HN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mid_per_sm, (k_tc_cta<MODE, WIN, false>),
                                                           kTcWarps * 32, dyn_mid));
     if (mid_per_sm < 1) mid_per_sm = 1;
     // small vertices by thread (only with the smaller-side assignment, which
@@ -1467,10 +1476,15 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     HN_LAUNCH((k_tc_warp<MODE, WIN>), gw, kTcWarps * 32, dyn_warp, s, view, g->nV, d_counts, d_total,
               counters, big, big_cap, warp_cap, mid_cap, warp_work, item_work, chunk, narrow_min,
               small_du, small_dc);
-    HN_LAUNCH((k_tc_cta<MODE, WIN>), (long long)g->info.sms * mid_per_sm, kTcWarps * 32, dyn_mid, s, view,
-              g->nV, d_counts, d_total, counters, big, big_cap, item_work, narrow_min, 0, mid_cap);
-    HN_LAUNCH((k_tc_cta<MODE, WIN>), (long long)g->info.sms, kTcWarps * 32, dyn_huge, s, view, g->nV,
-              d_counts, d_total, counters, big, big_cap, item_work, narrow_min, 1, cta_cap);
+    if constexpr (WIN != kNoWin)
+        HN_LAUNCH((k_tc_cta<MODE, WIN, true>), (long long)g->info.sms * bits_ctas(MODE), kTcWarps * 32, bits, s,
+                  view, g->nV, d_counts, d_total, counters, big, big_cap, item_work, narrow_min, 0,
+                  0);
+    HN_LAUNCH((k_tc_cta<MODE, WIN, false>), (long long)g->info.sms * mid_per_sm, kTcWarps * 32,
+              dyn_mid, s, view, g->nV, d_counts, d_total, counters, big, big_cap, item_work,
+              narrow_min, 0, mid_cap);
+    HN_LAUNCH((k_tc_cta<MODE, WIN, false>), (long long)g->info.sms, kTcWarps * 32, dyn_huge, s, view,
+              g->nV, d_counts, d_total, counters, big, big_cap, item_work, narrow_min, 1, cta_cap);
 }
 
 namespace {
