@@ -6,8 +6,12 @@
 // BatchUpdate.i.cuh).  Here the key is one 64-bit word of 2L significant bits,
 // sorted 8 bits per pass (ceil(2L / 8) passes: 6 at 2^24 vertices), ONE kernel
 // per pass over tiles of 8 keys per thread (4096 keys, or 2048 with values;
-// 1024 threads per SM either way: the pass waits on memory, so occupancy
-// pays):
+// 1024 threads per SM either way: 42 registers and 1536 threads measured the
+// same on 10 M keys and slower on 300 K).  A pass is bound by its instructions,
+// the ranking above all, and by the barriers between a tile's phases.  10 M
+// keys: 115 us a pass with 64-bit indexes and a leader per digit that hands its
+// peers their base, 90 us with tile-relative indexes, no bounds checks in full
+// tiles and every lane reading its digit's count itself:
 //   * tiles take their numbers from a counter as they start, so every
 //     lower-numbered tile is already running;
 //   * a tile ranks its keys stably by digit (warp by warp, 32 keys a round in
@@ -28,6 +32,8 @@
 // the host reports the error at its synchronisation.  (The wait cannot
 // actually run out: a lower-numbered tile took its number, so it is running,
 // and it publishes its counts before any wait of its own.)
+#include <type_traits>
+
 #include "hn_graph.cuh"
 
 namespace hn {
@@ -38,12 +44,17 @@ constexpr int kOsIpt = 8;          // keys per thread of a pass
 constexpr int kBins = 256;
 constexpr int kMaxPasses = 8;
 constexpr long long kWaitLimit = 1 << 22;
-constexpr int kLook = 4;   // statuses a look-back step reads at once
+constexpr int kLook = 8;   // statuses a look-back step reads at once
 constexpr long long kStatusBytes = 64 << 20;
 
-constexpr unsigned long long kFlagAgg = 1ull << 62;    // the tile's own counts
-constexpr unsigned long long kFlagIncl = 2ull << 62;   // counts of tiles 0..t
-constexpr unsigned long long kValMask = (1ull << 62) - 1;
+// A status: a flag in the top two bits, a count of keys below them.
+template <typename S>
+struct Status {
+    static constexpr int kShift = 8 * sizeof(S) - 2;
+    static constexpr S kAgg = (S)1 << kShift;    // the tile's own counts
+    static constexpr S kIncl = (S)2 << kShift;   // counts of tiles 0..t
+    static constexpr S kVal = kAgg - 1;
+};
 
 struct SortState {
     unsigned ghist[kMaxPasses][kBins];   // keys per digit, per pass
@@ -91,11 +102,11 @@ __device__ __forceinline__ unsigned warp_incl(unsigned x, int lane) {
 
 // One pass over one tile of NT * kOsIpt keys (NT threads, NT >= kBins);
 // threads 0..255 also act for the 256 digits.
-template <bool VALS, int NT>
+template <bool VALS, int NT, typename S>
 __global__ void __launch_bounds__(NT, 1024 / NT)
 k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict__ vin,
           unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, long long n,
-          int pass, int shift, int next_shift, unsigned long long* status, SortState* ss,
+          int pass, int shift, int next_shift, S* status, SortState* ss,
           int* err) {
     constexpr int NW = NT / 32;
     constexpr int TILE = NT * kOsIpt;
@@ -104,7 +115,8 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict
     __shared__ uint32_t sval[VALS ? TILE : 1];
     __shared__ unsigned short wcnt[NW][kBins];   // per warp, then warp prefix
     __shared__ unsigned s_start[kBins];   // first slot of digit d in the reordered tile
-    __shared__ unsigned s_out[kBins];     // output slot of the tile's first key of digit d
+    __shared__ unsigned s_out[kBins];     // output slot of the tile's first key of digit d, less its
+                                          // slot in the reordered tile (modulo 2^32)
     __shared__ unsigned s_next[kBins];    // next pass's digit counts of this tile
     __shared__ unsigned s_wsum[DW], s_bsum[DW];
     __shared__ int s_tile, s_fail;
@@ -118,37 +130,49 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict
     if (d < kBins) s_next[d] = 0;
     __syncthreads();
     const int tile = s_tile;
-    // warp w: keys tile*TILE + w*32*kOsIpt + r*32 + lane, r = 0..kOsIpt-1
-    const long long t0 = (long long)tile * TILE + w * (32 * kOsIpt);
+    const long long tile0 = (long long)tile * TILE;
+    const int tile_n = n - tile0 < TILE ? (int)(n - tile0) : TILE;   // keys of the tile
+    const bool full = tile_n == TILE;
+    // warp w: keys t0 + r*32 + lane of the tile, r = 0..kOsIpt-1
+    const int t0 = w * (32 * kOsIpt) + lane;
     unsigned long long k[kOsIpt];
     uint32_t v[kOsIpt];
     unsigned short rank[kOsIpt];
+    {
+        const unsigned long long* kt = kin + tile0 + t0;
+        const uint32_t* vt = VALS ? vin + tile0 + t0 : nullptr;
 #pragma unroll
-    for (int r = 0; r < kOsIpt; r++) {
-        const long long i = t0 + r * 32 + lane;
-        k[r] = i < n ? kin[i] : 0ull;
-        if (VALS) v[r] = i < n ? vin[i] : 0u;
-    }
-#pragma unroll
-    for (int r = 0; r < kOsIpt; r++) {
-        const bool valid = t0 + r * 32 + lane < n;
-        const unsigned active = __ballot_sync(0xFFFFFFFFu, valid);
-        const unsigned dg = digit_of(k[r], shift);
-        const unsigned peers = same_digit_lanes(dg, active);
-        const int leader = valid ? __ffs(peers) - 1 : lane;
-        unsigned base = 0;
-        if (valid && lane == leader) base = wcnt[w][dg];
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
-        if (valid) {
-            rank[r] = (unsigned short)(base + __popc(peers & ((1u << lane) - 1u)));
-            if (lane == leader) wcnt[w][dg] = (unsigned short)(base + __popc(peers));
-            if (next_shift >= 0) atomicAdd(&s_next[digit_of(k[r], next_shift)], 1u);
+        for (int r = 0; r < kOsIpt; r++) {
+            const bool valid = full || t0 + r * 32 < tile_n;
+            k[r] = valid ? kt[r * 32] : 0ull;
+            if (VALS) v[r] = valid ? vt[r * 32] : 0u;
         }
-        __syncwarp();
     }
+    unsigned short* const wc = wcnt[w];
+    auto rank_keys = [&](auto all) {   // all: every key of the tile exists
+        constexpr bool ALL = decltype(all)::value;
+#pragma unroll
+        for (int r = 0; r < kOsIpt; r++) {
+            const bool valid = ALL || t0 + r * 32 < tile_n;
+            const unsigned active = ALL ? 0xFFFFFFFFu : __ballot_sync(0xFFFFFFFFu, valid);
+            const unsigned dg = digit_of(k[r], shift);
+            const unsigned peers = same_digit_lanes(dg, active);
+            // every lane reads its digit's count, the last of its peers adds them
+            if (valid) {
+                const unsigned base = wc[dg];
+                rank[r] = (unsigned short)(base + __popc(peers & ((1u << lane) - 1u)));
+                if (next_shift >= 0) atomicAdd(&s_next[digit_of(k[r], next_shift)], 1u);
+            }
+            __syncwarp();
+            if (valid && peers >> lane == 1u) wc[dg] = (unsigned short)(rank[r] + 1);
+            __syncwarp();
+        }
+    };
+    if (full) rank_keys(std::true_type());
+    else rank_keys(std::false_type());
     __syncthreads();
     unsigned cnt = 0, tot = 0, ci = 0, ti = 0;
-    unsigned long long excl = 0;
+    unsigned excl = 0;
     if (d < kBins) {
         // digit d's count in this tile (warp counts -> warp prefixes)
 #pragma unroll
@@ -160,8 +184,8 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict
         // publish the counts now; the look-back for the earlier tiles'
         // counts waits until this tile's keys are reordered, so that the
         // tiles before it have had that long to publish theirs
-        *(volatile unsigned long long*)(status + (long long)tile * kBins + d) =
-            (tile == 0 ? kFlagIncl : kFlagAgg) | cnt;
+        *(volatile S*)(status + (long long)tile * kBins + d) =
+            (tile == 0 ? Status<S>::kIncl : Status<S>::kAgg) | cnt;
         // this tile's digit starts (exclusive scan of cnt over d) and the
         // digits' bases in the output (exclusive scan of the pass histogram)
         tot = ss->ghist[pass][d];
@@ -186,9 +210,9 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict
     // reorder in shared memory
 #pragma unroll
     for (int r = 0; r < kOsIpt; r++) {
-        if (t0 + r * 32 + lane < n) {
+        if (full || t0 + r * 32 < tile_n) {
             const unsigned dd = digit_of(k[r], shift);
-            const unsigned at = s_start[dd] + wcnt[w][dd] + rank[r];
+            const unsigned at = s_start[dd] + wc[dd] + rank[r];
             skey[at] = k[r];
             if (VALS) sval[at] = v[r];
         }
@@ -204,17 +228,17 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict
             long long polls = 0;
             bool done = false;
             while (!done) {
-                unsigned long long sv[kLook];
+                S sv[kLook];
 #pragma unroll
                 for (int q = 0; q < kLook; q++)
                     sv[q] = j - q >= 0
-                                ? *(volatile const unsigned long long*)(status + (j - q) * kBins + d)
-                                : kFlagIncl;
+                                ? *(volatile const S*)(status + (j - q) * kBins + d)
+                                : Status<S>::kIncl;
                 int q = 0;
                 for (; q < kLook; q++) {
-                    const unsigned f = (unsigned)(sv[q] >> 62);
+                    const unsigned f = (unsigned)(sv[q] >> Status<S>::kShift);
                     if (f == 0) break;
-                    excl += sv[q] & kValMask;
+                    excl += (unsigned)(sv[q] & Status<S>::kVal);
                     if (f == 2) {
                         done = true;
                         break;
@@ -230,23 +254,20 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const uint32_t* __restrict
                     __nanosleep(32);
                 }
             }
-            *(volatile unsigned long long*)(status + (long long)tile * kBins + d) =
-                kFlagIncl | (excl + cnt);
+            *(volatile S*)(status + (long long)tile * kBins + d) = Status<S>::kIncl | (excl + cnt);
         }
         if (fail) s_fail = 1;
-        s_out[d] = tpre + ti - tot + (unsigned)excl;
+        s_out[d] = tpre + ti - tot + excl - s_start[d];
     }
     __syncthreads();
     if (s_fail) {
         if (threadIdx.x == 0) atomicExch(err, HN_ERR_TIMEOUT);
         return;
     }
-    const long long rem = n - (long long)tile * TILE;
-    const int tile_n = rem < TILE ? (int)rem : TILE;
     for (int j = threadIdx.x; j < tile_n; j += NT) {
         const unsigned long long key = skey[j];
         const unsigned dd = digit_of(key, shift);
-        const long long at = (long long)s_out[dd] + (j - (long long)s_start[dd]);
+        const unsigned at = s_out[dd] + (unsigned)j;   // (wraps: see s_out)
         if (at < n) {   // always: the counts add up to n
             kout[at] = key;
             if (VALS) vout[at] = sval[j];
@@ -287,8 +308,11 @@ void radix_sort_u64(hn_graph* g, unsigned long long*& keys, unsigned long long*&
     // the state and every pass's statuses are cleared at once; only when the
     // statuses would take more than kStatusBytes do the passes share one array
     const long long per_pass = ntiles * kBins;
-    const bool all = per_pass * passes * (long long)sizeof(unsigned long long) <= kStatusBytes;
-    DevBuf<unsigned long long> mem(sizeof(SortState) / 8 + (size_t)per_pass * (all ? passes : 1), s,
+    // 32-bit statuses while their 30 bits hold the counts
+    const bool narrow = n < (1ll << 30);
+    const long long pass_words = narrow ? (per_pass + 1) / 2 : per_pass;   // 8 bytes each
+    const bool all = pass_words * passes * 8 <= kStatusBytes;
+    DevBuf<unsigned long long> mem(sizeof(SortState) / 8 + (size_t)pass_words * (all ? passes : 1), s,
                                    arena);
     SortState* ss = (SortState*)mem.get();
     unsigned long long* status0 = mem.get() + sizeof(SortState) / 8;
@@ -299,15 +323,20 @@ void radix_sort_u64(hn_graph* g, unsigned long long*& keys, unsigned long long*&
     for (int p = 0; p < passes; p++) {
         const int shift = 8 * p;
         const int next = p + 1 < passes ? shift + 8 : -1;
-        unsigned long long* status = status0 + (all ? p * per_pass : 0);
-        if (!all) HN_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * per_pass, s));
-        if (vals)
-            HN_LAUNCH((k_rs_pass<true, 256>), ntiles, 256, 0, s, keys, vals, keys_alt, vals_alt,
-                      n, p, shift, next, status, ss, err);
-        else
-            HN_LAUNCH((k_rs_pass<false, 512>), ntiles, 512, 0, s, keys,
-                      (const uint32_t*)nullptr, keys_alt, (uint32_t*)nullptr, n, p, shift, next,
-                      status, ss, err);
+        unsigned long long* status = status0 + (all ? p * pass_words : 0);
+        if (!all) HN_CUDA(cudaMemsetAsync(status, 0, 8 * pass_words, s));
+        auto pass = [&](auto* st) {
+            using S = std::remove_pointer_t<decltype(st)>;
+            if (vals)
+                HN_LAUNCH((k_rs_pass<true, 256, S>), ntiles, 256, 0, s, keys, vals, keys_alt,
+                          vals_alt, n, p, shift, next, st, ss, err);
+            else
+                HN_LAUNCH((k_rs_pass<false, 512, S>), ntiles, 512, 0, s, keys,
+                          (const uint32_t*)nullptr, keys_alt, (uint32_t*)nullptr, n, p, shift, next,
+                          st, ss, err);
+        };
+        if (narrow) pass((unsigned*)status);
+        else pass(status);
         std::swap(keys, keys_alt);
         if (vals) std::swap(vals, vals_alt);
     }
