@@ -274,7 +274,8 @@ def roofline_entry(H, prefixes, algo_bytes_fn, peak, peak_kind, report, workload
     whose bandwidth `peak` is."""
     if isinstance(prefixes, str):
         prefixes = [prefixes]
-    cand = {k: v for k, v in report.items() if any(k.startswith(p) for p in prefixes)}
+    # (kernels launched with several template arguments are named in parentheses)
+    cand = {k: v for k, v in report.items() if any(k.lstrip("(").startswith(p) for p in prefixes)}
     if not cand:
         return None
     name, rec = max(cand.items(), key=lambda kv: kv[1]["ms"])
@@ -390,7 +391,7 @@ def bench_static(args, H, h, deg, nV, nE, stream, dev, rank, world, peak, peak_k
     prof_edges, prof_vis = run_steps(W, min(K, 16))
     rep = H.profile_report()
     H.profile_enable(False)
-    roof = roofline_entry(H, ["k_bfs_level<false>", "k_bfs_wlevel<false>"], lambda: 8 * prof_edges + 20 * prof_vis, peak,
+    roof = roofline_entry(H, ["k_bfs_level<false>", "k_bfs_run<false>"], lambda: 8 * prof_edges + 20 * prof_vis, peak,
                           peak_kind, rep, f"R-MAT scale {scale} BFS, {min(K, 16)} sources")
 
     also = {}
@@ -477,7 +478,7 @@ def static_extras(args, H, h, nV, nE, stream, dev, peak, peak_kind, scale, tunin
     # is served by L2 (the oriented graph, 0.29 GB, is read from DRAM about
     # once), so the path is measured against L2 bandwidth, not HBM
     l2_gbs = measure_l2_gbs(H, h, dev)
-    troof = roofline_entry(H, ["k_orient", "k_cand", "k_tc_", "k_degrees"], lambda: tc_bytes,
+    troof = roofline_entry(H, ["k_orient", "k_rank", "k_cand", "k_tc_", "k_dplus", "k_pad", "k_max_int", "k_local_sample"], lambda: tc_bytes,
                            round(l2_gbs, 1),
                            "measured now: L2 read bandwidth of a 48 MiB buffer resident in L2 "
                            "(16-byte loads, 20 passes, CUDA events; hn_read_bandwidth)", rep,
