@@ -176,6 +176,7 @@ enum Knob {
     kKnobUpdateBigMin,
     kKnobUpdateInPlace,
     kKnobUpdateOwnSort,
+    kKnobMsCheckMin,
     kNumKnobs
 };
 long long knob(Knob k);

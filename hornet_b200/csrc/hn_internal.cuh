@@ -90,6 +90,14 @@ __device__ __forceinline__ int warp_append(int* counter, bool pred) {
     return pred ? base + __popc(ballot & ((1u << lane) - 1)) : -1;
 }
 
+// SplitMix64's mixing function (S. Vigna), a permutation of 64-bit words.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
+    x += 0x9E3779B97F4A7C15ull;
+    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
+    return x ^ (x >> 31);
+}
+
 // First index i in [0,n) with a[i] >= x (n when none).
 template <typename T>
 __device__ __forceinline__ long long lower_bound_dev(const T* a, long long n, T x) {

@@ -22,6 +22,7 @@
 // distance when they sit in different components (a disjoint union of
 // graphs, one source per graph per slot).
 #include "hn_graph.cuh"
+#include "hn_window.cuh"
 
 namespace hn {
 
@@ -31,7 +32,10 @@ constexpr int kMaxSlots = 64;
 
 // A level pushes and applies the touched vertices it listed, pulls (apply
 // does the work), or pushes without a list and applies in a pass over all
-// vertices.
+// vertices.  A pull looks for a vertex's predecessors in its own list, so it
+// is right only where every edge is stored both ways: the first level that
+// would pull leaves the loop, the host has the edges checked (k_ms_one_way)
+// and goes on with the loop, pulling or not.
 enum { kMsPush, kMsPull, kMsPushAll };
 
 struct MsState {
@@ -59,8 +63,13 @@ struct MsState {
     int prev_nq;                    // size of the previous frontier (its fronts are cleared)
     int bottom_up;                  // bottom-up levels allowed
     int alpha, beta;                // direction switch thresholds
+    long long nE;                   // edges of the graph
+    long long check_min;            // edges of a frontier that the check is made for
     long long open_edges;           // degrees of the vertices that miss a slot
     unsigned long long all_mask;    // slots that hold at least one source
+    int symmetric;                  // 1: every edge is stored both ways, 0: not known, -1: no
+    int ask;                        // the loop has ended to have that found out
+    unsigned long long one_way;     // sum over the edges, 0 when symmetric
 };
 
 struct MsGraph {
@@ -76,8 +85,8 @@ struct MsGraph {
     int32_t* touched = nullptr;
     unsigned long long* stat = nullptr;
     unsigned long long* h_stat = nullptr;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    cudaGraph_t graph[2] = {nullptr, nullptr};      // [0] from the start, [1] the next levels
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
     int block = 256;      // msbfs.block knob baked into the graph
     unsigned grid = 0;    // msbfs.ctas_per_sm x SMs
 };
@@ -524,17 +533,112 @@ k_ms_apply(MsState* st, cudaGraphConditionalHandle cond) {
             // pull while the next frontier's edges (which a push reads) exceed
             // those of the vertices that still miss a slot (which a pull reads
             // at most) -- alpha / kMsScan, about 1 by default -- and the
-            // frontier holds nV/beta vertices or more
+            // frontier holds nV/beta vertices or more.  The check for symmetry
+            // reads all edges and takes a round trip to the host (60 us on a
+            // small graph, 0.58 ms at 128 M edges), so a frontier of fewer than
+            // check_min edges or a quarter of the graph's is pushed instead
+            // (16 M edges: 8 slots 490 us pushed, 433 checked and pulled, one
+            // slot 335 and 368; 8 M edges, 8 slots: 331 and 362; 128 M edges, 8
+            // slots: 2.40 and 1.73 ms)
             const long long mf = (long long)(c >> 32);
+            const bool more = nn > 0 && level < nV;
             int next = mf * kMsAll > nV ? kMsPushAll : kMsPush;
-            if (st->bottom_up) {
+            int ask = 0;
+            if (st->bottom_up && st->symmetric >= 0 && more) {
                 const long long open = (long long)atomicAdd((unsigned long long*)&st->open_edges, 0ull);
-                if (mf * st->alpha > kMsScan * open && (long long)nn * st->beta >= nV) next = kMsPull;
+                if (mf * st->alpha > kMsScan * open && (long long)nn * st->beta >= nV) {
+                    if (st->symmetric) next = kMsPull;
+                    else if (mf >= st->check_min && 4 * mf >= st->nE) ask = 1;
+                }
             }
             st->mode = next;
-            cudaGraphSetConditional(cond, (nn > 0 && level < nV) ? 1u : 0u);
+            st->ask = ask;
+            cudaGraphSetConditional(cond, more && !ask ? 1u : 0u);
         }
     }
+}
+
+// Is every edge stored both ways?  The sum over the edges (u, v) of
+// mix64({min, max}), counted negative where u > v: 0 when each pair is stored
+// as often one way as the other.  A single one-way edge never gives 0, others
+// with a probability of 2^-64.  Loops do not count.  A warp per merge-path
+// tile, windows of 32 vertices, four rows of 32 edges in flight; bound by HBM
+// (4 bytes an edge).
+constexpr int kMsTile = 1024;
+constexpr int kOneWayBlock = 256;
+
+__global__ void __launch_bounds__(kOneWayBlock)
+k_ms_one_way(const long long* __restrict__ prefix, int nV, long long nE,
+             const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,
+             const long long* __restrict__ splits, long long ntiles, MsState* st) {
+    constexpr int ROWS = 4;
+    const unsigned kFull = 0xFFFFFFFFu;
+    __shared__ unsigned long long s_sum[kOneWayBlock / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long nwarps = (long long)gridDim.x * (kOneWayBlock / 32);
+    unsigned long long sum = 0;
+    for (long long tile = blockIdx.x * (long long)(kOneWayBlock / 32) + warp; tile < ntiles;
+         tile += nwarps) {
+        const WarpTile wt = warp_tile(splits, tile, kMsTile, nE, nV);
+        if (wt.nitems == 0) continue;
+        for (long long v0 = wt.seg0; v0 <= wt.seg1; v0 += 32) {
+            const long long v = v0 + lane < nV ? v0 + lane : nV;
+            const long long first = prefix[v];
+            const long long next = v0 + 32 <= nV ? prefix[v0 + 32] : nE;
+            const long long off = v < nV ? vtab[v].off : 0;
+            const WarpWindow w = warp_window(wt, v0, first, next);
+            if (w.n == 0) continue;
+            const long long base = __shfl_sync(kFull, off - first, w.lane_of) + wt.item0;
+            const int id = (int)v0 + w.lane_of;
+            for (int r = w.begin; r < w.end; r += 32 * ROWS) {
+                int x[ROWS], u[ROWS];
+#pragma unroll
+                for (int k = 0; k < ROWS; k++) {
+                    const int row = r + 32 * k;
+                    x[k] = u[k] = 0;
+                    if (row >= w.end) continue;   // uniform
+                    const int j = warp_owner(w, row) & 31;
+                    const long long b = __shfl_sync(kFull, base, j);
+                    u[k] = __shfl_sync(kFull, id, j);
+                    x[k] = row + lane < w.end ? __ldcs(pool + b + row + lane) : u[k];
+                }
+#pragma unroll
+                for (int k = 0; k < ROWS; k++) {
+                    const unsigned lo = (unsigned)min(x[k], u[k]), hi = (unsigned)max(x[k], u[k]);
+                    const unsigned long long h = mix64((unsigned long long)lo << 32 | hi);
+                    if (u[k] < x[k]) sum += h;
+                    if (u[k] > x[k]) sum -= h;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+    if (lane == 0) s_sum[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < kOneWayBlock / 32; i++) sum += s_sum[i];
+        if (sum) atomicAdd(&st->one_way, sum);
+    }
+}
+
+// One thread: the answer, and with it the direction of the level asked for.
+__global__ void k_ms_answer(MsState* st) {
+    st->symmetric = st->one_way ? -1 : 1;
+    if (!st->one_way) st->mode = kMsPull;
+    st->ask = 0;
+}
+
+void check_symmetry(hn_graph* g, MsGraph& mg) {
+    cudaStream_t s = g->stream;
+    DevBuf<long long> prefix((size_t)g->nV + 1, s), splits;
+    degree_prefix(g, nullptr, g->nV, prefix.get());
+    lb_splits(g, prefix.get(), g->nV, g->nE, kMsTile, splits);
+    const long long ntiles = (g->nE + g->nV + kMsTile - 1) / kMsTile;
+    HN_LAUNCH(k_ms_one_way, grid_for(g, ntiles, kOneWayBlock / 32), kOneWayBlock, 0, s,
+              (const long long*)prefix.get(), g->nV, (long long)g->nE, (const VRec*)g->vtab,
+              (const int32_t*)g->pool, (const long long*)splits.get(), ntiles, mg.state);
+    HN_LAUNCH(k_ms_answer, 1, 1, 0, s, mg.state);
 }
 
 void build_ms_graph(hn_graph* g, MsGraph& mg) {
@@ -554,55 +658,54 @@ void build_ms_graph(hn_graph* g, MsGraph& mg) {
     mg.nV = nV;
     mg.nchunk_cap = nchunk_cap;
 
-    HN_CUDA(cudaGraphCreate(&mg.graph, 0));
-    cudaGraphNode_t fill, seed, condn, push, apply;
-    {
+    for (int part = 0; part < 2; part++) {
+        cudaGraph_t& graph = mg.graph[part];
+        HN_CUDA(cudaGraphCreate(&graph, 0));
+        cudaGraphNode_t fill, seed, condn, push, apply;
         void* args[] = {&mg.state};
         cudaKernelNodeParams p = {};
-        p.func = (void*)k_ms_fill;
-        p.gridDim = dim3((unsigned)g->info.sms * 8);
-        p.blockDim = dim3(256);
         p.kernelParams = args;
-        HN_CUDA(cudaGraphAddKernelNode(&fill, mg.graph, nullptr, 0, &p));
-        p.func = (void*)k_ms_seed;
-        p.gridDim = dim3(1);
-        p.blockDim = dim3(kSeedBlock);
-        HN_CUDA(cudaGraphAddKernelNode(&seed, mg.graph, &fill, 1, &p));
-    }
-    cudaGraphConditionalHandle handle;
-    HN_CUDA(cudaGraphConditionalHandleCreate(&handle, mg.graph, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = handle;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    HN_CUDA(cudaGraphAddNode(&condn, mg.graph, &seed, 1, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    {
-        void* args[] = {&mg.state};
-        cudaKernelNodeParams p = {};
+        if (part == 0) {
+            p.func = (void*)k_ms_fill;
+            p.gridDim = dim3((unsigned)g->info.sms * 8);
+            p.blockDim = dim3(256);
+            HN_CUDA(cudaGraphAddKernelNode(&fill, graph, nullptr, 0, &p));
+            p.func = (void*)k_ms_seed;
+            p.gridDim = dim3(1);
+            p.blockDim = dim3(kSeedBlock);
+            HN_CUDA(cudaGraphAddKernelNode(&seed, graph, &fill, 1, &p));
+        }
+        cudaGraphConditionalHandle handle;
+        HN_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = handle;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        HN_CUDA(cudaGraphAddNode(&condn, graph, part == 0 ? &seed : nullptr, part == 0 ? 1 : 0, &cp));
+        cudaGraph_t body = cp.conditional.phGraph_out[0];
         p.func = mg.block == 128 ? (void*)k_ms_push<128>
                : mg.block == 512 ? (void*)k_ms_push<512> : (void*)k_ms_push<256>;
         p.gridDim = dim3(mg.grid);
         p.blockDim = dim3(mg.block);
-        p.kernelParams = args;
         HN_CUDA(cudaGraphAddKernelNode(&push, body, nullptr, 0, &p));
         void* args2[] = {&mg.state, &handle};
         p.func = mg.block == 128 ? (void*)k_ms_apply<128>
                : mg.block == 512 ? (void*)k_ms_apply<512> : (void*)k_ms_apply<256>;
-        p.gridDim = dim3(mg.grid);
         p.kernelParams = args2;
         HN_CUDA(cudaGraphAddKernelNode(&apply, body, &push, 1, &p));
+        HN_CUDA(cudaGraphInstantiate(&mg.exec[part], graph, 0));
     }
-    HN_CUDA(cudaGraphInstantiate(&mg.exec, mg.graph, 0));
 }
 
 }  // namespace
 
 void free_ms_graph(MsGraph* mg) {
     if (!mg) return;
-    if (mg->exec) cudaGraphExecDestroy(mg->exec);
-    if (mg->graph) cudaGraphDestroy(mg->graph);
+    for (int i = 0; i < 2; i++) {
+        if (mg->exec[i]) cudaGraphExecDestroy(mg->exec[i]);
+        if (mg->graph[i]) cudaGraphDestroy(mg->graph[i]);
+    }
     if (mg->state) cudaFree(mg->state);
     if (mg->h_state) cudaFreeHost(mg->h_state);
     if (mg->qbuf) cudaFree(mg->qbuf);
@@ -700,20 +803,27 @@ extern "C" int hn_bfs_batch(hn_graph_t* g, const int32_t* sources, const int32_t
     h.bottom_up = (int)knob(kKnobMsBottomUp);
     h.alpha = (int)knob(kKnobBfsDoAlpha);
     h.beta = (int)knob(kKnobBfsDoBeta);
-    h.open_edges = g->nE;
+    h.nE = h.open_edges = g->nE;
+    h.check_min = knob(kKnobMsCheckMin);
     HN_CUDA(cudaMemcpyAsync(mg.state, &h, sizeof(MsState), cudaMemcpyHostToDevice, s));
-    cudaEvent_t ev0 = nullptr;
-    if (g_profiling) profile_begin(s, &ev0);
-    HN_CUDA(cudaGraphLaunch(mg.exec, s));
-    if (ev0) profile_end("k_ms_push+apply", s, ev0);
-    count_launch(3);
-    HN_CUDA(cudaMemcpyAsync(mg.h_stat, mg.stat, sizeof(unsigned long long) * 3 * kMaxSlots,
-                            cudaMemcpyDeviceToHost, s));
-    HN_CUDA(cudaMemcpyAsync(mg.h_state, mg.state, sizeof(MsState), cudaMemcpyDeviceToHost, s));
-    if (mem == HN_MEM_HOST)
+    for (int part = 0; part < 2; part++) {   // at most twice: the answer is then known
+        cudaEvent_t ev0 = nullptr;
+        if (g_profiling) profile_begin(s, &ev0);
+        HN_CUDA(cudaGraphLaunch(mg.exec[part], s));
+        if (ev0) profile_end("k_ms_push+apply", s, ev0);
+        count_launch(part == 0 ? 3 : 2);
+        HN_CUDA(cudaMemcpyAsync(mg.h_stat, mg.stat, sizeof(unsigned long long) * 3 * kMaxSlots,
+                                cudaMemcpyDeviceToHost, s));
+        HN_CUDA(cudaMemcpyAsync(mg.h_state, mg.state, sizeof(MsState), cudaMemcpyDeviceToHost, s));
+        HN_CUDA(cudaStreamSynchronize(s));
+        if (!h.ask) break;
+        check_symmetry(g, mg);
+    }
+    if (mem == HN_MEM_HOST) {
         HN_CUDA(cudaMemcpyAsync(dist, out, sizeof(int32_t) * (size_t)nslots * nV,
                                 cudaMemcpyDeviceToHost, s));
-    HN_CUDA(cudaStreamSynchronize(s));
+        HN_CUDA(cudaStreamSynchronize(s));
+    }
     if (slot_stats)
         for (int b = 0; b < nslots; b++) {
             slot_stats[b].levels =

@@ -22,13 +22,6 @@ __global__ void k_vertex_degree(hornet::HornetDevice hd, int32_t* out) {
         out[v] = hd.vertex((int)v).degree();
 }
 
-__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
-    x += 0x9E3779B97F4A7C15ull;
-    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
-    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
-    return x ^ (x >> 31);
-}
-
 // Order-independent checksum of the edge multiset: sum over edges (u, v) of
 // SplitMix64(u << 32 | v), a warp per vertex, one atomic per warp.
 __global__ void k_adjacency_hash(const VRec* __restrict__ vtab, const int32_t* __restrict__ pool,

@@ -122,7 +122,12 @@ int hn_profile_report(char* buf, int64_t len);
  *                       merging sorted lists (0 turns it off) (0..64, 16;
  *                       1..1024, 32)
  *   msbfs.bottom_up     1: batched BFS runs bottom-up levels while the
- *                       frontier is large (bfs.do_alpha / do_beta switch) (0..1, 1)
+ *                       frontier's edges exceed those still open
+ *                       (bfs.do_alpha / do_beta shift the switch), on graphs
+ *                       that store every edge both ways, which it checks
+ *                       first (0..1, 1)
+ *   msbfs.check_min     frontier edges from which it makes that check, which
+ *                       reads all edges (1..2^32, 2^23)
  *   tc.warp_ctas_per_sm CTAs per SM of the warp-per-vertex kernel (1..16, 8)
  *   bfs.dynamic_chunks  1: BFS CTAs take frontier chunks from a counter
  *                       instead of round-robin (0..1, 0)

@@ -138,10 +138,11 @@ def test_batch_block_size_knobs(block, ctas, bu):
         H.tune_reset()
 
 
-@pytest.mark.parametrize("alpha,beta", [(1, 1 << 20), (1 << 20, 1), (14, 24)])
+@pytest.mark.parametrize("alpha,beta", [(1, 1 << 20), (1 << 20, 1), (14, 24), (1 << 20, 1 << 20)])
 def test_batch_bottom_up_switching(alpha, beta):
-    """Bottom-up levels from the first level on (alpha 1), never (huge
-    alpha), and the default switch: distances and statistics unchanged."""
+    """Bottom-up levels for the largest frontiers only (alpha 1), never (beta
+    1: no frontier holds all vertices), from alpha 14 and beta 24, and from the
+    first level on (both huge): distances and statistics unchanged."""
     g = T.rmat_graph(12, 16, seed=23)
     h = build(g)
     srcs = np.arange(0, 4096, 97, dtype=np.int32)
@@ -201,4 +202,93 @@ def test_batch_levels_without_a_touched_list(extra, slots):
             out, st = H.BfsTopDown(h).run_batch(srcs)
             check(out, st, ref, ref_stats)
     finally:
+        H.tune_reset()
+
+
+def one_way_layers(width, layers):
+    """Vertex 0, then layers of `width` vertices with four edges each to the
+    next layer; the last layer has no edges.  Nothing leads back."""
+    n = 1 + width * layers
+    at = 1 + width * np.arange(layers)
+    i = np.arange(width)
+    src, dst = [np.zeros(width, np.int64)], [at[0] + i]
+    for a, b in zip(at[:-1], at[1:]):
+        for step in (0, 1, 3, 7):
+            src.append(a + i)
+            dst.append(b + (i + step) % width)
+    return one_way(n, np.concatenate(src), np.concatenate(dst))
+
+
+def one_way(n, src, dst):
+    order = np.lexsort((dst, src))
+    off = np.zeros(n + 1, np.int64)
+    np.add.at(off, src + 1, 1)
+    return O.Csr(np.cumsum(off), dst[order].astype(np.int32))
+
+
+@pytest.mark.parametrize("width,layers", [(30, 20), (1000, 20), (1000, 3)])
+@pytest.mark.parametrize("slots", [1, 9])
+def test_batch_one_way_graph(width, layers, slots):
+    """Edges stored one way only: no level may look for predecessors in a
+    vertex's own list, whichever directions are allowed."""
+    g = one_way_layers(width, layers)
+    h = build(g)
+    srcs = (np.arange(slots) * 7 % (1 + width)).astype(np.int32)
+    ref, ref_stats = oracle_slots(g, srcs, range(slots), slots)
+    try:
+        for alpha, beta in ((4, 24), (14, 24), (1 << 20, 1 << 20)):
+            H.tune_set("bfs.do_alpha", alpha)
+            H.tune_set("bfs.do_beta", beta)
+            for _ in range(2):
+                out, st = H.BfsTopDown(h).run_batch(srcs)
+                check(out, st, ref, ref_stats)
+    finally:
+        H.tune_reset()
+
+
+def test_batch_graph_loses_and_regains_an_edge():
+    """A symmetric graph, the same after updates that store the only edge to
+    a vertex one way, and after one that stores it both ways again."""
+    core = T.rmat_graph(11, 16, seed=17)
+    n = core.nV + 1
+    s, d = core.coo()
+    hub = int(np.diff(core.off).argmax())
+    g = one_way(n, np.concatenate([s, [hub, n - 1]]), np.concatenate([d, [n - 1, hub]]))
+    h = build(g)
+    srcs = np.concatenate([[hub], np.arange(0, 2000, 61)]).astype(np.int32)
+
+    def same():
+        ref, ref_stats = oracle_slots(g, srcs, range(len(srcs)), len(srcs))
+        out, st = H.BfsTopDown(h).run_batch(srcs)
+        check(out, st, ref, ref_stats)
+
+    try:
+        H.tune_set("bfs.do_alpha", 1 << 20)
+        H.tune_set("bfs.do_beta", 1 << 20)
+        same()
+        back = np.array([n - 1], np.int32), np.array([hub], np.int32)
+        assert h.erase(H.BatchUpdate(h, *back)) == 1
+        g, _ = O.erase(g, *back, 0)
+        same()
+        assert h.insert(H.BatchUpdate(h, *back), True, True) == 1
+        g, _ = O.insert(g, *back, 3)
+        same()
+    finally:
+        H.tune_reset()
+
+
+@pytest.mark.parametrize("run", [lambda: test_batch_bottom_up_switching(1 << 20, 1 << 20),
+                                 lambda: test_batch_bottom_up_long_lists(256),
+                                 lambda: test_batch_one_way_graph(1000, 3, 9),
+                                 test_batch_graph_loses_and_regains_an_edge])
+def test_batch_small_graphs_checked_for_one_way_edges(run):
+    """The check for edges stored one way, and the pulls after it, on graphs
+    below the size from which it is made by default."""
+    H.tune_set("msbfs.check_min", 1)
+    H.profile_enable(True)
+    try:
+        run()
+        assert "k_ms_one_way" in H.profile_report()
+    finally:
+        H.profile_enable(False)
         H.tune_reset()
