@@ -410,6 +410,7 @@ struct BfsArgs {
     int alpha, beta;             // direction switch (DO)
     int first;                   // 1: a new BFS (0: the next levels of one)
     int max_levels;
+    unsigned wait_polls;         // limit of a wait at the grid barrier
 };
 
 // Warp-private shared memory of the grid-wide levels.
@@ -1144,7 +1145,7 @@ __device__ __forceinline__ void grid_sync(const BfsArgs& a, Seal seal) {
     BfsCtl* ctl = a.ctl;
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (!grid_barrier(&ctl->bar, lo.gen, seal)) {
+        if (!grid_barrier(&ctl->bar, lo.gen, a.wait_polls, seal)) {
             *(volatile int*)&a.out->error = HN_ERR_TIMEOUT;
             lo.error = 1;
         }
@@ -1689,6 +1690,7 @@ void launch_run(hn_graph* g, BfsGraph& bg, int src, int32_t* dist, BfsOut* out,
     // bfs.host_levels: one launch per level, so that each can be profiled
     const bool host_driven = knob(kKnobBfsHostLevels) != 0;
     a.max_levels = host_driven ? 1 : INT_MAX;
+    a.wait_polls = (unsigned)knob(kKnobGridWaitPolls);
     cudaEvent_t ev0 = nullptr;
     if (g_profiling) profile_begin(s, &ev0);
     while (true) {
@@ -1791,7 +1793,8 @@ void bfs_run(hn_graph* g, const int32_t* sources, int k, int32_t* dist, int mem,
             if (bg.kernel) {
                 res[i] = bg.h_out[r];
                 if (res[i].error) {
-                    // waits that gave up leave the barrier mid-count
+                    // the sources queued behind this one were refused at
+                    // their first barrier (kGridDead), and have finished
                     HN_CUDA(cudaMemsetAsync(bg.ctl, 0, sizeof(BfsCtl), s));
                     HN_CUDA(cudaStreamSynchronize(s));
                     throw Error(HN_ERR_TIMEOUT, "BFS: a bounded wait gave up");

@@ -68,6 +68,7 @@ const KnobDef kKnobs[kNumKnobs] = {
     {"update.in_place", 1, 0, 1, false},
     {"update.own_sort", 1, 0, 1, false},
     {"msbfs.check_min", 1 << 23, 1, 1ll << 32, false},
+    {"grid.wait_polls", 1 << 24, 1024, 1 << 24, false},
 };
 std::atomic<long long> g_knob[kNumKnobs];
 // every knob starts at its default (static initialisation, in definition

@@ -177,6 +177,7 @@ enum Knob {
     kKnobUpdateInPlace,
     kKnobUpdateOwnSort,
     kKnobMsCheckMin,
+    kKnobGridWaitPolls,
     kNumKnobs
 };
 long long knob(Knob k);

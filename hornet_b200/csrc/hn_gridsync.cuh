@@ -7,33 +7,40 @@
 namespace hn {
 
 // In device memory, zeroed once; a launch that ends without a timeout leaves
-// it ready for the next.
+// it ready for the next.  After a timeout `arrive` may count CTAs that have
+// left, and a barrier counted on from it would open with CTAs still outside.
+// So the wait that gives up sets kGridDead in it, which no barrier clears:
+// every later barrier of this launch, and of launches queued behind it, is
+// refused until the host zeroes the struct.
 struct GridBar {
-    unsigned arrive;   // CTAs at the barrier
+    unsigned arrive;   // CTAs at the barrier, kGridDead
     unsigned gen;      // barriers passed
     unsigned beat;     // moved by a CTA that works on while the others wait
     unsigned pad;
 };
-
-// Polls without progress (neither the barrier nor `beat` moved) before a wait
-// gives up: seconds.
-constexpr unsigned kGridWait = 1u << 24;
+constexpr unsigned kGridDead = 1u << 31;
 
 // One thread of each CTA, between two __syncthreads.  The last CTA to arrive
 // runs `seal` before it opens the barrier.  `gen` is the CTA's count of
 // barriers passed, first read from bar->gen before the CTA's first arrival.
-// Writes before the barrier are visible to every CTA after it.  False: the
-// wait gave up, and the CTA must leave the kernel.
+// `limit`: polls without progress (neither the barrier nor `beat` moved) before
+// a wait gives up (the grid.wait_polls knob; its default is seconds).
+// Writes before the barrier are visible to every CTA after it.  False: a wait
+// gave up, here or in another CTA, and the CTA must leave the kernel.
 template <typename Seal>
-__device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned& gen, Seal seal) {
+__device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned& gen, unsigned limit,
+                                             Seal seal) {
     bool ok = true;
     __threadfence();
-    if (atomicAdd(&bar->arrive, 1u) == gridDim.x - 1) {
+    const unsigned before = atomicAdd(&bar->arrive, 1u);
+    if (before == gridDim.x - 1) {
         __threadfence();
         seal();
-        bar->arrive = 0;
+        atomicSub(&bar->arrive, gridDim.x);   // (not a store: kGridDead stays)
         __threadfence();
         atomicAdd(&bar->gen, 1u);
+    } else if (before & kGridDead) {
+        ok = false;
     } else {
         unsigned polls = 0, beat = 0;
         while (*(volatile unsigned*)&bar->gen == gen) {
@@ -44,7 +51,8 @@ __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned& gen, Seal s
                     beat = b;
                     polls = 64;
                 }
-                if (polls >= kGridWait) {
+                if (polls >= limit || (*(volatile unsigned*)&bar->arrive & kGridDead)) {
+                    atomicOr(&bar->arrive, kGridDead);
                     ok = false;
                     break;
                 }

@@ -371,6 +371,7 @@ struct KtArgs {
     int32_t* state;
     int32_t* sup;
     int32_t* truss;
+    unsigned wait_polls;      // limit of a wait at the grid barrier
 };
 
 // x loses a triangle; the thread that takes it below K - 2 puts it on the
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(kKtThreads, 1) k_kt_run(const __grid_constant_
     auto sync = [&](auto seal) {
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (!grid_barrier(&ctl->bar, s_gen, seal)) {
+            if (!grid_barrier(&ctl->bar, s_gen, a.wait_polls, seal)) {
                 *(volatile int*)&ctl->error = HN_ERR_TIMEOUT;
                 s_error = 1;
             }
@@ -768,7 +769,8 @@ int ktruss_run(hn_graph* g, int32_t* d_edge_truss) {
             h.minsup = INT_MAX;
             HN_CUDA(cudaMemcpyAsync(ctl.get(), &h, sizeof(KtCtl), cudaMemcpyHostToDevice, s));
             KtArgs a{ctl.get(), loff, ladj, lcanon, lm, {F.get(), NF.get()}, {L.get(), L2.get()},
-                     src.get(), adj.get(), state.get(), sup.get(), truss.get()};
+                     src.get(), adj.get(), state.get(), sup.get(), truss.get(),
+                     (unsigned)knob(kKnobGridWaitPolls)};
             void* args[] = {&a};
             cudaEvent_t ev = nullptr;
             if (g_profiling) profile_begin(s, &ev);
