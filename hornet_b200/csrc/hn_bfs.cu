@@ -1784,6 +1784,13 @@ void bfs_run(hn_graph* g, const int32_t* sources, int k, int32_t* dist, int mem,
     // copy stream drains buffer (i - 1) % 2 to the host
     DevBuf<int32_t> d_dist;
     if (host_out) d_dist.alloc((size_t)2 * nV, s);
+    // an early end waits for the copies before d_dist and the caller's array go
+    struct CopiesEnd {
+        cudaStream_t copy;
+        ~CopiesEnd() {
+            if (copy) cudaStreamSynchronize(copy);
+        }
+    } copies_end{host_out ? bg.copy : nullptr};
     std::vector<BfsOut> res((size_t)k);
     // results of the ring entries of sources [from, to)
     auto collect = [&](int from, int to) {

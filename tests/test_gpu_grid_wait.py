@@ -69,6 +69,31 @@ def test_bfs_wait_gives_up():
         H.tune_reset()
 
 
+def test_bfs_wait_gives_up_with_copies_queued():
+    """Distances to pinned host memory: when the call has reported the error,
+    no copy into the caller's array is still to come."""
+    import torch
+    h, dist = hub_off_the_frontier(1_000_000)
+    out = torch.empty((70, len(dist)), dtype=torch.int32, pin_memory=True).numpy()
+    bfs = H.BfsTopDown(h)
+    try:
+        for k, v in BOTTOM_UP.items():
+            H.tune_set(k, v)
+        H.tune_set("grid.wait_polls", 1024)
+        with pytest.raises(H.HornetError) as e:
+            bfs.run_multi([0] * 70, out=out, direction_optimizing=True)
+        out[:, -1] = -7
+        assert e.value.code == H.HN_ERR_TIMEOUT
+        torch.cuda.synchronize()
+        assert (out[:, -1] == -7).all()
+        H.tune_set("grid.wait_polls", 1 << 24)
+        bfs.run_multi([0] * 70, out=out, direction_optimizing=True)
+        for i in (0, 1, 63, 64, 69):
+            np.testing.assert_array_equal(out[i], dist)
+    finally:
+        H.tune_reset()
+
+
 def test_ktruss_wait_gives_up():
     h = double_star(200_000)
     kt = H.KTruss(h)
