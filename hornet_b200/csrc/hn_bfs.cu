@@ -842,6 +842,9 @@ __device__ __noinline__ void frontier_bits() {
 // measured 5 % slower).  A warp owns whole words of the visited and
 // next-frontier bitmaps, so both are written with plain stores.
 constexpr int kBuLane = 16;
+// Entries of long lists that a warp reads between two signs of progress (2,048
+// steps, 1.2 ms): its share of a level has no bound but the edge count.
+constexpr int kBuBeat = 1 << 17;
 
 __device__ __noinline__ int bottom_up_level() {
     const LevelSmem& lo = level_smem();
@@ -862,6 +865,7 @@ __device__ __noinline__ int bottom_up_level() {
     const unsigned units = ((unsigned)nV + kWChunk - 1) >> kChunkShiftWarp;
     const unsigned nwords = ((unsigned)nV + 31) / 32;
     unsigned long long queued = 0;   // (degree sum << 32) | vertices with edges
+    int beat = 0;                    // entries of long lists since the last sign of progress
     for (unsigned c = gw; c < units; c += nwarps) {
         const unsigned word = c * kWIpt + lane;
         const bool own = lane < kWIpt && word < nwords;
@@ -910,6 +914,11 @@ __device__ __noinline__ int bottom_up_level() {
                     unsigned any = x >= 0 ? __ldca(fb + (x >> 5)) >> (x & 31) : 0u;
                     any |= y >= 0 ? __ldca(fb + (y >> 5)) >> (y & 31) : 0u;
                     got = __any_sync(kFull, any & 1u);
+                    beat += 64;
+                    if (beat >= kBuBeat) {
+                        if (lane == 0) grid_progress(&a.ctl->bar);
+                        beat = 0;
+                    }
                 }
                 if (lane == l) hit = got;
             }
@@ -1090,6 +1099,7 @@ __device__ __noinline__ int small_levels() {
                 out->t_end[level - 1] = global_ns();
                 out->lvl_edges[level - 1] = total;
             }
+            // (a store: only this CTA works, and a 5 us level feels an atomic)
             *(volatile unsigned*)&ctl->bar.beat = (unsigned)level;
         }
         cur = nx;

@@ -15,10 +15,14 @@ namespace hn {
 struct GridBar {
     unsigned arrive;   // CTAs at the barrier, kGridDead
     unsigned gen;      // barriers passed
-    unsigned beat;     // moved by a CTA that works on while the others wait
+    unsigned beat;     // moved by CTAs that work on while others wait (grid_progress)
     unsigned pad;
 };
 constexpr unsigned kGridDead = 1u << 31;
+
+// Work of one CTA or warp between two barriers that may take longer than a
+// wait's limit tells the others, every few milliseconds, that it goes on.
+__device__ __forceinline__ void grid_progress(GridBar* bar) { atomicAdd(&bar->beat, 1u); }
 
 // One thread of each CTA, between two __syncthreads.  The last CTA to arrive
 // runs `seal` before it opens the barrier.  `gen` is the CTA's count of

@@ -342,6 +342,7 @@ constexpr int kKtThreads = 1024;
 constexpr int kKtFew = 512;      // edges staged per CTA
 constexpr int kKtSolo = 16;      // edges that CTA 0 takes alone
 constexpr int kKtSoloMax = 64;
+constexpr int kKtBeat = 256;     // chunks of a warp between two signs of progress (1 ms with lists of 4 M)
 static_assert(kKtSoloMax <= kKtFew, "CTA 0 stages its frontiers");
 constexpr int kAlive = INT_MAX;
 
@@ -473,6 +474,7 @@ __global__ void __launch_bounds__(kKtThreads, 1) k_kt_run(const __grid_constant_
         load();
     }
     __syncthreads();
+    int beat = 0;   // chunks since this warp's last sign of progress
     while (true) {
         // the frontier of K: alive edges with support < K - 2
         {
@@ -538,6 +540,10 @@ __global__ void __launch_bounds__(kKtThreads, 1) k_kt_run(const __grid_constant_
                     }
                     const int i = (c - s_pre[lo]) * 32 + lane;
                     if (i < s_na[lo]) probe(s_e[lo], s_pa[lo], s_pb[lo], s_nb[lo], i, r, n_next);
+                    if (++beat == kKtBeat) {
+                        if (lane == 0) grid_progress(&ctl->bar);
+                        beat = 0;
+                    }
                 }
             };
             // the round is over: its counters are free for the one after next
@@ -551,7 +557,7 @@ __global__ void __launch_bounds__(kKtThreads, 1) k_kt_run(const __grid_constant_
                     while (n > 0 && n <= (r == round ? kKtSolo : kKtSoloMax)) {
                         if (threadIdx.x == 0) {
                             s_next = 0;
-                            vc->bar.beat = (unsigned)r;
+                            grid_progress(&ctl->bar);
                         }
                         __syncthreads();
                         few(0, n, r, warp, NW, &s_next);
@@ -584,6 +590,7 @@ __global__ void __launch_bounds__(kKtThreads, 1) k_kt_run(const __grid_constant_
                 for (int f0 = blockIdx.x * per; f0 < end; f0 += kKtFew) {
                     few(f0, min(kKtFew, end - f0), round, warp, NW, n_next);
                     __syncthreads();   // the staged edges are replaced
+                    if (threadIdx.x == 0) grid_progress(&ctl->bar);
                 }
             }
             if (!sync(end_round)) return;

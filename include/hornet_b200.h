@@ -161,7 +161,8 @@ int hn_profile_report(char* buf, int64_t len);
  *   grid.wait_polls     polls without progress after which a CTA of a
  *                       one-launch BFS or k-truss stops waiting for the others
  *                       and the call returns HN_ERR_TIMEOUT; the default is
- *                       some ten seconds (1024..2^24, 2^24)
+ *                       a few seconds, 1024 a quarter of a millisecond
+ *                       (1024..2^24, 2^24)
  * hn_tune_name(i) enumerates the names (NULL past the last one). */
 int hn_tune_set(const char* name, int64_t value);
 int hn_tune_get(const char* name, int64_t* value);

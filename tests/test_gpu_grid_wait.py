@@ -1,6 +1,6 @@
 """Waits of the cooperative launches (one-launch BFS, k-truss rounds) that run
-out: the limit is set to a fraction of a millisecond and one warp or CTA has
-a list of 200,000 neighbours to read while the others wait.  The call
+out: the limit is set to a quarter of a millisecond and one warp or CTA has
+a long list to read while the others wait.  The call
 reports HN_ERR_TIMEOUT, and the next call on the handle is right."""
 import numpy as np
 import pytest
@@ -94,8 +94,27 @@ def test_bfs_wait_gives_up_with_copies_queued():
         H.tune_reset()
 
 
+def test_slow_work_is_progress():
+    """A warp that reads 4 M neighbours (37 ms), and a CTA that intersects lists
+    of 6 M (25 ms), take several times as long as the limit (8 and 4 ms) but
+    tell the others every 1.2 and 1 ms that they go on."""
+    h, dist = hub_off_the_frontier(4_000_000)
+    try:
+        for k, v in BOTTOM_UP.items():
+            H.tune_set(k, v)
+        H.tune_set("grid.wait_polls", 1 << 15)
+        out, _ = H.BfsTopDown(h).run_multi([0], direction_optimizing=True)
+        np.testing.assert_array_equal(out[0], dist)
+        H.tune_set("grid.wait_polls", 1 << 14)
+        kt = H.KTruss(double_star(6_000_000))
+        assert kt.run() == 2
+        assert (kt.edge_truss == 2).all()
+    finally:
+        H.tune_reset()
+
+
 def test_ktruss_wait_gives_up():
-    h = double_star(200_000)
+    h = double_star(800_000)
     kt = H.KTruss(h)
     try:
         H.tune_set("grid.wait_polls", 1024)
