@@ -1604,6 +1604,7 @@ extern "C" int hn_tc_owner(hn_graph_t* g, uint64_t* counts, int mem, uint64_t* t
     HN_API_BEGIN
     HN_REQUIRE(g && counts, "null argument");
     HN_REQUIRE(mem == HN_MEM_HOST || mem == HN_MEM_DEVICE, "bad memory kind");
+    HandleUse use(g);
     HN_CUDA(cudaSetDevice(g->device));
     cudaStream_t s = g->stream;
     if (g->nV == 0) {

@@ -121,3 +121,32 @@ def test_close_ids_use_bitmaps_of_ids(case):
             np.testing.assert_array_equal(ow, ow0)
         finally:
             H.tune_reset()
+
+
+def test_a_busy_handle_is_refused():
+    """Owner counts called on a handle that another thread is counting on:
+    each call returns the counts or HN_ERR_STATE."""
+    import threading
+    g = T.rmat_graph(18, 16, seed=7)
+    h = build(g)
+    ref = O.tc(g)
+    assert owner(h)[1] == ref
+    codes, wrong, start = [], [], threading.Barrier(2)
+
+    def count():
+        start.wait()
+        for _ in range(50):
+            try:
+                if owner(h)[1] != ref:
+                    wrong.append(1)
+                codes.append(0)
+            except H.HornetError as e:
+                codes.append(e.code)
+
+    threads = [threading.Thread(target=count) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong and set(codes) == {0, H.HN_ERR_STATE}
+    assert owner(h)[1] == ref
