@@ -1279,9 +1279,18 @@ void build_oriented(hn_graph* g, Oriented& o, const int32_t* canon) {
     HN_LAUNCH(k_orient_flags, grid, kB, 0, s, o.prefix.get(), nV, g->vtab, g->pool, pos.get(),
               splits.get(), (long long)splits.n - 1);
     exclusive_scan(g, (const int32_t*)pos.get(), pos.get(), m + 1, s);
+    // arrays of the kept edges alone, about half of m (a count above 2^31 would
+    // not fit its 32 bits: the bound then)
+    o.total = m;
+    if (m <= INT_MAX) {
+        HN_CUDA(cudaMemcpyAsync(g->h_scalar + 5, pos.get() + m, sizeof(int32_t),
+                                cudaMemcpyDeviceToHost, s));
+        HN_CUDA(cudaStreamSynchronize(s));
+        o.total = *(const int*)(g->h_scalar + 5);
+    }
     o.offp.alloc((size_t)nV + 1, s);
-    o.fwd.alloc((size_t)(m + 4), s);
-    if (canon) o.feid.alloc((size_t)(m + 4), s);
+    o.fwd.alloc((size_t)(o.total + 4), s);
+    if (canon) o.feid.alloc((size_t)(o.total + 4), s);
     HN_LAUNCH(k_orient_fill, grid, kB, 0, s, o.prefix.get(), nV, g->vtab, g->pool, pos.get(),
               o.fwd.get(), o.offp.get(), splits.get(), (long long)splits.n - 1, canon,
               canon ? o.feid.get() : (int32_t*)nullptr);
@@ -1358,12 +1367,16 @@ static bool build_padded(hn_graph* g, Oriented& o) {
     HN_LAUNCH(k_padded, grid_for(g, (long long)nV + 1, kB), kB, 0, s, (const int*)o.dplus.get(),
               nV, cnt.get());
     exclusive_scan(g, (const int*)cnt.get(), o.offp.get(), (long long)nV + 1, s);
+    HN_CUDA(cudaMemcpyAsync(g->h_scalar + 5, o.offp.get() + nV, sizeof(long long),
+                            cudaMemcpyDeviceToHost, s));
     HN_CUDA(cudaStreamSynchronize(s));
     if (((const int*)(g->h_scalar + 4))[1] > knob(kKnobTcCtaTableCap)) return false;
-    o.fwd.alloc((size_t)(m + 3ll * nV + 4), s);
+    o.total = g->h_scalar[5];
+    o.fwd.alloc((size_t)(o.total + 4), s);
     orient(std::true_type());
     HN_LAUNCH(k_pad_lists, grid_for(g, nV, kB), kB, 0, s, (const long long*)o.offp.get(),
               (const int*)o.dplus.get(), nV, o.fwd.get());
+    o.prefix.release();
     o.padded = true;
     o.ranked = ranked;
     return true;
@@ -1378,8 +1391,7 @@ void build_candidates(hn_graph* g, const Oriented& o, DevBuf<long long>& coff,
                       DevBuf<int32_t>& cand, DevBuf<int32_t>* ceid) {
     cudaStream_t s = g->stream;
     const int nV = g->nV;
-    // bound on the oriented entries, pads included (their number is read on the device)
-    const long long m = g->nE + (o.padded ? 3ll * nV : 0);
+    const long long m = o.total;
     const long long ntiles = (m + nV + kOrientTile - 1) / kOrientTile;
     const long long grid = (ntiles + kB / 32 - 1) / (kB / 32);
     DevBuf<long long> splits, fbase((size_t)nV, s);

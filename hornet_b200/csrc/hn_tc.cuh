@@ -6,11 +6,12 @@
 namespace hn {
 
 struct Oriented {
-    DevBuf<long long> prefix;  // degree prefix of the undirected graph (nV+1)
+    DevBuf<long long> prefix;  // degree prefix of the undirected graph (nV+1; while it is built)
     DevBuf<long long> offp;    // oriented offsets (nV+1)
     DevBuf<int32_t> fwd;       // oriented, sorted neighbour lists
     DevBuf<int32_t> feid;      // edge id of each fwd entry (when built with canon)
     DevBuf<int> dplus;         // oriented degrees (nV)
+    long long total = 0;       // entries of fwd, pads included
     // build_for_counting: offp and dplus are indexed by number (the id, or
     // ranked 0 = highest rank) and fwd holds numbers, in the order of ids;
     // padded: each list starts on 16 bytes and is padded to four entries
