@@ -1182,7 +1182,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     Arena* ar = arena.cap ? &arena : nullptr;
     const bool small = n <= kSmallBatch && !g->weighted && !new_triangles;
     DevBuf<int32_t> cdst(n, s, ar), cseg(n, s, ar), seg_u(n, s, ar), seg_kstart(n + 1, s, ar),
-        seg_ncap(n, s, ar), seg_base(n, s, ar), capos(n, s, ar), big_list(n + 1, s, ar);
+        seg_ncap(n, s, ar), seg_base(n, s, ar), capos(n, s, ar), big_list;
     DevBuf<long long> seg_work(n + 1, s, ar), seg_new_off(n, s, ar), seg_old_off(n, s, ar);
     DevBuf<uint32_t> cw;
     long long* totals = g->d_scalar;
@@ -1191,6 +1191,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     const int big_min = g->weighted ? INT_MAX : (int)knob(kKnobUpdateBigMin);
     const bool in_place = !g->weighted && knob(kKnobUpdateInPlace) != 0;
     if (small) {
+        big_list.alloc(n + 1, s, ar);
         SmallPlan* h_plan = (SmallPlan*)g->h_scalar;
         if (insert)
             HN_LAUNCH(k_small_front<true>, 1, kSmallThreads, 0, s, b->src, b->dst, sorted, (int)n,
@@ -1273,6 +1274,7 @@ void run_update(hn_graph* g, hn_batch* b, unsigned flags, bool insert, int64_t* 
     keys2.release();
     scan.release();
     // 4. plan
+    big_list.alloc(n + 1, s, ar);   // (in the keys' place)
     DevBuf<unsigned long long> big_ctr(2, s, ar);   // [0] hubs listed, [1] snapshot slots
     HN_CUDA(cudaMemsetAsync(big_ctr.get(), 0, 2 * sizeof(unsigned long long), s));
     HN_LAUNCH(k_plan, grid_for(g, n + 1, kB), kB, 0, s, seg_u.get(), seg_kstart.get(), totals,

@@ -54,3 +54,18 @@ def test_triangle_counts(scale, flip, cap):
         assert peak(tc.run) < bound
     finally:
         H.tune_reset()
+
+
+@pytest.mark.parametrize("n", [(1 << 20) + 1, 3_000_003])
+def test_large_updates(n):
+    """Keys twice, their places and counters (32 bytes an entry) and the plan's
+    arrays (48); the list of hubs takes the keys' place."""
+    import torch
+    h = rmat(18, 16)
+    s = torch.empty(n, dtype=torch.int32, device="cuda")
+    d = torch.empty_like(s)
+    H.gen_rmat_device(18, n, 9, s, d, a=0.25, b=0.25, c=0.25)
+    torch.cuda.synchronize()
+    b = H.BatchUpdate(h, s, d)
+    assert peak(lambda: h.insert(b, True, True)) < 81 * n
+    assert peak(lambda: h.erase(b, True)) < 81 * n
