@@ -1668,11 +1668,28 @@ BfsGraph& bfs_graph_of(hn_graph* g) {
     return *g->bfs;
 }
 
+constexpr int64_t kShareMax = 1 << 26;   // edges
+
+hn_graph* bfs_root(hn_graph* g) { return g->parent ? g->parent : g; }
+
 // Launches one BFS from `src` into `dist` with k_bfs_run; its result arrives
 // in `out` (pinned).
 void launch_run(hn_graph* g, BfsGraph& bg, int src, int32_t* dist, BfsOut* out,
                 bool direction_optimizing) {
     cudaStream_t s = g->stream;
+    // A cooperative launch of a CTA on every SM leaves no room for another one,
+    // so BFS calls on several views would queue, though a small traversal has
+    // work for few CTAs.  Each call takes its share of the SMs instead.  us per
+    // BFS with 1 / 2 / 4 / 8 views at work, queued and shared: street grid 3390 /
+    // 3370 / 3350 / 3350 and 3390 / 2120 / 1270 / 740; R-MAT scale 12 70 / 47 / 46
+    // / 46 and 70 / 41 / 22 / 16, scale 16 91 / 72 / 71 / 78 and 93 / 50 / 28 / 20,
+    // scale 20 234 / 214 / 214 / 216 and 232 / 177 / 155 / 141.  Larger ones fill
+    // the GPU (scale 22: 278 queued, 259 / 220 / 195 shared), and the second of
+    // two calls alone would have half of it (scale 25 under load: no difference).
+    unsigned grid = bg.grid;
+    if (g->nE <= kShareMax)
+        grid = std::max(1u, grid / (unsigned)std::max(1, bfs_root(g)->bfs_running.load(
+                                                             std::memory_order_relaxed)));
     void* fn = direction_optimizing ? (void*)k_bfs_run<true> : (void*)k_bfs_run<false>;
     // set per call: the attribute belongs to the device in use
     HN_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem));
@@ -1705,7 +1722,7 @@ void launch_run(hn_graph* g, BfsGraph& bg, int src, int32_t* dist, BfsOut* out,
     if (g_profiling) profile_begin(s, &ev0);
     while (true) {
         void* args[] = {&a};
-        HN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(bg.grid), dim3(bg.threads), args, kRunSmem, s));
+        HN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(bg.threads), args, kRunSmem, s));
         count_launch();
         if (!host_driven) break;
         HN_CUDA(cudaStreamSynchronize(s));
@@ -1788,6 +1805,11 @@ void bfs_run(hn_graph* g, const int32_t* sources, int k, int32_t* dist, int mem,
     // edge offsets are 32-bit, and a chunk's end (offset + 256) must not wrap
     if (g->nE > 0xFFFFFE00ll) throw Error(HN_ERR_CAPACITY, "BFS needs nE < 2^32 - 512");
     if (k == 0) return;
+    struct Running {
+        std::atomic<int>& n;
+        explicit Running(std::atomic<int>& c) : n(c) { n.fetch_add(1, std::memory_order_relaxed); }
+        ~Running() { n.fetch_sub(1, std::memory_order_relaxed); }
+    } running(bfs_root(g)->bfs_running);
     BfsGraph& bg = bfs_graph_of(g);
     const bool host_out = mem == HN_MEM_HOST;
     // host output: two device buffers; BFS i writes buffer i % 2 while the

@@ -256,6 +256,8 @@ struct hn_graph {
 
     // set while a call that uses this handle's stream and scratch runs
     std::atomic<int> in_use{0};
+    // BFS calls running on this graph and its views (counted on the graph)
+    std::atomic<int> bfs_running{0};
 };
 
 namespace hn {

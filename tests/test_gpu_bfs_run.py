@@ -91,3 +91,33 @@ def test_unaligned_distance_rows():
     assert out[0] == -7
     for i, s in enumerate(srcs):
         np.testing.assert_array_equal(out[1 + i * 3001:1 + (i + 1) * 3001], O.bfs(g, s)[0])
+
+
+@pytest.mark.parametrize("views", [2, 3, 8])
+def test_views_share_the_gpu(views):
+    """BFS calls on several views at once: launches of all grid sizes from the
+    whole GPU to a share of it, also down to one CTA's levels."""
+    import threading
+    import torch
+    g = shape("rmat")
+    h = build(g)
+    vs = [h.view() for _ in range(views)]
+    srcs = [0, g.nV - 1, g.nV // 2, 5]
+    refs = np.stack([O.bfs(g, s)[0] for s in srcs])
+    wrong, start = [], threading.Barrier(views)
+
+    def traverse(i):
+        bfs = H.BfsTopDown(vs[i])
+        out = torch.empty((len(srcs), g.nV), dtype=torch.int32, device="cuda:0")
+        start.wait()
+        for r in range(10):
+            bfs.run_multi(srcs, out=out, direction_optimizing=(i + r) % 2 == 1)
+            if not (out.cpu().numpy() == refs).all():
+                wrong.append((i, r))
+
+    threads = [threading.Thread(target=traverse, args=(i,)) for i in range(views)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
