@@ -1450,11 +1450,9 @@ void launch_counting(hn_graph* g, const TcView& view, unsigned long long* d_coun
     constexpr bool by_rank = WIN == kRankWin;
     // lists by rank are not sorted: nothing to narrow
     const int narrow_min = by_rank ? INT_MAX : (int)knob(kKnobTcNarrowMin);
-    // by rank, with a bitmap to set up per item and cheaper pairs: items four
-    // times as long on graphs with enough of them (rmat scale 22, 46,000 items:
-    // 30.6 -> 27.3 ms)
-    const long long warp_work = knob(kKnobTcWarpWork);
-    const long long item_work = knob(kKnobTcItemWork) * (by_rank && g->nE >= (1ll << 26) ? 4 : 1);
+    // (items of 2^20 pairs by rank instead of 2^18: R-MAT graphs of 63 and 69 M
+    // edges 9.0 -> 9.3 and 8.9 -> 9.1 ms, of 128 M edges 17.2 -> 17.1)
+    const long long warp_work = knob(kKnobTcWarpWork), item_work = knob(kKnobTcItemWork);
     constexpr bool eid = MODE == 3;
     const int cap_max = eid ? kCtaCapEid : kCtaCap;
     // (the bitmap holds most members: a smaller table leaves room for four CTAs
