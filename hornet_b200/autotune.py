@@ -7,10 +7,15 @@ The knobs are load-balancing bin thresholds and launch shapes:
   tc.warp_ctas_per_sm — grid of the warp kernel;
 * msbfs.block — block size of the batched BFS (128/256/512 threads, the
   same 2048-edge chunks); msbfs.ctas_per_sm — its grid;
-* bfs.kernel — the warp-chunk (1) or CTA-chunk (0) BFS level kernel;
+* bfs.kernel — the BFS in one launch (1) or a kernel per level (0);
   bfs.warp_ctas_per_sm / bfs.ctas_per_sm — their grids; bfs.dynamic_chunks —
-  frontier chunks taken from a counter instead of round-robin (CTA kernel);
-  bfs.do_alpha / do_beta — the direction-optimising switch thresholds.
+  frontier chunks taken from a counter instead of round-robin (kernel per
+  level); bfs.do_alpha / do_beta — the direction-optimising switch thresholds.
+
+A space holds no two values that are the same setting (bfs.warp_ctas_per_sm
+above 3 fills the SM like 3; tc.mid_cap above 2,048 is 2,048 wherever the
+counts use bitmaps), and a knob that another knob's value leaves without
+effect (REQUIRES) is not tried.
 
 `tune` runs coordinate descent over a knob space: every candidate value of a
 knob is timed (median of `reps` runs, after one warm-up run that also
@@ -35,7 +40,7 @@ import numpy as np
 from . import tune_get, tune_names, tune_reset, tune_set
 
 SPACES: Dict[str, Dict[str, List[int]]] = {
-    "bfs": {"bfs.kernel": [1, 0], "bfs.warp_ctas_per_sm": [2, 3, 4, 6, 8],
+    "bfs": {"bfs.kernel": [1, 0], "bfs.warp_ctas_per_sm": [1, 2, 4],
             "bfs.ctas_per_sm": [4, 6, 8, 9, 12, 16], "bfs.dynamic_chunks": [0, 1],
             "bfs.warp_strided": [0, 1]},
     "bfs_do": {"bfs.do_alpha": [4, 8, 14, 24, 48], "bfs.do_beta": [8, 24, 64, 256]},
@@ -43,9 +48,15 @@ SPACES: Dict[str, Dict[str, List[int]]] = {
               "msbfs.bottom_up": [0, 1]},
     "tc": {"tc.warp_cap": [64, 128, 256, 512], "tc.chunk": [4, 16, 64],
            "tc.warp_ctas_per_sm": [4, 8, 12, 16], "tc.narrow_min": [0, 8, 32, 128],
-           "tc.mid_cap": [1024, 2048, 4096], "tc.warp_work": [16384, 65536, 262144],
+           "tc.mid_cap": [512, 1024, 4096], "tc.warp_work": [16384, 65536, 262144],
            "tc.item_work": [65536, 262144, 1048576], "tc.flip": [0, 1],
            "tc.thread_du": [0, 8, 16, 32], "tc.thread_dc": [16, 32, 128]},
+}
+
+# knob -> (other knob, the value of it that the knob needs)
+REQUIRES: Dict[str, Tuple[str, int]] = {
+    "bfs.warp_ctas_per_sm": ("bfs.kernel", 1), "bfs.ctas_per_sm": ("bfs.kernel", 0),
+    "bfs.dynamic_chunks": ("bfs.kernel", 0), "bfs.warp_strided": ("bfs.kernel", 0),
 }
 
 DEFAULT_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned.json")
@@ -81,6 +92,8 @@ def tune(run: Callable[[], object], same: Callable[[object, object], bool],
     best_t = base_t
     log = [{"knobs": dict(best), "s": base_t, "default": True}]
     for knob, values in space.items():
+        if knob in REQUIRES and tune_get(REQUIRES[knob][0]) != REQUIRES[knob][1]:
+            continue
         start = best[knob]
         for v in values:
             if v == start:

@@ -100,15 +100,20 @@ int hn_profile_report(char* buf, int64_t len);
  *   msbfs.ctas_per_sm   batched-BFS CTAs per SM (1..8, 4)
  *   tc.warp_cap         oriented-degree bin boundary between the warp-per-
  *                       vertex and CTA-per-vertex counting kernels (32..512, 512)
- *   tc.chunk            vertices handed to a warp per atomic (1..256, 16)
+ *   tc.chunk            vertices handed to a warp per atomic, at most one in
+ *                       512 per SM of the graph's (1..256, 16)
  *   tc.narrow_min       candidate lists longer than this are first narrowed
- *                       to the [min, max] of N+(u) by two searches (0..1024, 0)
+ *                       to the [min, max] of N+(u) by two searches; hash
+ *                       tables under vertex ids only (0..1024, 0)
  *   tc.mid_cap          listed vertices (oriented degree above tc.warp_cap)
  *                       up to this go to the CTA kernel with small tables,
- *                       several CTAs per SM (32..4096, 4096)
+ *                       several CTAs per SM; 2048 at most beside bitmaps
+ *                       (32..4096, 4096)
  *   tc.cta_table_cap    table capacity of the CTA kernel for the larger
- *                       listed vertices; above it N+(u) is binary-searched
- *                       in global memory (32..16384, 16384)
+ *                       listed vertices.  One oriented list above it sends
+ *                       the whole count to hash tables under vertex ids,
+ *                       without bitmaps; that list is binary-searched in
+ *                       global memory (32..16384, 16384)
  *   tc.warp_work        bound on a vertex's pairs (candidates x d+(u)) for
  *                       the warp-per-vertex kernel; above it, or with d+(u)
  *                       above tc.warp_cap, the vertex goes to CTA work
@@ -135,15 +140,16 @@ int hn_profile_report(char* buf, int64_t len);
  *                       round-robin (coalesced loads) instead of 8
  *                       consecutive edges per thread (0..1, 0)
  *   bfs.host_levels     1: launch the BFS levels one by one from the host
- *                       (for per-level profiling) instead of the CUDA
- *                       graph's device-side loop (0..1, 0)
+ *                       (for per-level profiling) instead of all in one
+ *                       launch, or in the CUDA graph of bfs.kernel 0 (0..1, 0)
  *   bfs.kernel          1 = a BFS in one cooperative launch (independent warps
  *                       on 256-edge chunks), 0 = a kernel per level in a CUDA
  *                       graph, 128-thread CTAs on 1024-edge chunks
  *                       (bfs.ctas_per_sm, bfs.dynamic_chunks and
  *                       bfs.warp_strided apply to it) (0..1, 1)
  *   bfs.warp_ctas_per_sm  256s of threads per SM of the one-launch BFS, of
- *                       which three fill an SM's registers (1..8, 4)
+ *                       which three fill an SM's registers: 3 to 8 are the
+ *                       same (1..8, 4)
  *   ktruss.device_rounds  1: the peel rounds of all K run in cooperative
  *                       launches (no host round trip per round or K); 0: one
  *                       host round trip per round, launches sized to the
@@ -343,9 +349,11 @@ int hn_bfs_multi(hn_graph_t* g, const int32_t* sources, int32_t k,
 
 /* Direction-optimising BFS (top-down levels switch to bottom-up ones while
  * the frontier is large; the counterpart of hornetsnest's BottomUpBFS,
- * src/Static/BottomUpBreadthFirstSearch/BottomUpBFS.cu).  Same arguments
- * and the same distances as hn_bfs_multi; stats count the same edges
- * (sum of degrees of reached vertices), although fewer are read. */
+ * src/Static/BottomUpBreadthFirstSearch/BottomUpBFS.cu).  The graph must
+ * store every edge both ways: a bottom-up level takes a vertex's neighbours
+ * for its predecessors.  Same arguments and then the same distances as
+ * hn_bfs_multi; stats count the same edges (sum of degrees of reached
+ * vertices), although fewer are read. */
 int hn_bfs_do(hn_graph_t* g, const int32_t* sources, int32_t k, int32_t* dist,
               int mem, hn_bfs_stats_t* stats);
 

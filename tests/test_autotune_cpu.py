@@ -75,6 +75,26 @@ def test_search_spaces_and_saved_knobs_are_registered():
                 assert H.tune_get(knob) == v
 
 
+def test_every_trial_is_another_setting():
+    """No two values of a space are the same setting, and knobs that the best
+    values so far leave without effect are not timed."""
+    same_from = {"bfs.warp_ctas_per_sm": 3, "tc.mid_cap": 2048}
+    for space in A.SPACES.values():
+        for knob, values in space.items():
+            eff = [min(v, same_from.get(knob, v)) for v in values]
+            assert len(set(eff)) == len(eff), knob
+            default = min(H.tune_get(knob), same_from.get(knob, H.tune_get(knob)))
+            assert H.tune_get(knob) in values or default not in eff, knob
+    for kernel in (0, 1):
+        best, log = A.tune(lambda: time.sleep(0.001 if H.tune_get("bfs.kernel") == kernel else 0.02),
+                           lambda a, b: True, A.SPACES["bfs"], reps=1)
+        assert best["bfs.kernel"] == kernel
+        tried = {k for t in log for k, v in t["knobs"].items() if v != log[0]["knobs"][k]}
+        assert ("bfs.warp_ctas_per_sm" in tried) == (kernel == 1)
+        assert ("bfs.ctas_per_sm" in tried) == (kernel == 0)
+        H.tune_reset()
+
+
 def test_knobs_start_at_their_defaults():
     """In a fresh process every knob already holds its default before any
     hn_tune_reset (the values are not a second hand-kept list)."""
