@@ -30,7 +30,7 @@
 //
 // Two kernels share this frontier format (knob bfs.kernel):
 //   * k_bfs_run (default): the whole BFS in one cooperative launch of one CTA
-//     per SM, with a grid barrier between levels (about 2 us; a kernel per
+//     per SM (launch_run: fewer beside other BFS calls), with a grid barrier between levels (about 2 us; a kernel per
 //     level in a WHILE node cost 8-15 us, whatever the level held).  A level
 //     runs in one of four ways:
 //       - up to 4,096 frontier edges: CTA 0 alone, level after level without
@@ -51,10 +51,11 @@
 //     shared memory and a CTA-wide enqueue (one atomic per chunk).
 // Distances equal the reference's: level-synchronous, INF = INT32_MAX.
 //
-// hn_bfs_do runs the same graph with a level kernel that may switch to
-// bottom-up steps (Beamer's direction-optimising BFS, the counterpart of
-// hornetsnest's BottomUpBFS, src/Static/BottomUpBreadthFirstSearch/
-// BottomUpBFS.cu); distances are identical, fewer edges are read.
+// hn_bfs_do runs the same kernel with levels that may run bottom-up (Beamer's
+// direction-optimising BFS, the counterpart of hornetsnest's BottomUpBFS,
+// src/Static/BottomUpBreadthFirstSearch/BottomUpBFS.cu); on a graph that
+// stores every edge both ways distances are identical, and fewer edges are
+// read.
 #include <algorithm>
 #include <climits>
 

@@ -247,8 +247,8 @@ struct hn_graph {
     long long* d_scalar = nullptr;        // device scalars (16)
 
     hn::Persist scratch[8];               // reusable device scratch
-    hn::BfsGraph* bfs = nullptr;          // instantiated BFS CUDA graph
-    hn::MsGraph* ms = nullptr;            // instantiated batched-BFS CUDA graph
+    hn::BfsGraph* bfs = nullptr;          // BFS arrays (and the CUDA graph of bfs.kernel 0)
+    hn::MsGraph* ms = nullptr;            // batched-BFS arrays and CUDA graphs
 
     // a query view (hn_graph_view_create): shares the parent's vertex table
     // and edge pool read-only, owns its stream and scratch

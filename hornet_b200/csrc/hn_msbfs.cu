@@ -3,7 +3,7 @@
 // Multi-Source Graph Traversal", VLDB 2015).
 //
 // Batching: many BFS sources (and, on a disjoint union, many small graphs)
-// in one persistent launch captured in a CUDA graph.  Each vertex carries three 64-bit masks:
+// in one launch of a CUDA graph (two where pulls are asked for).  Each vertex carries three 64-bit masks:
 //   seen[v]  slots that have reached v,
 //   front[v] slots for which v is on the current frontier,
 //   nxt[v]   slots that reach v at this level (OR-accumulated).

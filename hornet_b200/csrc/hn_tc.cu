@@ -497,8 +497,9 @@ __global__ void k_cand_flip_base(const long long* __restrict__ coff, const int* 
 //   and the (v, w) pairs of 32 candidates at a time are dealt to the lanes,
 //   about 40 instructions each.
 // R-MAT scale 22, 11.8 G pairs, both kernels: 36.5 ms by tables alone, 24.0
-// with a bitmap and pairs dealt to the lanes, 14.5 this way.  512 graphs (74 M
-// oriented edges), owner counts: 13.4 ms by tables, 6.6 this way.  What bounds
+// with a bitmap and pairs dealt to the lanes, 13.5 this way (k_tc_cta 8.9,
+// k_tc_warp 4.6).  512 graphs (74 M oriented edges), owner counts: 13.4 ms by
+// tables, 6.6 this way.  What bounds
 // it: the shared-memory reads of the bits (random words: about 3.5 wavefronts a
 // warp) beside 47 GB of list reads, mostly from L2.
 //   k_tc_warp: one warp per vertex with d+(u) <= warp_cap (the tc.warp_cap
@@ -653,8 +654,8 @@ __device__ __forceinline__ void tc_credit_edges(int* esup, int e_uv, int e_vw, i
 // the wn numbers from wb on, which hold all of N+(u), with a zero bit behind
 // them; kBitsHash: the bitmap for those numbers, the table for the others.
 enum { kSearch, kHash, kBits, kBitsHash };
-constexpr int kTcLong = 128;
-constexpr int kQuads = 4;   // kBits: lists read by the whole warp from this length on
+constexpr int kTcLong = 128;   // kBits: lists read by the whole warp from this length on
+constexpr int kQuads = 4;      // kBits: 16-byte quads of short lists in flight a lane
 // CTAs an SM of the bitmap-only kernel: it waits on list loads, so occupancy
 // pays.  Totals (32 registers), R-MAT scale 22: 9.7 ms at 4, 9.1 at 5, 8.8 at 8;
 // owner counts, which spill below 48 registers, 512 graphs: 1.43 ms at 4, 1.38 at
@@ -1058,8 +1059,9 @@ k_tc_thread(TcView g, int nV, int small_du, int small_dc,
     }
 }
 
-// Five CTAs per SM for the plain count (48 registers, no spills); the
-// modes that credit vertices or edges carry more state and get 64.
+// With bitmaps three CTAs per SM (their 64 KB a CTA), with tables alone five
+// for the plain count (48 registers, no spills), four for the modes that credit
+// vertices or edges, which carry more state.
 template <int MODE, int WIN>
 __global__ void __launch_bounds__(kTcWarps * 32, WIN != kNoWin ? 3 : MODE == 0 ? 5 : 4)
 k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
@@ -1163,7 +1165,8 @@ k_tc_warp(TcView g, int nV, unsigned long long* __restrict__ per_vertex,
 }
 
 // Listed vertices (d+(u) > warp_cap): one CTA each, its warps claiming
-// groups of 32 candidates from a shared counter.  Two launches: the mid list
+// groups of 32 candidates from a shared counter.  Two launches (with bitmaps
+// three, see WIN): the mid list
 // (d+(u) <= tc.mid_cap, several CTAs per SM) and the huge list (d+(u) up to
 // tc.cta_table_cap in a table, binary search of N+(u) beyond that).  A
 // table of d entries takes the power of two >= 2*d slots, so the dynamic

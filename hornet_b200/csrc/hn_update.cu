@@ -20,12 +20,16 @@
 //      from the bump pointer (largest class first, so blocks >= 4 slots stay
 //      16-byte aligned); grow the pool / lists if needed;
 //   6. assign blocks (warp-aggregated per-class ranks);
-//   7. scatter-merge into the new block: old element A[r] goes to
-//      r + |{B < A[r]}|, batch element B[j] to j + |{A <= B[j]}| (insert);
-//      for erase a kept A[r] goes to r - |{B <= A[r]}|;
+//   7. scatter-merge: old element A[r] goes to r + |{B < A[r]}|, batch element
+//      B[j] to j + |{A <= B[j]}| (insert); for erase a kept A[r] goes to
+//      r - |{B <= A[r]}|;
 //   8. commit vertex records and push old blocks on their free lists.
-// Every touched vertex is rewritten out of place, so no kernel ever reads
-// a slot another thread of the same launch writes.
+// A vertex whose block class stays is updated in its own block (its list from
+// the first entry that moves), by one warp or CTA that reads a group of entries
+// before it writes it, or with the boundaries between chunks saved first; any
+// other list moves to a new block.  So no kernel reads a slot that another
+// warp of the same launch may have written.  Up to kSmallBatch entries, steps 1
+// to 4 are one kernel, and 7 and 8 another.
 #include <cub/cub.cuh>
 
 #include <algorithm>

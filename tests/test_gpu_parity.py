@@ -703,7 +703,7 @@ def test_device_graph_save_and_reload(tmp_path):
 
 @pytest.mark.parametrize("device_rounds", [1, 0])
 def test_ktruss_round_drivers(device_rounds):
-    """The peel rounds driven on the device (a CUDA graph's WHILE node) and
+    """The peel rounds driven on the device (cooperative launches) and
     from the host give the oracle's truss numbers."""
     g = T.rmat_graph(9, 8, seed=3)
     h = build(g)
