@@ -342,7 +342,7 @@ constexpr int kKtThreads = 1024;
 constexpr int kKtFew = 512;      // edges staged per CTA
 constexpr int kKtSolo = 16;      // edges that CTA 0 takes alone
 constexpr int kKtSoloMax = 64;
-constexpr int kKtBeat = 256;     // chunks of a warp between two signs of progress (1 ms with lists of 4 M)
+constexpr int kKtBeat = 512;     // chunks of a warp between two signs of progress (2 ms with lists of 4 M)
 static_assert(kKtSoloMax <= kKtFew, "CTA 0 stages its frontiers");
 constexpr int kAlive = INT_MAX;
 
