@@ -132,6 +132,7 @@ def test_batch_block_size_knobs(block, ctas, bu):
         H.tune_set("msbfs.block", block)
         H.tune_set("msbfs.ctas_per_sm", ctas)
         H.tune_set("msbfs.bottom_up", bu)
+        H.tune_set("msbfs.check_min", 1)
         out, st = H.BfsTopDown(h).run_batch(srcs)
         check(out, st, ref, ref_stats)
     finally:
@@ -149,6 +150,7 @@ def test_batch_bottom_up_switching(alpha, beta):
     ref, ref_stats = oracle_slots(g, srcs, range(len(srcs)), len(srcs))
     try:
         H.tune_set("msbfs.bottom_up", 1)
+        H.tune_set("msbfs.check_min", 1)
         H.tune_set("bfs.do_alpha", alpha)
         H.tune_set("bfs.do_beta", beta)
         out, st = H.BfsTopDown(h).run_batch(srcs)
@@ -172,6 +174,7 @@ def test_batch_bottom_up_long_lists(block):
     ref, ref_stats = oracle_slots(g, srcs, slots, 40)
     try:
         H.tune_set("msbfs.block", block)
+        H.tune_set("msbfs.check_min", 1)
         for alpha, beta in ((1 << 20, 1), (1 << 20, 1 << 20), (2, 24)):
             H.tune_set("bfs.do_alpha", alpha)
             H.tune_set("bfs.do_beta", beta)
@@ -197,6 +200,7 @@ def test_batch_levels_without_a_touched_list(extra, slots):
     srcs = np.array([0, 2, n - 1, 1, d, 2 + d, 0, 5, 9][:slots], np.int32)
     ref, ref_stats = oracle_slots(g, srcs, range(slots), slots)
     try:
+        H.tune_set("msbfs.check_min", 1)
         for bu in (0, 1):
             H.tune_set("msbfs.bottom_up", bu)
             out, st = H.BfsTopDown(h).run_batch(srcs)
