@@ -1687,8 +1687,9 @@ void launch_run(hn_graph* g, BfsGraph& bg, int src, int32_t* dist, BfsOut* out,
     // 3370 / 3350 / 3350 and 3390 / 2120 / 1270 / 740; R-MAT scale 12 70 / 47 / 46
     // / 46 and 70 / 41 / 22 / 16, scale 16 91 / 72 / 71 / 78 and 93 / 50 / 28 / 20,
     // scale 20 234 / 214 / 214 / 216 and 232 / 177 / 155 / 141.  Larger ones fill
-    // the GPU (scale 22: 278 queued, 259 / 220 / 195 shared), and the second of
-    // two calls alone would have half of it (scale 25 under load: no difference).
+    // the GPU, and the second of two calls alone would have half of it (scale 22:
+    // 278 queued, 259 / 220 / 195 shared; a request mix on scale 25 with 1,000
+    // requests/s offered: 1,019 served queued, 944 shared).
     unsigned grid = bg.grid;
     if (g->nE <= kShareMax)
         grid = std::max(1u, grid / (unsigned)std::max(1, bfs_root(g)->bfs_running.load(
