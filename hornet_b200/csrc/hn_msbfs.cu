@@ -631,13 +631,19 @@ __global__ void k_ms_answer(MsState* st) {
 
 void check_symmetry(hn_graph* g, MsGraph& mg) {
     cudaStream_t s = g->stream;
-    DevBuf<long long> prefix((size_t)g->nV + 1, s), splits;
-    degree_prefix(g, nullptr, g->nV, prefix.get());
-    lb_splits(g, prefix.get(), g->nV, g->nE, kMsTile, splits);
-    const long long ntiles = (g->nE + g->nV + kMsTile - 1) / kMsTile;
-    HN_LAUNCH(k_ms_one_way, grid_for(g, ntiles, kOneWayBlock / 32), kOneWayBlock, 0, s,
-              (const long long*)prefix.get(), g->nV, (long long)g->nE, (const VRec*)g->vtab,
-              (const int32_t*)g->pool, (const long long*)splits.get(), ntiles, mg.state);
+    try {
+        DevBuf<long long> prefix((size_t)g->nV + 1, s), splits;
+        degree_prefix(g, nullptr, g->nV, prefix.get());
+        lb_splits(g, prefix.get(), g->nV, g->nE, kMsTile, splits);
+        const long long ntiles = (g->nE + g->nV + kMsTile - 1) / kMsTile;
+        HN_LAUNCH(k_ms_one_way, grid_for(g, ntiles, kOneWayBlock / 32), kOneWayBlock, 0, s,
+                  (const long long*)prefix.get(), g->nV, (long long)g->nE, (const VRec*)g->vtab,
+                  (const int32_t*)g->pool, (const long long*)splits.get(), ntiles, mg.state);
+    } catch (const Error& e) {
+        if (e.code != HN_ERR_OOM) throw;
+        // no room for the check (8 bytes a vertex): as if there were one-way edges
+        HN_CUDA(cudaMemsetAsync(&mg.state->one_way, 1, sizeof(mg.state->one_way), s));
+    }
     HN_LAUNCH(k_ms_answer, 1, 1, 0, s, mg.state);
 }
 
