@@ -51,7 +51,10 @@ struct ProfileScope {
 
 // Room for the temporary buffers of one call, from one stream-ordered
 // allocation: an update takes about 25 buffers, and at two driver calls each
-// they cost more host time than a small batch's kernels.
+// they cost more host time than a small batch's kernels.  Buffers released
+// early do not make room for later ones, so it is larger than what the call
+// holds at once; where that is not to be had it stays empty, and the buffers
+// are allocated one by one.
 struct Arena {
     char* p = nullptr;
     size_t cap = 0, used = 0;
@@ -59,7 +62,13 @@ struct Arena {
     Arena() = default;
     void open(size_t bytes, cudaStream_t st) {
         s = st;
-        HN_CUDA(cudaMallocAsync((void**)&p, bytes, st));
+        const cudaError_t e = cudaMallocAsync((void**)&p, bytes, st);
+        if (e == cudaErrorMemoryAllocation) {
+            p = nullptr;
+            (void)cudaGetLastError();
+            return;
+        }
+        HN_CUDA(e);
         cap = bytes;
     }
     void* take(size_t bytes) {   // null when it does not fit

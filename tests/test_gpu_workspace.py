@@ -69,3 +69,34 @@ def test_large_updates(n):
     b = H.BatchUpdate(h, s, d)
     assert peak(lambda: h.insert(b, True, True)) < 81 * n
     assert peak(lambda: h.erase(b, True)) < 81 * n
+
+
+def test_updates_without_room_for_one_allocation():
+    """2^20 entries with 120 MB free: too little for the one allocation of all
+    buffers (151 MB), enough for the buffers one by one (84 MB)."""
+    import numpy as np
+    import torch
+    h = rmat(18, 8)
+    n = 1 << 20
+    # edges that the graph does not hold: from isolated vertices
+    src, dst = h.getCOO(True)
+    isolated = np.flatnonzero(np.bincount(src, minlength=h.nV()) == 0).astype(np.int32)
+    rng = np.random.default_rng(3)
+    s = torch.from_numpy(isolated[rng.integers(0, len(isolated), n)]).cuda()
+    d = torch.from_numpy(rng.integers(0, h.nV(), n).astype(np.int32)).cuda()
+    torch.cuda.synchronize()
+    b = H.BatchUpdate(h, s, d)
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool = ctypes.c_void_p()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert cu.cuMemPoolTrimTo(pool, ctypes.c_size_t(0)) == 0
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (120 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 150 << 20
+        assert h.erase(b) == 0
+        assert h.nE() == len(src)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert h.erase(b) == 0
