@@ -647,6 +647,49 @@ void check_symmetry(hn_graph* g, MsGraph& mg) {
     HN_LAUNCH(k_ms_answer, 1, 1, 0, s, mg.state);
 }
 
+// The CUDA graph of part 0 (fill, seed and the levels) or 1 (the levels from
+// where they stand, built when a call first asks).
+void build_ms_loop(hn_graph* g, MsGraph& mg, int part) {
+    cudaGraph_t& graph = mg.graph[part];
+    if (graph) HN_CUDA(cudaGraphDestroy(graph));   // (of a build that failed)
+    graph = nullptr;
+    HN_CUDA(cudaGraphCreate(&graph, 0));
+    cudaGraphNode_t fill, seed, condn, push, apply;
+    void* args[] = {&mg.state};
+    cudaKernelNodeParams p = {};
+    p.kernelParams = args;
+    if (part == 0) {
+        p.func = (void*)k_ms_fill;
+        p.gridDim = dim3((unsigned)g->info.sms * 8);
+        p.blockDim = dim3(256);
+        HN_CUDA(cudaGraphAddKernelNode(&fill, graph, nullptr, 0, &p));
+        p.func = (void*)k_ms_seed;
+        p.gridDim = dim3(1);
+        p.blockDim = dim3(kSeedBlock);
+        HN_CUDA(cudaGraphAddKernelNode(&seed, graph, &fill, 1, &p));
+    }
+    cudaGraphConditionalHandle handle;
+    HN_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = handle;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    HN_CUDA(cudaGraphAddNode(&condn, graph, part == 0 ? &seed : nullptr, part == 0 ? 1 : 0, &cp));
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    p.func = mg.block == 128 ? (void*)k_ms_push<128>
+           : mg.block == 512 ? (void*)k_ms_push<512> : (void*)k_ms_push<256>;
+    p.gridDim = dim3(mg.grid);
+    p.blockDim = dim3(mg.block);
+    HN_CUDA(cudaGraphAddKernelNode(&push, body, nullptr, 0, &p));
+    void* args2[] = {&mg.state, &handle};
+    p.func = mg.block == 128 ? (void*)k_ms_apply<128>
+           : mg.block == 512 ? (void*)k_ms_apply<512> : (void*)k_ms_apply<256>;
+    p.kernelParams = args2;
+    HN_CUDA(cudaGraphAddKernelNode(&apply, body, &push, 1, &p));
+    HN_CUDA(cudaGraphInstantiate(&mg.exec[part], graph, 0));
+}
+
 void build_ms_graph(hn_graph* g, MsGraph& mg) {
     const int nV = g->nV;
     // room for the graph to grow by a quarter before a rebuild
@@ -664,44 +707,7 @@ void build_ms_graph(hn_graph* g, MsGraph& mg) {
     mg.nV = nV;
     mg.nchunk_cap = nchunk_cap;
 
-    for (int part = 0; part < 2; part++) {
-        cudaGraph_t& graph = mg.graph[part];
-        HN_CUDA(cudaGraphCreate(&graph, 0));
-        cudaGraphNode_t fill, seed, condn, push, apply;
-        void* args[] = {&mg.state};
-        cudaKernelNodeParams p = {};
-        p.kernelParams = args;
-        if (part == 0) {
-            p.func = (void*)k_ms_fill;
-            p.gridDim = dim3((unsigned)g->info.sms * 8);
-            p.blockDim = dim3(256);
-            HN_CUDA(cudaGraphAddKernelNode(&fill, graph, nullptr, 0, &p));
-            p.func = (void*)k_ms_seed;
-            p.gridDim = dim3(1);
-            p.blockDim = dim3(kSeedBlock);
-            HN_CUDA(cudaGraphAddKernelNode(&seed, graph, &fill, 1, &p));
-        }
-        cudaGraphConditionalHandle handle;
-        HN_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        HN_CUDA(cudaGraphAddNode(&condn, graph, part == 0 ? &seed : nullptr, part == 0 ? 1 : 0, &cp));
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        p.func = mg.block == 128 ? (void*)k_ms_push<128>
-               : mg.block == 512 ? (void*)k_ms_push<512> : (void*)k_ms_push<256>;
-        p.gridDim = dim3(mg.grid);
-        p.blockDim = dim3(mg.block);
-        HN_CUDA(cudaGraphAddKernelNode(&push, body, nullptr, 0, &p));
-        void* args2[] = {&mg.state, &handle};
-        p.func = mg.block == 128 ? (void*)k_ms_apply<128>
-               : mg.block == 512 ? (void*)k_ms_apply<512> : (void*)k_ms_apply<256>;
-        p.kernelParams = args2;
-        HN_CUDA(cudaGraphAddKernelNode(&apply, body, &push, 1, &p));
-        HN_CUDA(cudaGraphInstantiate(&mg.exec[part], graph, 0));
-    }
+    build_ms_loop(g, mg, 0);
 }
 
 }  // namespace
@@ -823,6 +829,7 @@ extern "C" int hn_bfs_batch(hn_graph_t* g, const int32_t* sources, const int32_t
         HN_CUDA(cudaMemcpyAsync(mg.h_state, mg.state, sizeof(MsState), cudaMemcpyDeviceToHost, s));
         HN_CUDA(cudaStreamSynchronize(s));
         if (!h.ask) break;
+        if (!mg.exec[1]) build_ms_loop(g, mg, 1);
         check_symmetry(g, mg);
     }
     if (mem == HN_MEM_HOST) {
