@@ -3,7 +3,7 @@
  *
  * A plain-C restatement of the reference algorithms on the Hornet hot path,
  * used only by tests/, __graft_entry__.smoke() and bench.py's CPU-baseline leg
- * as the checker.  Every function cites the reference file:line it follows
+ * to check results.  Every function cites the reference file:line it follows
  * (paths relative to the hornet-gt/hornet source tree).
  *
  * Pinning: the CSR builder, BFS and CC are checked against the reference's own

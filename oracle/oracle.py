@@ -5,7 +5,7 @@ oracle/hn_oracle.h for the reference lines each function follows) and to
 the reference's own host code compiled into oracle/_ref/ref_driver
 (xlib GraphStd / BFS / WCC, see oracle/ref_driver.cpp).  Only tests/,
 __graft_entry__.smoke() and bench.py's CPU-baseline leg use this module,
-always as the checker.
+always to check results.
 """
 from __future__ import annotations
 
